@@ -58,6 +58,7 @@ struct mpcd_ctx {
   cudaStream_t nst = nullptr;
   cudaEvent_t ev_tab = nullptr, ev_cls = nullptr, ev_end = nullptr, ev_list = nullptr, ev_free = nullptr;
   bool flight = true;
+  bool near_step = false;        // its substeps in one cooperative kernel (enq_step_near)
   cudaStream_t evs = nullptr;    // third stream (FP64 form): event passes and colloid finish
   cudaEvent_t ev_start = nullptr, ev_str = nullptr, ev_aux = nullptr, ev_finp[2] = {nullptr, nullptr};
 
@@ -67,6 +68,8 @@ struct mpcd_ctx {
   long long host_step = 0;       // completed steps (mirror of the device counter)
   int sort_every = 10;           // counting sort by cell every this many steps
   bool setup_done = false;
+  bool tables_stale = false;     // the last step was a free-flight one on k_near_step: the cell table of the next
+                                 // step's first substep is not built (ensure_tables)
   std::string err;
   int64_t launches = 0;
   bool profile = false;
@@ -159,6 +162,40 @@ static void launch_on(mpcd_ctx *c, cudaStream_t s, const char *name, void (*k)(K
     cudaEventRecordWithFlags(pe.a, s, c->tracing ? cudaEventRecordExternal : cudaEventRecordDefault);
   }
   k<<<g, b, 0, s>>>(args...);
+  c->launches++;
+  if (c->profile || c->tracing) {
+    cudaEventRecordWithFlags(pe.b, s, c->tracing ? cudaEventRecordExternal : cudaEventRecordDefault);
+    (c->tracing ? c->trace : c->pending).push_back(pe);
+  }
+}
+
+// a launch with one launch attribute: cooperative (its blocks wait on one another), or dependent (it
+// starts when every block of the kernel before it on the stream has let it, not when that has ended)
+template <typename... KArgs, typename... Args>
+static void launch_attr(mpcd_ctx *c, cudaStream_t s, const char *name, bool coop, void (*k)(KArgs...), int grid,
+                        int block, size_t smem, Args... args) {
+  ProfEvent pe{name, nullptr, nullptr};
+  if (c->profile || c->tracing) {
+    pe.a = pool_event(c);
+    pe.b = pool_event(c);
+    cudaEventRecordWithFlags(pe.a, s, c->tracing ? cudaEventRecordExternal : cudaEventRecordDefault);
+  }
+  cudaLaunchAttribute at;
+  if (coop) {
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+  } else {
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k, args...);
   c->launches++;
   if (c->profile || c->tracing) {
     cudaEventRecordWithFlags(pe.b, s, c->tracing ? cudaEventRecordExternal : cudaEventRecordDefault);
@@ -313,7 +350,7 @@ static void enq_run_shell(mpcd_ctx *c, cudaStream_t s, int fb) {
 
 static void enq_run_kick(mpcd_ctx *c) {
   const bool f32 = c->S.precision == MPCD_FP32C;
-  launch(c, "k_run_kick", f32 ? k_run_kick32 : k_run_kick, 152 * 4, 256, c->S, c->fbuf);
+  launch(c, "k_run_kick", f32 ? k_run_kick32 : k_run_kick, 152 * 4, 256, c->S, c->fbuf, 0);
 }
 
 static void enq_run_fluid(mpcd_ctx *c) {
@@ -454,15 +491,15 @@ static void enq_step_flight32(mpcd_ctx *c, bool sort) {
   launch(c, "k_cell_prep", k_cell_prep32, prep_blocks(S), 256, S);
   if (sort) enq_sort_scatter(c);
   cudaStreamWaitEvent(c->stream, c->ev_tab, 0);
-  launch(c, "k_rotate_classify", classify_kernel32(!sort), blocks_for(S.N, 256 * CLASSIFY32_U), 256, S, c->fbuf);
+  launch(c, "k_rotate_classify", classify_kernel32(!sort, false), blocks_for(S.N, 256 * CLASSIFY32_U), 256, S, c->fbuf);
   cudaEventRecord(c->ev_cls, c->stream);
   cudaStreamWaitEvent(c->nst, c->ev_cls, 0);
   cudaStreamWaitEvent(c->nst, c->ev_join, 0);
-  if (S.Nc > 0) launch_on(c, c->nst, "k_run_kick", k_run_kick32, 152 * 4, 256, S, c->fbuf);
+  if (S.Nc > 0) launch_on(c, c->nst, "k_run_kick", k_run_kick32, 152 * 4, 256, S, c->fbuf, 0);
   enq_fin_on(c, c->nst, M_KICK | M_ADVANCE, 0);
   for (int l = 1; l <= n; ++l) enq_substep_near32(c, c->nst, l);
   cudaEventRecord(c->ev_end, c->nst);
-  launch(c, "k_free_flight", k_free_flight32, free_blocks(c), 256, S, c->fbuf);
+  launch(c, "k_free_flight", k_free_flight32, free_blocks(c), 256, S, c->fbuf, 1);
   cudaStreamWaitEvent(c->stream, c->ev_end, 0);
   launch(c, "k_end_step", k_end_step, 1, 256, S);
 }
@@ -490,11 +527,11 @@ static void enq_step_flight64(mpcd_ctx *c, bool sort) {
   launch(c, "k_cell_prep", k_cell_prep, prep_blocks(S), 256, S);
   if (sort) enq_sort_scatter(c);
   cudaStreamWaitEvent(c->stream, c->ev_tab, 0);
-  launch(c, "k_rotate_classify", classify_kernel(!sort), blocks_for(S.N, 256), 256, S, c->fbuf);
+  launch(c, "k_rotate_classify", classify_kernel(!sort, false), blocks_for(S.N, 256), 256, S, c->fbuf);
   cudaEventRecord(c->ev_cls, c->stream);
   cudaStreamWaitEvent(c->nst, c->ev_cls, 0);
   cudaStreamWaitEvent(c->nst, c->ev_join, 0);
-  if (nc) launch_on(c, c->nst, "k_run_kick", k_run_kick, 152 * 4, 256, S, c->fbuf);
+  if (nc) launch_on(c, c->nst, "k_run_kick", k_run_kick, 152 * 4, 256, S, c->fbuf, 0);
   enq_fin_on(c, c->nst, M_KICK | M_ADVANCE, 0);
   cudaEventRecord(c->ev_start, c->nst);
   cudaStreamWaitEvent(c->evs, c->ev_start, 0);
@@ -520,14 +557,79 @@ static void enq_step_flight64(mpcd_ctx *c, bool sort) {
   // the free pass after the first substep's finish (by default): the chain's first event pass
   // then has the SMs to itself (the free pass holds half of every SM's registers)
   if (free_after(c) >= 1) cudaStreamWaitEvent(c->stream, c->ev_free, 0);
-  launch(c, "k_free_flight", k_free_flight, free_blocks(c), 256, S, c->fbuf);
+  launch(c, "k_free_flight", k_free_flight, free_blocks(c), 256, S, c->fbuf, 1);
   cudaStreamWaitEvent(c->stream, c->ev_end, 0);
   launch(c, "k_end_step", k_end_step, 1, 256, S);
+}
+
+// One step in the free-flight schedule with the substeps in one kernel (near_step.cuh).
+//   side stream: the flight table, run()'s rear-shell test, run()'s colloid kick and the first
+//                update_pos_md (k_fin), the step's rotational-diffusion normals;
+//   main:        the cell pass; the rotation with the classification (it needs the table); run()'s
+//                fluid kick (it needs the shell counts); the pass over the particles no sphere can
+//                reach in the step (free and near), beside
+//   near stream: the active particles' substeps with the colloids' (it needs the kick, the first
+//                colloid move and the pair list);
+//   main:        run() records of the near particles and the end of the step, after both.
+static void enq_step_near(mpcd_ctx *c, bool sort) {
+  const SysF64 &S = c->S;
+  const bool f32 = S.precision == MPCD_FP32C;
+  cudaEventRecord(c->ev_fork, c->stream);
+  cudaStreamWaitEvent(c->aux, c->ev_fork, 0);
+  launch_on(c, c->aux, "k_flight_table", k_flight_table32, S.Nc, 128, S);
+  cudaEventRecord(c->ev_tab, c->aux);
+  cudaStreamWaitEvent(c->evs, c->ev_fork, 0);
+  if (S.Dr > 0)
+    launch_on(c, c->evs, "k_rotdiff_step", k_rotdiff_step, blocks_for(2ll * S.Nc * S.n_sub, 256), 256, S);
+  enq_step_pairs(c, c->evs);
+  cudaEventRecord(c->ev_str, c->evs);
+  enq_run_shell(c, c->aux, c->fbuf);
+  cudaEventRecord(c->ev_join, c->aux);
+  SysF64 S1 = S;
+  S1.fin_table = 0;  // (no cell tables in this schedule)
+  {
+    const int g = S.Nc < c->n_sm ? S.Nc : c->n_sm, w = (int)blocks_for(S.Nc, g);
+    launch_on(c, c->aux, "k_fin", k_fin, w > 4 ? (int)blocks_for(S.Nc, 4) : g, 32 * (w > 4 ? 4 : w), S1,
+              M_KICK | M_ADVANCE | M_FLIGHT, 0);
+  }
+  cudaEventRecord(c->ev_aux, c->aux);
+  launch(c, "k_cell_prep", f32 ? k_cell_prep32 : k_cell_prep, prep_blocks(S), 256, S);
+  if (sort) enq_sort_scatter(c);
+  cudaStreamWaitEvent(c->stream, c->ev_tab, 0);
+  launch(c, "k_rotate_classify", f32 ? classify_kernel32(!sort, true) : classify_kernel(!sort, true),
+         blocks_for(S.N, f32 ? 256 * CLASSIFY32_U : 256), 256, S, c->fbuf);
+  cudaStreamWaitEvent(c->stream, c->ev_join, 0);
+  launch(c, "k_run_kick", f32 ? k_run_kick32 : k_run_kick, 152 * 4, 256, S, c->fbuf, 1);
+  cudaEventRecord(c->ev_cls, c->stream);
+  cudaStreamWaitEvent(c->nst, c->ev_cls, 0);
+  cudaStreamWaitEvent(c->nst, c->ev_aux, 0);
+  cudaStreamWaitEvent(c->nst, c->ev_str, 0);
+  launch_attr(c, c->nst, "k_stream_near", true, f32 ? k_near_step32 : k_near_step64, c->n_sm,
+              f32 ? NEAR32_BLOCK : NEAR64_BLOCK, f32 ? near_step32_smem() : near_step64_smem(), S, c->fbuf);
+  cudaEventRecord(c->ev_end, c->nst);
+  launch_attr(c, c->nst, "k_free_flight", false, f32 ? k_free_flight32 : k_free_flight, free_blocks(c), 256, 0, S,
+              c->fbuf, 2);
+  cudaEventRecord(c->ev_free, c->nst);
+  cudaStreamWaitEvent(c->stream, c->ev_end, 0);
+  cudaStreamWaitEvent(c->stream, c->ev_free, 0);
+  launch(c, "k_end_step", f32 ? k_end_flight32 : k_end_flight64, 1 + c->n_sm * 8, 256, S, c->fbuf);
+}
+
+// the cell table of the next step's first substep, for the schedules that read one, after a
+// step that left none
+static void ensure_tables(mpcd_ctx *c) {
+  if (!c->tables_stale) return;
+  if (c->S.Nc) launch(c, "k_table_next", k_table_next, c->S.Nc, 256, c->S);
+  c->tables_stale = false;
 }
 
 // one MPCD step: rotation_mpcd, run, n_sub substeps (cpp/active_brownian.cpp:25-38)
 static void enq_step(mpcd_ctx *c, bool sort) {
   const int n = c->S.n_sub;
+  if (c->flight && c->near_step) {
+    enq_step_near(c, sort);
+    return;
+  }
   if (c->flight) {
     if (c->S.precision == MPCD_FP32C) enq_step_flight32(c, sort);
     else enq_step_flight64(c, sort);
@@ -574,8 +676,13 @@ static const char *err_text(int bits) {
   if (bits & ERRB_SHELLSLOTS) return "a particle lies in more rear shells than a record holds";
   if (bits & ERRB_DELTA) return "a colloid momentum exchange left the range of the exact sums";
   if (bits & ERRB_EVENTS) return "the wall-collision event lists overflowed";
+  if (bits & ERRB_WAIT) return "a grid-wide wait of the near particles' substeps did not end within its limit";
   if (bits & ERRB_NBR) return "a colloid has more pair-list partners than the list holds";
   return "device error";
+}
+
+static int err_code(int bits) {
+  return (bits & ERRB_WAIT) ? MPCD_ERR_CUDA : (bits & (ERRB_VRANGE | ERRB_DELTA)) ? MPCD_ERR_RANGE : MPCD_ERR_CAPACITY;
 }
 
 // synchronise, read the device step state, turn error bits into a status
@@ -586,7 +693,7 @@ static int check_device(mpcd_ctx *c) {
   if (c->profile) collect_profile(c);
   int bits = c->ss_host->err;
   if (bits) {
-    int code = (bits & (ERRB_VRANGE | ERRB_DELTA)) ? MPCD_ERR_RANGE : MPCD_ERR_CAPACITY;
+    const int code = err_code(bits);
     char buf[160];
     snprintf(buf, sizeof buf, "device error bits 0x%x: %s", bits, err_text(bits));
     return fail(c, code, buf);
@@ -686,6 +793,7 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
   S.rT_coll = (float)(p.sigma * 0.5 + pmargin + cmargin + 0.01);
   S.rT_shell = (float)(p.sigma * 0.5 + 0.5 + pmargin + cmargin + 0.01);
   S.disp_margin2 = pmargin * pmargin;
+  S.disp_marginf = (float)pmargin;
   S.cmargin2 = cmargin * cmargin;
   S.cmarginf = (float)cmargin;
   S.max_per_cell = p.max_per_cell > 0 ? p.max_per_cell : 128;
@@ -701,6 +809,7 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
   S.vmaxf = (float)vmax;
   // free flight: a particle moving further than 5 thermal speeds' worth in a step is near
   S.flight_rv = (float)(5.0 * vth * p.ndt);
+  S.flight_rx = (float)fmax(5.0 * vth * p.ndt, pmargin + cmargin + 0.05);
   // the free-flight steps' forces from a pair list built at the start of each step
   S.vlist = p.n_colloid > 1 ? 1 : 0;
   // the FP64 form sums displacements w = v dt, the FP32 form velocities
@@ -738,6 +847,7 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
     S.Xcq[b] = m.get<float4>(Nc);
     S.Xco[b] = m.get<float4>(Nc);
     S.cbox[b] = m.get<int>(Nc);
+    S.ccell[b] = m.get<int4>(Nc);
     S.Tcnt[b] = m.get<unsigned long long>(S.C);
     S.Tlist[b] = m.get<uint16_t>((size_t)S.C * TCAP);
   }
@@ -764,6 +874,24 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
   S.near = m.get<int>(N);
   S.fnear = m.get<uint8_t>(N);
   S.ftab = m.get<FlightCell>(S.C);
+  S.act = m.get<int>(N);
+  S.bar = m.get<unsigned>(BAR_WORDS);
+  {
+    // A free-flight step takes the active particles through its substeps in one cooperative
+    // kernel where there are colloids and at least two substeps, unless the flight table's cells
+    // would overflow as a rule: with more than eight colloids expected within its reach of a cell
+    // (12 fit), the particles of overflowing cells would scan every colloid, which the
+    // per-substep cell tables avoid.  (The normals of a step: 24 bytes per colloid and substep.)
+    const double reach = S.r_shell + S.flight_rx + S.n_sub * cmargin + 0.02 + 0.62;  // + a cell's radius as a ball
+    const double expected = (double)S.Nc / (double)S.C * 4.0 / 3.0 * M_PI * reach * reach * reach;
+    c->near_step = S.Nc > 0 && S.n_sub >= 2 && expected <= 8.0 && (long long)S.Nc * S.n_sub <= (1ll << 24);
+    if (c->near_step && p.Dr > 0) S.xi_all = m.get<double>(3 * Nc * (size_t)S.n_sub);
+    if (c->near_step) S.w_all = m.get<double>(3 * Nc * (size_t)S.n_sub);
+    if (c->near_step && p.precision == MPCD_FP64) {
+      S.evx_cap = S.events_cap;
+      S.evx = m.get<char>((size_t)EV_STATE_BYTES * S.evx_cap);
+    }
+  }
   if (S.precision == MPCD_FP64) {
     S.newrec[0] = m.get<EventRec>(S.events_cap);
     S.newrec[1] = m.get<EventRec>(S.events_cap);
@@ -834,6 +962,21 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && nsm > 0)
       c->n_sm = nsm;
+    int coop = 0;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) c->near_step = false;
+  }
+  if (c->near_step) {
+    // the free-flight pass shares the SMs with the substeps' kernel: the same shared-memory split
+    const bool f32 = p.precision == MPCD_FP32C;
+    const void *k = f32 ? (const void *)k_near_step32 : (const void *)k_near_step64;
+    const void *ff = f32 ? (const void *)k_free_flight32 : (const void *)k_free_flight;
+    const int smem = (int)(f32 ? near_step32_smem() : near_step64_smem());
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess ||
+        cudaFuncSetAttribute(ff, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess) {
+      mpcd_destroy(c);
+      return MPCD_ERR_CUDA;
+    }
   }
   cudaDeviceSynchronize();
   *out = c;
@@ -965,6 +1108,7 @@ static int invalidate_tables(mpcd_ctx *c) {
   if (S.Nc) CUDA_OK(c, cudaMemsetAsync(S.exch, 0, sizeof(ExchAcc) * S.Nc, c->stream));
   if (S.ftab) CUDA_OK(c, cudaMemsetAsync(S.ftab, 0, sizeof(FlightCell) * S.C, c->stream));
   c->setup_done = false;
+  c->tables_stale = false;  // (mpcd_setup builds them)
   c->phase = 0;
   c->next_sub = 1;
   c->rseq = 0;
@@ -1140,6 +1284,7 @@ extern "C" int mpcd_rotation_mpcd(mpcd_ctx *c) {
   int r;
   if ((r = need_setup(c))) return r;
   if (c->phase != 0) return fail(c, MPCD_ERR_STATE, "rotation_mpcd starts a step: finish the substeps of this one");
+  ensure_tables(c);
   enq_rotation(c, sorts_at(c, c->host_step));
   c->phase = 1;
   c->next_sub = 0;
@@ -1180,12 +1325,19 @@ extern "C" int mpcd_substep(mpcd_ctx *c, int l) {
   return check_device(c);
 }
 
+// before whole steps are enqueued: the table their schedule reads, or the note that they leave none
+static void begin_steps(mpcd_ctx *c) {
+  if (c->flight && c->near_step) c->tables_stale = true;
+  else ensure_tables(c);
+}
+
 // nsteps steps enqueued on the context's stream (graph replays), nothing waited for
 static int enq_steps(mpcd_ctx *c, int nsteps) {
   int r;
   if ((r = need_setup(c))) return r;
   if (nsteps < 0) return MPCD_ERR_PARAM;
   if (c->phase != 0) return fail(c, MPCD_ERR_STATE, "a step begun routine by routine is unfinished");
+  if (nsteps > 0) begin_steps(c);
   if (c->profile) {
     for (int s = 0; s < nsteps; ++s) {
       enq_step(c, sorts_at(c, c->host_step));
@@ -1263,7 +1415,7 @@ extern "C" int mpcd_diag(mpcd_ctx *c, mpcd_diag_t *out) {
   if (int bits = c->ss_host->err) {
     char buf[200];
     snprintf(buf, sizeof buf, "device error bits 0x%x: %s", bits, err_text(bits));
-    return fail(c, (bits & (ERRB_VRANGE | ERRB_DELTA)) ? MPCD_ERR_RANGE : MPCD_ERR_CAPACITY, buf);
+    return fail(c, err_code(bits), buf);
   }
   const double *part = h;
   double sw[3] = {0, 0, 0}, s2 = 0, n = 0;
@@ -1364,6 +1516,7 @@ extern "C" int mpcd_trace_step(mpcd_ctx *c, char names[][48], double *t0_ms, dou
   if ((r = need_setup(c))) return r;
   if (c->phase != 0) return fail(c, MPCD_ERR_STATE, "a step begun routine by routine is unfinished");
   if (c->profile) return fail(c, MPCD_ERR_STATE, "profiling is on");
+  begin_steps(c);
   const int sort = sorts_at(c, c->host_step) ? 1 : 0, b = c->fbuf;
   cudaEvent_t start = pool_event(c);
   cudaGraph_t g;

@@ -31,6 +31,20 @@ static __device__ __forceinline__ bool in_block(const SysF64 &S, int cb, int lin
   return off_ok(bx - cx, S.Lx) && off_ok(by - cy, S.Ly) && off_ok(bz - cz, S.Lz);
 }
 
+// the coordinates of cell number cb, with w = (cb < C)
+static __device__ __forceinline__ int4 cell_coords(const SysF64 &S, int cb) {
+  const int t = cb / S.Lx;
+  return make_int4(cb - t * S.Lx, t % S.Ly, t / S.Ly, cb < S.C ? 1 : 0);
+}
+
+// in_block for the cell with coordinates ix, iy, iz (inside the box) and a colloid's
+// cell_coords, without divisions
+static __device__ __forceinline__ bool in_block3(const SysF64 &S, int4 c, int ix, int iy, int iz) {
+  const int dx = abs(ix - c.x), dy = abs(iy - c.y), dz = abs(iz - c.z);
+  const bool in = (dx <= 3 || dx >= S.Lx - 3) && (dy <= 3 || dy >= S.Ly - 3) && (dz <= 3 || dz >= S.Lz - 3);
+  return c.w != 0 && in && (S.physics != 0 || (dx | dy | dz) != 0);
+}
+
 // 1 + cell(pos) - 1: the reference's truncating linear cell of a wrapped position.
 // A wrapped coordinate lies in [0, L], so each integer part is at most L and the
 // cell number stays below Cpad; anything else (NaN, a negative or runaway
@@ -246,6 +260,15 @@ static __device__ __forceinline__ void exch_add6(ExchAcc *e, d3 dv, d3 dl, int *
     atomicAdd((unsigned long long *)&e->hi[k], (unsigned long long)hi[k]);
     atomicAdd((unsigned long long *)&e->lo[k], (unsigned long long)lo[k]);
   }
+}
+
+// one component (c) of a collision's exchange
+static __device__ __forceinline__ void exch_add1(ExchAcc *e, int c, double v, int *err) {
+  if ((dbits(v) & 0x7FFFFFFFFFFFFFFFll) >= 0x4130000000000000ll) atomicOr(err, ERRB_DELTA);
+  long long hi, lo;
+  exch_split(v, hi, lo);
+  atomicAdd((unsigned long long *)&e->hi[c], (unsigned long long)hi);
+  atomicAdd((unsigned long long *)&e->lo[c], (unsigned long long)lo);
 }
 
 static __device__ __forceinline__ double exch_val(const ExchAcc &e, int comp) {
@@ -797,6 +820,42 @@ static __device__ void for_reach_cells(const SysF64 &S, int cb, float4 xc, float
 static __device__ __forceinline__ void shift_of(const SysF64 &S, long long nn, double rr[3]) {
   const uint4 r = draw4(S.key, DOM_SHIFT, 0, 0, 0, (uint32_t)nn);
   rr[0] = u01(r.x) - 0.5; rr[1] = u01(r.y) - 0.5; rr[2] = u01(r.z) - 0.5;
+}
+
+static __device__ __forceinline__ int colloid_cell(const SysF64 &S, d3 X) {
+  bool alias;
+  return cell_of_pos(S, X.x, X.y, X.z, alias);
+}
+
+// colloid position as integer cell + FP32 offset (the FP32 form's coordinates)
+static __device__ __forceinline__ void colloid_q(const SysF64 &S, int b, int j, d3 X) {
+  double v[3] = {X.x, X.y, X.z};
+  const int L[3] = {S.Lx, S.Ly, S.Lz};
+  float c[3], o[3];
+  for (int k = 0; k < 3; ++k) {
+    double f = floor(v[k]);
+    float of = (float)(v[k] - f);
+    int ci = (int)f;
+    if (of >= 1.f) { of = 0.f; ci += 1; }
+    ci %= L[k];
+    if (ci < 0) ci += L[k];
+    c[k] = (float)ci;
+    o[k] = of;
+  }
+  S.Xcq[b][j] = make_float4(c[0], c[1], c[2], 0.f);
+  S.Xco[b][j] = make_float4(o[0], o[1], o[2], 0.f);
+}
+
+// grid shift of the SRD binning the coming streaming pass performs (rotation_mpcd
+// of that step draws it first, cpp/rotation_mpcd.cpp:9), keyed by that step
+static __device__ __forceinline__ void set_shift(const SysF64 &S, long long nn) {
+  S.ss->nshell = 0;
+  double rr[3];
+  shift_of(S, nn, rr);
+  for (int k = 0; k < 3; ++k) {
+    S.ss->rr[k] = rr[k];
+    S.ss->rrf[k] = (float)rr[k];
+  }
 }
 
 // reach of the cell table of substep e: the run() shell on the last substep of a

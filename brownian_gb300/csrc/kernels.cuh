@@ -5,7 +5,8 @@
 namespace bgb {
 
 enum : int { F_STREAM = 1, F_COLLIDE = 2, F_SHELL = 4, F_BINROT = 8, F_PIPE = 16 };
-enum : int { M_FINISH = 1, M_KICK = 2, M_ADVANCE = 4, M_ACT = 8, M_COLL = 16 };
+// M_FLIGHT: the first colloid move of a free-flight step, whose lists and grid shift are not k_fin's
+enum : int { M_FINISH = 1, M_KICK = 2, M_ADVANCE = 4, M_ACT = 8, M_COLL = 16, M_FLIGHT = 32 };
 
 // k_stream<FLAGS> instantiations, by flag set (nullptr for a set not built)
 using StreamKernel = void (*)(const SysF64, int, int);
@@ -46,8 +47,8 @@ __global__ void k_flight_table32(__grid_constant__ const SysF64 S);
 // FP32 form's takes CLASSIFY32_U particles per thread (grid: N / (256 CLASSIFY32_U) blocks)
 constexpr int CLASSIFY32_U = 2;
 using ClassifyKernel = void (*)(const SysF64, int);
-ClassifyKernel classify_kernel32(bool rotate);
-__global__ void k_free_flight32(__grid_constant__ const SysF64 S, int fb);
+ClassifyKernel classify_kernel32(bool rotate, bool split);
+__global__ void k_free_flight32(__grid_constant__ const SysF64 S, int fb, int thr);
 StreamKernel stream_kernel32_near(int flags);
 // the same over a batch of systems (persistent, batch_for)
 __global__ void k_flight_table32_b(const SysF64 *Ss, const int *boff, int nrep);
@@ -55,16 +56,26 @@ using ClassifyKernelB = void (*)(const SysF64 *, const int *, int, int);
 ClassifyKernelB classify_kernel32_b(bool rotate);
 __global__ void k_free_flight32_b(const SysF64 *Ss, const int *boff, int nrep, int fb);
 StreamKernelB stream_kernel32_near_b(int flags);
-ClassifyKernel classify_kernel(bool rotate);
-__global__ void k_free_flight(const SysF64 S, int fb);
+ClassifyKernel classify_kernel(bool rotate, bool split);
+__global__ void k_free_flight(const SysF64 S, int fb, int thr);
 __global__ void k_bin_near(const SysF64 S, int fb);
 StreamKernel stream_kernel_near(int flags);
+// the active particles' substeps in one cooperative kernel (near_step.cuh), and what goes with it
+__global__ void k_near_step64(__grid_constant__ const SysF64 S, int fb);
+__global__ void k_near_step32(__grid_constant__ const SysF64 S, int fb);
+constexpr int NEAR64_BLOCK = 256, NEAR32_BLOCK = 384;
+size_t near_step64_smem();
+size_t near_step32_smem();
+__global__ void k_rotdiff_step(__grid_constant__ const SysF64 S);
+__global__ void k_table_next(const SysF64 S);
+__global__ void k_end_flight64(__grid_constant__ const SysF64 S, int fb);
+__global__ void k_end_flight32(__grid_constant__ const SysF64 S, int fb);
 // the FP64 event pass fused with the substep's colloid side work (grid: nevb event blocks,
 // then one block per two colloids)
 using EventAuxKernel = void (*)(const SysF64, int, int, int, int);
 EventAuxKernel event_aux_kernel(int flags);
 __global__ void k_run_shell32(__grid_constant__ const SysF64 S, int fb);
-__global__ void k_run_kick32(__grid_constant__ const SysF64 S, int fb);
+__global__ void k_run_kick32(__grid_constant__ const SysF64 S, int fb, int split);
 __global__ void k_aos_to_q(const SysF64 S, const double *pos, const double *vel, int fb);
 __global__ void k_q_to_aos(const SysF64 S, double *pos, double *vel, int fb);
 __global__ void k_cell_prep(const SysF64 S);
@@ -72,7 +83,7 @@ __global__ void k_scan_blocks(__grid_constant__ const SysF64 S, int nblk);
 __global__ void k_rotate_sort(const SysF64 S, int src, int dst);
 __global__ void k_rotate(const SysF64 S, int fb);
 __global__ void k_run_shell(const SysF64 S, int fb);
-__global__ void k_run_kick(const SysF64 S, int fb);
+__global__ void k_run_kick(const SysF64 S, int fb, int split);
 __global__ void k_fin(__grid_constant__ const SysF64 S, int mode, int l);
 __global__ void k_aux(__grid_constant__ const SysF64 S, int l, int act, int vl);
 __global__ void k_colloid_setup(const SysF64 S);

@@ -14,7 +14,7 @@
 // Kernels mirror the FP64 form: k_stream32 (stream, FP32 scan of nearby colloids,
 // event list, last-substep binning), k_events32 (wall collisions in FP32, one per
 // lane), k_cell_prep32, k_rotate32 / k_rotate_sort32, k_run_shell32 / k_run_kick32.
-#include "device.cuh"
+#include "near_step.cuh"
 
 namespace bgb {
 
@@ -139,44 +139,104 @@ struct f3 { float x, y, z; };
 __device__ __forceinline__ f3 fm(float x, float y, float z) { f3 r; r.x = x; r.y = y; r.z = z; return r; }
 __device__ __forceinline__ f3 fcross(f3 a, f3 b) { return fm(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x); }
 
-// stochastic_reflection (cpp/fluid_colloid_collision.cpp:7-24) in FP32 with the
-// same keyed draws as the FP64 form: Rayleigh normal speed along rs plus one
-// Gaussian tangential component along unit(un x t)
-__device__ f3 reflect32(const SysF64 &S, uint32_t a, uint32_t b, uint32_t t, f3 rf, f3 rs) {
-  int idx = 0;
-  uint4 buf = make_uint4(0, 0, 0, 0);
-  auto next = [&]() {
-    int s = idx & 3;
-    if (s == 0) buf = draw4(S.key, DOM_COLL, (uint32_t)(idx >> 2), a, b, t);
-    idx++;
-    uint32_t w = s == 0 ? buf.x : s == 1 ? buf.y : s == 2 ? buf.z : buf.w;
-    return u01f(w);
-  };
-  float u = next();
-  float om = 1.f - u;
-  float val = sqrtf(-logf(om * om) * (float)S.inv_m_beta);
-  float ir = rsqrtf(rs.x * rs.x + rs.y * rs.y + rs.z * rs.z);
-  f3 un = fm(rs.x * ir * val, rs.y * ir * val, rs.z * ir * val);
-  float t0 = next(), t1 = next(), t2 = next();
-  f3 tt = fm(t0 * S.Lxf - rf.x, t1 * S.Lyf - rf.y, t2 * S.Lzf - rf.z);
-  tt.x -= S.Lxf * rintf(tt.x / S.Lxf); tt.y -= S.Lyf * rintf(tt.y / S.Lyf); tt.z -= S.Lzf * rintf(tt.z / S.Lzf);
-  f3 ut = fcross(un, tt);
-  float iu = rsqrtf(ut.x * ut.x + ut.y * ut.y + ut.z * ut.z);
-  float x1 = 0.f, x2 = 0.f, z = 2.f;
-  for (int it = 0; z > 1.f && it < 256; ++it) {
-    x1 = 2.f * next() - 1.f;
-    x2 = 2.f * next() - 1.f;
-    z = x1 * x1 + x2 * x2;
+// One wall collision of a particle in two halves.  bounce32_draw: everything that the colloid's
+// state does not enter, into Bounce32: the point half a substep back (cell and offset) and, from
+// stochastic_reflection (cpp/fluid_colloid_collision.cpp:7-24, in FP32 with the same keyed draws
+// as the FP64 form), the random point seen from there (part 0), the Rayleigh normal speed (part
+// 1), the tangential Gaussians (part 2; the second only for the fixed rules).  bounce32_apply: the
+// reflection in the colloid's frame, Rayleigh normal speed along rs plus the Gaussian along
+// unit(un x t), the exchange (dv, dl), half a substep forward.
+struct Bounce32 {
+  int cx, cy, cz;
+  float ox, oy, oz;
+  f3 tt;
+  float val, v1, v2;
+};
+
+// (explicitly rounded: the collisions run in several kernels, and left to the compiler the
+// products and sums would be fused differently from one to the next)
+static __device__ __forceinline__ float xd2(f3 a) {
+  return __fmaf_rn(a.z, a.z, __fmaf_rn(a.x, a.x, __fmul_rn(a.y, a.y)));
+}
+static __device__ __forceinline__ float xdet(float a, float b, float c, float d) {  // a b - c d
+  return __fmaf_rn(a, b, -__fmul_rn(c, d));
+}
+static __device__ __forceinline__ f3 xcross(f3 a, f3 b) {
+  return fm(xdet(a.y, b.z, a.z, b.y), xdet(a.z, b.x, a.x, b.z), xdet(a.x, b.y, a.y, b.x));
+}
+static __device__ __forceinline__ void bounce32_draw(const SysF64 &S, long long gs, int j, int id, int part, int cx,
+                                                     int cy, int cz, float ox, float oy, float oz, float vx, float vy,
+                                                     float vz, Bounce32 &o) {
+  const uint32_t a = (uint32_t)(id + 1), b = (uint32_t)(j + 1), t = (uint32_t)gs;
+  if (part == 0) {
+    ox = __fmaf_rn(__fmul_rn(-0.5f, vx), S.dtf, ox); oy = __fmaf_rn(__fmul_rn(-0.5f, vy), S.dtf, oy);
+    oz = __fmaf_rn(__fmul_rn(-0.5f, vz), S.dtf, oz);
+    carry(cx, ox, S.Lx); carry(cy, oy, S.Ly); carry(cz, oz, S.Lz);
+    const f3 rf = fm(__fadd_rn((float)cx, ox), __fadd_rn((float)cy, oy), __fadd_rn((float)cz, oz));
+    const uint4 r = draw4(S.key, DOM_COLL, 0, a, b, t);
+    const float t0 = u01f(r.y), t1 = u01f(r.z), t2 = u01f(r.w);
+    f3 tt = fm(__fmaf_rn(t0, S.Lxf, -rf.x), __fmaf_rn(t1, S.Lyf, -rf.y), __fmaf_rn(t2, S.Lzf, -rf.z));
+    tt.x = __fmaf_rn(-S.Lxf, rintf(tt.x / S.Lxf), tt.x); tt.y = __fmaf_rn(-S.Lyf, rintf(tt.y / S.Lyf), tt.y); tt.z = __fmaf_rn(-S.Lzf, rintf(tt.z / S.Lzf), tt.z);
+    o.cx = cx; o.cy = cy; o.cz = cz;
+    o.ox = ox; o.oy = oy; o.oz = oz;
+    o.tt = tt;
+  } else if (part == 1) {
+    const float u = u01f(draw4(S.key, DOM_COLL, 0, a, b, t).x);
+    const float om = 1.f - u;
+    o.val = sqrtf(-logf(om * om) * (float)S.inv_m_beta);
+  } else {
+    // pairs of Box-Muller tries from the second block of draws on
+    float x1 = 0.f, x2 = 0.f, z = 2.f;
+    uint4 r = make_uint4(0, 0, 0, 0);
+    for (int it = 0; z > 1.f && it < 256; ++it) {
+      if ((it & 1) == 0) r = draw4(S.key, DOM_COLL, 1u + (uint32_t)(it >> 1), a, b, t);
+      x1 = __fmaf_rn(2.f, u01f((it & 1) ? r.z : r.x), -1.f);
+      x2 = __fmaf_rn(2.f, u01f((it & 1) ? r.w : r.y), -1.f);
+      z = __fmaf_rn(x1, x1, __fmul_rn(x2, x2));
+    }
+    z = sqrtf(-2.f * logf(z) / z);
+    o.v1 = x1 * z * (float)S.sqrt_kt_m;
+    o.v2 = x2 * z * (float)S.sqrt_kt_m;
   }
-  z = sqrtf(-2.f * logf(z) / z);
-  float v1 = x1 * z * (float)S.sqrt_kt_m;
-  f3 res = fm(ut.x * iu * v1 + un.x, ut.y * iu * v1 + un.y, ut.z * iu * v1 + un.z);
+}
+
+static __device__ __forceinline__ void bounce32_apply(const SysF64 &S, int j, float4 cq, float4 co, f3 vdump,
+                                                      const Bounce32 &o, int &cx, int &cy, int &cz, float &ox,
+                                                      float &oy, float &oz, float &vx, float &vy, float &vz, f3 &dv,
+                                                      f3 &dl) {
+  cx = o.cx; cy = o.cy; cz = o.cz;
+  ox = o.ox; oy = o.oy; oz = o.oz;
+  const f3 rs = fm(rel(cx, ox, cq.x, co.x, S.Lx), rel(cy, oy, cq.y, co.y, S.Ly), rel(cz, oz, cq.z, co.z, S.Lz));
+  const float ir = rsqrtf(xd2(rs));
+  const f3 n = fm(__fmul_rn(rs.x, ir), __fmul_rn(rs.y, ir), __fmul_rn(rs.z, ir));
+  const f3 un = fm(__fmul_rn(n.x, o.val), __fmul_rn(n.y, o.val), __fmul_rn(n.z, o.val));
+  const f3 ut = xcross(un, o.tt);
+  const float iu = rsqrtf(xd2(ut));
+  const f3 ti = fm(__fmul_rn(ut.x, iu), __fmul_rn(ut.y, iu), __fmul_rn(ut.z, iu));
+  f3 u = fm(__fmaf_rn(ti.x, o.v1, un.x), __fmaf_rn(ti.y, o.v1, un.y), __fmaf_rn(ti.z, o.v1, un.z));
   if (S.physics) {  // the fixed rules: the second tangential component along n x unit(ut)
-    const float v2 = x2 * z * (float)S.sqrt_kt_m;
-    const f3 t2 = fcross(fm(rs.x * ir, rs.y * ir, rs.z * ir), fm(ut.x * iu, ut.y * iu, ut.z * iu));
-    res = fm(res.x + t2.x * v2, res.y + t2.y * v2, res.z + t2.z * v2);
+    const f3 t2 = xcross(n, ti);
+    u = fm(__fmaf_rn(t2.x, o.v2, u.x), __fmaf_rn(t2.y, o.v2, u.y), __fmaf_rn(t2.z, o.v2, u.z));
   }
-  return res;
+  const f3 V = fm((float)S.V[3 * j], (float)S.V[3 * j + 1], (float)S.V[3 * j + 2]);
+  const f3 W = fm((float)S.W[3 * j], (float)S.W[3 * j + 1], (float)S.W[3 * j + 2]);
+  const f3 wr = xcross(W, rs);
+  vx = __fadd_rn(__fadd_rn(u.x, V.x), wr.x); vy = __fadd_rn(__fadd_rn(u.y, V.y), wr.y); vz = __fadd_rn(__fadd_rn(u.z, V.z), wr.z);
+  dv = fm(vdump.x - vx, vdump.y - vy, vdump.z - vz);
+  dl = xcross(rs, dv);
+  ox = __fmaf_rn(__fmul_rn(0.5f, vx), S.dtf, ox); oy = __fmaf_rn(__fmul_rn(0.5f, vy), S.dtf, oy);
+  oz = __fmaf_rn(__fmul_rn(0.5f, vz), S.dtf, oz);
+  carry(cx, ox, S.Lx); carry(cy, oy, S.Ly); carry(cz, oz, S.Lz);
+}
+
+// both halves at once, with the exchange added
+static __device__ void bounce32(const SysF64 &S, long long gs, int j, float4 cq, float4 co, int id, f3 vdump, int &cx,
+                                int &cy, int &cz, float &ox, float &oy, float &oz, float &vx, float &vy, float &vz) {
+  Bounce32 o;
+  for (int part = 0; part < 3; ++part) bounce32_draw(S, gs, j, id, part, cx, cy, cz, ox, oy, oz, vx, vy, vz, o);
+  f3 dv, dl;
+  bounce32_apply(S, j, cq, co, vdump, o, cx, cy, cz, ox, oy, oz, vx, vy, vz, dv, dl);
+  exch_add6(S.exch + j, mk(dv.x, dv.y, dv.z), mk(dl.x, dl.y, dl.z), &S.ss->err);
 }
 
 // One warp's wall collisions (cpp/fluid_colloid_collision.cpp:26-49) of the particles its
@@ -213,21 +273,7 @@ __device__ __forceinline__ void collide32_warp(const SysF64 &S, long long gs, in
     }
     __syncwarp();
     if (j == 0x7FFFFFFF) continue;
-    // back half a substep, reflect, forward half a substep
-    ox -= 0.5f * vx * S.dtf; oy -= 0.5f * vy * S.dtf; oz -= 0.5f * vz * S.dtf;
-    carry(cx, ox, S.Lx); carry(cy, oy, S.Ly); carry(cz, oz, S.Lz);
-    f3 rs = fm(rel(cx, ox, cq.x, co.x, S.Lx), rel(cy, oy, cq.y, co.y, S.Ly), rel(cz, oz, cq.z, co.z, S.Lz));
-    f3 rf = fm((float)cx + ox, (float)cy + oy, (float)cz + oz);
-    f3 u = reflect32(S, (uint32_t)(id + 1), (uint32_t)(j + 1), (uint32_t)gs, rf, rs);
-    f3 V = fm((float)S.V[3 * j], (float)S.V[3 * j + 1], (float)S.V[3 * j + 2]);
-    f3 W = fm((float)S.W[3 * j], (float)S.W[3 * j + 1], (float)S.W[3 * j + 2]);
-    f3 wr = fcross(W, rs);
-    vx = u.x + V.x + wr.x; vy = u.y + V.y + wr.y; vz = u.z + V.z + wr.z;
-    f3 dv = fm(vdump.x - vx, vdump.y - vy, vdump.z - vz);
-    f3 dl = fcross(rs, dv);
-    exch_add6(S.exch + j, mk(dv.x, dv.y, dv.z), mk(dl.x, dl.y, dl.z), &S.ss->err);
-    ox += 0.5f * vx * S.dtf; oy += 0.5f * vy * S.dtf; oz += 0.5f * vz * S.dtf;
-    carry(cx, ox, S.Lx); carry(cy, oy, S.Ly); carry(cz, oz, S.Lz);
+    bounce32(S, gs, j, cq, co, id, vdump, cx, cy, cz, ox, oy, oz, vx, vy, vz);
   }
 }
 
@@ -451,7 +497,7 @@ int stream32_per_thread(int flags) { return stream32_u(flags); }
 // reach of the flight table: colloids within it of a cell's box can come within a
 // particle's near radius of a particle in the cell
 static __device__ __forceinline__ float flight_reach(const SysF64 &S) {
-  return S.r_shell + S.flight_rv + (float)S.n_sub * S.ss->cm + 0.02f;
+  return S.r_shell + S.flight_rx + (float)S.n_sub * S.ss->cm + 0.02f;
 }
 
 // the flight table of this step (both forms: the colloids' cell + offset copies are kept by
@@ -463,11 +509,16 @@ static __device__ __forceinline__ void k_flight_table32_body(const SysF64 &S, co
   const long long step = S.ss->step;
   if (j == 0 && threadIdx.x == 0) {
     S.ss->nnear = 0;
+    S.ss->nact = 0;
+    S.ss->cm_f = S.ss->cm;
+    S.ss->step_f = step;
+    S.bar[BAR_COLL] = S.bar[BAR_MOVE] = S.bar[BAR_EVX] = 0;
     shift_of(S, step + 2, S.ss->rrn);
   }
   if (j >= S.Nc) return;
   const int b0 = (int)((step * S.n_sub - 1) & 1);
   const float reach = flight_reach(S);
+  if (threadIdx.x == 0) S.ccell[b0][j] = cell_coords(S, S.cbox[b0][j]);
   const float4 cq = S.Xcq[b0][j], co = S.Xco[b0][j];
   const int K = (int)ceilf(reach) + 1, side = 2 * K + 1;
   const int tot = side * side * side;
@@ -485,6 +536,7 @@ static __device__ __forceinline__ void k_flight_table32_body(const SysF64 &S, co
     atomicMax(&fc->tc, tag);
     const int slot = (int)(unsigned)atomicAdd(&fc->tc, 1ull);
     if (slot < FLIGHT_CAP) fc->id[slot] = (uint16_t)j;
+    if (slot == TCAP) S.ss->crowd = step + 1;  // (a cell table, whose reach is shorter, may overflow)
   }
 }
 
@@ -503,20 +555,22 @@ __global__ void __launch_bounds__(128) k_flight_table32_b(const SysF64 *Ss, cons
 // the near list (one atomic per block).
 // U particles per thread (thread t of virtual block b: particles b 256 U + t + 256 u), their
 // loads issued together so that more gathers are in flight
-template <bool ROT, int U>
+// SPLIT: of the near ones, those whose straight path may meet a sphere are also listed as
+// active (k_near_step32)
+template <bool ROT, bool SPLIT, int U>
 static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S, const int VB, int fb) {
   const Fluid32 F = fluid32_at(S, fb);
   const long long step = S.ss->step;
   const int b0 = (int)((step * S.n_sub - 1) & 1);
   int pp[U], cc[U];
-  bool valid[U], near[U];
+  bool valid[U], near[U], active[U];
   float vx[U], vy[U], vz[U];
   uint4 qq[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     pp[u] = VB * (256 * U) + (int)threadIdx.x + 256 * u;
     valid[u] = pp[u] < S.N;
-    near[u] = false;
+    near[u] = active[u] = false;
     if (valid[u]) {
       const int p = pp[u];
       cc[u] = ROT ? S.rotcell[p] : S.C;
@@ -540,10 +594,11 @@ static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S,
     }
     const float travel = (float)S.n_sub * S.dtf * sqrtf(vx[u] * vx[u] + vy[u] * vy[u] + vz[u] * vz[u]);
     const int cnt = tcount(((unsigned long long)w0.y << 32) | w0.x, step);
-    bool nr = false;
+    bool nr = false, ac = false;
     if (!inb || !(travel <= S.flight_rv) || cnt > FLIGHT_CAP) {
-      nr = true;  // faster than the table allows (or not finite), or a crowded cell
+      nr = ac = true;  // faster than the table allows (or not finite), or a crowded cell
     } else if (cnt > 0) {
+      const float rad = near_radius(S, S.ss->cm, S.n_sub), T = (float)S.n_sub * S.dtf;
       const float r = S.r_shell + travel + (float)S.n_sub * S.ss->cm + 0.01f, r2 = r * r;
       const unsigned ids[6] = {w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
       const float4 *Xq = S.Xcq[b0], *Xo = S.Xco[b0];
@@ -552,11 +607,15 @@ static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S,
         const float4 cq = Xq[j], co = Xo[j];
         const float dx = rel(cx, ox, cq.x, co.x, S.Lx), dy = rel(cy, oy, cq.y, co.y, S.Ly),
                     dz = rel(cz, oz, cq.z, co.z, S.Lz);
-        nr = nr || !(dx * dx + dy * dy + dz * dz > r2);
+        if (!(dx * dx + dy * dy + dz * dz > r2)) {
+          nr = true;
+          if (SPLIT) ac = ac || path_meets(dx, dy, dz, T * vx[u], T * vy[u], T * vz[u], rad);
+        }
       }
     }
     near[u] = nr;
-    S.fnear[p] = nr ? 1 : 0;
+    active[u] = ac;
+    S.fnear[p] = nr ? (SPLIT && ac ? 2 : 1) : 0;
   }
   // the near list: one atomic per block for all U rounds
   const int lane = threadIdx.x & 31;
@@ -574,18 +633,31 @@ static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S,
     if (near[u]) S.near[base + __popc(m[u] & lt)] = pp[u];
     base += __popc(m[u]);
   }
+  if (!SPLIT) return;
+  tot = 0;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    m[u] = __ballot_sync(FULL, active[u]);
+    tot += __popc(m[u]);
+  }
+  base = block_base_n(&S.ss->nact, tot, lane);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (active[u]) S.act[base + __popc(m[u] & lt)] = pp[u];
+    base += __popc(m[u]);
+  }
 }
 
-template <bool ROT>
+template <bool ROT, bool SPLIT>
 __global__ void __launch_bounds__(256) k_rotate_classify32(__grid_constant__ const SysF64 S, int fb) {
-  k_rotate_classify32_body<ROT, CLASSIFY32_U>(S, blockIdx.x, fb);
+  k_rotate_classify32_body<ROT, SPLIT, CLASSIFY32_U>(S, blockIdx.x, fb);
 }
 
 // the same over a batch of systems (persistent: batch_for)
 template <bool ROT>
 __global__ void __launch_bounds__(256) k_rotate_classify32_b(const SysF64 *Ss, const int *boff, int nrep, int fb) {
   __shared__ SysF64 sS;
-  batch_for(Ss, boff, nrep, sS, [&](int VB, int) { k_rotate_classify32_body<ROT, CLASSIFY32_U>(sS, VB, fb); });
+  batch_for(Ss, boff, nrep, sS, [&](int VB, int) { k_rotate_classify32_body<ROT, false, CLASSIFY32_U>(sS, VB, fb); });
 }
 
 // the free particles' whole step: n_sub streaming substeps (update_pos_mpcd, the
@@ -593,13 +665,16 @@ __global__ void __launch_bounds__(256) k_rotate_classify32_b(const SysF64 *Ss, c
 // next step's grid shift.  Runs beside the near particles' substeps, which touch none of
 // its particles; a grid of a few blocks per SM walks the fluid (it shares the SMs with the
 // substeps' latency-bound chain).
-static __device__ __forceinline__ void k_free_flight32_body(const SysF64 &S, const int VB, const int NVB, int fb) {
+// (thr: the flag from which on a particle is not this pass's: 1, or 2 where the near ones that
+// no sphere can reach are streamed here too)
+static __device__ __forceinline__ void k_free_flight32_body(const SysF64 &S, const int VB, const int NVB, int fb,
+                                                            int thr) {
   const Fluid32 F = fluid32_at(S, fb);
   const float rr[3] = {(float)S.ss->rrn[0], (float)S.ss->rrn[1], (float)S.ss->rrn[2]};
   for (int p0 = VB * blockDim.x; p0 < S.N; p0 += NVB * blockDim.x) {
     const int p = p0 + threadIdx.x;
     BinTerm32 bt{-1, 0, 0, 0, 0};
-    if (p < S.N && !S.fnear[p]) {
+    if (p < S.N && S.fnear[p] < thr) {
       int cx, cy, cz;
       float ox, oy, oz;
       unpack(F.q[p], cx, cy, cz, ox, oy, oz);
@@ -615,15 +690,15 @@ static __device__ __forceinline__ void k_free_flight32_body(const SysF64 &S, con
   }
 }
 
-__global__ void __launch_bounds__(256) k_free_flight32(__grid_constant__ const SysF64 S, int fb) {
-  k_free_flight32_body(S, blockIdx.x, gridDim.x, fb);
+__global__ void __launch_bounds__(256) k_free_flight32(__grid_constant__ const SysF64 S, int fb, int thr) {
+  k_free_flight32_body(S, blockIdx.x, gridDim.x, fb, thr);
 }
 
 // the same over a batch of systems (persistent: batch_for; each virtual block walks its
 // system's fluid with the system's virtual blocks as stride)
 __global__ void __launch_bounds__(256) k_free_flight32_b(const SysF64 *Ss, const int *boff, int nrep, int fb) {
   __shared__ SysF64 sS;
-  batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_free_flight32_body(sS, VB, NVB, fb); });
+  batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_free_flight32_body(sS, VB, NVB, fb, 1); });
 }
 
 // the per-substep pass over the near list (stride over chunks of 256 U)
@@ -647,8 +722,9 @@ __global__ void __launch_bounds__(256) k_stream32_near_b(const SysF64 *Ss, const
   batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_stream32_near_body<FLAGS>(sS, VB, NVB, l, fb); });
 }
 
-ClassifyKernel classify_kernel32(bool rotate) {
-  return rotate ? k_rotate_classify32<true> : k_rotate_classify32<false>;
+ClassifyKernel classify_kernel32(bool rotate, bool split) {
+  return rotate ? (split ? k_rotate_classify32<true, true> : k_rotate_classify32<true, false>)
+                : (split ? k_rotate_classify32<false, true> : k_rotate_classify32<false, false>);
 }
 
 ClassifyKernelB classify_kernel32_b(bool rotate) {
@@ -895,6 +971,30 @@ __global__ void __launch_bounds__(256) k_rotate_sort32_b(const SysF64 *Ss, const
   batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_rotate_sort32_body(sS, VB, NVB, src, dst); });
 }
 
+// candidates of a particle for its next `rem` substeps, packed: the colloids its straight path
+// comes near, from the flight table of its cell (positions in buffer b); NEAR_WILD where that
+// does not cover them
+static __device__ __forceinline__ unsigned near_cand32(const SysF64 &S, long long step, int rem, int b, int cx,
+                                                       int cy, int cz, float ox, float oy, float oz, float vx,
+                                                       float vy, float vz) {
+  if (!(cx < S.Lx && cy < S.Ly && cz < S.Lz)) return NEAR_WILD;
+  const float T = (float)rem * S.dtf;
+  const float wx = T * vx, wy = T * vy, wz = T * vz;
+  if (!(sqrtf(wx * wx + wy * wy + wz * wz) <= S.flight_rv)) return NEAR_WILD;
+  const NearList q = near_list(S, step, lin_cell(S, cx, cy, cz), false);
+  if (q.brute) return NEAR_WILD;
+  const float rad = near_radius(S, S.ss->cm, rem);
+  unsigned cand = NEAR_NONE;
+  for (int k = 0; k < q.cnt; ++k) {
+    const int j = q.ids[k];
+    const float4 cq = S.Xcq[b][j], co = S.Xco[b][j];
+    if (path_meets(rel(cx, ox, cq.x, co.x, S.Lx), rel(cy, oy, cq.y, co.y, S.Ly), rel(cz, oz, cq.z, co.z, S.Lz), wx,
+                   wy, wz, rad))
+      cand = near_add(cand, j);
+  }
+  return cand;
+}
+
 // run() (cpp/run.cpp:17-24) on the FP32 fluid: rear-shell test against V + v0 ra
 static __device__ __forceinline__ void k_run_shell32_body(const SysF64 &S, const int VB, const int NVB, int fb) {
   const int n = min(S.ss->nshell, S.shell_cap);
@@ -933,7 +1033,9 @@ __global__ void k_run_shell32_b(const SysF64 *Ss, const int *boff, int nrep, int
   batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_run_shell32_body(sS, VB, NVB, fb); });
 }
 
-static __device__ __forceinline__ void k_run_kick32_body(const SysF64 &S, const int VB, const int NVB, int fb) {
+// (split: a near particle whose kicked path may meet a sphere becomes active)
+static __device__ __forceinline__ void k_run_kick32_body(const SysF64 &S, const int VB, const int NVB, int fb,
+                                                         bool split) {
   const int n = min(S.ss->nshell, S.shell_cap);
   const Fluid32 F = fluid32_at(S, fb);
   for (int i = VB * blockDim.x + threadIdx.x; i < n; i += NVB * blockDim.x) {
@@ -949,17 +1051,387 @@ static __device__ __forceinline__ void k_run_kick32_body(const SysF64 &S, const 
       vx -= (float)S.ra[3 * j] * f; vy -= (float)S.ra[3 * j + 1] * f; vz -= (float)S.ra[3 * j + 2] * f;
     }
     F.vx[p] = vx; F.vy[p] = vy; F.vz[p] = vz;
+    if (split && S.fnear[p] == 1) {
+      int cx, cy, cz;
+      float ox, oy, oz;
+      unpack(F.q[p], cx, cy, cz, ox, oy, oz);
+      const int b0 = (int)((S.ss->step * S.n_sub - 1) & 1);
+      if (near_cand32(S, S.ss->step, S.n_sub, b0, cx, cy, cz, ox, oy, oz, vx, vy, vz) != NEAR_NONE) {
+        S.fnear[p] = 2;
+        S.act[atomicAdd(&S.ss->nact, 1)] = p;
+      }
+    }
   }
 }
 
-__global__ void k_run_kick32(__grid_constant__ const SysF64 S, int fb) {
-  k_run_kick32_body(S, blockIdx.x, gridDim.x, fb);
+__global__ void k_run_kick32(__grid_constant__ const SysF64 S, int fb, int split) {
+  k_run_kick32_body(S, blockIdx.x, gridDim.x, fb, split != 0);
 }
 
 // the same over a batch of systems (persistent: batch_for)
 __global__ void k_run_kick32_b(const SysF64 *Ss, const int *boff, int nrep, int fb) {
   __shared__ SysF64 sS;
-  batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_run_kick32_body(sS, VB, NVB, fb); });
+  batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_run_kick32_body(sS, VB, NVB, fb, false); });
+}
+
+// ------------------------------------------------- active particles' substeps (FP32 form)
+
+constexpr int NEAR32_ACT = 3584, NEAR32_CHK = 128, NEAR32_IDX = 1024;
+
+// A listed particle of k_near_step32 (entry k), as NearEv of the FP64 form: the colloids it can
+// be inside of in the substep, and what its reflection off the first of them (jc) needs that no
+// colloid position enters
+struct NearChk {
+  int k, id, jc, nc;
+  Bounce32 b;
+  uint16_t cd[4];
+  bool slow;
+};
+
+// Per block: NEAR32_ACT active particles in shared memory (32 bytes each; more stay in the
+// other fluid buffer, which is free between sorts), the list of those to test exactly (more
+// than NEAR32_IDX: in that buffer too) and their preparations (beyond NEAR32_CHK: none).
+struct Near32 {
+  uint4 q[NEAR32_ACT];
+  float v[3][NEAR32_ACT];
+  unsigned cand[NEAR32_ACT];
+  int idx[NEAR32_IDX];
+  NearChk chk[NEAR32_CHK];
+};
+
+// run() candidate record of a particle after the last substep: the colloids, in ascending
+// order, whose boxes (of the substep before, buffer buf ^ 1) hold cell lin and whose run()
+// shell holds the particle; hit: it collided in this substep (its record then ends silently at
+// the first SHELL_J colloids, as the event pass's does)
+static __device__ __forceinline__ void near_shell32(const SysF64 &S, long long step, int buf, int cx, int cy, int cz,
+                                                    float ox, float oy, float oz, const NearCell &c, int id, bool hit,
+                                                    ShellRec &rec) {
+  const NearList q = near_list(S, step, c.lin, false);
+  const float rs2 = S.r_shell * S.r_shell;
+  rec.p = id;
+  rec.n = 0;
+  rec.pass = 0;
+  int last = -1;
+  for (int k = 0;; ++k) {
+    int j;
+    if (q.brute) {
+      j = last = near_next(S, q, last, c, buf ^ 1);
+      if (j < 0) break;
+    } else {
+      if (k >= q.cnt) break;
+      j = q.ids[k];
+    }
+    const float4 cq = S.Xcq[buf][j], co = S.Xco[buf][j];
+    const float dx = rel(cx, ox, cq.x, co.x, S.Lx), dy = rel(cy, oy, cq.y, co.y, S.Ly), dz = rel(cz, oz, cq.z, co.z, S.Lz);
+    if (!(xd2(fm(dx, dy, dz)) <= rs2) || !near_in_block(S, j, c, buf ^ 1)) continue;
+    if (rec.n == SHELL_J) {
+      if (!hit) atomicOr(&S.ss->err, ERRB_SHELLSLOTS);
+      if (rec.j[SHELL_J - 1] < j) continue;
+      --rec.n;
+    }
+    int at = rec.n++;
+    for (; at > 0 && rec.j[at - 1] > j; --at) rec.j[at] = rec.j[at - 1];
+    rec.j[at] = (uint16_t)j;
+  }
+}
+
+// see near_step.cuh.  Eight particle warps; per substep the listed particles' collisions run one
+// per lane, what does not wait for the colloids (Philox, logarithms) prepared beside the
+// colloids' finish.
+// (112 registers: the free-flight pass's two blocks fit beside it)
+__global__ void __maxnreg__(112) k_near_step32(__grid_constant__ const SysF64 S, int fb) {
+  constexpr int NT = NEAR32_BLOCK - 32 * (NEAR_CW + 1), NW = NT / 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Near32 &sm = *reinterpret_cast<Near32 *>(smem_raw);
+  __shared__ double s_hx[NT][6];  // the exchanges of a round's collisions, and their colloids
+  __shared__ int s_hj[NT];
+  __shared__ int s_nh, s_nchk, s_hits, s_fin;
+  __shared__ int s_flag[2];
+  const int t = threadIdx.x, VB = blockIdx.x, G = gridDim.x;
+  const int n = S.n_sub;
+  if (t == 0) s_nh = s_nchk = s_hits = s_fin = 0;
+  if (VB == 0 && t == NT) set_shift(S, S.ss->step + 2);  // (the records of this step are all kicked)
+  near_let_dependents();
+  __syncthreads();
+  if (t >= NT + 32 * NEAR_CW) {
+    near_orient(S, VB, G, t & 31, &s_fin);
+    return;
+  }
+  if (t >= NT) {
+    near_colloids(S, VB, G, t - NT, 2, &s_flag[1], &s_fin);
+    return;
+  }
+  const long long step = S.ss->step, g0 = step * n;
+  const float cm = S.ss->cm;
+  const Fluid32 F = fluid32_at(S, fb), O = fluid32_at(S, 1 - fb);
+  const int nact = min(S.ss->nact, S.N);
+  const int a0 = (int)((long long)VB * nact / G), cnt = (int)((long long)(VB + 1) * nact / G) - a0;
+  auto sync = [] { group_sync(1, NT); };
+  auto pq = [&](int k) -> uint4 * { return k < NEAR32_ACT ? &sm.q[k] : O.q + a0 + k; };
+  auto pv = [&](int c, int k) -> float * {
+    if (k < NEAR32_ACT) return &sm.v[c][k];
+    return (c == 0 ? O.vx : c == 1 ? O.vy : O.vz) + a0 + k;
+  };
+  auto idx = [&](int i) -> int * { return i < NEAR32_IDX ? &sm.idx[i] : O.id + a0 + i; };
+#pragma unroll 4
+  for (int k = t; k < cnt; k += NT) {
+    const int p = S.act[a0 + k];
+    const uint4 q = F.q[p];
+    const float vx = F.vx[p], vy = F.vy[p], vz = F.vz[p];
+    *pq(k) = q;
+    *pv(0, k) = vx; *pv(1, k) = vy; *pv(2, k) = vz;
+  }
+  for (int k = t; k < cnt && k < NEAR32_ACT; k += NT) {
+    int cx, cy, cz;
+    float ox, oy, oz;
+    unpack(sm.q[k], cx, cy, cz, ox, oy, oz);
+    sm.cand[k] = near_cand32(S, step, n, (int)((g0 - 1) & 1), cx, cy, cz, ox, oy, oz, sm.v[0][k], sm.v[1][k],
+                             sm.v[2][k]);
+  }
+
+  // update_pos_mpcd of substep l and a test against the positions of l - 1 with the
+  // displacement bound as margin: the particles to test exactly at X(l) are listed and prepared
+  auto advance = [&](int l) {
+    const long long gs = g0 + (l - 1);
+    const int xb = (int)(gs & 1) ^ 1;
+    const float4 *Xq = S.Xcq[xb], *Xo = S.Xco[xb];
+    const float ch = S.r_coll + 1e-3f + cm, far = ch + S.disp_marginf + 1e-3f;
+    for (int k = t; k < cnt; k += NT) {
+      uint4 *q = pq(k);
+      const float vx = *pv(0, k), vy = *pv(1, k), vz = *pv(2, k);
+      int cx, cy, cz;
+      float ox, oy, oz;
+      unpack(*q, cx, cy, cz, ox, oy, oz);
+      unsigned cand = k < NEAR32_ACT ? sm.cand[k] : NEAR_WILD;
+      if (cand == NEAR_STALE)
+        cand = sm.cand[k] = near_cand32(S, step, n - l + 1, xb, cx, cy, cz, ox, oy, oz, vx, vy, vz);
+      ox = fmaf(vx, S.dtf, ox); oy = fmaf(vy, S.dtf, oy); oz = fmaf(vz, S.dtf, oz);
+      carry(cx, ox, S.Lx); carry(cy, oy, S.Ly); carry(cz, oz, S.Lz);
+      *q = pack(cx, cy, cz, ox, oy, oz);
+      auto dist2 = [&](int j) {
+        const float4 cq = Xq[j], co = Xo[j];
+        const float dx = rel(cx, ox, cq.x, co.x, S.Lx), dy = rel(cy, oy, cq.y, co.y, S.Ly),
+                    dz = rel(cz, oz, cq.z, co.z, S.Lz);
+        return dx * dx + dy * dy + dz * dz;
+      };
+      bool e = false;
+      if (cand == NEAR_WILD) {
+        const NearList c = near_list(S, step, lin_cell(S, cx, cy, cz), false);
+        if (c.brute) {
+          for (int j = 0; j < S.Nc && !e; ++j) e = dist2(j) <= ch * ch;
+        } else {
+          for (int m = 0; m < c.cnt && !e; ++m) e = dist2(c.ids[m]) <= ch * ch;
+        }
+      } else {
+        const int j0 = (int)(cand & 0xFFFFu), j1 = (int)(cand >> 16);
+        if (j0 != 0xFFFF) e = e || dist2(j0) <= ch * ch;
+        if (j1 != 0xFFFF) e = e || dist2(j1) <= ch * ch;
+      }
+      if (!e) continue;
+      const int i = atomicAdd(&s_nchk, 1);
+      *idx(i) = k;
+      if (i >= NEAR32_CHK) continue;
+      // the colloids it may be inside of (a second sphere is reached through a collision with the
+      // first), ascending; jc: the first one the sphere and the colloid's move alone reach
+      NearChk &v = sm.chk[i];
+      const NearList c = near_list(S, step, lin_cell(S, cx, cy, cz), false);
+      v.k = k;
+      v.jc = -1;
+      v.nc = 0;
+      v.slow = c.brute;
+      for (int m = 0; m < c.cnt && !v.slow; ++m) {
+        const int j = c.ids[m];
+        const float d2 = dist2(j);
+        if (d2 > far * far || !in_block3(S, S.ccell[xb][j], cx, cy, cz)) continue;
+        if (v.nc == 4) {
+          v.slow = true;
+          break;
+        }
+        int at = v.nc++;
+        for (; at > 0 && v.cd[at - 1] > j; --at) v.cd[at] = v.cd[at - 1];
+        v.cd[at] = (uint16_t)j;
+        if (d2 <= ch * ch && (v.jc < 0 || j < v.jc)) v.jc = j;
+      }
+      if (v.jc < 0) v.nc = 0;
+      if (v.slow || v.nc) v.id = F.id[S.act[a0 + k]];
+    }
+    sync();
+    // the preparations, 32 particles at a time, in three parts on different warps
+    const int nchk = min(s_nchk, NEAR32_CHK);
+    for (int q = t >> 5; q < 3 * ((nchk + 31) / 32); q += NW) {
+      const int i = (q / 3) * 32 + (t & 31);
+      if (i >= nchk) continue;
+      NearChk &v = sm.chk[i];
+      if (v.slow || v.nc == 0) continue;
+      int cx, cy, cz;
+      float ox, oy, oz;
+      unpack(*pq(v.k), cx, cy, cz, ox, oy, oz);
+      bounce32_draw(S, gs, v.jc, v.id, q % 3, cx, cy, cz, ox, oy, oz, *pv(0, v.k), *pv(1, v.k), *pv(2, v.k), v.b);
+    }
+    if (t == 0) s_nh = 0;
+  };
+
+  advance(1);
+  for (int l = 1; l <= n; ++l) {
+    const long long gs = g0 + (l - 1);
+    const int buf = (int)(gs & 1);
+    if (l > 1) {
+      const unsigned Gm = (unsigned)(G < S.Nc ? G : S.Nc);
+      if (!group_wait(S, BAR_MOVE, Gm * (unsigned)(l - 1), t, 1, NT, &s_flag[0])) return;
+    } else {
+      sync();
+    }
+    // the listed particles' wall collisions at X(l), one per lane
+    const int nchk = s_nchk;
+    for (int base = 0;; base += NT) {
+      const int i = base + t;
+      const bool last_round = base + NT >= nchk;
+      if (i < nchk) {
+        const int k = *idx(i);
+        NearChk *v = i < NEAR32_CHK ? &sm.chk[i] : nullptr;
+        if (!v || v->slow || v->nc) {
+          int cx, cy, cz;
+          float ox, oy, oz;
+          unpack(*pq(k), cx, cy, cz, ox, oy, oz);
+          float vx = *pv(0, k), vy = *pv(1, k), vz = *pv(2, k);
+          const int cx0 = cx, cy0 = cy, cz0 = cz;
+          const float ox0 = ox, oy0 = oy, oz0 = oz;
+          const f3 vdump = fm(vx, vy, vz);
+          const NearCell c{lin_cell(S, cx, cy, cz), cx, cy, cz, false};
+          const float4 *Xq = S.Xcq[buf], *Xo = S.Xco[buf];
+          const float rc2 = S.r_coll * S.r_coll;
+          auto inside = [&](int j) {
+            const float4 cq = Xq[j], co = Xo[j];
+            return xd2(fm(rel(cx, ox, cq.x, co.x, S.Lx), rel(cy, oy, cq.y, co.y, S.Ly),
+                          rel(cz, oz, cq.z, co.z, S.Lz))) <= rc2;
+          };
+          int hits = 0;
+          int id = v ? v->id : -1;
+          // the collisions from colloid j on by the general routine
+          auto rest = [&](int j) {
+            const NearList q = near_list(S, step, c.lin, false);
+            for (; j >= 0; j = near_next(S, q, j, c, buf ^ 1)) {
+              if (!inside(j)) continue;
+              if (id < 0) id = F.id[S.act[a0 + k]];
+              ++hits;
+              bounce32(S, gs, j, Xq[j], Xo[j], id, vdump, cx, cy, cz, ox, oy, oz, vx, vy, vz);
+            }
+          };
+          if (!v || v->slow) {
+            rest(near_next(S, near_list(S, step, c.lin, false), -1, c, buf ^ 1));
+          } else {
+            int m = 0, j = -1;
+            for (; m < v->nc; ++m) {
+              j = v->cd[m];
+              if (inside(j)) break;
+            }
+            if (m < v->nc && j != v->jc) {
+              rest(j);
+            } else if (m < v->nc) {
+              ++hits;
+              f3 dv, dl;
+              bounce32_apply(S, j, Xq[j], Xo[j], vdump, v->b, cx, cy, cz, ox, oy, oz, vx, vy, vz, dv, dl);
+              const int h = atomicAdd(&s_nh, 1);
+              s_hj[h] = j;
+              s_hx[h][0] = dv.x; s_hx[h][1] = dv.y; s_hx[h][2] = dv.z;
+              s_hx[h][3] = dl.x; s_hx[h][4] = dl.y; s_hx[h][5] = dl.z;
+              if (m + 1 < v->nc) rest(near_next(S, near_list(S, step, c.lin, false), j, c, buf ^ 1));
+            }
+          }
+          if (hits) {
+            atomicAdd(&s_hits, 1);
+            // the candidates are looked up with a margin; a move beyond it could hide a colloid
+            const float ex = rel(cx, ox, (float)cx0, ox0, S.Lx), ey = rel(cy, oy, (float)cy0, oy0, S.Ly),
+                        ez = rel(cz, oz, (float)cz0, oz0, S.Lz);
+            if (ex * ex + ey * ey + ez * ez > (float)S.disp_margin2) atomicOr(&S.ss->err, ERRB_DISPLACE);
+            *pq(k) = pack(cx, cy, cz, ox, oy, oz);
+            *pv(0, k) = vx; *pv(1, k) = vy; *pv(2, k) = vz;
+            if (k < NEAR32_ACT) sm.cand[k] = NEAR_STALE;
+            const int p = S.act[a0 + k];
+            F.vx[p] = vx; F.vy[p] = vy; F.vz[p] = vz;
+            if (l == n) {
+              // its run() record (by the cell it collided in) and binning
+              ShellRec rec;
+              near_shell32(S, step, buf, cx, cy, cz, ox, oy, oz, c, id, true, rec);
+              if (rec.n) {
+                const int at = atomicAdd(&S.ss->nshell, 1);
+                if (at < S.shell_cap) S.shell[at] = rec;
+                else atomicOr(&S.ss->err, ERRB_SHELL);
+              }
+              const float rr[3] = {(float)S.ss->rrn[0], (float)S.ss->rrn[1], (float)S.ss->rrn[2]};
+              const BinTerm32 b = bin32_term(S, rr, p, cx, cy, cz, ox, oy, oz, vx, vy, vz);
+              bin_add(S.acc + b.c, 1, b.fx, b.fy, b.fz, b.f2);
+              S.fnear[p] = FN_DONE;
+            }
+          }
+        }
+      }
+      sync();
+      // the round's exchanges, a component per thread
+      const int nh = s_nh;
+      for (int q = t; q < 6 * nh; q += NT) exch_add1(S.exch + s_hj[q / 6], q % 6, s_hx[q / 6][q % 6], &S.ss->err);
+      sync();
+      if (t == 0) {
+        if (last_round) {
+          bar_arrive(S.bar + BAR_COLL);
+          s_nchk = 0;
+        } else {
+          s_nh = 0;
+        }
+      }
+      if (last_round) break;
+      sync();
+    }
+    sync();
+    if (l < n) advance(l + 1);
+  }
+
+  // after the last substep: the positions back to the fluid arrays (the run() candidate records
+  // and the binning are the end kernel's, except of what collided in this substep)
+  for (int k = t; k < cnt; k += NT) F.q[S.act[a0 + k]] = *pq(k);
+  if (t == 0 && s_hits) atomicAdd((unsigned long long *)&S.ss->ev_total, (unsigned long long)s_hits);
+}
+
+size_t near_step32_smem() { return sizeof(Near32); }
+
+// The end of a free-flight step, as k_end_flight64: the step counter and the next step's margin
+// (block 0); the run() candidate records of the near particles and the binning of the active
+// ones among them (the others)
+__global__ void __launch_bounds__(256) k_end_flight32(__grid_constant__ const SysF64 S, int fb) {
+  if (blockIdx.x == 0) {
+    k_end_step_body(S, 0, 1);
+    return;
+  }
+  const long long step = S.ss->step_f;
+  const int buf = (int)((step * S.n_sub + S.n_sub - 1) & 1);
+  const Fluid32 F = fluid32_at(S, fb);
+  const float rr[3] = {(float)S.ss->rrn[0], (float)S.ss->rrn[1], (float)S.ss->rrn[2]};
+  const int count = min(S.ss->nnear, S.N), lane = threadIdx.x & 31;
+  for (int base = (blockIdx.x - 1) * 256; base < count; base += (gridDim.x - 1) * 256) {
+    const int i = base + threadIdx.x;
+    ShellRec rec;
+    rec.n = 0;
+    BinTerm32 b{-1, 0, 0, 0, 0};
+    if (i < count) {
+      const int p = S.near[i];
+      const uint8_t fn = S.fnear[p];
+      if (fn != FN_DONE) {
+        int cx, cy, cz;
+        float ox, oy, oz;
+        unpack(F.q[p], cx, cy, cz, ox, oy, oz);
+        const NearCell c{lin_cell(S, cx, cy, cz), cx, cy, cz, false};
+        near_shell32(S, step, buf, cx, cy, cz, ox, oy, oz, c, F.id[p], false, rec);
+        if (fn != FN_NEAR) b = bin32_term(S, rr, p, cx, cy, cz, ox, oy, oz, F.vx[p], F.vy[p], F.vz[p]);
+      }
+    }
+    if (__any_sync(FULL, b.c >= 0)) bin_add_warp(S.acc, b.c, b.fx, b.fy, b.fz, b.f2);
+    const unsigned m = __ballot_sync(FULL, rec.n != 0);
+    const int at = block_base(&S.ss->nshell, m, lane) + __popc(m & ((1u << lane) - 1u));
+    if (rec.n) {
+      if (at < S.shell_cap) S.shell[at] = rec;
+      else atomicOr(&S.ss->err, ERRB_SHELL);
+    }
+  }
 }
 
 // AoS doubles (particle order) -> FP32 records; download scatters back by id

@@ -20,7 +20,7 @@
 //   k_fin         per colloid: end of fluid_colloid_collision, update_activity_direction,
 //                 update_velocity_colloid, then update_pos_md of the next substep
 #include "../../include/brownian_gb300.h"
-#include "device.cuh"
+#include "near_step.cuh"
 
 namespace bgb {
 // One particle's part of the SRD binning for the next step: its cell (recorded
@@ -403,17 +403,18 @@ __global__ void __launch_bounds__(256) k_bin_near(const SysF64 S, int fb) {
 
 // rotation_mpcd of one particle (w' = A w + b of its cell, as k_rotate; ROT false: a
 // counting-sort step, whose scatter rotated it) and its classification against the flight
-// table: a near particle is flagged and listed (one atomic per block).
-template <bool ROT>
+// table: a near particle is flagged and listed (one atomic per block).  SPLIT: of the near
+// ones, those whose straight path may meet a sphere are also listed as active (k_near_step64).
+template <bool ROT, bool SPLIT>
 __global__ void __launch_bounds__(256) k_rotate_classify(const SysF64 S, int fb) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = p < S.N;
   const Fluid F = fluid_at(S, fb);
   const long long step = S.ss->step;
   const int b0 = (int)((step * S.n_sub - 1) & 1);
-  bool near = false;
+  bool near = false, active = false;
   if (valid) {
-    S.pend[p] = 0;  // no particle is pending at the start of a step
+    if (!SPLIT) S.pend[p] = 0;  // no particle is pending at the start of a step
     const int c = ROT ? S.rotcell[p] : S.C;
     double wx = F.wx[p], wy = F.wy[p], wz = F.wz[p];
     const float px = d2f_trunc(F.x[p]), py = d2f_trunc(F.y[p]), pz = d2f_trunc(F.z[p]);
@@ -438,24 +439,33 @@ __global__ void __launch_bounds__(256) k_rotate_classify(const SysF64 S, int fb)
     const float travel = (float)S.n_sub * sqrtf(fx * fx + fy * fy + fz * fz);
     const int cnt = tcount(((unsigned long long)w0.y << 32) | w0.x, step);
     if (!inb || !(travel <= S.flight_rv) || cnt > FLIGHT_CAP) {
-      near = true;  // faster than the table allows (or not finite), or a crowded cell
+      near = active = true;  // faster than the table allows (or not finite), or a crowded cell
     } else if (cnt > 0) {
       const float r = S.r_shell + travel + (float)S.n_sub * S.ss->cm + 0.01f, r2 = r * r;
+      const float rad = near_radius(S, S.ss->cm, S.n_sub), fn = (float)S.n_sub;
       const unsigned ids[6] = {w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
       const float4 *Xf = S.Xf[b0];
       for (int k = 0; k < cnt; ++k) {
         const int j = (int)((ids[k >> 1] >> (16 * (k & 1))) & 0xFFFFu);
         const float4 q = Xf[j];
         const float dx = wrap_half(q.x - px, S.Lxf), dy = wrap_half(q.y - py, S.Lyf), dz = wrap_half(q.z - pz, S.Lzf);
-        near = near || !(dx * dx + dy * dy + dz * dz > r2);
+        if (!(dx * dx + dy * dy + dz * dz > r2)) {
+          near = true;
+          if (SPLIT) active = active || path_meets(-dx, -dy, -dz, fn * fx, fn * fy, fn * fz, rad);
+        }
       }
     }
-    S.fnear[p] = near ? 1 : 0;
+    S.fnear[p] = near ? (SPLIT && active ? 2 : 1) : 0;
   }
   const int lane = threadIdx.x & 31;
   const unsigned m = __ballot_sync(FULL, near);
   const int base = block_base_n(&S.ss->nnear, __popc(m), lane);
   if (near) S.near[base + __popc(m & ((1u << lane) - 1u))] = p;
+  if (SPLIT) {
+    const unsigned ma = __ballot_sync(FULL, active);
+    const int ba = block_base_n(&S.ss->nact, __popc(ma), lane);
+    if (active) S.act[ba + __popc(ma & ((1u << lane) - 1u))] = p;
+  }
 }
 
 // n substeps of update_pos_mpcd along one axis for a free particle: x = mod(x + w, L) n
@@ -550,12 +560,14 @@ static __device__ __forceinline__ double free_stream(double x, double w, int n, 
 // last substep with the next step's grid shift, beside the near particles' substeps,
 // which touch none of its particles.  A grid of a few blocks per SM walks the fluid (it
 // shares the SMs with the substeps' latency-bound chain).
-__global__ void __launch_bounds__(256) k_free_flight(const SysF64 S, int fb) {
+// (thr: the flag from which on a particle is not this pass's: 1, or 2 where the near ones that
+// no sphere can reach are streamed here too)
+__global__ void __launch_bounds__(256) k_free_flight(const SysF64 S, int fb, int thr) {
   const Fluid F = fluid_at(S, fb);
   for (int p0 = blockIdx.x * blockDim.x; p0 < S.N; p0 += gridDim.x * blockDim.x) {
     const int p = p0 + threadIdx.x;
     BinTerm t{-1, 0, 0, 0, 0};
-    if (p < S.N && !S.fnear[p]) {
+    if (p < S.N && S.fnear[p] < thr) {
       const double wx = F.wx[p], wy = F.wy[p], wz = F.wz[p];
       const double x = free_stream(F.x[p], wx, S.n_sub, S.dx), y = free_stream(F.y[p], wy, S.n_sub, S.dy),
                    z = free_stream(F.z[p], wz, S.n_sub, S.dz);
@@ -574,7 +586,10 @@ EventAuxKernel event_aux_kernel(int flags) {
   return nullptr;
 }
 
-ClassifyKernel classify_kernel(bool rotate) { return rotate ? k_rotate_classify<true> : k_rotate_classify<false>; }
+ClassifyKernel classify_kernel(bool rotate, bool split) {
+  return rotate ? (split ? k_rotate_classify<true, true> : k_rotate_classify<true, false>)
+                : (split ? k_rotate_classify<false, true> : k_rotate_classify<false, false>);
+}
 
 StreamKernel stream_kernel_near(int flags) {
   switch (flags) {
@@ -798,6 +813,31 @@ __global__ void __launch_bounds__(256) k_rotate(const SysF64 S, int fb) {
   F.wz[p] = fma(a67.x, wx, fma(a67.y, wy, fma(a8b0.x, wz, b12.y)));
 }
 
+// candidates of a particle for its next `rem` substeps, packed: the colloids its straight path
+// comes near, from the flight table of its cell (positions in buffer b); NEAR_WILD where that
+// does not cover them
+static __device__ __forceinline__ unsigned near_cand64(const SysF64 &S, long long step, int rem, int b, double x,
+                                                       double y, double z, double wx, double wy, double wz) {
+  const float px = d2f_trunc(x), py = d2f_trunc(y), pz = d2f_trunc(z);
+  int cx = (int)px, cy = (int)py, cz = (int)pz;  // positions in (0, L]: L is cell 0
+  cx -= cx == S.Lx ? S.Lx : 0; cy -= cy == S.Ly ? S.Ly : 0; cz -= cz == S.Lz ? S.Lz : 0;
+  if (!(cx >= 0 && cx < S.Lx && cy >= 0 && cy < S.Ly && cz >= 0 && cz < S.Lz)) return NEAR_WILD;
+  const float fr = (float)rem;
+  const float fx = fr * d2f_trunc(wx), fy = fr * d2f_trunc(wy), fz = fr * d2f_trunc(wz);
+  if (!(sqrtf(fx * fx + fy * fy + fz * fz) <= S.flight_rv)) return NEAR_WILD;
+  const NearList q = near_list(S, step, lin_cell(S, cx, cy, cz), false);
+  if (q.brute) return NEAR_WILD;
+  const float rad = near_radius(S, S.ss->cm, rem);
+  unsigned cand = NEAR_NONE;
+  for (int k = 0; k < q.cnt; ++k) {
+    const int j = q.ids[k];
+    const float4 c = S.Xf[b][j];
+    const float dx = wrap_half(c.x - px, S.Lxf), dy = wrap_half(c.y - py, S.Lyf), dz = wrap_half(c.z - pz, S.Lzf);
+    if (path_meets(-dx, -dy, -dz, fx, fy, fz, rad)) cand = near_add(cand, j);
+  }
+  return cand;
+}
+
 // --------------------------------------------------------------------- run()
 
 // rear-shell test of run() (cpp/run.cpp:17-19) against the kicked colloid
@@ -828,7 +868,8 @@ __global__ void k_run_shell(const SysF64 S, int fb) {
 
 // vel_fl -= v0 ra M / (m cnt) for each rear shell the particle is in, in colloid
 // order (cpp/run.cpp:20-24)
-__global__ void k_run_kick(const SysF64 S, int fb) {
+// (split: a near particle whose kicked path may meet a sphere becomes active)
+__global__ void k_run_kick(const SysF64 S, int fb, int split) {
   const int n = min(S.ss->nshell, S.shell_cap);
   const Fluid F = fluid_at(S, fb);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -845,46 +886,16 @@ __global__ void k_run_kick(const SysF64 S, int fb) {
       v = sub3(v, mul3s(del, f));
     }
     F.wx[p] = __dmul_rn(v.x, S.dt); F.wy[p] = __dmul_rn(v.y, S.dt); F.wz[p] = __dmul_rn(v.z, S.dt);
+    if (split && S.fnear[p] == 1 &&
+        near_cand64(S, S.ss->step, S.n_sub, (int)((S.ss->step * S.n_sub - 1) & 1), F.x[p], F.y[p], F.z[p],
+                    F.wx[p], F.wy[p], F.wz[p]) != NEAR_NONE) {
+      S.fnear[p] = 2;
+      S.act[atomicAdd(&S.ss->nact, 1)] = p;
+    }
   }
 }
 
 // ------------------------------------------------------------------ colloids
-
-__device__ __forceinline__ int colloid_cell(const SysF64 &S, d3 X) {
-  bool alias;
-  return cell_of_pos(S, X.x, X.y, X.z, alias);
-}
-
-// colloid position as integer cell + FP32 offset (the FP32 form's coordinates)
-__device__ __forceinline__ void colloid_q(const SysF64 &S, int b, int j, d3 X) {
-  double v[3] = {X.x, X.y, X.z};
-  const int L[3] = {S.Lx, S.Ly, S.Lz};
-  float c[3], o[3];
-  for (int k = 0; k < 3; ++k) {
-    double f = floor(v[k]);
-    float of = (float)(v[k] - f);
-    int ci = (int)f;
-    if (of >= 1.f) { of = 0.f; ci += 1; }
-    ci %= L[k];
-    if (ci < 0) ci += L[k];
-    c[k] = (float)ci;
-    o[k] = of;
-  }
-  S.Xcq[b][j] = make_float4(c[0], c[1], c[2], 0.f);
-  S.Xco[b][j] = make_float4(o[0], o[1], o[2], 0.f);
-}
-
-// grid shift of the SRD binning the coming streaming pass performs (rotation_mpcd
-// of that step draws it first, cpp/rotation_mpcd.cpp:9), keyed by that step
-__device__ __forceinline__ void set_shift(const SysF64 &S, long long nn) {
-  S.ss->nshell = 0;
-  double rr[3];
-  shift_of(S, nn, rr);
-  for (int k = 0; k < 3; ++k) {
-    S.ss->rr[k] = rr[k];
-    S.ss->rrf[k] = (float)rr[k];
-  }
-}
 
 // One warp per colloid (warp w of block b holds colloid b + gridDim.x * w), its
 // vector components on separate lanes so the FP64 latency chains run side by
@@ -906,7 +917,11 @@ static __device__ __forceinline__ void k_fin_body(const SysF64 &S, const int VB,
   const long long step = S.ss->step;
   const long long g = step * S.n_sub + (l - 1);  // substep finished (l >= 1)
   const long long gn = g + 1;                    // substep advanced to
-  if (VB == 0 && threadIdx.x == 0) {
+  if (VB == 0 && threadIdx.x == 0 && (mode & M_FLIGHT)) {
+    // events a pass before this step listed (the set-up's), which no list takes over
+    S.ss->ev_total += S.ss->nnew[0] + S.ss->nnew[1] + S.ss->nevents;
+    S.ss->nnew[0] = S.ss->nnew[1] = S.ss->nevents = 0;
+  } else if (VB == 0 && threadIdx.x == 0) {
     if (S.precision == MPCD_FP64) {
       // the list substep g's streaming pass filled has been taken over by the event
       // pass (into the pending list, empty again after the last substep); its
@@ -1012,6 +1027,7 @@ static __device__ __forceinline__ void k_fin_colloid(const SysF64 &S, int j, int
       if (d2 > S.ss->cm2) atomicOr(&S.ss->err, ERRB_DISPLACE);
       S.Xf[nxt][j] = make_float4((float)Xn.x, (float)Xn.y, (float)Xn.z, 0.f);
       S.cbox[nxt][j] = colloid_cell(S, Xn);
+      S.ccell[nxt][j] = cell_coords(S, S.cbox[nxt][j]);
       colloid_q(S, nxt, j, Xn);
     }
   }
@@ -1074,55 +1090,6 @@ __global__ void __launch_bounds__(128) k_colloid_pot(const SysF64 S, int b) {
   if (lane == 0) S.pot_part[j] = pot;
 }
 
-// completes a step: bumps the step counter
-static __device__ __forceinline__ void k_end_step_body(const SysF64 &S, const int VB, const int NVB) {
-  if (VB != 0) return;
-  // run()'s shell counts start from zero for the next step (its rear-shell test runs beside
-  // the next step's cell pass, so the cell pass cannot clear them)
-  for (int j = threadIdx.x; j < S.Nc; j += blockDim.x) S.shell_cnt[j] = 0;
-  if (S.Nc > 0) {
-    // the next step's colloid margin: twice the largest displacement a substep gives at
-    // the colloids' present speeds, within [0.005, the static bound], and never below the
-    // move the FP64 form's next first streaming pass assumes (from the last substep's
-    // positions to the present ones, already checked against this step's margin; from the
-    // FP32 copies of the positions, plus 2e-5 for their rounding).  A colloid that moves
-    // further in a substep fails the step (the finish checks every move), so the FP32
-    // form's free-flight classification may take n_sub times it as the colloids' move.
-    __shared__ float s_vm[32], s_dm[32];
-    const long long g = (S.ss->step + 1) * S.n_sub;  // the substep the colloids are at
-    const float4 *Fc = S.Xf[g & 1], *Fp = S.Xf[(g - 1) & 1];
-    float vm = 0.f, dm = 0.f;
-    for (int j = threadIdx.x; j < S.Nc; j += blockDim.x) {
-      const float vx = (float)S.V[3 * j], vy = (float)S.V[3 * j + 1], vz = (float)S.V[3 * j + 2];
-      vm = fmaxf(vm, vx * vx + vy * vy + vz * vz);
-      const float4 a = Fc[j], b = Fp[j];
-      const float ex = wrapf(a.x - b.x, S.Lxf), ey = wrapf(a.y - b.y, S.Lyf), ez = wrapf(a.z - b.z, S.Lzf);
-      dm = fmaxf(dm, ex * ex + ey * ey + ez * ez);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      vm = fmaxf(vm, __shfl_xor_sync(0xFFFFFFFFu, vm, o));
-      dm = fmaxf(dm, __shfl_xor_sync(0xFFFFFFFFu, dm, o));
-    }
-    const int w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    if ((threadIdx.x & 31) == 0) {
-      s_vm[w] = vm;
-      s_dm[w] = dm;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int k = 1; k < nw; ++k) {
-        vm = fmaxf(vm, s_vm[k]);
-        dm = fmaxf(dm, s_dm[k]);
-      }
-      float cm = fminf(fmaxf(2.f * (float)S.dt * sqrtf(vm), 0.005f), S.cmarginf);
-      cm = fmaxf(cm, sqrtf(dm) + 2e-5f);
-      S.ss->cm = cm;
-      S.ss->cm2 = (double)cm * (double)cm;
-    }
-  }
-  if (threadIdx.x == 0) S.ss->step += 1;
-}
-
 __global__ void k_end_step(__grid_constant__ const SysF64 S) {
   k_end_step_body(S, blockIdx.x, gridDim.x);
 }
@@ -1152,6 +1119,447 @@ __global__ void __launch_bounds__(256) k_diag_fluid(const SysF64 S, double *part
   }
   if (threadIdx.x == 0)
     for (int k = 0; k < 5; ++k) part[blockIdx.x * 5 + k] = sh[k][0];
+}
+
+// ------------------------------------------------- active particles' substeps (FP64 form)
+
+// A pending particle of k_near_step64: its state streamed to the substep in flight, the colloids
+// it can be inside of (ascending; none: nc = 0), and, prepared while the colloids move, what its
+// reflection off the first of them (jc) needs that no colloid position enters: the point half a
+// substep back, the random point seen from there, the Rayleigh speed and the Gaussians.
+struct NearEv : EvState {
+  double bx, by, bz, tx, ty, tz, val, v1, v2;
+  NearCell c;
+  int jc, nc;
+  uint16_t cd[4];
+  bool slow;  // more than four of them, or an aliased or overflowing cell: searched anew
+};
+static_assert(sizeof(NearEv) <= EV_STATE_BYTES, "records of SysF64::evx");
+
+static __device__ __forceinline__ NearCell near_cell64(const SysF64 &S, double x, double y, double z) {
+  NearCell c;
+  c.lin = cell_of_pos(S, x, y, z, c.alias);
+  c.ix = trunc_nonneg(x); c.iy = trunc_nonneg(y); c.iz = trunc_nonneg(z);
+  return c;
+}
+
+// The colloids a streamed particle may be inside of in this substep (prev: the buffer of the
+// positions before it): those whose boxes hold its cell within the sphere, the colloid's move
+// (mg) and a wall collision's displacement (a second sphere is reached through a collision
+// with the first); jc the first that the sphere and the move alone reach.
+static __device__ __forceinline__ void near_spheres64(const SysF64 &S, long long step, NearEv &e, int prev, float mg) {
+  const NearList q = near_list(S, step, e.c.lin, e.c.alias);
+  e.jc = -1;
+  e.nc = 0;
+  e.slow = q.brute;
+  if (q.brute) return;
+  const float px = d2f_trunc(e.x), py = d2f_trunc(e.y), pz = d2f_trunc(e.z);
+  const float ch = S.r_coll + 1e-3f + mg, far = ch + S.disp_marginf + 1e-3f;
+  for (int k = 0; k < q.cnt; ++k) {
+    const int j = q.ids[k];
+    const float4 c = S.Xf[prev][j];
+    const float dx = wrap_half(c.x - px, S.Lxf), dy = wrap_half(c.y - py, S.Lyf), dz = wrap_half(c.z - pz, S.Lzf);
+    const float d2 = dx * dx + dy * dy + dz * dz;
+    if (d2 > far * far || !in_block3(S, S.ccell[prev][j], e.c.ix, e.c.iy, e.c.iz)) continue;
+    if (e.nc == 4) {
+      e.slow = true;
+      return;
+    }
+    int at = e.nc++;
+    for (; at > 0 && e.cd[at - 1] > j; --at) e.cd[at] = e.cd[at - 1];
+    e.cd[at] = (uint16_t)j;
+    if (d2 <= ch * ch && (e.jc < 0 || j < e.jc)) e.jc = j;
+  }
+  if (e.jc < 0) e.nc = 0;  // no first collision
+}
+
+// the collisions of a particle from colloid j on (j < 0: from the first), one after another, by
+// the general routine: the rare cases that nothing was prepared for
+static __device__ __noinline__ void near_collide_rest(const SysF64 &S, NearEv &e, int j, long long step, long long gs,
+                                                      int buf) {
+  const NearList q = near_list(S, step, e.c.lin, e.c.alias);
+  if (j < 0) j = near_next(S, q, -1, e.c, buf ^ 1);
+  while (j >= 0) {
+    if (within(S, S.X[buf], S.Xf[buf][j], j, e.x, e.y, e.z, S.r_coll, S.sig2q)) ev_collide(S, e, j, gs, buf);
+    j = near_next(S, q, j, e.c, buf ^ 1);
+  }
+}
+
+// run() candidate record of a particle (id) at x, y, z after the last substep: the colloids, in
+// ascending order, whose boxes (of the substep before, buffer buf ^ 1) hold cell c and whose
+// run() shell holds it; *band: the FP32 test against the positions of the substep before
+// (margin mg) leaves the shell membership open, which the streaming pass counts as an event
+static __device__ __forceinline__ void near_shell64(const SysF64 &S, long long step, int buf, float mg, double x,
+                                                    double y, double z, const NearCell &c, int id, ShellRec &rec,
+                                                    bool *band) {
+  const NearList q = near_list(S, step, c.lin, c.alias);
+  const float px = d2f_trunc(x), py = d2f_trunc(y), pz = d2f_trunc(z);
+  const float sl = S.r_shell - 1e-3f - mg, sh = S.r_shell + 1e-3f + mg;
+  rec.p = id;
+  rec.n = 0;
+  rec.pass = 0;
+  *band = c.alias;
+  // (an unordered walk, the ids inserted in order; a colloid beyond the band is no member)
+  int last = -1;
+  for (int k = 0;; ++k) {
+    int j;
+    if (q.brute) {
+      j = last = near_next(S, q, last, c, buf ^ 1);
+      if (j < 0) break;
+    } else {
+      if (k >= q.cnt) break;
+      j = q.ids[k];
+    }
+    const float4 f = S.Xf[buf ^ 1][j];
+    const float dx = wrap_half(f.x - px, S.Lxf), dy = wrap_half(f.y - py, S.Lyf), dz = wrap_half(f.z - pz, S.Lzf);
+    const float d2 = dx * dx + dy * dy + dz * dz;
+    if (d2 > sh * sh || !near_in_block(S, j, c, buf ^ 1)) continue;
+    if (!(d2 < sl * sl)) *band = true;
+    if (!within(S, S.X[buf], S.Xf[buf][j], j, x, y, z, S.r_shell, S.rsh2)) continue;
+    if (rec.n == SHELL_J) {
+      atomicOr(&S.ss->err, ERRB_SHELLSLOTS);
+      continue;
+    }
+    int at = rec.n++;
+    for (; at > 0 && rec.j[at - 1] > j; --at) rec.j[at] = rec.j[at - 1];
+    rec.j[at] = (uint16_t)j;
+  }
+}
+
+// Particles per block kept in shared memory: NEAR64_ACT active ones (52 bytes each; more stay
+// in the other fluid buffer, which is free between sorts) and NEAR64_EV pending ones.
+constexpr int NEAR64_ACT = 1024, NEAR64_EV = 160;
+struct Near64 {
+  double st[6][NEAR64_ACT];
+  unsigned cand[NEAR64_ACT];
+  NearEv ev[NEAR64_EV];
+};
+
+// see near_step.cuh.  A particle the FP32 test cannot clear is pending for the rest of the step,
+// as in the overlapped substeps.  An FP64 instruction takes a warp about 60 cycles, and the SM's
+// FP64 unit 16 of them however many lanes are active, so a substep's collisions run one per lane
+// on as few warps as hold them, and everything that does not wait for the colloids (the
+// logarithms of the draws above all) is prepared beside the colloids' finish.
+__global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant__ const SysF64 S, int fb) {
+  constexpr int NT = NEAR64_BLOCK - 32 * (NEAR_CW + 1), NW = NT / 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Near64 &sm = *reinterpret_cast<Near64 *>(smem_raw);
+  __shared__ double s_hx[NT][6];  // the exchanges of a round's collisions, and their colloids
+  __shared__ int s_hj[NT];
+  __shared__ int s_nh, s_np, s_fin;
+  __shared__ int s_flag[2];
+  const int t = threadIdx.x, VB = blockIdx.x, G = gridDim.x;
+  const int n = S.n_sub;
+  if (t == 0) s_np = s_nh = s_fin = 0;
+  if (VB == 0 && t == NT) set_shift(S, S.ss->step + 2);  // (the records of this step are all kicked)
+  near_let_dependents();
+  __syncthreads();
+  if (t >= NT + 32 * NEAR_CW) {
+    near_orient(S, VB, G, t & 31, &s_fin);
+    return;
+  }
+  if (t >= NT) {
+    near_colloids(S, VB, G, t - NT, 2, &s_flag[1], &s_fin);
+    return;
+  }
+  const long long step = S.ss->step, g0 = step * n;
+  const float mg = S.ss->cm;
+  const Fluid F = fluid_at(S, fb), O = fluid_at(S, 1 - fb);
+  const int nact = min(S.ss->nact, S.N);
+  const int a0 = (int)((long long)VB * nact / G), cnt = (int)((long long)(VB + 1) * nact / G) - a0;
+  const int w = t >> 5, lane = t & 31;
+  auto sync = [] { group_sync(1, NT); };
+  // active particle k of the block: its state in shared memory or in the other fluid buffer
+  auto ptr = [&](int c, int k) -> double * {
+    if (k < NEAR64_ACT) return &sm.st[c][k];
+    double *o = c == 0 ? O.x : c == 1 ? O.y : c == 2 ? O.z : c == 3 ? O.wx : c == 4 ? O.wy : O.wz;
+    return o + a0 + k;
+  };
+  auto ev = [&](int i) -> NearEv & {
+    return i < NEAR64_EV ? sm.ev[i]
+                         : *reinterpret_cast<NearEv *>((char *)S.evx + (size_t)EV_STATE_BYTES * O.id[a0 + i]);
+  };
+#pragma unroll 2
+  for (int k = t; k < cnt; k += NT) {
+    const int p = S.act[a0 + k];
+    const double x = F.x[p], y = F.y[p], z = F.z[p], wx = F.wx[p], wy = F.wy[p], wz = F.wz[p];
+    *ptr(0, k) = x; *ptr(1, k) = y; *ptr(2, k) = z;
+    *ptr(3, k) = wx; *ptr(4, k) = wy; *ptr(5, k) = wz;
+  }
+  for (int k = t; k < cnt && k < NEAR64_ACT; k += NT)
+    sm.cand[k] = near_cand64(S, step, n, (int)((g0 - 1) & 1), sm.st[0][k], sm.st[1][k], sm.st[2][k], sm.st[3][k],
+                             sm.st[4][k], sm.st[5][k]);
+
+  // update_pos_mpcd of substep l and the FP32 test against the positions of l - 1 with the
+  // displacement bound as margin (np: pending particles of the substeps before), then what the
+  // pending ones' collisions can be given in advance
+  auto advance = [&](int l, int np) {
+    const long long gs = g0 + (l - 1);
+    const int xb = (int)(gs & 1) ^ 1;
+    const float4 *Xf = S.Xf[xb];
+    const float ch = S.r_coll + 1e-3f + mg;
+    for (int i = t; i < np; i += NT) {
+      NearEv &e = ev(i);
+      const double x = ref_mod(__dadd_rn(e.x, e.wx), S.dx), y = ref_mod(__dadd_rn(e.y, e.wy), S.dy),
+                   z = ref_mod(__dadd_rn(e.z, e.wz), S.dz);
+      e.c = near_cell64(S, x, y, z);
+      e.x = e.x0 = x; e.y = e.y0 = y; e.z = e.z0 = z;
+      e.dumped = false;
+      near_spheres64(S, step, e, xb, mg);
+    }
+    for (int k = t; k < cnt; k += NT) {
+      const unsigned cand = k < NEAR64_ACT ? sm.cand[k] : (S.fnear[S.act[a0 + k]] != FN_ACTIVE ? NEAR_GONE : NEAR_WILD);
+      if (cand == NEAR_GONE) continue;
+      double *px = ptr(0, k), *py = ptr(1, k), *pz = ptr(2, k);
+      const double wx = *ptr(3, k), wy = *ptr(4, k), wz = *ptr(5, k);
+      const double x = ref_mod(__dadd_rn(*px, wx), S.dx), y = ref_mod(__dadd_rn(*py, wy), S.dy),
+                   z = ref_mod(__dadd_rn(*pz, wz), S.dz);
+      const float fx = d2f_trunc(x), fy = d2f_trunc(y), fz = d2f_trunc(z);
+      auto close = [&](int j) {
+        const float4 c = Xf[j];
+        const float dx = wrap_half(c.x - fx, S.Lxf), dy = wrap_half(c.y - fy, S.Lyf), dz = wrap_half(c.z - fz, S.Lzf);
+        return dx * dx + dy * dy + dz * dz <= ch * ch;
+      };
+      const NearCell c = near_cell64(S, x, y, z);
+      bool e = c.alias;
+      if (cand == NEAR_WILD) {
+        const NearList q = near_list(S, step, c.lin, c.alias);
+        if (q.brute) {
+          for (int j = 0; j < S.Nc && !e; ++j) e = close(j) && near_in_block(S, j, c, xb);
+        } else {
+          for (int m = 0; m < q.cnt && !e; ++m) e = close(q.ids[m]) && near_in_block(S, q.ids[m], c, xb);
+        }
+      } else {
+        const int j0 = (int)(cand & 0xFFFFu), j1 = (int)(cand >> 16);
+        if (j0 != 0xFFFF) e = e || (close(j0) && near_in_block(S, j0, c, xb));
+        if (j1 != 0xFFFF) e = e || (close(j1) && near_in_block(S, j1, c, xb));
+      }
+      if (!e) {
+        *px = x; *py = y; *pz = z;
+        continue;
+      }
+      const int i = atomicAdd(&s_np, 1), p = S.act[a0 + k];
+      if (i >= NEAR64_EV) {
+        int o = (int)atomicAdd(S.bar + BAR_EVX, 1u);
+        if (o >= S.evx_cap) {
+          atomicOr(&S.ss->err, ERRB_EVENTS);
+          o = S.evx_cap - 1;
+        }
+        O.id[a0 + i] = o;
+      }
+      NearEv &v = ev(i);
+      v.x = v.x0 = x; v.y = v.y0 = y; v.z = v.z0 = z;
+      v.wx = wx; v.wy = wy; v.wz = wz;
+      v.vdx = v.vdy = v.vdz = 0.0;
+      v.p = p; v.id = F.id[p]; v.lin = c.lin; v.last = -1; v.cnt = 0; v.j = -1;
+      v.alias = c.alias; v.dumped = false; v.changed = false;
+      v.c = c;
+      near_spheres64(S, step, v, xb, mg);
+      S.fnear[p] = FN_PENDING;
+      if (k < NEAR64_ACT) sm.cand[k] = NEAR_GONE;
+    }
+    sync();
+    // the preparations of 32 pending particles at a time, the three independent FP64 chains on
+    // different warps (SM schedulers)
+    const int np1 = s_np;
+    for (int q = w; q < 3 * ((np1 + 31) / 32); q += NW) {
+      const int i = (q / 3) * 32 + lane, what = q % 3;
+      if (i >= np1) continue;
+      NearEv &e = ev(i);
+      if (e.slow || e.nc == 0) continue;
+      const uint32_t a = (uint32_t)(e.id + 1), b = (uint32_t)(e.jc + 1), tt = (uint32_t)gs;
+      if (what == 0) {
+        const double x = ref_mod(__dsub_rn(e.x, __dmul_rn(e.wx, 0.5)), S.dx);
+        const double y = ref_mod(__dsub_rn(e.y, __dmul_rn(e.wy, 0.5)), S.dy);
+        const double z = ref_mod(__dsub_rn(e.z, __dmul_rn(e.wz, 0.5)), S.dz);
+        const d3 tp = refl_point(S, draw4(S.key, DOM_COLL, 0, a, b, tt), mk(x, y, z));
+        e.bx = x; e.by = y; e.bz = z;
+        e.tx = tp.x; e.ty = tp.y; e.tz = tp.z;
+      } else if (what == 1) {
+        e.val = refl_speed(S, draw4(S.key, DOM_COLL, 0, a, b, tt));
+      } else {
+        double v2;
+        e.v1 = refl_gauss(S, draw4(S.key, DOM_COLL, 1, a, b, tt), a, b, tt, &v2);
+        e.v2 = v2;
+      }
+    }
+    if (t == 0) s_nh = 0;
+  };
+
+  advance(1, 0);
+  for (int l = 1; l <= n; ++l) {
+    const long long gs = g0 + (l - 1);
+    const int buf = (int)(gs & 1);
+    if (l > 1) {
+      const unsigned Gm = (unsigned)(G < S.Nc ? G : S.Nc);
+      if (!group_wait(S, BAR_MOVE, Gm * (unsigned)(l - 1), t, 1, NT, &s_flag[0])) return;
+    } else {
+      sync();
+    }
+    // the pending particles' wall collisions at X(l), one per lane
+    const int np = s_np;
+    for (int base = 0;; base += NT) {
+      const int i = base + t;
+      const bool last_round = base + NT >= np;
+      bool hit = false;
+      d3 vn = mk(0, 0, 0), xb = vn;
+      NearEv *e = nullptr;
+      // the particle after its collision
+      auto settle = [&] {
+        const double wx = __dmul_rn(vn.x, S.dt), wy = __dmul_rn(vn.y, S.dt), wz = __dmul_rn(vn.z, S.dt);
+        // step forward half a substep with the new velocity
+        const double x = ref_mod(__dadd_rn(xb.x, __dmul_rn(wx, 0.5)), S.dx);
+        const double y = ref_mod(__dadd_rn(xb.y, __dmul_rn(wy, 0.5)), S.dy);
+        const double z = ref_mod(__dadd_rn(xb.z, __dmul_rn(wz, 0.5)), S.dz);
+        // the candidates are looked up with a margin; a move beyond it could hide a colloid
+        const double ex = ref_img(__dsub_rn(x, e->x0), S.dx), ey = ref_img(__dsub_rn(y, e->y0), S.dy),
+                     ez = ref_img(__dsub_rn(z, e->z0), S.dz);
+        if (norm2_ref(ex, ey, ez) > S.disp_margin2) atomicOr(&S.ss->err, ERRB_DISPLACE);
+        e->x = x; e->y = y; e->z = z; e->wx = wx; e->wy = wy; e->wz = wz;
+      };
+      if (i < np) {
+        e = &ev(i);
+        if (e->slow) {
+          near_collide_rest(S, *e, -1, step, gs, buf);
+        } else if (e->nc > 0) {
+          int j = -1, c = 0;
+          for (; c < e->nc; ++c) {
+            j = e->cd[c];
+            if (within(S, S.X[buf], S.Xf[buf][j], j, e->x, e->y, e->z, S.r_coll, S.sig2q)) break;
+          }
+          if (c < e->nc && j != e->jc) {
+            near_collide_rest(S, *e, j, step, gs, buf);  // (inside a sphere the FP32 test had cleared)
+          } else if (c < e->nc) {
+            hit = true;
+            const d3 Vj = ldv(S.V, j), Wj = ldv(S.W, j), Xj = ldv(S.X[buf], j);
+            xb = mk(e->bx, e->by, e->bz);
+            const d3 rs = mk(ref_img(__dsub_rn(xb.x, Xj.x), S.dx), ref_img(__dsub_rn(xb.y, Xj.y), S.dy),
+                             ref_img(__dsub_rn(xb.z, Xj.z), S.dz));
+            const d3 u = refl_combine(S, refl_unit(rs), e->val, mk(e->tx, e->ty, e->tz), e->v1, e->v2);
+            // dump_vel_fl: the velocity when the collision routine began
+            const d3 vd = mk(__dmul_rn(e->wx, S.inv_dt), __dmul_rn(e->wy, S.inv_dt), __dmul_rn(e->wz, S.inv_dt));
+            vn = add3(add3(u, Vj), cross_ref(Wj, rs));
+            const d3 dv = sub3(vd, vn), dl = cross_ref(rs, dv);
+            const int h = atomicAdd(&s_nh, 1);
+            s_hj[h] = j;
+            s_hx[h][0] = dv.x; s_hx[h][1] = dv.y; s_hx[h][2] = dv.z;
+            s_hx[h][3] = dl.x; s_hx[h][4] = dl.y; s_hx[h][5] = dl.z;
+            e->vdx = vd.x; e->vdy = vd.y; e->vdz = vd.z;
+            e->dumped = e->changed = true;
+            if (c + 1 < e->nc) {  // a second sphere may hold it now
+              settle();
+              hit = false;
+              near_collide_rest(S, *e, near_next(S, near_list(S, step, e->c.lin, e->c.alias), j, e->c, buf ^ 1), step,
+                                gs, buf);
+            }
+          }
+        }
+      }
+      sync();
+      // the round's exchanges, a component per thread
+      const int nh = s_nh;
+      for (int q = t; q < 6 * nh; q += NT) exch_add1(S.exch + s_hj[q / 6], q % 6, s_hx[q / 6][q % 6], &S.ss->err);
+      sync();
+      if (t == 0) {
+        if (last_round) bar_arrive(S.bar + BAR_COLL);
+        else s_nh = 0;
+      }
+      if (hit) settle();
+      if (last_round) break;
+      sync();
+    }
+    if (l < n) advance(l + 1, np);
+  }
+
+  // after the last substep: the state back to the fluid arrays (the run() candidate records and
+  // the binning are the end kernel's, except of what collided in this substep)
+  sync();
+  const int np = s_np, buf = (int)((g0 + n - 1) & 1);
+  for (int base = 0; base < np; base += NT) {
+    const int i = base + t;
+    BinTerm b{-1, 0, 0, 0, 0};
+    ShellRec rec;
+    rec.n = 0;
+    if (i < np) {
+      const NearEv &e = ev(i);
+      const int p = e.p;
+      if (e.dumped) {
+        bool band;
+        near_shell64(S, step, buf, mg, e.x, e.y, e.z, e.c, e.id, rec, &band);
+        b = bin_term(S, S.ss->rrn, p, e.x, e.y, e.z, e.wx, e.wy, e.wz);
+        S.fnear[p] = FN_DONE;
+      }
+      F.x[p] = e.x; F.y[p] = e.y; F.z[p] = e.z;
+      F.wx[p] = e.wx; F.wy[p] = e.wy; F.wz[p] = e.wz;
+    }
+    near_record(S, rec, rec.n != 0);
+    bin_add_warp(S.acc, b.c, b.fx, b.fy, b.fz, b.f2);
+  }
+  for (int k = t; k < cnt; k += NT) {
+    const int p = S.act[a0 + k];
+    if (k < NEAR64_ACT ? sm.cand[k] == NEAR_GONE : S.fnear[p] != FN_ACTIVE) continue;
+    F.x[p] = *ptr(0, k); F.y[p] = *ptr(1, k); F.z[p] = *ptr(2, k);
+  }
+  if (t == 0 && np) atomicAdd((unsigned long long *)&S.ss->ev_total, (unsigned long long)np);
+}
+
+size_t near_step64_smem() { return sizeof(Near64); }
+
+__global__ void __launch_bounds__(256) k_rotdiff_step(__grid_constant__ const SysF64 S) {
+  rotdiff_step(S, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// the cell table of a step's first substep at the present positions (the free-flight steps
+// leave none; the per-substep passes read it), one block per colloid
+__global__ void __launch_bounds__(256) k_table_next(const SysF64 S) {
+  const int j = blockIdx.x;
+  if (j >= S.Nc) return;
+  const long long g = S.ss->step * S.n_sub;
+  const int b = (int)(g & 1);
+  int *err = &S.ss->err;
+  for_reach_cells(S, S.cbox[b ^ 1][j], S.Xf[b ^ 1][j], table_reach(S, g), threadIdx.x, blockDim.x,
+                  [&](int cell) { tappend(S.Tcnt[b], S.Tlist[b], cell, g, j, err); });
+}
+
+// The end of a free-flight step: the step counter and the next step's margin (block 0), and, in
+// the other blocks, the run() candidate records of the near particles and the binning of the
+// active ones among them (k_near_step64 wrote their final state).
+__global__ void __launch_bounds__(256) k_end_flight64(__grid_constant__ const SysF64 S, int fb) {
+  if (blockIdx.x == 0) {
+    k_end_step_body(S, 0, 1);
+    return;
+  }
+  const long long step = S.ss->step_f;
+  const float mg = S.ss->cm_f;
+  const int buf = (int)((step * S.n_sub + S.n_sub - 1) & 1);
+  const Fluid F = fluid_at(S, fb);
+  const int count = min(S.ss->nnear, S.N), lane = threadIdx.x & 31;
+  for (int base = (blockIdx.x - 1) * 256; base < count; base += (gridDim.x - 1) * 256) {
+    const int i = base + threadIdx.x;
+    ShellRec rec;
+    rec.n = 0;
+    bool band = false;
+    BinTerm b{-1, 0, 0, 0, 0};
+    if (i < count) {
+      const int p = S.near[i];
+      const uint8_t fn = S.fnear[p];
+      if (fn != FN_DONE) {
+        const double x = F.x[p], y = F.y[p], z = F.z[p];
+        near_shell64(S, step, buf, mg, x, y, z, near_cell64(S, x, y, z), F.id[p], rec, &band);
+        if (fn == FN_PENDING) band = false;  // (counted when it became pending)
+        if (fn != FN_NEAR) b = bin_term(S, S.ss->rrn, p, x, y, z, F.wx[p], F.wy[p], F.wz[p]);
+      }
+    }
+    if (__any_sync(FULL, b.c >= 0)) bin_add_warp(S.acc, b.c, b.fx, b.fy, b.fz, b.f2);
+    const unsigned mb = __ballot_sync(FULL, band);
+    if (lane == 0 && mb) atomicAdd((unsigned long long *)&S.ss->ev_total, (unsigned long long)__popc(mb));
+    const unsigned m = __ballot_sync(FULL, rec.n != 0);
+    const int at = block_base(&S.ss->nshell, m, lane) + __popc(m & ((1u << lane) - 1u));
+    if (rec.n) {
+      if (at < S.shell_cap) S.shell[at] = rec;
+      else atomicOr(&S.ss->err, ERRB_SHELL);
+    }
+  }
 }
 
 // error bits of every system of a batch, for one read-back

@@ -16,7 +16,8 @@ enum : int {
   ERRB_SHELLSLOTS = 32, // a particle sits in the rear shells of more colloids than a record holds
   ERRB_DELTA = 64,      // a colloid momentum exchange left the range of the exact sums
   ERRB_EVENTS = 128,    // the wall-collision event (or pending-particle) lists overflowed
-  ERRB_NBR = 256        // a colloid has more pair-list partners than the list holds
+  ERRB_NBR = 256,       // a colloid has more pair-list partners than the list holds
+  ERRB_WAIT = 512       // a grid-wide wait of the near particles' substeps ran out
 };
 
 constexpr int TCAP = 16;     // colloids per cell in the fluid-to-colloid table
@@ -71,7 +72,16 @@ struct StepState {
   double cm2;
   int nnear;        // free-flight schedule: particles listed for the near passes this step
   double rrn[3];    // free-flight schedule: the next step's grid shift (the free pass bins with it)
+  int nact;         // free-flight schedule: particles whose path may meet a sphere this step
+  float cm_f;       // this step's cm and step number, for the end of the step, whose first block
+  long long step_f; // sets the next step's while the others still record run() candidates
+  long long crowd;  // step + 1 if some flight cell lists more colloids than a cell table holds
 };
+
+// a particle in a free-flight step: free; near; of the near ones active, those of them that
+// became pending (FP64 form), and those that collided in the last substep (their run() record
+// and binning are done with the collision)
+enum : uint8_t { FN_FREE = 0, FN_NEAR = 1, FN_ACTIVE = 2, FN_PENDING = 3, FN_DONE = 4 };
 
 // one cell of the FP32 form's flight table: (step + 1) << 32 | count, and the first
 // FLIGHT_CAP colloids (a cell with more is treated as near for all its particles)
@@ -109,6 +119,7 @@ struct SysF64 {
   float rT_coll, rT_shell;   // cell-table reach (sphere or shell + margins), FP32
   float r_coll, r_shell;     // sphere radius sigma/2 and shell radius sigma/2 + 1/2, FP32
   double disp_margin2;       // squared bound on the displacement of one wall collision
+  float disp_marginf;        // that bound, FP32
   double cmargin2;           // squared bound on a colloid's displacement in one substep
   int kw;                    // fixed-point scale of the cell sums (w and |w|^2)
   double inv_sw;             // 2^-kw
@@ -134,6 +145,7 @@ struct SysF64 {
   double *X[2];        // [Nc][3] double-buffered by global substep parity
   float4 *Xf[2];       // FP32 copies for prefilters
   int *cbox[2];        // 0-based linear cell of each colloid (may alias or exceed C)
+  int4 *ccell[2];      // the coordinates of that cell number and (w) whether it is below C (free-flight steps)
   double *V, *W, *ra, *f;   // [Nc][3]
   double *fnew;             // [Nc][3] force at the positions of the substep in flight
   double *xi;               // [Nc][3] rotational-diffusion normals of the substep in flight
@@ -184,9 +196,20 @@ struct SysF64 {
   // cell the colloids that come within the flight reach of it at the start of the step
   // (tag step + 1, like Tcnt).
   int *near;                    // [N] slots of the near particles
-  uint8_t *fnear;               // [N] 1: the slot's particle is near this step
+  // of these, the ones whose straight path over the step may meet a sphere (or whose path the
+  // flight table does not cover) are active: k_near_step takes them through the substeps
+  int *act;                     // [N] slots of the active particles
+  uint8_t *fnear;               // [N] the slot's particle this step: FN_*
+  unsigned *bar;                // k_near_step's counters, 128 bytes apart (BAR_*)
+  double *xi_all;               // [n_sub][Nc][3] rotational-diffusion normals of the step's substeps
+  double *w_all;                // [n_sub][Nc][3] Omega after each substep of the step
+  void *evx;                    // [evx_cap] records of pending particles beyond a block's shared
+                                // memory (FP64 form; EvState)
+  int evx_cap;
   FlightCell *ftab;             // [C]
   float flight_rv;              // travel allowance: particles moving further in a step are near
+  float flight_rx;              // the table's reach beyond the run() shell: the travel allowance, and
+                                // at least a wall collision's and a colloid's displacement bounds
   int vlist;                    // the free-flight steps compute the forces from a pair list built
                                 // at the start of the step
   // step state
@@ -200,6 +223,11 @@ struct SysF64 {
   int *bkt_cur;        // [NBK_MAX^3] fill cursor of each bucket
   int *bkt_list;       // [Nc] colloids by bucket
 };
+
+// k_near_step's counters in SysF64::bar: blocks whose particles are through the substep's
+// collisions, blocks whose colloids have moved on, overflow records taken
+constexpr int EV_STATE_BYTES = 256;
+enum : int { BAR_COLL = 0, BAR_MOVE = 32, BAR_EVX = 64, BAR_WORDS = 96 };
 
 // the bucket grid of a colloid pair list: per axis nb buckets of width bs >= the list
 // radius (every partner within it is in a neighbouring bucket), r2 = radius^2

@@ -176,8 +176,11 @@ int mpcd_sync(mpcd_ctx *c);
  * in the step plus n_sub times the colloids' bound on a substep's move) is streamed through all
  * substeps and binned by one pass, with the operations the substep passes would apply to it,
  * beside the substeps of the other (near) particles, which the substep passes walk alone.  The
- * results are those of the schedule without it, bit for bit.  mpcd_get_flight gives the near
- * particles of the last step that used it. */
+ * results are those of the schedule without it, bit for bit.  The near particles whose path may
+ * meet a sphere go through the substeps, with the colloids, in one cooperative kernel (its waits
+ * are bounded: MPCD_ERR_CUDA if one runs out); in a system without colloids, with one substep, or
+ * with more colloids around a cell than its tables are made for, in launches per substep.
+ * mpcd_get_flight gives the near particles of the last step that used it. */
 int mpcd_set_flight(mpcd_ctx *c, int on);
 int mpcd_get_flight(mpcd_ctx *c, int32_t *near);
 /* diagnostics of the state now (cpp/active_brownian.cpp:39-55) */
@@ -214,13 +217,15 @@ enum { MPCD_LAUNCH_EVENTS = 0, /* wall-collision events: grid, block (<= 128, mu
                                   second stream beside the streaming and event passes): grid > 0
                                   sets, block = threads per colloid (64, 128 or 256) */
        MPCD_LAUNCH_FREE = 3 }; /* free-flight pass (a persistent grid beside the substeps): grid
-                                  blocks of 256 threads; block = in the FP64 form the substep
-                                  after whose colloid finish it starts (0: right after the
-                                  classification; the default is 1) */
+                                  blocks of 256 threads; block = in the FP64 form, where the
+                                  substeps are launches, the substep after whose colloid finish
+                                  it starts (0: right after the classification; the default is 1) */
 /* grid <= 0 restores the default (events: one block of 128 threads per SM; finish: one block of
  * 32 per SM; side work: 128 threads per colloid, 64 in the FP64 form, whose colloid finish builds
  * the cell tables; free flight: two blocks per SM); results do not depend on the shape (every
- * sum is exact); drops the captured step graphs */
+ * sum is exact); drops the captured step graphs.  The first three are the shapes of the
+ * per-substep launches (mpcd_substep, the routines, mpcd_set_flight(c, 0)); a free-flight step
+ * whose substeps are one kernel has none of these launches. */
 int mpcd_set_launch(mpcd_ctx *c, int which, int grid, int block);
 
 /* ---- exchange record (no counterpart in the reference) ------------------------------- */
