@@ -31,6 +31,20 @@ __device__ __host__ __forceinline__ uint4 philox(uint4 c, uint2 k) {
   return c;
 }
 
+// the same with the rounds as a loop (a tenth of the code), for kernels that run at the rate
+// their code is fetched
+__device__ __forceinline__ uint4 philox_loop(uint4 c, uint2 k) {
+#pragma unroll 1
+  for (int r = 0; r < 10; ++r) {
+    const uint32_t hi0 = __umulhi(0xD2511F53u, c.x), lo0 = 0xD2511F53u * c.x;
+    const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z), lo1 = 0xCD9E8D57u * c.z;
+    c = make_uint4(hi1 ^ c.y ^ k.x, lo1, hi0 ^ c.w ^ k.y, lo0);
+    k.x += 0x9E3779B9u;
+    k.y += 0xBB67AE85u;
+  }
+  return c;
+}
+
 // Draw domains: counter word w carries (domain << 24) | block.
 enum : uint32_t {
   DOM_SHIFT = 1, DOM_AXIS = 2, DOM_COLL = 3, DOM_TUMBLE = 4, DOM_ROTDIFF = 5,
@@ -40,6 +54,10 @@ enum : uint32_t {
 __device__ __host__ __forceinline__ uint4 draw4(uint2 key, uint32_t dom, uint32_t blk, uint32_t a, uint32_t b,
                                                  uint32_t t) {
   return philox(make_uint4(a, b, t, (dom << 24) | (blk & 0xFFFFFFu)), key);
+}
+
+__device__ __forceinline__ uint4 draw4_loop(uint2 key, uint32_t dom, uint32_t blk, uint32_t a, uint32_t b, uint32_t t) {
+  return philox_loop(make_uint4(a, b, t, (dom << 24) | (blk & 0xFFFFFFu)), key);
 }
 
 // The double v 2^-k for an odd v < 2^53 (negated if neg), assembled on the
@@ -94,6 +112,13 @@ struct Dim {
   long long img2_bits;  // bits of 1.49 L
 };
 
+// a - L lround((a - h) / L): the bands of mod and img that need the division, out of line (inlined
+// at every wrap it is most of the kernels' code, and the kernels run at the rate their code is
+// fetched)
+static __device__ __noinline__ double far_mod(double a, double L, double h) {
+  return __dsub_rn(a, __dmul_rn(L, (double)llround(__ddiv_rn(__dsub_rn(a, h), L))));
+}
+
 // The reference's mod(a, L) = a - L*lround((a - L/2)/L) (cpp/parameters.hpp:75).
 // The quotient rounds to 0 for a in [2^-30 L, L) (result a), to 1 for a in
 // [L, 1.49 L) (result a - L*1) and to -1 for a in (-0.49 L, -0] (result
@@ -105,8 +130,7 @@ __device__ __forceinline__ double ref_mod(double a, const Dim &d) {
   if (b >= d.lo_bits && b < d.L_bits) return a;
   if (b >= d.L_bits && b < d.img2_bits) return __dsub_rn(a, d.L);
   if (b < 0 && (b & 0x7FFFFFFFFFFFFFFFll) < d.img_bits) return __dsub_rn(a, -d.L);
-  double q = __ddiv_rn(__dsub_rn(a, d.halfL), d.L);
-  return __dsub_rn(a, __dmul_rn(d.L, (double)llround(q)));
+  return far_mod(a, d.L, d.halfL);
 }
 
 // The reference's img(a, L) = a - L*lround(a/L) (cpp/parameters.hpp:76).  For
@@ -117,7 +141,7 @@ __device__ __forceinline__ double ref_img(double a, const Dim &d) {
   long long b = dbits(a) & 0x7FFFFFFFFFFFFFFFll;
   if (b < d.img_bits) return a;
   if (b > d.img1_bits && b < d.img2_bits) return __dsub_rn(a, a > 0 ? d.L : -d.L);
-  return __dsub_rn(a, __dmul_rn(d.L, (double)llround(__ddiv_rn(a, d.L))));
+  return far_mod(a, d.L, 0.0);
 }
 
 // (x*x + y*y) + z*z with separately rounded products, as point::sum() of a*a.

@@ -2,11 +2,14 @@
 // device-resident state, the constants derived from the parameters, the launch
 // sequence of one MPCD step (captured once into a CUDA graph and replayed), the
 // routine-level entry points, initialisation and diagnostics.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <queue>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/brownian_gb300.h"
@@ -172,14 +175,7 @@ static void launch_on(mpcd_ctx *c, cudaStream_t s, const char *name, void (*k)(K
 // a launch with one launch attribute: cooperative (its blocks wait on one another), or dependent (it
 // starts when every block of the kernel before it on the stream has let it, not when that has ended)
 template <typename... KArgs, typename... Args>
-static void launch_attr(mpcd_ctx *c, cudaStream_t s, const char *name, bool coop, void (*k)(KArgs...), int grid,
-                        int block, size_t smem, Args... args) {
-  ProfEvent pe{name, nullptr, nullptr};
-  if (c->profile || c->tracing) {
-    pe.a = pool_event(c);
-    pe.b = pool_event(c);
-    cudaEventRecordWithFlags(pe.a, s, c->tracing ? cudaEventRecordExternal : cudaEventRecordDefault);
-  }
+static void launch_with(cudaStream_t s, bool coop, void (*k)(KArgs...), int grid, int block, size_t smem, Args... args) {
   cudaLaunchAttribute at;
   if (coop) {
     at.id = cudaLaunchAttributeCooperative;
@@ -196,6 +192,18 @@ static void launch_attr(mpcd_ctx *c, cudaStream_t s, const char *name, bool coop
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+template <typename... KArgs, typename... Args>
+static void launch_attr(mpcd_ctx *c, cudaStream_t s, const char *name, bool coop, void (*k)(KArgs...), int grid,
+                        int block, size_t smem, Args... args) {
+  ProfEvent pe{name, nullptr, nullptr};
+  if (c->profile || c->tracing) {
+    pe.a = pool_event(c);
+    pe.b = pool_event(c);
+    cudaEventRecordWithFlags(pe.a, s, c->tracing ? cudaEventRecordExternal : cudaEventRecordDefault);
+  }
+  launch_with(s, coop, k, grid, block, smem, args...);
   c->launches++;
   if (c->profile || c->tracing) {
     cudaEventRecordWithFlags(pe.b, s, c->tracing ? cudaEventRecordExternal : cudaEventRecordDefault);
@@ -238,9 +246,8 @@ static NListGeo nlist_geo(const mpcd_ctx *c, double rl) {
 // cmargin a substep; the colloid finish fails a step in which one moves further)
 static void enq_step_pairs(mpcd_ctx *c, cudaStream_t s) {
   if (!c->S.vlist) return;
-  const NListGeo geo = nlist_geo(c, c->S.r_cutoff + 2.0 * c->S.n_sub * sqrt(c->S.cmargin2) + 0.05);
-  launch_on(c, s, "k_cbucket", k_cbucket, 1, 1024, c->S, (const double *)nullptr, geo);
-  launch_on(c, s, "k_nlist_step", k_nlist_step, blocks_for(c->S.Nc, 4), 128, c->S, geo);
+  launch_on(c, s, "k_cbucket", k_cbucket, 1, 1024, c->S, (const double *)nullptr, c->S.step_geo);
+  launch_on(c, s, "k_nlist_step", k_nlist_step, blocks_for(c->S.Nc, 4), 128, c->S);
   cudaEventRecord(c->ev_list, s);
 }
 
@@ -812,6 +819,7 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
   S.flight_rx = (float)fmax(5.0 * vth * p.ndt, pmargin + cmargin + 0.05);
   // the free-flight steps' forces from a pair list built at the start of each step
   S.vlist = p.n_colloid > 1 ? 1 : 0;
+  S.step_geo = nlist_geo(c, S.r_cutoff + 2.0 * S.n_sub * sqrt(S.cmargin2) + 0.05);
   // the FP64 form sums displacements w = v dt, the FP32 form velocities
   const double wmax = p.precision == MPCD_FP64 ? vmax * dt : vmax;
   // one scale for the sums of w and |w|^2: max_per_cell * max(wmax, 3 wmax^2) * 2^kw < 2^62
@@ -875,16 +883,19 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
   S.fnear = m.get<uint8_t>(N);
   S.ftab = m.get<FlightCell>(S.C);
   S.act = m.get<int>(N);
+  S.actc = m.get<unsigned>(N);
   S.bar = m.get<unsigned>(BAR_WORDS);
   {
     // A free-flight step takes the active particles through its substeps in one cooperative
     // kernel where there are colloids and at least two substeps, unless the flight table's cells
     // would overflow as a rule: with more than eight colloids expected within its reach of a cell
     // (12 fit), the particles of overflowing cells would scan every colloid, which the
-    // per-substep cell tables avoid.  (The normals of a step: 24 bytes per colloid and substep.)
+    // per-substep cell tables avoid.  (The normals and spins of a step: 48 bytes per colloid and
+    // substep; substep numbers in 16 bits.)
     const double reach = S.r_shell + S.flight_rx + S.n_sub * cmargin + 0.02 + 0.62;  // + a cell's radius as a ball
     const double expected = (double)S.Nc / (double)S.C * 4.0 / 3.0 * M_PI * reach * reach * reach;
-    c->near_step = S.Nc > 0 && S.n_sub >= 2 && expected <= 8.0 && (long long)S.Nc * S.n_sub <= (1ll << 24);
+    c->near_step =
+        S.Nc > 0 && S.n_sub >= 2 && S.n_sub <= 4096 && expected <= 8.0 && (long long)S.Nc * S.n_sub <= (1ll << 24);
     if (c->near_step && p.Dr > 0) S.xi_all = m.get<double>(3 * Nc * (size_t)S.n_sub);
     if (c->near_step) S.w_all = m.get<double>(3 * Nc * (size_t)S.n_sub);
     if (c->near_step && p.precision == MPCD_FP64) {

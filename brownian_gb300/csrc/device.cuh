@@ -87,8 +87,10 @@ static __device__ __forceinline__ int block_base(int *counter, unsigned m, int l
 // boff[r+1] - boff[r] of its system r, with that system's SysF64 copied into shared
 // memory when the run reaches it (a run crosses a system boundary at most a few times).
 // body(VB, NVB) must be called by the whole block, as a kernel body would be.
+// batch_runs: the same shares, a run's part within one system in one piece: body(v0, v1, NVB)
+// for that system's virtual blocks [v0, v1) of NVB
 template <typename Body>
-static __device__ __forceinline__ void batch_for(const SysF64 *Ss, const int *boff, int nrep, SysF64 &sS, Body body) {
+static __device__ __forceinline__ void batch_runs(const SysF64 *Ss, const int *boff, int nrep, SysF64 &sS, Body body) {
   __shared__ int s_r;
   const int total = boff[nrep];
   const int v0 = (int)((long long)blockIdx.x * total / gridDim.x);
@@ -113,7 +115,7 @@ static __device__ __forceinline__ void batch_for(const SysF64 *Ss, const int *bo
   };
   load(r);
   __syncthreads();
-  for (int v = v0; v < v1; ++v) {
+  for (int v = v0; v < v1;) {
     if (v >= next) {  // the run reaches the next system (systems without blocks skipped)
       do {
         ++r;
@@ -123,9 +125,21 @@ static __device__ __forceinline__ void batch_for(const SysF64 *Ss, const int *bo
       load(r);
       __syncthreads();
     }
-    body(v - first, next - first);
+    const int e = min(next, v1);
+    body(v - first, e - first, next - first);
     __syncthreads();  // the body's shared memory and the descriptor are reused
+    v = e;
   }
+}
+
+template <typename Body>
+static __device__ __forceinline__ void batch_for(const SysF64 *Ss, const int *boff, int nrep, SysF64 &sS, Body body) {
+  batch_runs(Ss, boff, nrep, sS, [&](int v0, int v1, int nvb) {
+    for (int v = v0; v < v1; ++v) {
+      if (v > v0) __syncthreads();
+      body(v, nvb);
+    }
+  });
 }
 
 // A cell-table entry is (tag << 32) | count with tag = substep + 1: substeps
@@ -200,6 +214,13 @@ static __device__ __forceinline__ float d2f_trunc(double x) {
   if (fe >= 255) return __int_as_float(0x7f800000);
   unsigned m = (unsigned)((b >> 29) & 0x7FFFFF);
   return __uint_as_float(((unsigned)((unsigned long long)b >> 32) & 0x80000000u) | ((unsigned)fe << 23) | m);
+}
+
+// the same for a position inside the box ([2^-30 L, L)), whose exponent needs no checks (of any
+// other double: some float)
+static __device__ __forceinline__ float d2f_box(double x) {
+  const unsigned long long b = (unsigned long long)dbits(x);
+  return __uint_as_float(__funnelshift_l((unsigned)b, (unsigned)(b >> 32), 3) - (896u << 23));
 }
 
 static __device__ __forceinline__ float wrap_half(float d, float L) {
@@ -284,9 +305,9 @@ struct CollDraw {
   uint4 buf;
 };
 
-static __device__ __forceinline__ double cd_next(CollDraw &d) {
+static __device__ double cd_next(CollDraw &d) {
   int s = d.idx & 3;
-  if (s == 0) d.buf = draw4(d.key, DOM_COLL, (uint32_t)(d.idx >> 2), d.a, d.b, d.t);
+  if (s == 0) d.buf = draw4_loop(d.key, DOM_COLL, (uint32_t)(d.idx >> 2), d.a, d.b, d.t);
   d.idx++;
   uint32_t w = s == 0 ? d.buf.x : s == 1 ? d.buf.y : s == 2 ? d.buf.z : d.buf.w;
   return u01(w);
@@ -319,9 +340,23 @@ static __device__ __forceinline__ double refl_speed(const SysF64 &S, uint4 r0) {
 // tries never run out.  The second try is computed by every lane and selected
 // (2 ran - 1 is exact: pm1 builds it from the draw's bits); only two rejections
 // in a row (1 in 22) branch.
-static __device__ __forceinline__ double refl_gauss(const SysF64 &S, uint4 r1, uint32_t a, uint32_t b, uint32_t t,
-                                                    double *v2) {
-  double x1 = pm1(r1.x), x2 = pm1(r1.y);
+// (refl_try: the accepted try's x1, x2 and, returned, its z)
+static __device__ __noinline__ double refl_more(uint2 key, uint32_t a, uint32_t b, uint32_t t, double &x1, double &x2) {
+  CollDraw d;
+  d.key = key; d.a = a; d.b = b; d.t = t; d.idx = 8;
+  double z = 2.0;
+  for (int it = 2; z > 1.0 && it < 256; ++it) {
+    x1 = __dsub_rn(__dmul_rn(2.0, cd_next(d)), 1.0);
+    x2 = __dsub_rn(__dmul_rn(2.0, cd_next(d)), 1.0);
+    z = __dadd_rn(__dmul_rn(x1, x1), __dmul_rn(x2, x2));
+  }
+  return z;
+}
+
+static __device__ __forceinline__ double refl_try(const SysF64 &S, uint4 r1, uint32_t a, uint32_t b, uint32_t t,
+                                                  double &x1, double &x2) {
+  x1 = pm1(r1.x);
+  x2 = pm1(r1.y);
   double z = __dadd_rn(__dmul_rn(x1, x1), __dmul_rn(x2, x2));
   const double x1b = pm1(r1.z), x2b = pm1(r1.w);
   const double zb = __dadd_rn(__dmul_rn(x1b, x1b), __dmul_rn(x2b, x2b));
@@ -329,15 +364,14 @@ static __device__ __forceinline__ double refl_gauss(const SysF64 &S, uint4 r1, u
   x1 = second ? x1b : x1;
   x2 = second ? x2b : x2;
   z = second ? zb : z;
-  if (z > 1.0) {
-    CollDraw d;
-    d.key = S.key; d.a = a; d.b = b; d.t = t; d.idx = 8;
-    for (int it = 2; z > 1.0 && it < 256; ++it) {
-      x1 = __dsub_rn(__dmul_rn(2.0, cd_next(d)), 1.0);
-      x2 = __dsub_rn(__dmul_rn(2.0, cd_next(d)), 1.0);
-      z = __dadd_rn(__dmul_rn(x1, x1), __dmul_rn(x2, x2));
-    }
-  }
+  if (z > 1.0) z = refl_more(S.key, a, b, t, x1, x2);
+  return z;
+}
+
+static __device__ __forceinline__ double refl_gauss(const SysF64 &S, uint4 r1, uint32_t a, uint32_t b, uint32_t t,
+                                                    double *v2) {
+  double x1, x2;
+  const double z = refl_try(S, r1, a, b, t, x1, x2);
   // -2 log(z) / z as -2 log(z) times 1/z (the reciprocal overlaps the logarithm; within an ulp)
   const double g = __dsqrt_rn(__dmul_rn(__dmul_rn(-2.0, log(z)), __drcp_rn(z)));
   *v2 = __dmul_rn(__dmul_rn(x2, g), S.sqrt_kt_m);
@@ -630,6 +664,8 @@ static __device__ d3 activity_rot(const SysF64 &S, d3 ra, d3 sb, d3 cb, d3 xi) {
   return ra;
 }
 
+static __device__ __noinline__ void sincos_far(double x, double *s, double *c) { sincos(x, s, c); }
+
 // sin x and cos x: for |x| < 2^-6 (the Euler angles Omega dt of a substep) by their
 // Maclaurin series in Horner form, whose first omitted terms x^9/9! and x^10/10! are below
 // 1e-21, so the results are within a few ulp; else sincos
@@ -639,7 +675,7 @@ static __device__ __forceinline__ void sincos_small(double x, double *s, double 
     *s = x * (1.0 - x2 * (1.0 / 6.0) * (1.0 - x2 * (1.0 / 20.0) * (1.0 - x2 * (1.0 / 42.0))));
     *c = 1.0 - x2 * 0.5 * (1.0 - x2 * (1.0 / 12.0) * (1.0 - x2 * (1.0 / 30.0) * (1.0 - x2 * (1.0 / 56.0))));
   } else {
-    sincos(x, s, c);
+    sincos_far(x, s, c);
   }
 }
 

@@ -22,7 +22,7 @@ __global__ void k_cell_prep32_b(const SysF64 *Ss, const int *boff, int nrep);
 __global__ void k_rotate32_b(const SysF64 *Ss, const int *boff, int nrep, int fb);
 __global__ void k_rotate_sort32_b(const SysF64 *Ss, const int *boff, int nrep, int src, int dst);
 __global__ void k_run_shell32_b(const SysF64 *Ss, const int *boff, int nrep, int fb);
-__global__ void k_run_kick32_b(const SysF64 *Ss, const int *boff, int nrep, int fb);
+__global__ void k_run_kick32_b(const SysF64 *Ss, const int *boff, int nrep, int fb, int split);
 __global__ void k_aux_b(const SysF64 *Ss, const int *boff, int nrep, int l, int act);
 __global__ void k_fin_b(const SysF64 *Ss, const int *boff, int nrep, int mode, int l);
 __global__ void k_end_step_b(const SysF64 *Ss, const int *boff, int nrep);
@@ -45,7 +45,7 @@ __global__ void k_rotate_sort32(__grid_constant__ const SysF64 S, int src, int d
 __global__ void k_flight_table32(__grid_constant__ const SysF64 S);
 // the rotation with the classification (rotate false: after a counting-sort scatter); the
 // FP32 form's takes CLASSIFY32_U particles per thread (grid: N / (256 CLASSIFY32_U) blocks)
-constexpr int CLASSIFY32_U = 2;
+constexpr int CLASSIFY32_U = 2, FREE32_CHUNK = 1024;
 using ClassifyKernel = void (*)(const SysF64, int);
 ClassifyKernel classify_kernel32(bool rotate, bool split);
 __global__ void k_free_flight32(__grid_constant__ const SysF64 S, int fb, int thr);
@@ -53,8 +53,8 @@ StreamKernel stream_kernel32_near(int flags);
 // the same over a batch of systems (persistent, batch_for)
 __global__ void k_flight_table32_b(const SysF64 *Ss, const int *boff, int nrep);
 using ClassifyKernelB = void (*)(const SysF64 *, const int *, int, int);
-ClassifyKernelB classify_kernel32_b(bool rotate);
-__global__ void k_free_flight32_b(const SysF64 *Ss, const int *boff, int nrep, int fb);
+ClassifyKernelB classify_kernel32_b(bool rotate, bool split);
+__global__ void k_free_flight32_b(const SysF64 *Ss, const int *boff, int nrep, int fb, int thr);
 StreamKernelB stream_kernel32_near_b(int flags);
 ClassifyKernel classify_kernel(bool rotate, bool split);
 __global__ void k_free_flight(const SysF64 S, int fb, int thr);
@@ -63,13 +63,16 @@ StreamKernel stream_kernel_near(int flags);
 // the active particles' substeps in one cooperative kernel (near_step.cuh), and what goes with it
 __global__ void k_near_step64(__grid_constant__ const SysF64 S, int fb);
 __global__ void k_near_step32(__grid_constant__ const SysF64 S, int fb);
+__global__ void k_near_step32_b(const SysF64 *Ss, const int *boff, int nrep, int first, int fb);
 constexpr int NEAR64_BLOCK = 256, NEAR32_BLOCK = 384;
 size_t near_step64_smem();
 size_t near_step32_smem();
 __global__ void k_rotdiff_step(__grid_constant__ const SysF64 S);
+__global__ void k_rotdiff_step_b(const SysF64 *Ss, const int *boff, int nrep);
 __global__ void k_table_next(const SysF64 S);
 __global__ void k_end_flight64(__grid_constant__ const SysF64 S, int fb);
 __global__ void k_end_flight32(__grid_constant__ const SysF64 S, int fb);
+__global__ void k_end_flight32_b(const SysF64 *Ss, const int *boff, int nrep, int fb);
 // the FP64 event pass fused with the substep's colloid side work (grid: nevb event blocks,
 // then one block per two colloids)
 using EventAuxKernel = void (*)(const SysF64, int, int, int, int);
@@ -91,7 +94,9 @@ __global__ void k_colloid_pot(const SysF64 S, int b);
 // routine-by-routine substeps (routines.cu)
 __global__ void k_cbucket(const SysF64 S, const double *Xc, NListGeo geo);
 __global__ void k_nlist(const SysF64 S, const double *Xc, NListGeo geo);
-__global__ void k_nlist_step(const SysF64 S, NListGeo geo);
+__global__ void k_nlist_step(__grid_constant__ const SysF64 S);
+__global__ void k_cbucket_step_b(const SysF64 *Ss, const int *boff, int nrep);
+__global__ void k_nlist_step_b(const SysF64 *Ss, const int *boff, int nrep);
 __global__ void k_force_list(const SysF64 S, const double *Xc);
 __global__ void k_act_now(const SysF64 S, int l);
 __global__ void k_vel_colloid(const SysF64 S);

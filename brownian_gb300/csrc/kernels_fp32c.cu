@@ -168,12 +168,12 @@ static __device__ __forceinline__ void bounce32_draw(const SysF64 &S, long long 
                                                      int cy, int cz, float ox, float oy, float oz, float vx, float vy,
                                                      float vz, Bounce32 &o) {
   const uint32_t a = (uint32_t)(id + 1), b = (uint32_t)(j + 1), t = (uint32_t)gs;
+  uint4 r = draw4_loop(S.key, DOM_COLL, part == 2 ? 1 : 0, a, b, t);
   if (part == 0) {
     ox = __fmaf_rn(__fmul_rn(-0.5f, vx), S.dtf, ox); oy = __fmaf_rn(__fmul_rn(-0.5f, vy), S.dtf, oy);
     oz = __fmaf_rn(__fmul_rn(-0.5f, vz), S.dtf, oz);
     carry(cx, ox, S.Lx); carry(cy, oy, S.Ly); carry(cz, oz, S.Lz);
     const f3 rf = fm(__fadd_rn((float)cx, ox), __fadd_rn((float)cy, oy), __fadd_rn((float)cz, oz));
-    const uint4 r = draw4(S.key, DOM_COLL, 0, a, b, t);
     const float t0 = u01f(r.y), t1 = u01f(r.z), t2 = u01f(r.w);
     f3 tt = fm(__fmaf_rn(t0, S.Lxf, -rf.x), __fmaf_rn(t1, S.Lyf, -rf.y), __fmaf_rn(t2, S.Lzf, -rf.z));
     tt.x = __fmaf_rn(-S.Lxf, rintf(tt.x / S.Lxf), tt.x); tt.y = __fmaf_rn(-S.Lyf, rintf(tt.y / S.Lyf), tt.y); tt.z = __fmaf_rn(-S.Lzf, rintf(tt.z / S.Lzf), tt.z);
@@ -181,15 +181,14 @@ static __device__ __forceinline__ void bounce32_draw(const SysF64 &S, long long 
     o.ox = ox; o.oy = oy; o.oz = oz;
     o.tt = tt;
   } else if (part == 1) {
-    const float u = u01f(draw4(S.key, DOM_COLL, 0, a, b, t).x);
+    const float u = u01f(r.x);
     const float om = 1.f - u;
     o.val = sqrtf(-logf(om * om) * (float)S.inv_m_beta);
   } else {
     // pairs of Box-Muller tries from the second block of draws on
     float x1 = 0.f, x2 = 0.f, z = 2.f;
-    uint4 r = make_uint4(0, 0, 0, 0);
     for (int it = 0; z > 1.f && it < 256; ++it) {
-      if ((it & 1) == 0) r = draw4(S.key, DOM_COLL, 1u + (uint32_t)(it >> 1), a, b, t);
+      if (it > 0 && (it & 1) == 0) r = draw4_loop(S.key, DOM_COLL, 1u + (uint32_t)(it >> 1), a, b, t);
       x1 = __fmaf_rn(2.f, u01f((it & 1) ? r.z : r.x), -1.f);
       x2 = __fmaf_rn(2.f, u01f((it & 1) ? r.w : r.y), -1.f);
       z = __fmaf_rn(x1, x1, __fmul_rn(x2, x2));
@@ -230,7 +229,7 @@ static __device__ __forceinline__ void bounce32_apply(const SysF64 &S, int j, fl
 }
 
 // both halves at once, with the exchange added
-static __device__ void bounce32(const SysF64 &S, long long gs, int j, float4 cq, float4 co, int id, f3 vdump, int &cx,
+static __device__ __noinline__ void bounce32(const SysF64 &S, long long gs, int j, float4 cq, float4 co, int id, f3 vdump, int &cx,
                                 int &cy, int &cz, float &ox, float &oy, float &oz, float &vx, float &vy, float &vz) {
   Bounce32 o;
   for (int part = 0; part < 3; ++part) bounce32_draw(S, gs, j, id, part, cx, cy, cz, ox, oy, oz, vx, vy, vz, o);
@@ -563,14 +562,16 @@ static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S,
   const long long step = S.ss->step;
   const int b0 = (int)((step * S.n_sub - 1) & 1);
   int pp[U], cc[U];
-  bool valid[U], near[U], active[U];
+  bool valid[U], near[U];
+  unsigned cand[U];  // (SPLIT: the colloids its path comes near)
   float vx[U], vy[U], vz[U];
   uint4 qq[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     pp[u] = VB * (256 * U) + (int)threadIdx.x + 256 * u;
     valid[u] = pp[u] < S.N;
-    near[u] = active[u] = false;
+    near[u] = false;
+    cand[u] = NEAR_NONE;
     if (valid[u]) {
       const int p = pp[u];
       cc[u] = ROT ? S.rotcell[p] : S.C;
@@ -594,9 +595,10 @@ static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S,
     }
     const float travel = (float)S.n_sub * S.dtf * sqrtf(vx[u] * vx[u] + vy[u] * vy[u] + vz[u] * vz[u]);
     const int cnt = tcount(((unsigned long long)w0.y << 32) | w0.x, step);
-    bool nr = false, ac = false;
+    bool nr = false;
     if (!inb || !(travel <= S.flight_rv) || cnt > FLIGHT_CAP) {
-      nr = ac = true;  // faster than the table allows (or not finite), or a crowded cell
+      nr = true;  // faster than the table allows (or not finite), or a crowded cell
+      cand[u] = NEAR_WILD;
     } else if (cnt > 0) {
       const float rad = near_radius(S, S.ss->cm, S.n_sub), T = (float)S.n_sub * S.dtf;
       const float r = S.r_shell + travel + (float)S.n_sub * S.ss->cm + 0.01f, r2 = r * r;
@@ -609,13 +611,12 @@ static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S,
                     dz = rel(cz, oz, cq.z, co.z, S.Lz);
         if (!(dx * dx + dy * dy + dz * dz > r2)) {
           nr = true;
-          if (SPLIT) ac = ac || path_meets(dx, dy, dz, T * vx[u], T * vy[u], T * vz[u], rad);
+          if (SPLIT && path_meets(dx, dy, dz, T * vx[u], T * vy[u], T * vz[u], rad)) cand[u] = near_add(cand[u], j);
         }
       }
     }
     near[u] = nr;
-    active[u] = ac;
-    S.fnear[p] = nr ? (SPLIT && ac ? 2 : 1) : 0;
+    S.fnear[p] = nr ? (SPLIT && cand[u] != NEAR_NONE ? FN_ACTIVE : FN_NEAR) : FN_FREE;
   }
   // the near list: one atomic per block for all U rounds
   const int lane = threadIdx.x & 31;
@@ -637,13 +638,16 @@ static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S,
   tot = 0;
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    m[u] = __ballot_sync(FULL, active[u]);
+    m[u] = __ballot_sync(FULL, cand[u] != NEAR_NONE);
     tot += __popc(m[u]);
   }
   base = block_base_n(&S.ss->nact, tot, lane);
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    if (active[u]) S.act[base + __popc(m[u] & lt)] = pp[u];
+    if (cand[u] != NEAR_NONE) {
+      S.act[base + __popc(m[u] & lt)] = pp[u];
+      S.actc[base + __popc(m[u] & lt)] = cand[u];
+    }
     base += __popc(m[u]);
   }
 }
@@ -654,35 +658,71 @@ __global__ void __launch_bounds__(256) k_rotate_classify32(__grid_constant__ con
 }
 
 // the same over a batch of systems (persistent: batch_for)
-template <bool ROT>
+template <bool ROT, bool SPLIT>
 __global__ void __launch_bounds__(256) k_rotate_classify32_b(const SysF64 *Ss, const int *boff, int nrep, int fb) {
   __shared__ SysF64 sS;
-  batch_for(Ss, boff, nrep, sS, [&](int VB, int) { k_rotate_classify32_body<ROT, false, CLASSIFY32_U>(sS, VB, fb); });
+  batch_for(Ss, boff, nrep, sS, [&](int VB, int) { k_rotate_classify32_body<ROT, SPLIT, CLASSIFY32_U>(sS, VB, fb); });
+}
+
+// n streaming substeps along one axis: the streaming passes' o = fma(v, dt, o) and carry, n
+// times, without a branch: carry's floor leaves an offset in [0, 1) as it is, so it is taken
+// every time (a warp nearly always has a lane that needs it), and the cells carried are added up
+// and wrapped into the box once at the end (integer sums, the same cell).  What carry does with
+// a NaN or runaway offset is left out: its particle fails the range test of the binning.
+static __device__ __forceinline__ void free_axis32(int &c, float &o, float v, float dt, int n, int L) {
+  float k = 0.f;
+#pragma unroll 2
+  for (int l = 0; l < n; ++l) {
+    o = fmaf(v, dt, o);
+    const float f = floorf(o);
+    o -= f;
+    k += f;
+    if (o >= 1.f) { o = 0.f; k += 1.f; }
+  }
+  c += (int)k;
+  if (c < 0 || c >= L) {
+    c %= L;
+    if (c < 0) c += L;
+  }
 }
 
 // the free particles' whole step: n_sub streaming substeps (update_pos_mpcd, the
 // streaming passes' operations in order) and the binning of the last substep with the
 // next step's grid shift.  Runs beside the near particles' substeps, which touch none of
 // its particles; a grid of a few blocks per SM walks the fluid (it shares the SMs with the
-// substeps' latency-bound chain).
+// substeps' latency-bound chain), each thread's next particle loaded while this one is worked on.
 // (thr: the flag from which on a particle is not this pass's: 1, or 2 where the near ones that
 // no sphere can reach are streamed here too)
-static __device__ __forceinline__ void k_free_flight32_body(const SysF64 &S, const int VB, const int NVB, int fb,
-                                                            int thr) {
+// Particles p, p + stride, ... below end.
+static __device__ __forceinline__ void k_free_flight32_body(const SysF64 &S, int p, const int stride, const int end,
+                                                            int fb, int thr) {
   const Fluid32 F = fluid32_at(S, fb);
   const float rr[3] = {(float)S.ss->rrn[0], (float)S.ss->rrn[1], (float)S.ss->rrn[2]};
-  for (int p0 = VB * blockDim.x; p0 < S.N; p0 += NVB * blockDim.x) {
-    const int p = p0 + threadIdx.x;
+  const int n = S.n_sub;
+  uint4 q = make_uint4(0, 0, 0, 0);
+  float wx = 0.f, wy = 0.f, wz = 0.f;
+  int fn = 255;
+  auto load = [&](int i) {
+    fn = 255;
+    if (i < end) {
+      fn = S.fnear[i];
+      q = F.q[i];
+      wx = F.vx[i]; wy = F.vy[i]; wz = F.vz[i];
+    }
+  };
+  load(p);
+  for (int p0 = p - (int)threadIdx.x; p0 < end; p0 += stride, p += stride) {
+    const bool free = fn < thr;
+    const float vx = wx, vy = wy, vz = wz;
+    int cx, cy, cz;
+    float ox, oy, oz;
+    unpack(q, cx, cy, cz, ox, oy, oz);
+    load(p + stride);
     BinTerm32 bt{-1, 0, 0, 0, 0};
-    if (p < S.N && S.fnear[p] < thr) {
-      int cx, cy, cz;
-      float ox, oy, oz;
-      unpack(F.q[p], cx, cy, cz, ox, oy, oz);
-      const float vx = F.vx[p], vy = F.vy[p], vz = F.vz[p];
-      for (int l = 0; l < S.n_sub; ++l) {
-        ox = fmaf(vx, S.dtf, ox); oy = fmaf(vy, S.dtf, oy); oz = fmaf(vz, S.dtf, oz);
-        carry(cx, ox, S.Lx); carry(cy, oy, S.Ly); carry(cz, oz, S.Lz);
-      }
+    if (free) {
+      free_axis32(cx, ox, vx, S.dtf, n, S.Lx);
+      free_axis32(cy, oy, vy, S.dtf, n, S.Ly);
+      free_axis32(cz, oz, vz, S.dtf, n, S.Lz);
       bt = bin32_term(S, rr, p, cx, cy, cz, ox, oy, oz, vx, vy, vz);
       F.q[p] = pack(cx, cy, cz, ox, oy, oz);
     }
@@ -691,14 +731,16 @@ static __device__ __forceinline__ void k_free_flight32_body(const SysF64 &S, con
 }
 
 __global__ void __launch_bounds__(256) k_free_flight32(__grid_constant__ const SysF64 S, int fb, int thr) {
-  k_free_flight32_body(S, blockIdx.x, gridDim.x, fb, thr);
+  k_free_flight32_body(S, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, S.N, fb, thr);
 }
 
-// the same over a batch of systems (persistent: batch_for; each virtual block walks its
-// system's fluid with the system's virtual blocks as stride)
-__global__ void __launch_bounds__(256) k_free_flight32_b(const SysF64 *Ss, const int *boff, int nrep, int fb) {
+// the same over a batch of systems (persistent: batch_runs; a virtual block per FREE32_CHUNK particles)
+__global__ void __launch_bounds__(256, 5) k_free_flight32_b(const SysF64 *Ss, const int *boff, int nrep, int fb,
+                                                         int thr) {
   __shared__ SysF64 sS;
-  batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_free_flight32_body(sS, VB, NVB, fb, 1); });
+  batch_runs(Ss, boff, nrep, sS, [&](int v0, int v1, int) {
+    k_free_flight32_body(sS, v0 * FREE32_CHUNK + (int)threadIdx.x, 256, min(sS.N, v1 * FREE32_CHUNK), fb, thr);
+  });
 }
 
 // the per-substep pass over the near list (stride over chunks of 256 U)
@@ -727,8 +769,9 @@ ClassifyKernel classify_kernel32(bool rotate, bool split) {
                 : (split ? k_rotate_classify32<false, true> : k_rotate_classify32<false, false>);
 }
 
-ClassifyKernelB classify_kernel32_b(bool rotate) {
-  return rotate ? k_rotate_classify32_b<true> : k_rotate_classify32_b<false>;
+ClassifyKernelB classify_kernel32_b(bool rotate, bool split) {
+  return rotate ? (split ? k_rotate_classify32_b<true, true> : k_rotate_classify32_b<true, false>)
+                : (split ? k_rotate_classify32_b<false, true> : k_rotate_classify32_b<false, false>);
 }
 
 StreamKernelB stream_kernel32_near_b(int flags) {
@@ -1051,15 +1094,21 @@ static __device__ __forceinline__ void k_run_kick32_body(const SysF64 &S, const 
       vx -= (float)S.ra[3 * j] * f; vy -= (float)S.ra[3 * j + 1] * f; vz -= (float)S.ra[3 * j + 2] * f;
     }
     F.vx[p] = vx; F.vy[p] = vy; F.vz[p] = vz;
-    if (split && S.fnear[p] == 1) {
+    if (!split) continue;
+    // an active particle's candidates are looked up anew (k_near_step32); another may become active
+    if (S.fnear[p] == FN_ACTIVE) {
+      S.fnear[p] = FN_KICKED;
+    } else if (S.fnear[p] == FN_NEAR) {
       int cx, cy, cz;
       float ox, oy, oz;
       unpack(F.q[p], cx, cy, cz, ox, oy, oz);
       const int b0 = (int)((S.ss->step * S.n_sub - 1) & 1);
-      if (near_cand32(S, S.ss->step, S.n_sub, b0, cx, cy, cz, ox, oy, oz, vx, vy, vz) != NEAR_NONE) {
-        S.fnear[p] = 2;
-        S.act[atomicAdd(&S.ss->nact, 1)] = p;
-      }
+      const unsigned cand = near_cand32(S, S.ss->step, S.n_sub, b0, cx, cy, cz, ox, oy, oz, vx, vy, vz);
+      if (cand == NEAR_NONE) continue;
+      S.fnear[p] = FN_ACTIVE;
+      const int at = atomicAdd(&S.ss->nact, 1);
+      S.act[at] = p;
+      S.actc[at] = cand;
     }
   }
 }
@@ -1069,14 +1118,28 @@ __global__ void k_run_kick32(__grid_constant__ const SysF64 S, int fb, int split
 }
 
 // the same over a batch of systems (persistent: batch_for)
-__global__ void k_run_kick32_b(const SysF64 *Ss, const int *boff, int nrep, int fb) {
+__global__ void k_run_kick32_b(const SysF64 *Ss, const int *boff, int nrep, int fb, int split) {
   __shared__ SysF64 sS;
-  batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_run_kick32_body(sS, VB, NVB, fb, false); });
+  batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_run_kick32_body(sS, VB, NVB, fb, split != 0); });
 }
 
 // ------------------------------------------------- active particles' substeps (FP32 form)
 
 constexpr int NEAR32_ACT = 3584, NEAR32_CHK = 128, NEAR32_IDX = 1024;
+
+// what the tests need of a colloid
+struct __align__(16) NearCol32 {
+  float4 q, o;
+  int4 c;
+  static __device__ __forceinline__ NearCol32 get(const SysF64 &S, int b, int j) {
+    return {S.Xcq[b][j], S.Xco[b][j], S.ccell[b][j]};
+  }
+  static __device__ __forceinline__ void copy(const SysF64 &S, int b, int j, NearCol32 *to) {
+    near_copy16(&to->q, &S.Xcq[b][j]);
+    near_copy16(&to->o, &S.Xco[b][j]);
+    near_copy16(&to->c, &S.ccell[b][j]);
+  }
+};
 
 // A listed particle of k_near_step32 (entry k), as NearEv of the FP64 form: the colloids it can
 // be inside of in the substep, and what its reflection off the first of them (jc) needs that no
@@ -1097,6 +1160,7 @@ struct Near32 {
   unsigned cand[NEAR32_ACT];
   int idx[NEAR32_IDX];
   NearChk chk[NEAR32_CHK];
+  NearCols<NearCol32> col;
 };
 
 // run() candidate record of a particle after the last substep: the colloids, in ascending
@@ -1138,8 +1202,7 @@ static __device__ __forceinline__ void near_shell32(const SysF64 &S, long long s
 // see near_step.cuh.  Eight particle warps; per substep the listed particles' collisions run one
 // per lane, what does not wait for the colloids (Philox, logarithms) prepared beside the
 // colloids' finish.
-// (112 registers: the free-flight pass's two blocks fit beside it)
-__global__ void __maxnreg__(112) k_near_step32(__grid_constant__ const SysF64 S, int fb) {
+static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB, const int G, int fb) {
   constexpr int NT = NEAR32_BLOCK - 32 * (NEAR_CW + 1), NW = NT / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Near32 &sm = *reinterpret_cast<Near32 *>(smem_raw);
@@ -1147,9 +1210,10 @@ __global__ void __maxnreg__(112) k_near_step32(__grid_constant__ const SysF64 S,
   __shared__ int s_hj[NT];
   __shared__ int s_nh, s_nchk, s_hits, s_fin;
   __shared__ int s_flag[2];
-  const int t = threadIdx.x, VB = blockIdx.x, G = gridDim.x;
+  const int t = threadIdx.x;
   const int n = S.n_sub;
   if (t == 0) s_nh = s_nchk = s_hits = s_fin = 0;
+  sm.col.clear(S, t, NEAR32_BLOCK);
   if (VB == 0 && t == NT) set_shift(S, S.ss->step + 2);  // (the records of this step are all kicked)
   near_let_dependents();
   __syncthreads();
@@ -1173,76 +1237,119 @@ __global__ void __maxnreg__(112) k_near_step32(__grid_constant__ const SysF64 S,
     return (c == 0 ? O.vx : c == 1 ? O.vy : O.vz) + a0 + k;
   };
   auto idx = [&](int i) -> int * { return i < NEAR32_IDX ? &sm.idx[i] : O.id + a0 + i; };
-#pragma unroll 4
+#pragma unroll 2
   for (int k = t; k < cnt; k += NT) {
     const int p = S.act[a0 + k];
     const uint4 q = F.q[p];
     const float vx = F.vx[p], vy = F.vy[p], vz = F.vz[p];
+    unsigned cand = S.actc[a0 + k];
+    if (S.fnear[p] == FN_KICKED) {
+      int cx, cy, cz;
+      float ox, oy, oz;
+      unpack(q, cx, cy, cz, ox, oy, oz);
+      cand = near_cand32(S, step, n, (int)((g0 - 1) & 1), cx, cy, cz, ox, oy, oz, vx, vy, vz);
+      S.fnear[p] = FN_ACTIVE;
+    }
     *pq(k) = q;
     *pv(0, k) = vx; *pv(1, k) = vy; *pv(2, k) = vz;
+    if (k < NEAR32_ACT) {
+      sm.cand[k] = cand;
+      sm.col.note(cand);
+    }
   }
-  for (int k = t; k < cnt && k < NEAR32_ACT; k += NT) {
-    int cx, cy, cz;
-    float ox, oy, oz;
-    unpack(sm.q[k], cx, cy, cz, ox, oy, oz);
-    sm.cand[k] = near_cand32(S, step, n, (int)((g0 - 1) & 1), cx, cy, cz, ox, oy, oz, sm.v[0][k], sm.v[1][k],
-                             sm.v[2][k]);
-  }
+  sync();
+  sm.col.load(S, (int)((g0 - 1) & 1), t, NT);
+  for (int k = t; k < min(cnt, NEAR32_ACT); k += NT) sm.cand[k] = sm.col.slots(sm.cand[k]);
+  sync();
 
   // update_pos_mpcd of substep l and a test against the positions of l - 1 with the
   // displacement bound as margin: the particles to test exactly at X(l) are listed and prepared
   auto advance = [&](int l) {
     const long long gs = g0 + (l - 1);
     const int xb = (int)(gs & 1) ^ 1;
-    const float4 *Xq = S.Xcq[xb], *Xo = S.Xco[xb];
     const float ch = S.r_coll + 1e-3f + cm, far = ch + S.disp_marginf + 1e-3f;
-    for (int k = t; k < cnt; k += NT) {
+    // particle k by the general path
+    auto one = [&](int k, unsigned cand) {
       uint4 *q = pq(k);
       const float vx = *pv(0, k), vy = *pv(1, k), vz = *pv(2, k);
       int cx, cy, cz;
       float ox, oy, oz;
       unpack(*q, cx, cy, cz, ox, oy, oz);
-      unsigned cand = k < NEAR32_ACT ? sm.cand[k] : NEAR_WILD;
-      if (cand == NEAR_STALE)
-        cand = sm.cand[k] = near_cand32(S, step, n - l + 1, xb, cx, cy, cz, ox, oy, oz, vx, vy, vz);
       ox = fmaf(vx, S.dtf, ox); oy = fmaf(vy, S.dtf, oy); oz = fmaf(vz, S.dtf, oz);
       carry(cx, ox, S.Lx); carry(cy, oy, S.Ly); carry(cz, oz, S.Lz);
       *q = pack(cx, cy, cz, ox, oy, oz);
-      auto dist2 = [&](int j) {
-        const float4 cq = Xq[j], co = Xo[j];
-        const float dx = rel(cx, ox, cq.x, co.x, S.Lx), dy = rel(cy, oy, cq.y, co.y, S.Ly),
-                    dz = rel(cz, oz, cq.z, co.z, S.Lz);
+      auto dist2 = [&](const NearCol32 &o) {
+        const float dx = rel(cx, ox, o.q.x, o.o.x, S.Lx), dy = rel(cy, oy, o.q.y, o.o.y, S.Ly),
+                    dz = rel(cz, oz, o.q.z, o.o.z, S.Lz);
         return dx * dx + dy * dy + dz * dz;
       };
       bool e = false;
       if (cand == NEAR_WILD) {
         const NearList c = near_list(S, step, lin_cell(S, cx, cy, cz), false);
-        if (c.brute) {
-          for (int j = 0; j < S.Nc && !e; ++j) e = dist2(j) <= ch * ch;
-        } else {
-          for (int m = 0; m < c.cnt && !e; ++m) e = dist2(c.ids[m]) <= ch * ch;
-        }
+        for (int m = 0; m < (c.brute ? S.Nc : c.cnt) && !e; ++m)
+          e = dist2(sm.col.at(S, xb, c.brute ? m : c.ids[m])) <= ch * ch;
       } else {
-        const int j0 = (int)(cand & 0xFFFFu), j1 = (int)(cand >> 16);
-        if (j0 != 0xFFFF) e = e || dist2(j0) <= ch * ch;
-        if (j1 != 0xFFFF) e = e || dist2(j1) <= ch * ch;
+        for (unsigned r = cand; (r & 0xFFFFu) != 0xFFFFu && !e; r = (r >> 16) | 0xFFFF0000u)
+          e = dist2(sm.col.d[r & 0xFFFFu]) <= ch * ch;
       }
-      if (!e) continue;
-      const int i = atomicAdd(&s_nchk, 1);
-      *idx(i) = k;
-      if (i >= NEAR32_CHK) continue;
-      // the colloids it may be inside of (a second sphere is reached through a collision with the
-      // first), ascending; jc: the first one the sphere and the colloid's move alone reach
+      if (e) *idx(atomicAdd(&s_nchk, 1)) = k;
+    };
+    // Two at a time and without a branch where they stay inside their cell (the addition then
+    // carries nothing) and have one candidate, which is not near: about 50 instructions each,
+    // interleaved.  Everything else takes the general path.
+    const int kept = min(cnt, NEAR32_ACT);
+    for (int k0 = t; k0 < kept; k0 += 2 * NT) {
+      unsigned cand[2];
+      bool away[2];
+      uint4 q[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int k = min(k0 + u * NT, kept - 1);
+        cand[u] = k0 + u * NT < kept ? sm.cand[k] : NEAR_GONE;
+        q[u] = sm.q[k];
+        const NearCol32 &o = sm.col.d[min(cand[u] & 0xFFFFu, (unsigned)(NearCols<NearCol32>::MAX - 1))];
+        int cx, cy, cz;
+        float ox, oy, oz;
+        unpack(q[u], cx, cy, cz, ox, oy, oz);
+        ox = fmaf(sm.v[0][k], S.dtf, ox); oy = fmaf(sm.v[1][k], S.dtf, oy); oz = fmaf(sm.v[2][k], S.dtf, oz);
+        const float dx = rel(cx, ox, o.q.x, o.o.x, S.Lx), dy = rel(cy, oy, o.q.y, o.o.y, S.Ly),
+                    dz = rel(cz, oz, o.q.z, o.o.z, S.Lz);
+        away[u] = (cand[u] >> 16) == 0xFFFFu && ox >= 0.f && ox < 1.f && oy >= 0.f && oy < 1.f && oz >= 0.f &&
+                  oz < 1.f && dx * dx + dy * dy + dz * dz > (ch + 1e-4f) * (ch + 1e-4f);
+        q[u] = pack(cx, cy, cz, ox, oy, oz);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int k = k0 + u * NT;
+        if (away[u]) sm.q[k] = q[u];
+        else if (cand[u] != NEAR_GONE) one(k, cand[u]);
+      }
+    }
+    for (int k = NEAR32_ACT + t; k < cnt; k += NT) one(k, NEAR_WILD);  // beyond shared memory
+    sync();
+    // the listed ones, one per thread (what they read of global memory is one latency for all):
+    // the colloids each may be inside of (a second sphere is reached through a collision with the
+    // first), ascending; jc: the first one the sphere and the colloid's move alone reach
+    const int nchk = min(s_nchk, NEAR32_CHK);
+    for (int i = t; i < nchk; i += NT) {
       NearChk &v = sm.chk[i];
+      const int k = *idx(i);
+      int cx, cy, cz;
+      float ox, oy, oz;
+      unpack(*pq(k), cx, cy, cz, ox, oy, oz);
       const NearList c = near_list(S, step, lin_cell(S, cx, cy, cz), false);
       v.k = k;
+      v.id = F.id[S.act[a0 + k]];
       v.jc = -1;
       v.nc = 0;
       v.slow = c.brute;
       for (int m = 0; m < c.cnt && !v.slow; ++m) {
         const int j = c.ids[m];
-        const float d2 = dist2(j);
-        if (d2 > far * far || !in_block3(S, S.ccell[xb][j], cx, cy, cz)) continue;
+        const NearCol32 o = sm.col.at(S, xb, j);
+        const float dx = rel(cx, ox, o.q.x, o.o.x, S.Lx), dy = rel(cy, oy, o.q.y, o.o.y, S.Ly),
+                    dz = rel(cz, oz, o.q.z, o.o.z, S.Lz);
+        const float d2 = dx * dx + dy * dy + dz * dz;
+        if (d2 > far * far || !in_block3(S, o.c, cx, cy, cz)) continue;
         if (v.nc == 4) {
           v.slow = true;
           break;
@@ -1253,11 +1360,9 @@ __global__ void __maxnreg__(112) k_near_step32(__grid_constant__ const SysF64 S,
         if (d2 <= ch * ch && (v.jc < 0 || j < v.jc)) v.jc = j;
       }
       if (v.jc < 0) v.nc = 0;
-      if (v.slow || v.nc) v.id = F.id[S.act[a0 + k]];
     }
     sync();
     // the preparations, 32 particles at a time, in three parts on different warps
-    const int nchk = min(s_nchk, NEAR32_CHK);
     for (int q = t >> 5; q < 3 * ((nchk + 31) / 32); q += NW) {
       const int i = (q / 3) * 32 + (t & 31);
       if (i >= nchk) continue;
@@ -1281,11 +1386,13 @@ __global__ void __maxnreg__(112) k_near_step32(__grid_constant__ const SysF64 S,
     } else {
       sync();
     }
+    if (l < n) sm.col.copy(S, buf, t, NT);  // (for the tests of l + 1; it arrives meanwhile)
     // the listed particles' wall collisions at X(l), one per lane
     const int nchk = s_nchk;
     for (int base = 0;; base += NT) {
       const int i = base + t;
       const bool last_round = base + NT >= nchk;
+      int hit = -1;
       if (i < nchk) {
         const int k = *idx(i);
         NearChk *v = i < NEAR32_CHK ? &sm.chk[i] : nullptr;
@@ -1346,7 +1453,7 @@ __global__ void __maxnreg__(112) k_near_step32(__grid_constant__ const SysF64 S,
             if (ex * ex + ey * ey + ez * ez > (float)S.disp_margin2) atomicOr(&S.ss->err, ERRB_DISPLACE);
             *pq(k) = pack(cx, cy, cz, ox, oy, oz);
             *pv(0, k) = vx; *pv(1, k) = vy; *pv(2, k) = vz;
-            if (k < NEAR32_ACT) sm.cand[k] = NEAR_STALE;
+            hit = k;
             const int p = S.act[a0 + k];
             F.vx[p] = vx; F.vy[p] = vy; F.vz[p] = vz;
             if (l == n) {
@@ -1379,9 +1486,17 @@ __global__ void __maxnreg__(112) k_near_step32(__grid_constant__ const SysF64 S,
           s_nh = 0;
         }
       }
+      if (hit >= 0 && hit < NEAR32_ACT && l < n) {  // its candidates from here on
+        int cx, cy, cz;
+        float ox, oy, oz;
+        unpack(sm.q[hit], cx, cy, cz, ox, oy, oz);
+        sm.cand[hit] = sm.col.slots(near_cand32(S, step, n - l, buf, cx, cy, cz, ox, oy, oz, sm.v[0][hit],
+                                                sm.v[1][hit], sm.v[2][hit]));
+      }
       if (last_round) break;
       sync();
     }
+    near_copy_wait();
     sync();
     if (l < n) advance(l + 1);
   }
@@ -1392,13 +1507,35 @@ __global__ void __maxnreg__(112) k_near_step32(__grid_constant__ const SysF64 S,
   if (t == 0 && s_hits) atomicAdd((unsigned long long *)&S.ss->ev_total, (unsigned long long)s_hits);
 }
 
+// (104 registers: the free-flight pass's two blocks fit beside it)
+__global__ void __maxnreg__(104) k_near_step32(__grid_constant__ const SysF64 S, int fb) {
+  near_step32(S, blockIdx.x, gridDim.x, fb);
+}
+
+// The same over a batch of systems, each on blocks of its own (boff: where they begin; the launch
+// covers the blocks from `first` on), which meet only at their system's counters.
+__global__ void __maxnreg__(104) k_near_step32_b(const SysF64 *Ss, const int *boff, int nrep, int first, int fb) {
+  __shared__ SysF64 sS;
+  __shared__ int s_r;
+  const int v = first + blockIdx.x;
+  for (int r = threadIdx.x; r < nrep; r += blockDim.x)
+    if (boff[r] <= v && v < boff[r + 1]) s_r = r;
+  __syncthreads();
+  const int r = s_r;
+  const int *src = reinterpret_cast<const int *>(Ss + r);
+  int *dst = reinterpret_cast<int *>(&sS);
+  for (int k = threadIdx.x; k < (int)(sizeof(SysF64) / sizeof(int)); k += blockDim.x) dst[k] = src[k];
+  __syncthreads();
+  near_step32(sS, v - boff[r], boff[r + 1] - boff[r], fb);
+}
+
 size_t near_step32_smem() { return sizeof(Near32); }
 
 // The end of a free-flight step, as k_end_flight64: the step counter and the next step's margin
 // (block 0); the run() candidate records of the near particles and the binning of the active
 // ones among them (the others)
-__global__ void __launch_bounds__(256) k_end_flight32(__grid_constant__ const SysF64 S, int fb) {
-  if (blockIdx.x == 0) {
+static __device__ __forceinline__ void k_end_flight32_body(const SysF64 &S, const int VB, const int NVB, int fb) {
+  if (VB == 0) {
     k_end_step_body(S, 0, 1);
     return;
   }
@@ -1407,7 +1544,7 @@ __global__ void __launch_bounds__(256) k_end_flight32(__grid_constant__ const Sy
   const Fluid32 F = fluid32_at(S, fb);
   const float rr[3] = {(float)S.ss->rrn[0], (float)S.ss->rrn[1], (float)S.ss->rrn[2]};
   const int count = min(S.ss->nnear, S.N), lane = threadIdx.x & 31;
-  for (int base = (blockIdx.x - 1) * 256; base < count; base += (gridDim.x - 1) * 256) {
+  for (int base = (VB - 1) * 256; base < count; base += (NVB - 1) * 256) {
     const int i = base + threadIdx.x;
     ShellRec rec;
     rec.n = 0;
@@ -1432,6 +1569,16 @@ __global__ void __launch_bounds__(256) k_end_flight32(__grid_constant__ const Sy
       else atomicOr(&S.ss->err, ERRB_SHELL);
     }
   }
+}
+
+__global__ void __launch_bounds__(256) k_end_flight32(__grid_constant__ const SysF64 S, int fb) {
+  k_end_flight32_body(S, blockIdx.x, gridDim.x, fb);
+}
+
+// the same over a batch of systems (persistent: batch_for)
+__global__ void __launch_bounds__(256) k_end_flight32_b(const SysF64 *Ss, const int *boff, int nrep, int fb) {
+  __shared__ SysF64 sS;
+  batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_end_flight32_body(sS, VB, NVB, fb); });
 }
 
 // AoS doubles (particle order) -> FP32 records; download scatters back by id

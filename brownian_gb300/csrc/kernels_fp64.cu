@@ -412,7 +412,8 @@ __global__ void __launch_bounds__(256) k_rotate_classify(const SysF64 S, int fb)
   const Fluid F = fluid_at(S, fb);
   const long long step = S.ss->step;
   const int b0 = (int)((step * S.n_sub - 1) & 1);
-  bool near = false, active = false;
+  bool near = false;
+  unsigned cand = NEAR_NONE;  // (SPLIT: the colloids its path comes near)
   if (valid) {
     if (!SPLIT) S.pend[p] = 0;  // no particle is pending at the start of a step
     const int c = ROT ? S.rotcell[p] : S.C;
@@ -439,7 +440,8 @@ __global__ void __launch_bounds__(256) k_rotate_classify(const SysF64 S, int fb)
     const float travel = (float)S.n_sub * sqrtf(fx * fx + fy * fy + fz * fz);
     const int cnt = tcount(((unsigned long long)w0.y << 32) | w0.x, step);
     if (!inb || !(travel <= S.flight_rv) || cnt > FLIGHT_CAP) {
-      near = active = true;  // faster than the table allows (or not finite), or a crowded cell
+      near = true;  // faster than the table allows (or not finite), or a crowded cell
+      cand = NEAR_WILD;
     } else if (cnt > 0) {
       const float r = S.r_shell + travel + (float)S.n_sub * S.ss->cm + 0.01f, r2 = r * r;
       const float rad = near_radius(S, S.ss->cm, S.n_sub), fn = (float)S.n_sub;
@@ -451,20 +453,24 @@ __global__ void __launch_bounds__(256) k_rotate_classify(const SysF64 S, int fb)
         const float dx = wrap_half(q.x - px, S.Lxf), dy = wrap_half(q.y - py, S.Lyf), dz = wrap_half(q.z - pz, S.Lzf);
         if (!(dx * dx + dy * dy + dz * dz > r2)) {
           near = true;
-          if (SPLIT) active = active || path_meets(-dx, -dy, -dz, fn * fx, fn * fy, fn * fz, rad);
+          if (SPLIT && path_meets(-dx, -dy, -dz, fn * fx, fn * fy, fn * fz, rad)) cand = near_add(cand, j);
         }
       }
     }
-    S.fnear[p] = near ? (SPLIT && active ? 2 : 1) : 0;
+    S.fnear[p] = near ? (SPLIT && cand != NEAR_NONE ? FN_ACTIVE : FN_NEAR) : FN_FREE;
   }
   const int lane = threadIdx.x & 31;
   const unsigned m = __ballot_sync(FULL, near);
   const int base = block_base_n(&S.ss->nnear, __popc(m), lane);
   if (near) S.near[base + __popc(m & ((1u << lane) - 1u))] = p;
   if (SPLIT) {
+    const bool active = cand != NEAR_NONE;
     const unsigned ma = __ballot_sync(FULL, active);
-    const int ba = block_base_n(&S.ss->nact, __popc(ma), lane);
-    if (active) S.act[ba + __popc(ma & ((1u << lane) - 1u))] = p;
+    const int ba = block_base_n(&S.ss->nact, __popc(ma), lane) + __popc(ma & ((1u << lane) - 1u));
+    if (active) {
+      S.act[ba] = p;
+      S.actc[ba] = cand;
+    }
   }
 }
 
@@ -477,102 +483,84 @@ __global__ void __launch_bounds__(256) k_rotate_classify(const SysF64 S, int fb)
 // So while the results x + j k u stay at least u inside the binade (the exact sums then lie
 // inside it) and inside [2^-30 L, L), where mod is the identity, j additions give x + j k u,
 // built here on the integer pipe from the bits (the FP64 units stay free for the substeps'
-// chains).  free_stream takes such a run of steps, then the one addition that crosses a
-// binade or the box edge as the reference does it (mod(x + w, L) in FP64), then the next run
-// from the new x (a few crossings at most; a coordinate crosses one in a few per cent of the
-// steps of a step); on a tie, or past the crossings it allows, the additions one by one.
+// chains).
 
-// the largest j in [0, left] with j step <= room (step > 0; room < 2^53 and left <= 2^10, so
-// no product below overflows once step <= room)
-static __device__ __forceinline__ int seg_steps(long long room, long long step, int left) {
-  if (room < step) return 0;
-  if ((long long)left * step <= room) return left;
-  int j = (int)((float)room / (float)step);  // within one of the quotient (j < left < 2^23)
-  j = j < 0 ? 0 : (j > left ? left : j);
-  while (j < left && (long long)(j + 1) * step <= room) ++j;
-  while (j > 0 && (long long)j * step > room) --j;
-  return j;
-}
-
-// a run of up to `left` integer steps from x: false where the step does not apply (then x
-// is left as it is); else *j steps taken (0 when x sits at the edge it moves towards)
-static __device__ __forceinline__ bool free_run(double &x, double w, int left, const Dim &D, int *j) {
-  const long long bx = dbits(x), bw = dbits(w);
-  const long long aw = bw & 0x7FFFFFFFFFFFFFFFll;
-  const int ex = (int)((bx >> 52) & 0x7FF), ew = (int)((aw >> 52) & 0x7FF);
-  if (!(bx >= D.lo_bits && bx < D.L_bits && ex > 0 && (aw == 0 || ew > 0))) return false;
-  long long k = 0;
-  if (aw != 0) {
-    const long long mw = (aw & 0xFFFFFFFFFFFFFll) | 0x10000000000000ll;
-    const int sh = ex - ew;
-    if (sh <= 0) {
-      if (sh <= -8) return false;  // (a w that large leaves the binade at once)
-      k = mw << -sh;
-    } else if (sh <= 53) {
-      k = mw >> sh;
-      const long long rem = mw & ((1ll << sh) - 1), half = 1ll << (sh - 1);
-      if (rem == half) return false;  // a tie
-      k += rem > half ? 1 : 0;
-    }  // sh > 53: |w| < u/2, every sum rounds back to x (k = 0)
-    if (bw < 0) k = -k;
-  }
-  if (left < 1 || left > 1024) return false;
-  const long long mx = (bx & 0xFFFFFFFFFFFFFll) | 0x10000000000000ll;
-  const long long lo = 0x10000000000000ll + 1, hi = 0x20000000000000ll - 1;
-  int n;
-  if (k == 0) {
-    n = left;
-  } else if (k > 0) {
-    long long room = hi - mx;  // inside the binade, and below L where L lies in it
-    if ((int)((D.L_bits >> 52) & 0x7FF) == ex) {
-      const long long rl = ((D.L_bits & 0xFFFFFFFFFFFFFll) | 0x10000000000000ll) - 1 - mx;
-      room = rl < room ? rl : room;
-    }
-    n = seg_steps(room, k, left);
-  } else {
-    long long room = mx - lo;  // inside the binade, and at or above 2^-30 L where it lies in it
-    if ((int)((D.lo_bits >> 52) & 0x7FF) == ex) {
-      const long long rl = mx - ((D.lo_bits & 0xFFFFFFFFFFFFFll) | 0x10000000000000ll);
-      room = rl < room ? rl : room;
-    }
-    n = seg_steps(room, -k, left);
-  }
-  if (n > 0) x = __longlong_as_double(((long long)ex << 52) | ((mx + (long long)n * k) & 0xFFFFFFFFFFFFFll));
-  *j = n;
-  return true;
-}
-
-static __device__ __forceinline__ double free_stream(double x, double w, int n, const Dim &D) {
-  for (int seg = 0; seg < 3 && n > 0; ++seg) {
-    int j;
-    if (!free_run(x, w, n, D, &j)) break;
-    n -= j;
-    if (n == 0) return x;
-    x = ref_mod(__dadd_rn(x, w), D);  // the crossing step, as the reference does it
-    n -= 1;
-  }
-  for (; n > 0; --n) x = ref_mod(__dadd_rn(x, w), D);
+// the additions one by one, as the reference does them
+static __device__ __forceinline__ double seq(double x, double w, int n, const Dim &D) {
+#pragma unroll 1
+  for (int q = 0; q < n; ++q) x = ref_mod(__dadd_rn(x, w), D);
   return x;
 }
 
-// the free particles' whole step: update_pos_mpcd of every substep (free_stream: the
-// streaming passes' operations in order, or their exact result) and the binning of the
-// last substep with the next step's grid shift, beside the near particles' substeps,
-// which touch none of its particles.  A grid of a few blocks per SM walks the fluid (it
-// shares the SMs with the substeps' latency-bound chain).
+// All n steps at once where they lie in one run, without a branch: with x1 = fl(x + w) in the
+// binade of x (and no tie), x1 - x is the k u of the run above, as a difference of bit patterns
+// k, and the result's pattern is x's plus n k, if that too lies inside the binade (not on its
+// lower edge) and inside [2^-30 L, L).  Else x stays and the result is false.  One FP64 addition
+// and about 30 integer instructions an axis, the three axes independent of one another; it
+// applies to 98.9 % of axis moves, and the rest take the additions one by one (seq, a single
+// copy of it: the pass runs at the rate its instructions are fetched).  Measured, the 64^3
+// system's step (density 10, 500 colloids; the pass beside the substeps' kernel): runs of steps
+// between crossings, with branches and inlined per axis, 593 us; this 461 us.
+static __device__ __forceinline__ bool free_jump(double &x, double w, int n, const Dim &D) {
+  const long long bx = dbits(x), b1 = dbits(__dadd_rn(x, w)), aw = dbits(w) & 0x7FFFFFFFFFFFFFFFll;
+  const long long bn = (long long)((unsigned long long)bx + ((unsigned long long)b1 - (unsigned long long)bx) * n);
+  // (the same sign and exponent, x1's checked so that n k cannot have wrapped)
+  const bool in = (((b1 ^ bx) | (bn ^ bx)) >> 52) == 0 && (bn & 0xFFFFFFFFFFFFFll) != 0 && bx >= D.lo_bits &&
+                  bn >= D.lo_bits && bx < D.L_bits && bn < D.L_bits && n <= 1024;
+  // w / u halfway between two integers: the fraction of w's significand below u is one half
+  const int sh = (int)(bx >> 52) - (int)(aw >> 52);
+  const unsigned long long mw = ((unsigned long long)aw & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+  const bool tie = sh >= 1 && sh <= 53 && (mw << (64 - sh)) == 0x8000000000000000ull;
+  const bool ok = in && !tie;
+  if (ok) x = __longlong_as_double(bn);
+  return ok;
+}
+
+// the free particles' whole step: update_pos_mpcd of every substep (free_jump, or seq on the axes
+// it does not cover: the streaming passes' operations in order, or their exact result) and the
+// binning of the last substep with the next step's grid shift, beside the near particles'
+// substeps, which touch none of its particles.  A grid of a few blocks per SM walks the fluid
+// (it shares the SMs with the substeps' latency-bound chain), each thread's next particle loaded
+// while this one is worked on.
 // (thr: the flag from which on a particle is not this pass's: 1, or 2 where the near ones that
 // no sphere can reach are streamed here too)
-__global__ void __launch_bounds__(256) k_free_flight(const SysF64 S, int fb, int thr) {
+__global__ void __launch_bounds__(256, 4) k_free_flight(const SysF64 S, int fb, int thr) {
   const Fluid F = fluid_at(S, fb);
-  for (int p0 = blockIdx.x * blockDim.x; p0 < S.N; p0 += gridDim.x * blockDim.x) {
-    const int p = p0 + threadIdx.x;
+  const int n = S.n_sub, stride = gridDim.x * blockDim.x;
+  int p = blockIdx.x * blockDim.x + threadIdx.x;
+  double x = 0, y = 0, z = 0, wx = 0, wy = 0, wz = 0;
+  int fn = 255;
+  auto load = [&](int q) {
+    fn = 255;
+    if (q < S.N) {
+      fn = S.fnear[q];
+      x = F.x[q]; y = F.y[q]; z = F.z[q];
+      wx = F.wx[q]; wy = F.wy[q]; wz = F.wz[q];
+    }
+  };
+  load(p);
+  for (int p0 = p - (int)threadIdx.x; p0 < S.N; p0 += stride, p += stride) {
+    const bool free = fn < thr;
+    double ax = x, ay = y, az = z;
+    const double bx = wx, by = wy, bz = wz;
+    load(p + stride);
     BinTerm t{-1, 0, 0, 0, 0};
-    if (p < S.N && S.fnear[p] < thr) {
-      const double wx = F.wx[p], wy = F.wy[p], wz = F.wz[p];
-      const double x = free_stream(F.x[p], wx, S.n_sub, S.dx), y = free_stream(F.y[p], wy, S.n_sub, S.dy),
-                   z = free_stream(F.z[p], wz, S.n_sub, S.dz);
-      t = bin_term(S, S.ss->rrn, p, x, y, z, wx, wy, wz);
-      F.x[p] = x; F.y[p] = y; F.z[p] = z;
+    if (free) {
+      const bool ox = free_jump(ax, bx, n, S.dx), oy = free_jump(ay, by, n, S.dy), oz = free_jump(az, bz, n, S.dz);
+      // the axes it does not cover, one a lane at a time
+      unsigned left = (ox ? 0u : 1u) | (oy ? 0u : 2u) | (oz ? 0u : 4u);
+      while (left) {
+        const int a = __ffs(left) - 1;
+        left &= left - 1;
+        const double sel = a == 0 ? ax : a == 1 ? ay : az, sw = a == 0 ? bx : a == 1 ? by : bz;
+        const Dim &D = a == 0 ? S.dx : a == 1 ? S.dy : S.dz;
+        const double r = seq(sel, sw, n, D);
+        if (a == 0) ax = r;
+        else if (a == 1) ay = r;
+        else az = r;
+      }
+      t = bin_term(S, S.ss->rrn, p, ax, ay, az, bx, by, bz);
+      F.x[p] = ax; F.y[p] = ay; F.z[p] = az;
     }
     bin_add_warp(S.acc, t.c, t.fx, t.fy, t.fz, t.f2);  // the whole warp
   }
@@ -886,11 +874,18 @@ __global__ void k_run_kick(const SysF64 S, int fb, int split) {
       v = sub3(v, mul3s(del, f));
     }
     F.wx[p] = __dmul_rn(v.x, S.dt); F.wy[p] = __dmul_rn(v.y, S.dt); F.wz[p] = __dmul_rn(v.z, S.dt);
-    if (split && S.fnear[p] == 1 &&
-        near_cand64(S, S.ss->step, S.n_sub, (int)((S.ss->step * S.n_sub - 1) & 1), F.x[p], F.y[p], F.z[p],
-                    F.wx[p], F.wy[p], F.wz[p]) != NEAR_NONE) {
-      S.fnear[p] = 2;
-      S.act[atomicAdd(&S.ss->nact, 1)] = p;
+    if (!split) continue;
+    // an active particle's candidates are looked up anew (k_near_step64); another may become active
+    if (S.fnear[p] == FN_ACTIVE) {
+      S.fnear[p] = FN_KICKED;
+    } else if (S.fnear[p] == FN_NEAR) {
+      const unsigned cand = near_cand64(S, S.ss->step, S.n_sub, (int)((S.ss->step * S.n_sub - 1) & 1), F.x[p], F.y[p],
+                                        F.z[p], F.wx[p], F.wy[p], F.wz[p]);
+      if (cand == NEAR_NONE) continue;
+      S.fnear[p] = FN_ACTIVE;
+      const int i = atomicAdd(&S.ss->nact, 1);
+      S.act[i] = p;
+      S.actc[i] = cand;
     }
   }
 }
@@ -1123,6 +1118,17 @@ __global__ void __launch_bounds__(256) k_diag_fluid(const SysF64 S, double *part
 
 // ------------------------------------------------- active particles' substeps (FP64 form)
 
+// what the FP32 tests need of a colloid
+struct __align__(16) NearCol64 {
+  float4 x;
+  int4 c;
+  static __device__ __forceinline__ NearCol64 get(const SysF64 &S, int b, int j) { return {S.Xf[b][j], S.ccell[b][j]}; }
+  static __device__ __forceinline__ void copy(const SysF64 &S, int b, int j, NearCol64 *to) {
+    near_copy16(&to->x, &S.Xf[b][j]);
+    near_copy16(&to->c, &S.ccell[b][j]);
+  }
+};
+
 // A pending particle of k_near_step64: its state streamed to the substep in flight, the colloids
 // it can be inside of (ascending; none: nc = 0), and, prepared while the colloids move, what its
 // reflection off the first of them (jc) needs that no colloid position enters: the point half a
@@ -1131,6 +1137,7 @@ struct NearEv : EvState {
   double bx, by, bz, tx, ty, tz, val, v1, v2;
   NearCell c;
   int jc, nc;
+  unsigned cand;  // the slots of the colloids its path comes near; NEAR_STALE after a collision
   uint16_t cd[4];
   bool slow;  // more than four of them, or an aliased or overflowing cell: searched anew
 };
@@ -1144,23 +1151,35 @@ static __device__ __forceinline__ NearCell near_cell64(const SysF64 &S, double x
 }
 
 // The colloids a streamed particle may be inside of in this substep (prev: the buffer of the
-// positions before it): those whose boxes hold its cell within the sphere, the colloid's move
-// (mg) and a wall collision's displacement (a second sphere is reached through a collision
-// with the first); jc the first that the sphere and the move alone reach.
-static __device__ __forceinline__ void near_spheres64(const SysF64 &S, long long step, NearEv &e, int prev, float mg) {
-  const NearList q = near_list(S, step, e.c.lin, e.c.alias);
-  e.jc = -1;
-  e.nc = 0;
-  e.slow = q.brute;
-  if (q.brute) return;
+// positions before it): jc, the first in order that its boxes, the sphere and the colloid's move
+// (mg) alone allow, among the ones its path comes near; where there is one, all those within a
+// wall collision's displacement of that as well (a second sphere is reached through a collision
+// with the first).
+static __device__ __forceinline__ void near_spheres64(const SysF64 &S, long long step, NearEv &e, int prev, float mg,
+                                                      const NearCols<NearCol64> &cols) {
   const float px = d2f_trunc(e.x), py = d2f_trunc(e.y), pz = d2f_trunc(e.z);
   const float ch = S.r_coll + 1e-3f + mg, far = ch + S.disp_marginf + 1e-3f;
-  for (int k = 0; k < q.cnt; ++k) {
-    const int j = q.ids[k];
-    const float4 c = S.Xf[prev][j];
+  auto dist2 = [&](float4 c) {
     const float dx = wrap_half(c.x - px, S.Lxf), dy = wrap_half(c.y - py, S.Lyf), dz = wrap_half(c.z - pz, S.Lzf);
-    const float d2 = dx * dx + dy * dy + dz * dz;
-    if (d2 > far * far || !in_block3(S, S.ccell[prev][j], e.c.ix, e.c.iy, e.c.iz)) continue;
+    return dx * dx + dy * dy + dz * dz;
+  };
+  e.jc = -1;
+  e.nc = 0;
+  e.slow = e.c.alias;
+  if (e.slow) return;
+  if (e.cand != NEAR_WILD) {
+    bool any = false;
+    for (unsigned r = e.cand; (r & 0xFFFFu) != 0xFFFFu && !any; r = (r >> 16) | 0xFFFF0000u)
+      any = dist2(cols.d[r & 0xFFFFu].x) <= ch * ch;
+    if (!any) return;
+  }
+  const NearList q = near_list(S, step, e.c.lin, e.c.alias);
+  e.slow = q.brute;
+  for (int k = 0; k < q.cnt && !e.slow; ++k) {
+    const int j = q.ids[k];
+    const NearCol64 o = cols.at(S, prev, j);
+    const float d2 = dist2(o.x);
+    if (d2 > far * far || !in_block3(S, o.c, e.c.ix, e.c.iy, e.c.iz)) continue;
     if (e.nc == 4) {
       e.slow = true;
       return;
@@ -1233,6 +1252,7 @@ struct Near64 {
   double st[6][NEAR64_ACT];
   unsigned cand[NEAR64_ACT];
   NearEv ev[NEAR64_EV];
+  NearCols<NearCol64> col;
 };
 
 // see near_step.cuh.  A particle the FP32 test cannot clear is pending for the rest of the step,
@@ -1240,6 +1260,7 @@ struct Near64 {
 // FP64 unit 16 of them however many lanes are active, so a substep's collisions run one per lane
 // on as few warps as hold them, and everything that does not wait for the colloids (the
 // logarithms of the draws above all) is prepared beside the colloids' finish.
+// (112 registers: the free-flight pass's two blocks fit beside it)
 __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant__ const SysF64 S, int fb) {
   constexpr int NT = NEAR64_BLOCK - 32 * (NEAR_CW + 1), NW = NT / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1251,6 +1272,7 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
   const int t = threadIdx.x, VB = blockIdx.x, G = gridDim.x;
   const int n = S.n_sub;
   if (t == 0) s_np = s_nh = s_fin = 0;
+  sm.col.clear(S, t, NEAR64_BLOCK);
   if (VB == 0 && t == NT) set_shift(S, S.ss->step + 2);  // (the records of this step are all kicked)
   near_let_dependents();
   __syncthreads();
@@ -1283,12 +1305,22 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
   for (int k = t; k < cnt; k += NT) {
     const int p = S.act[a0 + k];
     const double x = F.x[p], y = F.y[p], z = F.z[p], wx = F.wx[p], wy = F.wy[p], wz = F.wz[p];
+    unsigned cand = S.actc[a0 + k];
+    if (S.fnear[p] == FN_KICKED) {
+      cand = near_cand64(S, step, n, (int)((g0 - 1) & 1), x, y, z, wx, wy, wz);
+      S.fnear[p] = FN_ACTIVE;
+    }
     *ptr(0, k) = x; *ptr(1, k) = y; *ptr(2, k) = z;
     *ptr(3, k) = wx; *ptr(4, k) = wy; *ptr(5, k) = wz;
+    if (k < NEAR64_ACT) {
+      sm.cand[k] = cand;
+      sm.col.note(cand);
+    }
   }
-  for (int k = t; k < cnt && k < NEAR64_ACT; k += NT)
-    sm.cand[k] = near_cand64(S, step, n, (int)((g0 - 1) & 1), sm.st[0][k], sm.st[1][k], sm.st[2][k], sm.st[3][k],
-                             sm.st[4][k], sm.st[5][k]);
+  sync();
+  sm.col.load(S, (int)((g0 - 1) & 1), t, NT);
+  for (int k = t; k < min(cnt, NEAR64_ACT); k += NT) sm.cand[k] = sm.col.slots(sm.cand[k]);
+  sync();
 
   // update_pos_mpcd of substep l and the FP32 test against the positions of l - 1 with the
   // displacement bound as margin (np: pending particles of the substeps before), then what the
@@ -1296,47 +1328,36 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
   auto advance = [&](int l, int np) {
     const long long gs = g0 + (l - 1);
     const int xb = (int)(gs & 1) ^ 1;
-    const float4 *Xf = S.Xf[xb];
     const float ch = S.r_coll + 1e-3f + mg;
-    for (int i = t; i < np; i += NT) {
-      NearEv &e = ev(i);
-      const double x = ref_mod(__dadd_rn(e.x, e.wx), S.dx), y = ref_mod(__dadd_rn(e.y, e.wy), S.dy),
-                   z = ref_mod(__dadd_rn(e.z, e.wz), S.dz);
-      e.c = near_cell64(S, x, y, z);
-      e.x = e.x0 = x; e.y = e.y0 = y; e.z = e.z0 = z;
-      e.dumped = false;
-      near_spheres64(S, step, e, xb, mg);
-    }
-    for (int k = t; k < cnt; k += NT) {
-      const unsigned cand = k < NEAR64_ACT ? sm.cand[k] : (S.fnear[S.act[a0 + k]] != FN_ACTIVE ? NEAR_GONE : NEAR_WILD);
-      if (cand == NEAR_GONE) continue;
+    // active particle k by the general path
+    auto one = [&](int k, unsigned cand) {
       double *px = ptr(0, k), *py = ptr(1, k), *pz = ptr(2, k);
       const double wx = *ptr(3, k), wy = *ptr(4, k), wz = *ptr(5, k);
       const double x = ref_mod(__dadd_rn(*px, wx), S.dx), y = ref_mod(__dadd_rn(*py, wy), S.dy),
                    z = ref_mod(__dadd_rn(*pz, wz), S.dz);
       const float fx = d2f_trunc(x), fy = d2f_trunc(y), fz = d2f_trunc(z);
-      auto close = [&](int j) {
-        const float4 c = Xf[j];
+      auto close = [&](float4 c) {
         const float dx = wrap_half(c.x - fx, S.Lxf), dy = wrap_half(c.y - fy, S.Lyf), dz = wrap_half(c.z - fz, S.Lzf);
         return dx * dx + dy * dy + dz * dz <= ch * ch;
       };
       const NearCell c = near_cell64(S, x, y, z);
+      auto block = [&](int4 cc, int j) { return c.alias ? near_in_block(S, j, c, xb) : in_block3(S, cc, c.ix, c.iy, c.iz); };
       bool e = c.alias;
       if (cand == NEAR_WILD) {
         const NearList q = near_list(S, step, c.lin, c.alias);
-        if (q.brute) {
-          for (int j = 0; j < S.Nc && !e; ++j) e = close(j) && near_in_block(S, j, c, xb);
-        } else {
-          for (int m = 0; m < q.cnt && !e; ++m) e = close(q.ids[m]) && near_in_block(S, q.ids[m], c, xb);
+        for (int m = 0; m < (q.brute ? S.Nc : q.cnt) && !e; ++m) {
+          const int j = q.brute ? m : q.ids[m];
+          e = close(sm.col.at(S, xb, j).x) && near_in_block(S, j, c, xb);
         }
       } else {
-        const int j0 = (int)(cand & 0xFFFFu), j1 = (int)(cand >> 16);
-        if (j0 != 0xFFFF) e = e || (close(j0) && near_in_block(S, j0, c, xb));
-        if (j1 != 0xFFFF) e = e || (close(j1) && near_in_block(S, j1, c, xb));
+        for (unsigned r = cand; (r & 0xFFFFu) != 0xFFFFu && !e; r = (r >> 16) | 0xFFFF0000u) {
+          const NearCol64 &o = sm.col.d[r & 0xFFFFu];
+          e = close(o.x) && block(o.c, sm.col.id[r & 0xFFFFu]);
+        }
       }
       if (!e) {
         *px = x; *py = y; *pz = z;
-        continue;
+        return;
       }
       const int i = atomicAdd(&s_np, 1), p = S.act[a0 + k];
       if (i >= NEAR64_EV) {
@@ -1347,40 +1368,117 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
         }
         O.id[a0 + i] = o;
       }
+      *px = x; *py = y; *pz = z;
       NearEv &v = ev(i);
-      v.x = v.x0 = x; v.y = v.y0 = y; v.z = v.z0 = z;
-      v.wx = wx; v.wy = wy; v.wz = wz;
-      v.vdx = v.vdy = v.vdz = 0.0;
-      v.p = p; v.id = F.id[p]; v.lin = c.lin; v.last = -1; v.cnt = 0; v.j = -1;
-      v.alias = c.alias; v.dumped = false; v.changed = false;
-      v.c = c;
-      near_spheres64(S, step, v, xb, mg);
+      v.j = k;  // (the record is made below)
+      v.p = p;
+      v.cand = cand;
       S.fnear[p] = FN_PENDING;
       if (k < NEAR64_ACT) sm.cand[k] = NEAR_GONE;
+    };
+    // The active ones, two at a time and without a branch where they stay inside the box (so the
+    // additions need no mod) and have one candidate, which is not near: about 60 instructions
+    // each, interleaved.  Everything else takes the general path.
+    const int kept = min(cnt, NEAR64_ACT);
+    for (int k0 = t; k0 < kept; k0 += 2 * NT) {
+      unsigned cand[2];
+      bool far[2];
+      double x[2][3];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int k = min(k0 + u * NT, kept - 1);
+        cand[u] = k0 + u * NT < kept ? sm.cand[k] : NEAR_GONE;
+        const NearCol64 &o = sm.col.d[min(cand[u] & 0xFFFFu, (unsigned)(NearCols<NearCol64>::MAX - 1))];
+        float d2 = 0.f;
+        far[u] = (cand[u] >> 16) == 0xFFFFu;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const Dim &D = a == 0 ? S.dx : (a == 1 ? S.dy : S.dz);
+          const float L = a == 0 ? S.Lxf : (a == 1 ? S.Lyf : S.Lzf);
+          x[u][a] = __dadd_rn(sm.st[a][k], sm.st[3 + a][k]);
+          const long long b = dbits(x[u][a]);
+          far[u] = far[u] && b >= D.lo_bits && b < D.L_bits;
+          const float d = wrap_half((a == 0 ? o.x.x : a == 1 ? o.x.y : o.x.z) - d2f_box(x[u][a]), L);
+          d2 = a == 0 ? d * d : fmaf(d, d, d2);
+        }
+        far[u] = far[u] && d2 > (ch + 1e-4f) * (ch + 1e-4f);  // (the general path's rounding may differ)
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int k = k0 + u * NT;
+        if (far[u]) {
+          sm.st[0][k] = x[u][0]; sm.st[1][k] = x[u][1]; sm.st[2][k] = x[u][2];
+        } else if (cand[u] != NEAR_GONE) {
+          one(k, cand[u]);
+        }
+      }
+    }
+    for (int k = NEAR64_ACT + t; k < cnt; k += NT)  // beyond shared memory
+      if (S.fnear[S.act[a0 + k]] == FN_ACTIVE) one(k, NEAR_WILD);
+    sync();
+    // the pending ones, old and new, one per thread: what they read of global memory (the flight
+    // table, ids) is one latency for all
+    const int np1 = s_np;
+    for (int i = t; i < np1; i += NT) {
+      NearEv &e = ev(i);
+      unsigned cand = e.cand;
+      if (i < np) {
+        if (cand == NEAR_STALE)
+          cand = e.cand = sm.col.slots(near_cand64(S, step, n - l + 1, xb, e.x, e.y, e.z, e.wx, e.wy, e.wz));
+        e.x = ref_mod(__dadd_rn(e.x, e.wx), S.dx);
+        e.y = ref_mod(__dadd_rn(e.y, e.wy), S.dy);
+        e.z = ref_mod(__dadd_rn(e.z, e.wz), S.dz);
+      } else {
+        const int k = e.j;
+        e.x = *ptr(0, k); e.y = *ptr(1, k); e.z = *ptr(2, k);
+        e.wx = *ptr(3, k); e.wy = *ptr(4, k); e.wz = *ptr(5, k);
+        e.vdx = e.vdy = e.vdz = 0.0;
+        e.id = F.id[e.p]; e.last = -1; e.cnt = 0; e.j = -1;
+        e.changed = false;
+      }
+      e.c = near_cell64(S, e.x, e.y, e.z);
+      e.lin = e.c.lin;
+      e.alias = e.c.alias;
+      e.x0 = e.x; e.y0 = e.y; e.z0 = e.z;
+      e.dumped = false;
+      near_spheres64(S, step, e, xb, mg, sm.col);
     }
     sync();
     // the preparations of 32 pending particles at a time, the three independent FP64 chains on
     // different warps (SM schedulers)
-    const int np1 = s_np;
     for (int q = w; q < 3 * ((np1 + 31) / 32); q += NW) {
       const int i = (q / 3) * 32 + lane, what = q % 3;
       if (i >= np1) continue;
       NearEv &e = ev(i);
       if (e.slow || e.nc == 0) continue;
       const uint32_t a = (uint32_t)(e.id + 1), b = (uint32_t)(e.jc + 1), tt = (uint32_t)gs;
+      const uint4 r = draw4_loop(S.key, DOM_COLL, what == 2 ? 1 : 0, a, b, tt);
       if (what == 0) {
         const double x = ref_mod(__dsub_rn(e.x, __dmul_rn(e.wx, 0.5)), S.dx);
         const double y = ref_mod(__dsub_rn(e.y, __dmul_rn(e.wy, 0.5)), S.dy);
         const double z = ref_mod(__dsub_rn(e.z, __dmul_rn(e.wz, 0.5)), S.dz);
-        const d3 tp = refl_point(S, draw4(S.key, DOM_COLL, 0, a, b, tt), mk(x, y, z));
+        const d3 tp = refl_point(S, r, mk(x, y, z));
         e.bx = x; e.by = y; e.bz = z;
         e.tx = tp.x; e.ty = tp.y; e.tz = tp.z;
-      } else if (what == 1) {
-        e.val = refl_speed(S, draw4(S.key, DOM_COLL, 0, a, b, tt));
+        continue;
+      }
+      // the Rayleigh speed sqrt(-log((1 - u)^2) kT/m), or the Gaussians' sqrt(-2 log(z) / z)
+      // (refl_speed, refl_gauss: one logarithm and one root in the code for both)
+      double x1 = 0, x2 = 0, z, iz = 1.0;
+      if (what == 1) {
+        const double om = __dsub_rn(1.0, u01(r.x));
+        z = __dmul_rn(om, om);
       } else {
-        double v2;
-        e.v1 = refl_gauss(S, draw4(S.key, DOM_COLL, 1, a, b, tt), a, b, tt, &v2);
-        e.v2 = v2;
+        z = refl_try(S, r, a, b, tt, x1, x2);
+        iz = __drcp_rn(z);
+      }
+      const double lz = log(z);
+      const double g = __dsqrt_rn(what == 1 ? __dmul_rn(-lz, S.inv_m_beta) : __dmul_rn(__dmul_rn(-2.0, lz), iz));
+      if (what == 1) {
+        e.val = g;
+      } else {
+        e.v1 = __dmul_rn(__dmul_rn(x1, g), S.sqrt_kt_m);
+        e.v2 = __dmul_rn(__dmul_rn(x2, g), S.sqrt_kt_m);
       }
     }
     if (t == 0) s_nh = 0;
@@ -1396,6 +1494,7 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
     } else {
       sync();
     }
+    if (l < n) sm.col.copy(S, buf, t, NT);  // (for the tests of l + 1; it arrives meanwhile)
     // the pending particles' wall collisions at X(l), one per lane
     const int np = s_np;
     for (int base = 0;; base += NT) {
@@ -1421,17 +1520,20 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
         e = &ev(i);
         if (e->slow) {
           near_collide_rest(S, *e, -1, step, gs, buf);
+          if (e->dumped) e->cand = NEAR_STALE;
         } else if (e->nc > 0) {
           int j = -1, c = 0;
+          // (the colloid prepared for, loaded beside the test)
+          const d3 Vj = ldv(S.V, e->jc), Wj = ldv(S.W, e->jc), Xj = ldv(S.X[buf], e->jc);
           for (; c < e->nc; ++c) {
             j = e->cd[c];
             if (within(S, S.X[buf], S.Xf[buf][j], j, e->x, e->y, e->z, S.r_coll, S.sig2q)) break;
           }
           if (c < e->nc && j != e->jc) {
-            near_collide_rest(S, *e, j, step, gs, buf);  // (inside a sphere the FP32 test had cleared)
+            near_collide_rest(S, *e, j, step, gs, buf);  // (not the colloid that was prepared for)
+            if (e->dumped) e->cand = NEAR_STALE;
           } else if (c < e->nc) {
             hit = true;
-            const d3 Vj = ldv(S.V, j), Wj = ldv(S.W, j), Xj = ldv(S.X[buf], j);
             xb = mk(e->bx, e->by, e->bz);
             const d3 rs = mk(ref_img(__dsub_rn(xb.x, Xj.x), S.dx), ref_img(__dsub_rn(xb.y, Xj.y), S.dy),
                              ref_img(__dsub_rn(xb.z, Xj.z), S.dz));
@@ -1446,6 +1548,7 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
             s_hx[h][3] = dl.x; s_hx[h][4] = dl.y; s_hx[h][5] = dl.z;
             e->vdx = vd.x; e->vdy = vd.y; e->vdz = vd.z;
             e->dumped = e->changed = true;
+            e->cand = NEAR_STALE;
             if (c + 1 < e->nc) {  // a second sphere may hold it now
               settle();
               hit = false;
@@ -1468,6 +1571,8 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
       if (last_round) break;
       sync();
     }
+    near_copy_wait();
+    sync();
     if (l < n) advance(l + 1, np);
   }
 
@@ -1507,6 +1612,12 @@ size_t near_step64_smem() { return sizeof(Near64); }
 
 __global__ void __launch_bounds__(256) k_rotdiff_step(__grid_constant__ const SysF64 S) {
   rotdiff_step(S, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// the same over a batch of systems (persistent: batch_for)
+__global__ void __launch_bounds__(256) k_rotdiff_step_b(const SysF64 *Ss, const int *boff, int nrep) {
+  __shared__ SysF64 sS;
+  batch_for(Ss, boff, nrep, sS, [&](int VB, int) { rotdiff_step(sS, (long long)VB * blockDim.x + threadIdx.x); });
 }
 
 // the cell table of a step's first substep at the present positions (the free-flight steps

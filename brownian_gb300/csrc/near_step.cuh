@@ -20,10 +20,12 @@
 // stage boundary is one counter in L2 (about 1 us), the state stays on the SM, and the
 // streaming of l + 1 runs while the colloids of l are finished.  Bound: the latency of that
 // cycle (fence and counter 1.2 us twice, exact collisions 2 us FP32 / 4 us FP64, colloid finish
-// 2 us).  Measured per step, launches per stage -> this: 24^3 FP32 system (30 colloids) 205 ->
-// 131 us (a substep 16 -> 7 us), 20^3 FP64 (20 colloids) 252 -> 169 us, 64^3 FP32 (500
-// colloids) 383 -> 275 us, 128^3 FP32 (2,000 colloids, 20 substeps) 3.08 -> 2.19 ms; 64^3 FP64
-// 600 -> 590 us (there the free-flight pass beside it is the longer half).
+// 2 us), and with that the rate at which the code of a cycle is fetched: what is rarely taken is
+// out of line, and the common test runs two particles at a time without a branch.  Measured per
+// step, launches per stage -> this (with the free-flight pass as it is beside it): 24^3 FP32
+// system (30 colloids) 204 -> 134 us, 20^3 FP64 (20 colloids) 251 -> 167 us, 64^3 (500 colloids)
+// FP32 388 -> 280 us, FP64 605 -> 461 us, 128^3 FP32 (2,000 colloids, 20 substeps) 3.08 -> 1.81 ms;
+// 32 FP32 systems of 16^3 to 48^3 stepped together, each on blocks of its own, 2.28 -> 1.74 ms.
 //
 // The arithmetic is that of the per-substep passes, in their order: the results are theirs
 // bit for bit.  The candidates of a particle come from the flight table of its cell (every
@@ -162,6 +164,68 @@ static __device__ __forceinline__ unsigned near_add(unsigned cand, int j) {
   return NEAR_WILD;
 }
 
+// An asynchronous 16-byte copy from global to shared memory (through L2: what the grid-wide
+// counters have made visible there is what arrives), and the wait for this thread's copies
+static __device__ __forceinline__ void near_copy16(void *to, const void *from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from)
+               : "memory");
+}
+static __device__ __forceinline__ void near_copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The colloids around a block's active particles, kept in shared memory for the tests of the next
+// substep: seeing BAR_MOVE empties the SM's L1, so each test would otherwise wait for L2 again
+// (three to four dependent 0.4 us reads a substep).  T: what a test needs of a colloid.  The first
+// MAX colloids noted are kept; any other is read from global memory.
+template <typename T>
+struct NearCols {
+  static constexpr int MAX = 192, TAB = 2048;
+  T d[MAX];
+  int at_[TAB];  // colloid -> slot (-1: none)
+  uint16_t id[MAX];
+  int n;
+  __device__ __forceinline__ void clear(const SysF64 &S, int t, int nt) {
+    if (t == 0) n = 0;
+    for (int j = t; j < min(S.Nc, TAB); j += nt) at_[j] = -1;
+  }
+  // the candidates of a packed pair get slots
+  __device__ __forceinline__ void note(unsigned cand) {
+    if (cand == NEAR_WILD) return;
+    for (int k = 0; k < 2; ++k, cand >>= 16) {
+      const int j = (int)(cand & 0xFFFFu);
+      if (j >= TAB || at_[j] != -1 || atomicCAS(&at_[j], -1, -2) != -1) continue;  // (none is beyond the table)
+      const int i = atomicAdd(&n, 1);
+      if (i >= MAX) continue;
+      id[i] = (uint16_t)j;
+      at_[j] = i;
+    }
+  }
+  // the pair by slots; NEAR_WILD where one has none
+  __device__ __forceinline__ unsigned slots(unsigned cand) const {
+    if (cand == NEAR_WILD) return NEAR_WILD;
+    unsigned r = NEAR_NONE;
+    for (int k = 0; k < 2; ++k, cand >>= 16) {
+      const int j = (int)(cand & 0xFFFFu);
+      if (j == 0xFFFF) continue;
+      const int i = j < TAB ? at_[j] : -1;
+      if (i < 0) return NEAR_WILD;
+      r = near_add(r, i);
+    }
+    return r;
+  }
+  __device__ __forceinline__ int kept() const { return min(n, MAX); }
+  __device__ __forceinline__ void load(const SysF64 &S, int b, int t, int nt) {
+    for (int i = t; i < kept(); i += nt) d[i] = T::get(S, b, id[i]);
+  }
+  __device__ __forceinline__ void copy(const SysF64 &S, int b, int t, int nt) {
+    for (int i = t; i < kept(); i += nt) T::copy(S, b, id[i], &d[i]);
+  }
+  // colloid j (positions in buffer b)
+  __device__ __forceinline__ T at(const SysF64 &S, int b, int j) const {
+    const int i = j < TAB ? at_[j] : -1;
+    return i >= 0 ? d[i] : T::get(S, b, j);
+  }
+};
+
 // append run() candidate records, one atomic per warp (the whole warp calls it)
 static __device__ __forceinline__ void near_record(const SysF64 &S, const ShellRec &rec, bool has) {
   const int lane = threadIdx.x & 31;
@@ -205,9 +269,7 @@ static __device__ __forceinline__ void near_colloids(const SysF64 &S, const int 
     // compute_force_md at X(l): a warp per colloid
     for (int s = w; s < M; s += NEAR_CW) {
       const int j = VB + G * s;
-      double pot;
-      const d3 fn = S.vlist ? wca_force_vlist(S, S.X[cur], S.Xf[cur], j, lane)
-                            : wca_force(S, S.X[cur], S.Xf[cur], j, lane, false, pot);
+      const d3 fn = S.vlist ? wca_force_vlist(S, S.X[cur], S.Xf[cur], j, lane) : mk(0, 0, 0);  // (no list: one colloid)
       if (lane == 0) stv(S.fnew, j, fn);
     }
     group_sync(bar_id, NT);

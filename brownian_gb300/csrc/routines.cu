@@ -32,7 +32,7 @@ static __device__ __forceinline__ int bucket_of(const double *Xc, int j, const N
 // The colloids by bucket (a counting sort, one block of 1024 threads): bkt_start[b]
 // the first slot of bucket b in bkt_list, bkt_start[nbk] = Nc.
 // (Xc null: the positions at the start of the present step, the free-flight schedule's list)
-__global__ void __launch_bounds__(1024) k_cbucket(const SysF64 S, const double *Xc, NListGeo geo) {
+static __device__ __forceinline__ void cbucket_body(const SysF64 &S, const double *Xc, const NListGeo &geo) {
   __shared__ int wsum[32];
   __shared__ int carry;
   if (!Xc) Xc = S.X[(int)((S.ss->step * S.n_sub - 1) & 1)];
@@ -72,6 +72,16 @@ __global__ void __launch_bounds__(1024) k_cbucket(const SysF64 S, const double *
     const int slot = atomicAdd(&S.bkt_cur[bucket_of(Xc, j, geo)], 1);
     if (slot >= 0 && slot < S.Nc) S.bkt_list[slot] = j;
   }
+}
+
+__global__ void __launch_bounds__(1024) k_cbucket(const SysF64 S, const double *Xc, NListGeo geo) {
+  cbucket_body(S, Xc, geo);
+}
+
+// the free-flight schedule's over a batch of systems (persistent: batch_for; one virtual block each)
+__global__ void __launch_bounds__(1024) k_cbucket_step_b(const SysF64 *Ss, const int *boff, int nrep) {
+  __shared__ SysF64 sS;
+  batch_for(Ss, boff, nrep, sS, [&](int, int) { cbucket_body(sS, nullptr, sS.step_geo); });
 }
 
 // The pair list of colloid j (one warp per colloid, four per block): every colloid k
@@ -148,10 +158,10 @@ __global__ void __launch_bounds__(128) k_nlist(const SysF64 S, const double *Xc,
 // of the step, ascending, for the forces of the step's substeps.  The candidates of the
 // buckets next to j's are flattened across the warp (a prefix over the buckets' counts), so
 // a colloid takes a round per 32 candidates instead of a round per bucket.
-__global__ void __launch_bounds__(128) k_nlist_step(const SysF64 S, NListGeo geo) {
+static __device__ __forceinline__ void nlist_step_body(const SysF64 &S, const int VB, const NListGeo &geo) {
   __shared__ uint16_t sbuf[4][NBR_CAP];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int j = blockIdx.x * 4 + w;
+  const int j = VB * 4 + w;
   if (j >= S.Nc) return;
   const double *Xc = S.X[(int)((S.ss->step * S.n_sub - 1) & 1)];
   const d3 Xj = ldv(Xc, j);
@@ -223,6 +233,16 @@ __global__ void __launch_bounds__(128) k_nlist_step(const SysF64 S, NListGeo geo
     out[rank] = v;
   }
   if (lane == 0) S.nbr_n[j] = n;
+}
+
+__global__ void __launch_bounds__(128) k_nlist_step(__grid_constant__ const SysF64 S) {
+  nlist_step_body(S, blockIdx.x, S.step_geo);
+}
+
+// the same over a batch of systems (persistent: batch_for)
+__global__ void __launch_bounds__(128) k_nlist_step_b(const SysF64 *Ss, const int *boff, int nrep) {
+  __shared__ SysF64 sS;
+  batch_for(Ss, boff, nrep, sS, [&](int VB, int) { nlist_step_body(sS, VB, sS.step_geo); });
 }
 
 // compute_force_md over the pair list: f of every colloid (its old value was saved as

@@ -80,8 +80,9 @@ struct StepState {
 
 // a particle in a free-flight step: free; near; of the near ones active, those of them that
 // became pending (FP64 form), and those that collided in the last substep (their run() record
-// and binning are done with the collision)
-enum : uint8_t { FN_FREE = 0, FN_NEAR = 1, FN_ACTIVE = 2, FN_PENDING = 3, FN_DONE = 4 };
+// and binning are done with the collision); an active one that run() kicked, whose path is
+// looked up anew
+enum : uint8_t { FN_FREE = 0, FN_NEAR = 1, FN_ACTIVE = 2, FN_PENDING = 3, FN_DONE = 4, FN_KICKED = 5 };
 
 // one cell of the FP32 form's flight table: (step + 1) << 32 | count, and the first
 // FLIGHT_CAP colloids (a cell with more is treated as near for all its particles)
@@ -89,6 +90,14 @@ constexpr int FLIGHT_CAP = 12;
 struct __align__(32) FlightCell {
   unsigned long long tc;
   uint16_t id[FLIGHT_CAP];
+};
+
+// the bucket grid of a colloid pair list: per axis nb buckets of width bs >= the list
+// radius (every partner within it is in a neighbouring bucket), r2 = radius^2
+struct NListGeo {
+  int nb[3];
+  double bs[3];
+  double r2;
 };
 
 struct SysF64 {
@@ -199,6 +208,7 @@ struct SysF64 {
   // of these, the ones whose straight path over the step may meet a sphere (or whose path the
   // flight table does not cover) are active: k_near_step takes them through the substeps
   int *act;                     // [N] slots of the active particles
+  unsigned *actc;               // [N] and the colloids their paths come near (NEAR_*)
   uint8_t *fnear;               // [N] the slot's particle this step: FN_*
   unsigned *bar;                // k_near_step's counters, 128 bytes apart (BAR_*)
   double *xi_all;               // [n_sub][Nc][3] rotational-diffusion normals of the step's substeps
@@ -212,6 +222,7 @@ struct SysF64 {
                                 // at least a wall collision's and a colloid's displacement bounds
   int vlist;                    // the free-flight steps compute the forces from a pair list built
                                 // at the start of the step
+  NListGeo step_geo;            // its bucket grid
   // step state
   StepState *ss;
   double *pot_part;    // [Nc] per-colloid share of the WCA potential
@@ -228,14 +239,6 @@ struct SysF64 {
 // collisions, blocks whose colloids have moved on, overflow records taken
 constexpr int EV_STATE_BYTES = 256;
 enum : int { BAR_COLL = 0, BAR_MOVE = 32, BAR_EVX = 64, BAR_WORDS = 96 };
-
-// the bucket grid of a colloid pair list: per axis nb buckets of width bs >= the list
-// radius (every partner within it is in a neighbouring bucket), r2 = radius^2
-struct NListGeo {
-  int nb[3];
-  double bs[3];
-  double r2;
-};
 
 // view of one fluid buffer
 struct Fluid {
