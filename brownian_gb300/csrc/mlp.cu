@@ -9,17 +9,11 @@
 // a colloid's per-step momentum and angular-momentum exchange with the fluid,
 // trained by the Gaussian negative log-likelihood.
 //
-// One GEMM kernel serves every product: C[M x N] = A[M x K] B[K x N] with A and B
-// addressed through arbitrary strides (forward x W, backward dZ W^T and A^T dZ),
-// 32 x 64 block tiles, 32-wide K steps staged in shared memory through 16-byte
-// loads (the next tile prefetched into registers), four warps of 32 x 16 each,
-// and a fused epilogue (bias, SiLU, the SiLU derivative of the
-// backward pass, BF16 / FP32 stores, FP32 atomic accumulation for split-K
-// weight gradients).  Training runs every product on the 5th-generation tensor cores
-// instead (tcgen05.mma with the accumulator in tensor memory, TMEM): the layer products
-// (forward x W and backward dZ W^T, K and N <= 256) on k_gemm_tc, the weight gradients (a
-// reduction over the batch) on k_gemm_tc_wgrad; inference (mpcd_mlp_forward) keeps the
-// warp-level kernel, whose arithmetic the colloid-only step's network reproduces bit for bit.
+// Training runs its products on the 5th-generation tensor cores (tcgen05.mma with the
+// accumulator in tensor memory, TMEM): the layer products (forward x W and backward dZ W^T, K and N
+// <= 256) on k_gemm_tc, the weight gradients (a reduction over the batch) on k_gemm_tc_wgrad.
+// Inference (mpcd_mlp_forward) is one kernel over all layers (k_mlp_infer) on warp-level products,
+// whose arithmetic the colloid-only step's network reproduces bit for bit.
 #include <cuda_bf16.h>
 
 #include <cmath>
@@ -38,7 +32,6 @@ typedef __nv_bfloat16 bf16;
 
 constexpr int IN = MPCD_MLP_IN, INP = MLP_IN_PADDED, H = MPCD_MLP_HIDDEN, OUT = MPCD_MLP_OUT, OUTP = MLP_OUT_PADDED,
               NY = OUT / 2;
-constexpr int BM = 32, BN = 64, BK = 32;
 // normalised log-variances are used within [-6, 6] (variances between 0.0025 and 400 times
 // the target's): beyond that the likelihood's gradient is zero and inference clamps
 constexpr float kLogVarClamp = MLP_LOGVAR_CLAMP;
@@ -77,150 +70,6 @@ __device__ __forceinline__ void mma_bf16(float c[4], const uint32_t a[4], const 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// Staging of one operand tile into shared memory as T[row][k] (rows: m for A, n for
-// B), 8 elements per 16-byte load along whichever dimension is contiguous in
-// memory (scalar loads where a vector would leave the matrix, is misaligned or
-// neither stride is 1).  ROWS x KT elements, 128 threads.
-template <int ROWS, int KT>
-struct Stage {
-  static constexpr int NV = ROWS * KT / 8 / 128;  // vectors per thread
-  uint4 v[NV];
-  __device__ __forceinline__ static void slot(int t, bool kfast, int &r, int &k) {
-    if (kfast) { r = t / (KT / 8); k = (t % (KT / 8)) * 8; }
-    else { k = t / (ROWS / 8); r = (t % (ROWS / 8)) * 8; }
-  }
-  __device__ __forceinline__ void load(const bf16 *base, long long rs, long long ks, int r0, int k0, int rmax, int kmax,
-                                       bool kfast) {
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      int r, k;
-      slot(threadIdx.x + 128 * i, kfast, r, k);
-      r += r0; k += k0;
-      const bf16 *p = base + r * rs + k * ks;
-      const bool full = kfast ? (r < rmax && k + 8 <= kmax) : (k < kmax && r + 8 <= rmax);
-      if (full && (kfast ? ks == 1 : rs == 1) && ((reinterpret_cast<uintptr_t>(p) & 15) == 0)) {
-        v[i] = *reinterpret_cast<const uint4 *>(p);
-      } else {
-        bf16 e[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int rr = kfast ? r : r + q, kk = kfast ? k + q : k;
-          e[q] = (rr < rmax && kk < kmax) ? base[rr * rs + kk * ks] : __float2bfloat16(0.f);
-        }
-        v[i] = *reinterpret_cast<const uint4 *>(e);
-      }
-    }
-  }
-  template <int LD>
-  __device__ __forceinline__ void store(bf16 (*T)[LD], bool kfast) const {
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      int r, k;
-      slot(threadIdx.x + 128 * i, kfast, r, k);
-      const bf16 *e = reinterpret_cast<const bf16 *>(&v[i]);
-      if (kfast) {
-        *reinterpret_cast<uint4 *>(&T[r][k]) = v[i];
-      } else {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) T[r + q][k] = e[q];
-      }
-    }
-  }
-};
-
-// one element of C after the product: bias, pre-activation store, SiLU derivative
-// (backward), SiLU, stores; or FP32 accumulation (split-K weight gradients)
-__device__ __forceinline__ void epilogue(const Gemm &g, int m, int n, float v) {
-  if (g.Cacc) {
-    atomicAdd(&g.Cacc[m * g.ldca + n], v);
-    return;
-  }
-  if (g.bias) v += g.bias[n];
-  if (g.Zb) g.Zb[m * g.ldzb + n] = __float2bfloat16(v);
-  if (g.dz) {
-    const float z = __bfloat162float(g.dz[m * g.lddz + n]), s = sigm(z);
-    v *= s * (1.f + z * (1.f - s));
-  }
-  if (g.silu) v = v * sigm(v);
-  if (g.Cf) g.Cf[m * g.ldcf + n] = v;
-  if (g.Cb) g.Cb[m * g.ldcb + n] = __float2bfloat16(v);
-}
-
-// C tile TM x TN per block of 4 warps side by side along N (each TM x TN/4: TM/16
-// m16 by TN/32 n8 mma tiles), K in steps of TK; the next K tile is loaded into
-// registers while the current one is multiplied.  Two shapes: TK = 256 takes a
-// whole layer's K in one staging (inference-sized GEMMs: every load in flight at
-// once), TK = 32 streams long reductions (weight gradients over the batch).
-template <int TM, int TN, int TK>
-__global__ void __launch_bounds__(128) k_gemm(const Gemm g) {
-  constexpr int LD = TK + 8, MT = TM / 16, NT = TN / 32;
-  __shared__ __align__(16) bf16 As[TM][LD];
-  __shared__ __align__(16) bf16 Bs[TN][LD];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-  const int kbeg = blockIdx.z * g.kchunk, kend = min(g.K, kbeg + g.kchunk);
-  float acc[MT][NT][4];
-#pragma unroll
-  for (int i = 0; i < MT; ++i)
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.f;
-  const bool a_kfast = g.sak == 1, b_kfast = g.sbk == 1;
-  Stage<TM, TK> sa;
-  Stage<TN, TK> sb;
-  if (kbeg < kend) {
-    sa.load(g.A, g.sam, g.sak, m0, kbeg, g.M, kend, a_kfast);
-    sb.load(g.B, g.sbn, g.sbk, n0, kbeg, g.N, kend, b_kfast);
-  }
-  const int gq = lane >> 2, q = lane & 3;
-  for (int k0 = kbeg; k0 < kend; k0 += TK) {
-    sa.store(As, a_kfast);
-    sb.store(Bs, b_kfast);
-    __syncthreads();
-    if (k0 + TK < kend) {
-      sa.load(g.A, g.sam, g.sak, m0, k0 + TK, g.M, kend, a_kfast);
-      sb.load(g.B, g.sbn, g.sbk, n0, k0 + TK, g.N, kend, b_kfast);
-    }
-    const int kspan = min(TK, kend - k0);
-#pragma unroll 4
-    for (int kk = 0; kk < kspan; kk += 16) {
-      uint32_t af[MT][4], bfr[NT][2];
-#pragma unroll
-      for (int i = 0; i < MT; ++i) {
-        const int r0 = i * 16 + gq;
-        af[i][0] = *reinterpret_cast<const uint32_t *>(&As[r0][kk + q * 2]);
-        af[i][1] = *reinterpret_cast<const uint32_t *>(&As[r0 + 8][kk + q * 2]);
-        af[i][2] = *reinterpret_cast<const uint32_t *>(&As[r0][kk + q * 2 + 8]);
-        af[i][3] = *reinterpret_cast<const uint32_t *>(&As[r0 + 8][kk + q * 2 + 8]);
-      }
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const int cc = warp * (TN / 4) + j * 8 + gq;
-        bfr[j][0] = *reinterpret_cast<const uint32_t *>(&Bs[cc][kk + q * 2]);
-        bfr[j][1] = *reinterpret_cast<const uint32_t *>(&Bs[cc][kk + q * 2 + 8]);
-      }
-#pragma unroll
-      for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int j = 0; j < NT; ++j) mma_bf16(acc[i][j], af[i], bfr[j]);
-    }
-    __syncthreads();
-  }
-  // epilogue
-#pragma unroll
-  for (int i = 0; i < MT; ++i)
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int m = m0 + i * 16 + gq + (r >= 2 ? 8 : 0);
-        const int n = n0 + warp * (TN / 4) + j * 8 + q * 2 + (r & 1);
-        if (m >= g.M || n >= g.N) continue;
-        epilogue(g, m, n, acc[i][j][r]);
-      }
-}
-
 // ------------------------------------------------------------- tcgen05 products
 //
 // C[M x N] = A[M x K] B[K x N] for A with K contiguous (sak = 1) and B with K contiguous
@@ -233,7 +82,7 @@ __global__ void __launch_bounds__(128) k_gemm(const Gemm g) {
 // accumulator of 128 lanes x N columns, their completion signalled on an mbarrier
 // (tcgen05.commit) and waited for with a time limit (a wait that runs out sets *err and
 // skips the epilogue); then each warp reads its 32 TMEM lanes (rows) 16 columns at a time
-// (tcgen05.ld) into the same epilogue as k_gemm.
+// (tcgen05.ld) into the epilogue.
 constexpr int TC_M = 128;
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -617,16 +466,6 @@ __global__ void k_nll(const float *o, const float *y, int n, const float *ymean,
   if (threadIdx.x == 0) atomicAdd(loss, (double)sh[0]);
 }
 
-// normalised outputs -> physical units: mean * std + mean, log-variance + 2 log std
-__global__ void k_denorm(const float *o, int n, const float *ymean, const float *yistd, float *out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n * OUT) return;
-  const int r = i / OUT, k = i % OUT;
-  const float v = o[r * OUTP + k];
-  out[i] = k < NY ? v / yistd[k] + ymean[k]
-                  : fminf(fmaxf(v, -kLogVarClamp), kLogVarClamp) - 2.f * __logf(yistd[k - NY]);
-}
-
 // column sums of a BF16 matrix into FP32 (bias gradients), one atomic per (block, column)
 __global__ void k_colsum(const bf16 *a, int n, int cols, long long lda, float *out) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -635,6 +474,152 @@ __global__ void k_colsum(const bf16 *a, int n, int cols, long long lda, float *o
   float s = 0.f;
   for (int r = r0; r < r1; ++r) s += __bfloat162float(a[r * lda + c]);
   atomicAdd(&out[c], s);
+}
+
+// ------------------------------------------------------------------ inference
+//
+// The whole network for TM = 16 MT WM rows per CTA of eight warps (WM along the rows, 8 / WM
+// along the columns): normalisation, the four layers with the activations in shared memory, the
+// outputs in physical units, in one launch.  The weights stream from L2 through three stages
+// of 32 k rows by asynchronous copies, the next layer's first stages while this one's epilogue runs.
+// Each output element is K steps of 16 in ascending order into one FP32 accumulator, bias, SiLU and
+// the BF16 rounding between layers, as in the colloid-only step's network, whose bits these are.
+// Bound: L2 reads of the weights (311 KB a CTA) and the SiLU's two special-function operations
+// per element.  Measured, six launches with the activations through memory -> this: 16,384 rows
+// 197 -> 43 us a call, one row 50 -> 26.5 us (the rule at infer() has the rest).
+template <int MT, int WM, int ST>
+struct Infer {
+  static constexpr int TM = 16 * MT * WM, WN = 8 / WM, NT = H / WN / 8, LDA = H + 8, LDW = H + 8, KS = 32;
+  static constexpr size_t smem = (size_t)TM * LDA * 2 + (size_t)ST * KS * LDW * 2 + (size_t)H * 24 * 2;
+};
+
+__device__ __forceinline__ void ldsm4(uint32_t r[4], const void *p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t r[4], const void *p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void cp16(void *to, const void *from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from)
+               : "memory");
+}
+
+struct InferArgs {
+  const float *x, *xmean, *xistd, *ymean, *yistd, *bias;
+  const bf16 *w[4];
+  float *out;
+  int n;
+};
+
+template <int MT, int WM, int ST>
+__global__ void __launch_bounds__(256) k_mlp_infer(const InferArgs g) {
+  using T = Infer<MT, WM, ST>;
+  extern __shared__ __align__(16) uint8_t tc_smem[];
+  bf16(*A)[T::LDA] = reinterpret_cast<bf16(*)[T::LDA]>(tc_smem);
+  bf16(*W)[T::KS][T::LDW] = reinterpret_cast<bf16(*)[T::KS][T::LDW]>(tc_smem + sizeof(bf16) * T::TM * T::LDA);
+  bf16(*W4)[24] = reinterpret_cast<bf16(*)[24]>(tc_smem + sizeof(bf16) * (T::TM * T::LDA + ST * T::KS * T::LDW));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp % WM, wn = warp / WM;
+  const int gq = lane >> 2, q = lane & 3;
+  const int m0 = blockIdx.x * T::TM, rows = min(T::TM, g.n - m0);
+  // the weight stages in the order they are used: layer 1 (96 k rows), 2, 3
+  constexpr int S1 = INP / T::KS, S2 = H / T::KS, NS = S1 + 2 * S2;
+  auto stage = [&](int s) {
+    if (s < NS) {
+      const int k0 = (s < S1 ? s : (s - S1) % S2) * T::KS;
+      const bf16 *src = (s < S1 ? g.w[0] : s < S1 + S2 ? g.w[1] : g.w[2]) + (size_t)k0 * H;
+      for (int v = tid; v < T::KS * (H / 8); v += 256)
+        cp16(&W[s % ST][v / (H / 8)][(v % (H / 8)) * 8], src + (size_t)v * 8);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int v = tid; v < H * 2; v += 256) cp16(&W4[v >> 1][(v & 1) * 8], g.w[3] + (size_t)v * 8);  // (the first group)
+#pragma unroll
+  for (int q = 0; q < ST - 1; ++q) stage(q);
+  // normalised inputs, clipped (k_features_in)
+  for (int i = tid; i < T::TM * INP; i += 256) {
+    const int r = i / INP, c = i % INP;
+    const float z = c < IN && r < rows ? (g.x[(size_t)(m0 + r) * IN + c] - g.xmean[c]) * g.xistd[c] : 0.f;
+    A[r][c] = __float2bfloat16(fminf(fmaxf(z, -kInputClip), kInputClip));
+  }
+  float acc[MT][T::NT][4];
+  int s = 0;
+  for (int l = 0; l < 3; ++l) {
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int j = 0; j < T::NT; ++j)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.f;
+    const int ns = l == 0 ? S1 : S2;
+    for (int t = 0; t < ns; ++t, ++s) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+      __syncthreads();  // stage s has arrived, and the buffer of stage s - 1 is free
+      stage(s + ST - 1);
+      const bf16(*Ws)[T::LDW] = W[s % ST];
+#pragma unroll
+      for (int kk = 0; kk < T::KS; kk += 16) {
+        uint32_t af[MT][4];
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+          ldsm4(af[i], &A[(wm * MT + i) * 16 + (lane & 15)][t * T::KS + kk + (lane >> 4) * 8]);
+#pragma unroll
+        for (int j = 0; j < T::NT; j += 2) {
+          uint32_t b[4];  // k 0-7 and 8-15 of the tile's first 8 columns, then of its next 8
+          ldsm4t(b, &Ws[kk + (lane & 15)][wn * T::NT * 8 + j * 8 + (lane >> 4) * 8]);
+#pragma unroll
+          for (int i = 0; i < MT; ++i) {
+            mma_bf16(acc[i][j], af[i], b);
+            mma_bf16(acc[i][j + 1], af[i], b + 2);
+          }
+        }
+      }
+    }
+    __syncthreads();  // every warp has read the layer's inputs
+    const float *bias = g.bias + l * H;
+#pragma unroll
+    for (int j = 0; j < T::NT; ++j) {
+      const int c = wn * T::NT * 8 + j * 8 + q * 2;
+      const float b0 = bias[c], b1 = bias[c + 1];
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = (wm * MT + i) * 16 + gq + h * 8;
+          float v0 = acc[i][j][2 * h] + b0, v1 = acc[i][j][2 * h + 1] + b1;
+          v0 = v0 * sigm(v0);
+          v1 = v1 * sigm(v1);
+          *reinterpret_cast<__nv_bfloat162 *>(&A[r][c]) = __nv_bfloat162(__float2bfloat16(v0), __float2bfloat16(v1));
+        }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  // the output layer: 16 rows x 8 columns a warp, in physical units (k_denorm)
+  for (int p = warp; p < T::TM / 16 * 2; p += 8) {
+    const int r0 = (p >> 1) * 16, c0 = (p & 1) * 8;
+    float o[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int kk = 0; kk < H; kk += 32) {
+      uint32_t b[4], a0[4], a1[4];
+      ldsm4t(b, &W4[kk + lane][c0]);
+      ldsm4(a0, &A[r0 + (lane & 15)][kk + (lane >> 4) * 8]);
+      ldsm4(a1, &A[r0 + (lane & 15)][kk + 16 + (lane >> 4) * 8]);
+      mma_bf16(o, a0, b);
+      mma_bf16(o, a1, b + 2);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int r = r0 + gq + (e >= 2 ? 8 : 0), k = c0 + q * 2 + (e & 1);
+      if (r >= rows || k >= OUT) continue;
+      const float v = o[e] + g.bias[3 * H + k];
+      g.out[(size_t)(m0 + r) * OUT + k] =
+          k < NY ? v / g.yistd[k] + g.ymean[k]
+                 : fminf(fmaxf(v, -kLogVarClamp), kLogVarClamp) - 2.f * __logf(g.yistd[k - NY]);
+    }
+  }
 }
 
 // the parameter layout: flat FP32 vector (W1 [IN][H], b1, W2 [H][H], b2, W3, b3, W4 [H][OUT], b4)
@@ -699,6 +684,7 @@ __global__ void k_adam(float *p, const float *gr, float *m, float *v, long long 
 
 struct mpcd_mlp {
   int max_batch = 0;
+  int n_sm = 152;  // multiprocessors of the device
   Layout L;
   float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;  // flat FP32 params, grads, Adam moments
   bf16 *w[4] = {nullptr, nullptr, nullptr, nullptr};               // padded BF16 weights [k][n]
@@ -782,20 +768,6 @@ void gemm_tc_wgrad(mpcd_mlp *nn, cudaStream_t s, Gemm g) {
                                                                                            nn->tc_fault);
 }
 
-void gemm(cudaStream_t s, Gemm g, int ksplit = 1) {
-  if (g.K <= 256 && ksplit == 1) {
-    // whole K in one staging, 32 x 32 tiles: many blocks for inference-sized M
-    g.kchunk = g.K;
-    dim3 grid((g.N + 31) / 32, (g.M + 31) / 32, 1);
-    k_gemm<32, 32, 256><<<grid, 128, 0, s>>>(g);
-    return;
-  }
-  g.kchunk = ksplit > 1 ? ((g.K + ksplit - 1) / ksplit + BK - 1) / BK * BK : g.K;
-  const int kz = ksplit > 1 ? (g.K + g.kchunk - 1) / g.kchunk : 1;
-  dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, kz);
-  k_gemm<BM, BN, BK><<<grid, 128, 0, s>>>(g);
-}
-
 Gemm base() {
   Gemm g;
   memset(&g, 0, sizeof g);
@@ -812,18 +784,14 @@ long long bias_off(int l) {
 }
 
 // forward of rows [0, n) of n->X; stores Z (pre-activations) and A (activations) for the backward
-// pass.  tc: the products on the tcgen05 path (training), else the warp-level kernel (inference)
-void forward(mpcd_mlp *nn, int n, cudaStream_t s, bool tc) {
+// pass
+void forward(mpcd_mlp *nn, int n, cudaStream_t s) {
   const bf16 *in = nn->X;
   long long ldin = INP;
   for (int l = 0; l < 4; ++l) {
     Gemm g = base();
     g.A = in; g.sam = ldin; g.sak = 1;
-    if (tc) {
-      g.B = nn->wt[l]; g.sbk = 1; g.sbn = kKpad[l];
-    } else {
-      g.B = nn->w[l]; g.sbk = kNpad[l]; g.sbn = 1;
-    }
+    g.B = nn->wt[l]; g.sbk = 1; g.sbn = kKpad[l];
     g.M = n; g.N = kNpad[l]; g.K = kKpad[l];
     g.bias = nn->bias + bias_off(l);
     if (l < 3) {
@@ -835,8 +803,7 @@ void forward(mpcd_mlp *nn, int n, cudaStream_t s, bool tc) {
     } else {
       g.Cf = nn->O; g.ldcf = OUTP;
     }
-    if (tc) gemm_tc(nn, s, g);
-    else gemm(s, g);
+    gemm_tc(nn, s, g);
   }
 }
 
@@ -896,6 +863,38 @@ int upload_params(mpcd_mlp *nn, const float *h) {
   return cudaDeviceSynchronize() == cudaSuccess ? MPCD_OK : mfail(nn, MPCD_ERR_CUDA, "parameter upload");
 }
 
+template <int MT, int WM, int ST>
+void infer_launch(const InferArgs &g, cudaStream_t s) {
+  using T = Infer<MT, WM, ST>;
+  k_mlp_infer<MT, WM, ST><<<(unsigned)((g.n + T::TM - 1) / T::TM), 256, T::smem, s>>>(g);
+}
+
+template <int MT, int WM, int ST>
+bool infer_attr() {
+  return cudaFuncSetAttribute(k_mlp_infer<MT, WM, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)Infer<MT, WM, ST>::smem) == cudaSuccess;
+}
+
+// Rows per CTA: the smallest of 16, 32 and 64 that gives the device at most one CTA per SM (the
+// weights are then read the fewest times that keep every SM busy), and 64 beyond, where two CTAs share an
+// SM and one's epilogue runs under the other's products.  Measured per call, layer by layer -> 16 /
+// 32 / 64 rows a CTA: 1 row 50 -> 26.5 / 26.9 / 32 us, 2,432 rows 62 -> 29 / 30 / 34, 4,864 rows 90
+// -> 40 / 32 / 34, 16,384 rows 197 -> 96 / 54 / 43, 65,536 rows 663 -> 311 / 141 / 108 (128 rows a
+// CTA, one per SM: 47 and 136).
+void infer(mpcd_mlp *nn, const float *x, int n, float *out, cudaStream_t s) {
+  InferArgs g;
+  g.x = x;
+  g.xmean = nn->xmean; g.xistd = nn->xistd;
+  g.ymean = nn->ymean; g.yistd = nn->yistd;
+  g.bias = nn->bias;
+  for (int l = 0; l < 4; ++l) g.w[l] = nn->w[l];
+  g.out = out;
+  g.n = n;
+  if (n <= 16 * nn->n_sm) infer_launch<1, 1, 6>(g, s);
+  else if (n <= 32 * nn->n_sm) infer_launch<2, 1, 4>(g, s);
+  else infer_launch<4, 1, 3>(g, s);
+}
+
 int stage_inputs(mpcd_mlp *nn, const float *x, int n, cudaStream_t s) {
   if (n < 1 || n > nn->max_batch) return mfail(nn, MPCD_ERR_CAPACITY, "batch larger than max_batch");
   const long long tot = (long long)n * INP;
@@ -910,6 +909,10 @@ extern "C" int mpcd_mlp_create(int max_batch, uint64_t seed, mpcd_mlp **out) {
   *out = nullptr;
   mpcd_mlp *nn = new mpcd_mlp();
   nn->max_batch = max_batch;
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && nsm > 0)
+    nn->n_sm = nsm;
   nn->L = layout();
   const long long P = nn->L.total;
   nn->p = dalloc<float>(nn, P); nn->g = dalloc<float>(nn, P); nn->m = dalloc<float>(nn, P); nn->v = dalloc<float>(nn, P);
@@ -939,6 +942,10 @@ extern "C" int mpcd_mlp_create(int max_batch, uint64_t seed, mpcd_mlp **out) {
   std::vector<float> one(IN, 1.f), zero(IN, 0.f);
   cudaMemcpy(nn->xistd, one.data(), sizeof(float) * IN, cudaMemcpyHostToDevice);
   cudaMemcpy(nn->yistd, one.data(), sizeof(float) * NY, cudaMemcpyHostToDevice);
+  if (!infer_attr<1, 1, 6>() || !infer_attr<2, 1, 4>() || !infer_attr<4, 1, 3>()) {
+    mpcd_mlp_destroy(nn);
+    return MPCD_ERR_CUDA;
+  }
   std::vector<float> h;
   init_params(nn, seed, h);
   int r = upload_params(nn, h.data());
@@ -991,10 +998,8 @@ extern "C" int mpcd_mlp_set_params(mpcd_mlp *nn, const float *in) {
 extern "C" int mpcd_mlp_forward(mpcd_mlp *nn, const float *x, int n, float *out, void *stream) {
   if (!nn || !x || !out) return MPCD_ERR_PARAM;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  int r = stage_inputs(nn, x, n, s);
-  if (r) return r;
-  forward(nn, n, s, false);
-  k_denorm<<<(n * OUT + 255) / 256, 256, 0, s>>>(nn->O, n, nn->ymean, nn->yistd, out);
+  if (n < 1 || n > nn->max_batch) return mfail(nn, MPCD_ERR_CAPACITY, "batch larger than max_batch");
+  infer(nn, x, n, out, s);
   return cudaGetLastError() == cudaSuccess ? MPCD_OK : mfail(nn, MPCD_ERR_CUDA, "forward launch");
 }
 
@@ -1002,7 +1007,7 @@ extern "C" int mpcd_mlp_grad(mpcd_mlp *nn, const float *x, const float *y, int n
   if (!nn || !x || !y) return MPCD_ERR_PARAM;
   int r = stage_inputs(nn, x, n, nullptr);
   if (r) return r;
-  forward(nn, n, nullptr, true);
+  forward(nn, n, nullptr);
   cudaMemset(nn->loss, 0, sizeof(double));
   k_nll<<<(n + 255) / 256, 256>>>(nn->O, y, n, nn->ymean, nn->yistd, nn->dO, nn->loss);
   backward(nn, n, nullptr);
