@@ -6,19 +6,24 @@
 // forces, the active kick (run(), cpp/run.cpp:13) and the orientation update
 // (cpp/update.cpp:34-46, plus rotational diffusion Dr), in FP32.
 //
-// Per step, two kernels (one CUDA graph):
+// Per step, two kernels (CUDA graphs of one and of eight steps):
 //   k_sur_net, one block per 16 colloids over the whole GPU (16 compute warps, one
 //     producer warp): each colloid's neighbours (from candidate lists kept with a
 //     skin, all pairs when they expire), its 81 network inputs and its force partners
 //     for the step, the whole network (four layers, BF16 mma.sync with FP32
 //     accumulation, activations in shared memory, the weights streamed through a
-//     ring of shared-memory stages by bulk copies while the block computes), the
-//     Gaussian draw of the exchange, the step's rotational-diffusion draws and the
-//     orientation through the substeps;
-//   the substeps, k_sur_md1 (one block, up to 1024 colloids) or k_sur_md (one cluster
-//     of 8 blocks): the active kick and the n_sub velocity-Verlet substeps (each needs
-//     every colloid's new position: a block barrier, or distributed shared memory and
-//     one cluster barrier, per substep).
+//     ring of shared-memory stages by bulk copies while the block computes) and the
+//     Gaussian draw of the exchange;
+//   the substeps, k_sur_md1 (one block) or k_sur_md (one cluster of 8 blocks): the active
+//     kick and the n_sub velocity-Verlet substeps (each needs every colloid's new position: a
+//     block barrier, or distributed shared memory and one cluster barrier, per substep); beside
+//     them, on blocks of their own, the rotational-diffusion draws and the orientations.
+// Within a graph each kernel is launched before the one before it has ended: its blocks are then
+// placed, its weights and constants loaded, and it waits only for the state.
+// Bound: the latency of that chain (500 colloids: 12 us of network, half of it the layers' shared-memory
+// traffic, 13 us of substeps).  Measured, us a step, 500 / 2,000 colloids at volume fractions
+// 0.1 / 0.2: 39.8 / 50.5 -> 28.4 / 41.5 (the orientation behind the network and the
+// substeps behind its whole end: 37.7 / 48.4; a branch per pair in contact before that).
 // The packed weights (the layout k_sur_net reads) are rebuilt from the network at
 // every mpcd_surrogate_step call.  k_sur_features computes the inputs of the
 // current state on request.
@@ -45,6 +50,11 @@ typedef __nv_bfloat16 bf16;
 constexpr int NF = MPCD_MLP_IN, NO = MPCD_MLP_OUT, KNEAR = 12, MAXC = MPCD_SURROGATE_MAX_COLLOIDS, CAND = 64;
 constexpr int H = MPCD_MLP_HIDDEN, INP = MLP_IN_PADDED, OUTP = MLP_OUT_PADDED;
 constexpr uint32_t DOM_SUR_KICK = 20, DOM_SUR_ROT = 21;
+// Colloids up to which the substeps run in one block, else in a cluster of eight: the block's barrier
+// is 0.6 us a substep cheaper, but its SM shares the pair forces among few schedulers.  Measured,
+// us a step, block / cluster: 30 colloids 22.9 / 24.8, 200 26.1 / 27.0, 300 (volume fraction 0.2)
+// 30.9 / 29.3, 500 37.7 / 36.3, 1,024 55.6 / 41.2 (the last two before the kernels overlapped).
+constexpr int kMdBlockMax = 256;
 constexpr int MAXF = 32;  // force partners per colloid (within the WCA cutoff plus the skin)
 
 struct Sur {
@@ -61,7 +71,7 @@ struct Sur {
   float *feat;      // the last step's network inputs [Nc][81]
   float *out;       // the last step's normalised network outputs [Nc][16]
   float4 *imp;      // per-substep linear impulse of the drawn exchange [Nc], orientation at the step's start [Nc],
-                    // Omega and orientation at the step's end [Nc] [Nc] (stored by the substep kernel)
+                    // per-substep share of the angular exchange [Nc] (w: the step's number)
   uint16_t *fpart;  // force partners [Nc][MAXF], ascending index
   uint8_t *fpn;     // their count
   uint16_t *nbl;    // candidate neighbours [Nc][CAND] (within rlist at the last rebuild), ascending index
@@ -77,7 +87,18 @@ struct Sur {
   const float *ymean, *yistd;         // output normalisation
 };
 
-__device__ __forceinline__ float wrapd(float d, float L, float iL) { return d - L * rintf(d * iL); }
+// rintf and floorf of |t| < 2^22 by additions: the conversion unit that rounds takes four times as
+// long, and the pair loops round three times a pair
+__device__ __forceinline__ float rint_add(float t) { return __fadd_rn(__fadd_rn(t, 12582912.f), -12582912.f); }
+__device__ __forceinline__ float floor_add(float t) {
+  const float r = rint_add(t);
+  return r > t ? r - 1.f : r;
+}
+
+// minimum image of a difference of two positions inside the box
+__device__ __forceinline__ float wrapd(float d, float L, float iL) { return d - L * rint_add(__fmul_rn(d, iL)); }
+// back into the box after a substep's move
+__device__ __forceinline__ float boxed(float x, float L, float iL) { return x - L * floor_add(__fmul_rn(x, iL)); }
 
 // the skin of a step's force partners (pairs within the cutoff plus it): 2.5 times the
 // largest displacement the last step's speeds give, within [0.5, 2]; the candidate lists
@@ -94,7 +115,7 @@ __device__ __forceinline__ float2 normal2(uint32_t a, uint32_t b) {
   const float r = sqrtf(-2.f * __logf(u01f(a)));
   float s, c;
   __sincosf(6.283185307179586f * u01f(b), &s, &c);
-  return make_float2(r * c, r * s);
+  return make_float2(__fmul_rn(r, c), __fmul_rn(r, s));  // (rounded, whatever they are added to)
 }
 
 // features of colloid j (one warp): V, Omega, ra, then the 12 nearest colloids
@@ -167,10 +188,13 @@ __global__ void __launch_bounds__(128) k_sur_features(const Sur S) {
 // 8 t + (l >> 2)), so that a warp's fragments are one conflict-free 16-byte shared
 // load each.  Chunks 0-2: layer 1 (K 96), 3-10: layer 2, 11-18: layer 3 (32 K rows
 // x 256 columns, 16 KB each), 19: layer 4 (K 256 x 16 columns, 8 KB).
-constexpr int ROWS = 16, NCW = 16, TPW = 32 / NCW, NET_THREADS = 32 * (NCW + 1), CHUNK_U4 = 1024, NCHUNK = 20, NSTAGE = 6,
+constexpr int ROWS = 16, NCW = 16, TPW = 32 / NCW, NET_THREADS = 32 * (NCW + 1), CHUNK_U4 = 1024, NCHUNK = 20, NSTAGE = 8,
               LDA = H + 8;
+constexpr int FAULT_FIRST = 6;  // the first weight chunk that the tests' fault may leave out
 constexpr int PACK_U4 = 19 * CHUNK_U4 + 512;
 static_assert(ROWS == NCW, "one row per compute warp");
+
+constexpr int CPW = 4;  // weight chunks per wait of a compute warp (at most half the ring)
 
 constexpr int MAXSUB = 32;  // substeps per MPCD step the colloid-only step supports
 
@@ -182,8 +206,6 @@ struct __align__(128) NetSmem {
       float4 cx[ROWS][CAND], cv[ROWS][CAND];  // the candidates' positions and velocities
     } c;
   } u;
-  float4 nz[ROWS][MAXSUB];     // rotational-diffusion Gaussians of the step's substeps
-  float4 rm[ROWS][MAXSUB][3];  // the Euler matrix of Omega dt per substep (rows)
   float4 row[4][ROWS];       // the rows' X, V, Omega, ra at the step's start
   float dp[ROWS][NO / 2];    // the drawn exchange (momentum, angular momentum)
   bf16 act[2][ROWS][LDA];
@@ -329,10 +351,16 @@ __device__ __forceinline__ void a_frag(const bf16 (*A)[LDA], int kk, uint32_t a[
                : "memory");
 }
 
+// A step's kernels are launched before the one before them has ended (each then finds its blocks
+// placed and its constants loaded): wait_before holds until that one has ended and its writes are
+// visible, let_dependents lets the next one start
+__device__ __forceinline__ void wait_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ float sigm(float z) { return __fdividef(1.f, 1.f + __expf(-z)); }  // as mlp.cu
 
-// One block per 16 colloids: eight compute warps (two colloids each in the
-// neighbour and feature phases, 32 columns each in the network) and one producer
+// One block per 16 colloids: sixteen compute warps (a colloid each in the
+// neighbour and feature phases, 16 columns each in the network) and one producer
 // warp that streams the weights.
 //   neighbours within max(three radii, the force cutoff plus the skin): from each
 //   colloid's candidate list (colloids within that distance plus a skin of 2 at the
@@ -342,25 +370,19 @@ __device__ __forceinline__ float sigm(float z) { return __fdividef(1.f, 1.f + __
 //   ties by index, zero padded: the layout of brownian_gb300.closure.features), raw
 //   to S.feat and normalised (clipped to six standard deviations) as the BF16 input
 //   rows; the force partners (within the cutoff plus the skin, ascending index);
-//   the step's draws (rotational diffusion, the exchange's Gaussians);
+//   the exchange's Gaussians;
 //   the four layers (the mlp.cu forward pass: K steps in ascending order into one
 //   FP32 accumulator, bias, SiLU, BF16 between layers), the weights streamed by bulk
 //   copies NSTAGE chunks ahead (full / empty barriers per stage); from the outputs
-//   the Gaussian draw of the exchange (per-substep impulses for k_sur_md);
-//   the orientation over the step's substeps: Omega takes its share of the angular
-//   exchange each substep and ra the Euler rotation and the rotational diffusion
-//   (update_activity_direction); neither depends on positions or forces.
+//   the Gaussian draw of the exchange (per-substep shares for the substeps' kernel).
 __global__ void __launch_bounds__(NET_THREADS) k_sur_net(const Sur S) {
   extern __shared__ __align__(128) unsigned char net_smem[];
   NetSmem &sm = *reinterpret_cast<NetSmem *>(net_smem);
-  if (*S.err & 4) return;  // a weight copy of an earlier step of this call did not arrive: no more steps
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gq = lane >> 2, q = lane & 3;
   const unsigned lt = (1u << lane) - 1u;
   const int j0 = blockIdx.x * ROWS;
-  const uint32_t step = (uint32_t)*S.step;
   const bool producer = warp == NCW;
-  const float rfp = S.rc + partner_skin(S), rforce2 = rfp * rfp;
   if (tid == NCW * 32) {
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(&sm.full[s], 1);
@@ -370,16 +392,10 @@ __global__ void __launch_bounds__(NET_THREADS) k_sur_net(const Sur S) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     sm.abort = 0;
     // the first weight chunks stream in while the neighbours are found
-    for (int g = 0; g < NSTAGE; ++g) issue_chunk(S, sm, g);
+    for (int g = 0; g < NSTAGE; ++g)
+      if (g != S.drop_chunk) issue_chunk(S, sm, g);
   }
-  // the rows' state, the biases, the normalisation and the candidate lists (or every
-  // position, for a rebuild): independent loads, all in flight together
-  const bool rebuild = *S.rebuild != 0;
-  if (tid < 4 * ROWS) {
-    const int r = tid % ROWS, f = tid / ROWS, j = j0 + r;
-    const float4 *src = f == 0 ? S.X : (f == 1 ? S.V : (f == 2 ? S.W : S.ra));
-    if (j < S.Nc) sm.row[f][r] = src[j];
-  }
+  // what no step changes
   static_assert((3 * H + OUTP) / 4 <= NET_THREADS && NF <= NET_THREADS, "one load per thread");
   if (tid < (3 * H + OUTP) / 4) reinterpret_cast<uint4 *>(sm.bias)[tid] = reinterpret_cast<const uint4 *>(S.bias)[tid];
   if (tid < NF) {
@@ -390,6 +406,20 @@ __global__ void __launch_bounds__(NET_THREADS) k_sur_net(const Sur S) {
     sm.ym[tid] = S.ymean[tid];
     sm.ys[tid] = S.yistd[tid];
   }
+  // the substeps of the step before have ended, and what they wrote is here
+  wait_before();
+  let_dependents();
+  // the rows' state and the candidate lists (or every position, for a rebuild): independent loads,
+  // all in flight together
+  const int err = *S.err;
+  const uint32_t step = (uint32_t)*S.step;
+  const float rfp = S.rc + partner_skin(S), rforce2 = rfp * rfp;
+  const bool rebuild = *S.rebuild != 0;
+  if (tid < 4 * ROWS) {
+    const int r = tid % ROWS, f = tid / ROWS, j = j0 + r;
+    const float4 *src = f == 0 ? S.X : (f == 1 ? S.V : (f == 2 ? S.W : S.ra));
+    if (j < S.Nc) sm.row[f][r] = src[j];
+  }
   // the lists (read on every step, so that no load waits for the flag; a rebuild replaces them)
   static_assert(ROWS * CAND / 8 <= NET_THREADS, "one 16-byte piece of the lists per thread");
   if (tid < ROWS * CAND / 8) {
@@ -398,6 +428,14 @@ __global__ void __launch_bounds__(NET_THREADS) k_sur_net(const Sur S) {
       reinterpret_cast<uint4 *>(sm.lst[r])[qv] = reinterpret_cast<const uint4 *>(S.nbl + (size_t)j * CAND)[qv];
   }
   if (tid < ROWS) sm.lstn[tid] = j0 + tid < S.Nc ? S.nbn[j0 + tid] : 0;
+  if (err & 4) {
+    // a weight copy of an earlier step of this call did not arrive: no more steps (the copies in
+    // flight land first)
+    if (tid == NCW * 32)
+      for (int g = 0; g < NSTAGE; ++g)
+        if (g != S.drop_chunk) mbar_wait_bounded(&sm.full[g], 0);
+    return;
+  }
   if (rebuild) {
     for (int i0 = tid; i0 < S.Nc; i0 += 8 * NET_THREADS) {  // eight loads in flight per thread
       float4 v[8];
@@ -552,24 +590,16 @@ __global__ void __launch_bounds__(NET_THREADS) k_sur_net(const Sur S) {
     }
     }
   }
-  // the step's draws: rotational diffusion per substep, the exchange's six Gaussians
-  for (int i = tid; i < ROWS * (S.n_sub + 1); i += NET_THREADS) {
-    const int r = i % ROWS, l = i / ROWS, j = j0 + r;
-    if (j >= S.Nc) continue;
-    if (l < S.n_sub) {
-      if (S.rotdiff_s > 0.f) {
-        const uint4 d = draw4(S.key, DOM_SUR_ROT, 0, (uint32_t)(j + 1), 0, step * S.n_sub + l);
-        const float2 g0 = normal2(d.x, d.y), g1 = normal2(d.z, d.w);
-        sm.nz[r][l] = make_float4(g0.x, g0.y, g1.x, 0.f);
-      }
-    } else {
-      const uint4 r0 = draw4(S.key, DOM_SUR_KICK, 0, (uint32_t)(j + 1), 0, step);
-      const uint4 r1 = draw4(S.key, DOM_SUR_KICK, 1, (uint32_t)(j + 1), 0, step);
-      const float2 g0 = normal2(r0.x, r0.y), g1 = normal2(r0.z, r0.w), g2 = normal2(r1.x, r1.y);
-      sm.xi[r][0] = g0.x; sm.xi[r][1] = g0.y; sm.xi[r][2] = g1.x;
-      sm.xi[r][3] = g1.y; sm.xi[r][4] = g2.x; sm.xi[r][5] = g2.y;
-    }
+  // the exchange's six Gaussians, on the producer's lanes meanwhile
+  if (producer && lane < ROWS && j0 + lane < S.Nc) {
+    const int r = lane, j = j0 + r;
+    const uint4 r0 = draw4(S.key, DOM_SUR_KICK, 0, (uint32_t)(j + 1), 0, step);
+    const uint4 r1 = draw4(S.key, DOM_SUR_KICK, 1, (uint32_t)(j + 1), 0, step);
+    const float2 g0 = normal2(r0.x, r0.y), g1 = normal2(r0.z, r0.w), g2 = normal2(r1.x, r1.y);
+    sm.xi[r][0] = g0.x; sm.xi[r][1] = g0.y; sm.xi[r][2] = g1.x;
+    sm.xi[r][3] = g1.y; sm.xi[r][4] = g2.x; sm.xi[r][5] = g2.y;
   }
+  static_assert(ROWS <= 32, "a lane per row");
   __syncthreads();
   // raw inputs to S.feat, normalised BF16 rows to act[0]
   for (int i = tid; i < ROWS * INP; i += NET_THREADS) {
@@ -604,8 +634,9 @@ __global__ void __launch_bounds__(NET_THREADS) k_sur_net(const Sur S) {
         if (c != S.drop_chunk) mbar_wait_bounded(&sm.full[c % NSTAGE], (uint32_t)((c / NSTAGE) & 1));
     }
   } else {
-    // three hidden layers: compute warp w takes columns 8 TPW w .. 8 TPW (w + 1) - 1, two
-    // weight chunks per wait
+    // three hidden layers: compute warp w takes columns 8 TPW w .. 8 TPW (w + 1) - 1, four
+    // weight chunks per wait (their fragments and the rows' loaded together, then a chain of
+    // eight products per tile)
     int g = 0;
 #pragma unroll 1
     for (int layer = 0; layer < 3; ++layer) {
@@ -618,35 +649,32 @@ __global__ void __launch_bounds__(NET_THREADS) k_sur_net(const Sur S) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[t][e] = 0.f;
 #pragma unroll 1
-      for (int c = 0; c < nch; c += 2) {
-        const bool two = c + 1 < nch;
-        const bool ok0 = chunk_ready(S, sm, g), ok1 = two ? chunk_ready(S, sm, g + 1) : true;
-        const uint4 *B0 = sm.ring[g % NSTAGE], *B1 = sm.ring[(g + 1) % NSTAGE];
-        uint4 b0[TPW], b1[TPW];
+      for (int c = 0; c < nch; c += CPW) {
+        bool ok[CPW];
+        uint4 b[CPW][TPW];
+        uint32_t a[CPW][2][4];
 #pragma unroll
-        for (int t = 0; t < TPW; ++t) b0[t] = B0[(TPW * warp + t) * 32 + lane];
-        if (two) {
+        for (int u = 0; u < CPW; ++u) {
+          if (c + u >= nch) continue;
+          a_frag(A, 32 * (c + u), a[u][0]);
+          a_frag(A, 32 * (c + u) + 16, a[u][1]);
+          ok[u] = chunk_ready(S, sm, g + u);
+          const uint4 *B = sm.ring[(g + u) % NSTAGE];
 #pragma unroll
-          for (int t = 0; t < TPW; ++t) b1[t] = B1[(TPW * warp + t) * 32 + lane];
+          for (int t = 0; t < TPW; ++t) b[u][t] = B[(TPW * warp + t) * 32 + lane];
         }
-        uint32_t a[4];
-        a_frag(A, 32 * c, a);
 #pragma unroll
-        for (int t = 0; t < TPW; ++t) mma_bf16(acc[t], a, b0[t].x, b0[t].y);
-        a_frag(A, 32 * c + 16, a);
+        for (int u = 0; u < CPW; ++u) {
+          if (c + u >= nch) continue;
 #pragma unroll
-        for (int t = 0; t < TPW; ++t) mma_bf16(acc[t], a, b0[t].z, b0[t].w);
-        if (two) {
-          a_frag(A, 32 * c + 32, a);
+          for (int t = 0; t < TPW; ++t) mma_bf16(acc[t], a[u][0], b[u][t].x, b[u][t].y);
 #pragma unroll
-          for (int t = 0; t < TPW; ++t) mma_bf16(acc[t], a, b1[t].x, b1[t].y);
-          a_frag(A, 32 * c + 48, a);
-#pragma unroll
-          for (int t = 0; t < TPW; ++t) mma_bf16(acc[t], a, b1[t].z, b1[t].w);
+          for (int t = 0; t < TPW; ++t) mma_bf16(acc[t], a[u][1], b[u][t].z, b[u][t].w);
         }
-        chunk_release(sm, g, ok0);
-        if (two) chunk_release(sm, g + 1, ok1);
-        g += two ? 2 : 1;
+#pragma unroll
+        for (int u = 0; u < CPW; ++u)
+          if (c + u < nch) chunk_release(sm, g + u, ok[u]);
+        g += min(CPW, nch - c);
       }
       const float *bias = sm.bias + H * layer;
 #pragma unroll
@@ -703,58 +731,56 @@ __global__ void __launch_bounds__(NET_THREADS) k_sur_net(const Sur S) {
     sm.dp[r][k] = (o[k] + S.noise * __expf(0.5f * lv) * sm.xi[r][k]) / sm.ys[k] + sm.ym[k];
   }
   __syncthreads();
-  // per (row, substep): Omega after the substep's share of the angular exchange (spread
-  // in equal parts over the substeps: the fluid collides every substep; the same
-  // sequence of additions as the substeps make) and the Euler matrix of Omega dt
+  // for the substeps: the exchange in equal shares (the fluid collides every substep), and the
+  // orientation run()'s kick uses
   const float fm = 1.f / (S.M * S.n_sub), fi = 1.f / (S.I * S.n_sub);
-  for (int i = tid; i < ROWS * S.n_sub; i += NET_THREADS) {
-    const int r = i % ROWS, l = i / ROWS, j = j0 + r;
-    if (j >= S.Nc) continue;
-    if (l == 0) {
-      S.imp[j] = make_float4(sm.dp[r][0] * fm, sm.dp[r][1] * fm, sm.dp[r][2] * fm, 0.f);
-      S.imp[S.Nc + j] = sm.row[3][r];  // the orientation run()'s kick uses
-    }
-    const float pax = sm.dp[r][3] * fi, pay = sm.dp[r][4] * fi, paz = sm.dp[r][5] * fi;
-    float4 w = sm.row[2][r];
-    for (int s = 0; s <= l; ++s) {
-      w.x += pax; w.y += pay; w.z += paz;
-    }
-    float sx, cx, sy, cy, sz, cz;
-    __sincosf(w.x * S.dt, &sx, &cx); __sincosf(w.y * S.dt, &sy, &cy); __sincosf(w.z * S.dt, &sz, &cz);
-    sm.rm[r][l][0] = make_float4(cy * cz, -(cy * sz), sy, 0.f);
-    sm.rm[r][l][1] = make_float4(sx * sy * cz + cx * sz, -sx * sy * sz + cx * cz, -(sx * cy), 0.f);
-    sm.rm[r][l][2] = make_float4(-cx * sy * cz + sx * sz, cx * sy * sz + sx * cz, cx * cy, 0.f);
-  }
-  __syncthreads();
-  // the orientation through the substeps: the Euler rotation, then the rotational
-  // diffusion (update_activity_direction plus Dr)
   if (tid < ROWS && j0 + tid < S.Nc) {
     const int r = tid, j = j0 + r;
-    const float pax = sm.dp[r][3] * fi, pay = sm.dp[r][4] * fi, paz = sm.dp[r][5] * fi;
-    float4 w = sm.row[2][r], a = sm.row[3][r];
-    float4 n0 = sm.rm[r][0][0], n1 = sm.rm[r][0][1], n2 = sm.rm[r][0][2];
-    for (int l = 0; l < S.n_sub; ++l) {
-      w.x += pax; w.y += pay; w.z += paz;
-      const float4 m0 = n0, m1 = n1, m2 = n2;
-      if (l + 1 < S.n_sub) {  // the next substep's matrix, in flight meanwhile
-        n0 = sm.rm[r][l + 1][0]; n1 = sm.rm[r][l + 1][1]; n2 = sm.rm[r][l + 1][2];
-      }
-      float ax = m0.x * a.x + m0.y * a.y + m0.z * a.z;
-      float ay = m1.x * a.x + m1.y * a.y + m1.z * a.z;
-      float az = m2.x * a.x + m2.y * a.y + m2.z * a.z;
-      if (S.rotdiff_s > 0.f) {
-        const float4 gz = sm.nz[r][l];
-        const float d = gz.x * ax + gz.y * ay + gz.z * az;
-        ax += S.rotdiff_s * (gz.x - d * ax); ay += S.rotdiff_s * (gz.y - d * ay); az += S.rotdiff_s * (gz.z - d * az);
-      }
-      const float in = rsqrtf(ax * ax + ay * ay + az * az);
-      a = make_float4(ax * in, ay * in, az * in, 0.f);
-    }
-    // the step's end state of Omega and ra, which the substep kernel stores (so a step
-    // whose network failed leaves them as they were)
-    S.imp[2 * S.Nc + j] = w;
-    S.imp[3 * S.Nc + j] = a;
+    S.imp[j] = make_float4(sm.dp[r][0] * fm, sm.dp[r][1] * fm, sm.dp[r][2] * fm, 0.f);
+    S.imp[S.Nc + j] = sm.row[3][r];
+    S.imp[2 * S.Nc + j] =
+        make_float4(sm.dp[r][3] * fi, sm.dp[r][4] * fi, sm.dp[r][5] * fi, __uint_as_float(step));
   }
+}
+
+// Omega and orientation of colloid j through the step's substeps: Omega takes its share of the
+// angular exchange each substep, and the orientation the Euler rotation by Omega dt, then the
+// rotational diffusion (update_activity_direction plus Dr).  Neither depends on positions or forces,
+// so it runs on blocks of its own beside the substeps.  (Every rounding is written out: the bits do
+// not depend on what the compiler fuses.)
+__device__ __noinline__ void orient(const Sur &S, int j) {
+  const float4 pa = S.imp[2 * S.Nc + j];
+  const uint32_t step = __float_as_uint(pa.w);
+  float4 w = S.W[j], a = S.ra[j];
+#pragma unroll 2
+  for (int l = 0; l < S.n_sub; ++l) {
+    w.x += pa.x; w.y += pa.y; w.z += pa.z;
+    float sx, cx, sy, cy, sz, cz;
+    __sincosf(w.x * S.dt, &sx, &cx); __sincosf(w.y * S.dt, &sy, &cy); __sincosf(w.z * S.dt, &sz, &cz);
+    const float ss = __fmul_rn(sx, sy), cs = __fmul_rn(cx, sy);
+    const float4 m0 = make_float4(__fmul_rn(cy, cz), -__fmul_rn(cy, sz), sy, 0.f);
+    const float4 m1 = make_float4(__fmaf_rn(cx, sz, __fmul_rn(ss, cz)), __fmaf_rn(-ss, sz, __fmul_rn(cx, cz)),
+                                  -__fmul_rn(sx, cy), 0.f);
+    const float4 m2 = make_float4(__fmaf_rn(sx, sz, -__fmul_rn(cs, cz)), __fmaf_rn(cs, sz, __fmul_rn(sx, cz)),
+                                  __fmul_rn(cx, cy), 0.f);
+    auto row = [&](const float4 &m) { return __fmaf_rn(m.z, a.z, __fmaf_rn(m.y, a.y, __fmul_rn(m.x, a.x))); };
+    auto dot = [](float x, float y, float z, float p, float q, float r) {
+      return __fmaf_rn(z, r, __fmaf_rn(x, p, __fmul_rn(y, q)));
+    };
+    float ax = row(m0), ay = row(m1), az = row(m2);
+    if (S.rotdiff_s > 0.f) {
+      const uint4 d4 = draw4(S.key, DOM_SUR_ROT, 0, (uint32_t)(j + 1), 0, step * S.n_sub + l);
+      const float2 g0 = normal2(d4.x, d4.y), g1 = normal2(d4.z, d4.w);
+      const float d = dot(g0.x, g0.y, g1.x, ax, ay, az);
+      ax = __fmaf_rn(S.rotdiff_s, __fmaf_rn(-d, ax, g0.x), ax);
+      ay = __fmaf_rn(S.rotdiff_s, __fmaf_rn(-d, ay, g0.y), ay);
+      az = __fmaf_rn(S.rotdiff_s, __fmaf_rn(-d, az, g1.x), az);
+    }
+    const float in = rsqrtf(dot(ax, ay, az, ax, ay, az));
+    a = make_float4(ax * in, ay * in, az * in, 0.f);
+  }
+  S.W[j] = w;
+  S.ra[j] = a;
 }
 
 // ---- the substeps ---------------------------------------------------------------
@@ -767,113 +793,103 @@ __device__ __forceinline__ float step_moved2(const Sur &S, float4 x, float4 xs) 
 
 // the WCA forces on a colloid at x from its n partners (ids in row, ascending; positions
 // in P): the force-shifted WCA pair force (cpp/update.cpp:14-32) in FP32 for the pairs
-// within the cutoff (1/r by the fast reciprocal square root, 1/r^6 from 1/r^2), four
-// positions fetched together, summed in partner order
+// within the cutoff (1/r by the fast reciprocal square root, 1/r^6 from 1/r^2), summed in
+// partner order.  Four partners at a time without a branch (a pair beyond the cutoff gets the
+// factor 0, which leaves the sums as they are): the four chains of some 40 dependent operations
+// run beside one another, where a branch per pair in contact made them wait in turn.
 __device__ __forceinline__ float3 partner_forces(const Sur &S, float4 x, const float4 *P, const uint16_t *row, int n,
                                                  int self) {
   float3 fn = make_float3(0.f, 0.f, 0.f);
+#pragma unroll 1
   for (int e = 0; e < n; e += 4) {
     const uint2 kk = *reinterpret_cast<const uint2 *>(row + e);
     const int k4[4] = {(int)(kk.x & 0xFFFFu), (int)(kk.x >> 16), (int)(kk.y & 0xFFFFu), (int)(kk.y >> 16)};
-    float4 xk[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) xk[i] = P[e + i < n ? k4[i] : self];
+    float f[4], dx[4], dy[4], dz[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float dx = wrapd(x.x - xk[i].x, S.L[0], S.iL[0]), dy = wrapd(x.y - xk[i].y, S.L[1], S.iL[1]),
-                  dz = wrapd(x.z - xk[i].z, S.L[2], S.iL[2]);
-      const float r2 = dx * dx + dy * dy + dz * dz;
-      if (e + i < n && r2 < S.rc2) {
-        const float ir = rsqrtf(r2), ir2 = ir * ir, ir6 = ir2 * ir2 * ir2;
-        const float f = (4.f * S.eps * (12.f * S.sig12 * ir6 * ir6 * ir - 6.f * S.sig6 * ir6 * ir) - S.fc) * ir;
-        fn.x += f * dx; fn.y += f * dy; fn.z += f * dz;
-      }
+      const float4 xk = P[e + i < n ? k4[i] : self];
+      dx[i] = wrapd(x.x - xk.x, S.L[0], S.iL[0]);
+      dy[i] = wrapd(x.y - xk.y, S.L[1], S.iL[1]);
+      dz[i] = wrapd(x.z - xk.z, S.L[2], S.iL[2]);
+      const float r2 = dx[i] * dx[i] + dy[i] * dy[i] + dz[i] * dz[i];
+      const float ir = rsqrtf(r2), ir2 = ir * ir, ir6 = ir2 * ir2 * ir2;
+      const float g = (4.f * S.eps * (12.f * S.sig12 * ir6 * ir6 * ir - 6.f * S.sig6 * ir6 * ir) - S.fc) * ir;
+      f[i] = e + i < n && r2 < S.rc2 ? g : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      fn.x += f[i] * dx[i]; fn.y += f[i] * dy[i]; fn.z += f[i] * dz[i];
     }
   }
   return fn;
 }
 
-// One block, PER colloids per thread (position, velocity, force and the step's impulse
+// One block, a colloid per thread (position, velocity, force and the step's impulse
 // in registers; positions, two copies by substep parity, and force partners in shared
 // memory): run()'s kick along the orientation at the step's start, then n_sub substeps
 // of update_pos_md, the substep's share of the exchange, compute_force_md at the new
 // positions and update_velocity_colloid, one block barrier per substep (the copy a
 // substep writes was last read two substeps before).  At the end: whether a colloid has
 // moved more than half the skin since the candidate lists were built.
-template <int PER>
-__global__ void __launch_bounds__(1024) k_sur_md1(const Sur S) {
+// Blocks 1, 2, ...: the orientations.
+__global__ void __launch_bounds__(kMdBlockMax) k_sur_md1(const Sur S) {
   extern __shared__ float4 smem[];
-  if (*S.err & 4) return;  // the network's outputs of this step are incomplete: the state stays as it was
   __shared__ unsigned s_vmax;  // the largest speed at the end (float bits, non-negative)
-  const float hs = 0.5f * partner_skin(S), hs2 = hs * hs;
-  uint16_t *sF = reinterpret_cast<uint16_t *>(smem + 2 * MAXC);  // [MAXC][MAXF] force partners
-  uint8_t *sFn = reinterpret_cast<uint8_t *>(sF + MAXC * MAXF);   // [MAXC] their count
+  uint16_t *sF = reinterpret_cast<uint16_t *>(smem + 2 * kMdBlockMax);  // [kMdBlockMax][MAXF] force partners
   const int T = blockDim.x, tid = threadIdx.x;
+  wait_before();
+  let_dependents();
+  if (blockIdx.x > 0) {
+    const int j = (blockIdx.x - 1) * T + tid;
+    if (!(*S.err & 4) && j < S.Nc) orient(S, j);
+    return;
+  }
   if (tid == 0) s_vmax = 0u;
-  {
-    const uint4 *src = reinterpret_cast<const uint4 *>(S.fpart);
-    uint4 *dst = reinterpret_cast<uint4 *>(sF);
-    const int nq = S.Nc * (MAXF * 2 / 16);
-    for (int i0 = tid; i0 < nq; i0 += 4 * T) {  // four loads in flight per thread
-      uint4 qv[4];
+  const int j = tid;
+  const bool own = j < S.Nc;
+  const int err = *S.err;
+  const float hs = 0.5f * partner_skin(S), hs2 = hs * hs;
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f), v = x, fo = x, pl = x;
+  int n = 0;
+  if (own) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(S.fpart + (size_t)j * MAXF);
+    uint4 *dst = reinterpret_cast<uint4 *>(sF + j * MAXF);
+    uint4 pp[MAXF * 2 / 16];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (i0 + u * T < nq) qv[u] = src[i0 + u * T];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (i0 + u * T < nq) dst[i0 + u * T] = qv[u];
-    }
-    for (int i = tid; i < S.Nc; i += T) sFn[i] = S.fpn[i];
-  }
-  float4 x[PER], v[PER], fo[PER], pl[PER];
-#pragma unroll
-  for (int u = 0; u < PER; ++u) {
-    const int j = tid + T * u;
-    if (j >= S.Nc) continue;
-    x[u] = S.X[j]; v[u] = S.V[j]; fo[u] = S.f[j]; pl[u] = S.imp[j];
+    for (int i = 0; i < MAXF * 2 / 16; ++i) pp[i] = src[i];
+    n = S.fpn[j];
+    x = S.X[j]; v = S.V[j]; fo = S.f[j]; pl = S.imp[j];
     const float4 a = S.imp[S.Nc + j];
-    v[u].x += S.v0 * a.x; v[u].y += S.v0 * a.y; v[u].z += S.v0 * a.z;
+#pragma unroll
+    for (int i = 0; i < MAXF * 2 / 16; ++i) dst[i] = pp[i];
+    v.x += S.v0 * a.x; v.y += S.v0 * a.y; v.z += S.v0 * a.z;
   }
+  if (err & 4) return;  // the network's outputs of this step are incomplete: the state stays as it was
   const float hdt2m = 0.5f * S.dt * S.dt / S.M, hdtm = 0.5f * S.dt / S.M;
   for (int l = 0; l < S.n_sub; ++l) {
-    float4 *P = (l & 1) ? smem : smem + MAXC;  // this substep's copy
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {  // update_pos_md
-      const int j = tid + T * u;
-      if (j >= S.Nc) continue;
-      float4 &xx = x[u];
-      xx.x += v[u].x * S.dt + fo[u].x * hdt2m; xx.y += v[u].y * S.dt + fo[u].y * hdt2m;
-      xx.z += v[u].z * S.dt + fo[u].z * hdt2m;
-      xx.x -= S.L[0] * floorf(xx.x * S.iL[0]); xx.y -= S.L[1] * floorf(xx.y * S.iL[1]);
-      xx.z -= S.L[2] * floorf(xx.z * S.iL[2]);
-      P[j] = xx;
+    float4 *P = (l & 1) ? smem : smem + kMdBlockMax;  // this substep's copy
+    if (own) {  // update_pos_md
+      x.x += v.x * S.dt + fo.x * hdt2m; x.y += v.y * S.dt + fo.y * hdt2m; x.z += v.z * S.dt + fo.z * hdt2m;
+      x.x = boxed(x.x, S.L[0], S.iL[0]); x.y = boxed(x.y, S.L[1], S.iL[1]); x.z = boxed(x.z, S.L[2], S.iL[2]);
+      P[j] = x;
     }
     __syncthreads();
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-      const int j = tid + T * u;
-      if (j >= S.Nc) continue;
+    if (own) {
       // this substep's share of the fluid exchange (fluid_colloid_collision)
-      v[u].x += pl[u].x; v[u].y += pl[u].y; v[u].z += pl[u].z;
+      v.x += pl.x; v.y += pl.y; v.z += pl.z;
       // compute_force_md at the new positions, update_velocity_colloid
-      const float3 fn = partner_forces(S, x[u], P, sF + j * MAXF, sFn[j], j);
-      v[u].x += (fo[u].x + fn.x) * hdtm; v[u].y += (fo[u].y + fn.y) * hdtm; v[u].z += (fo[u].z + fn.z) * hdtm;
-      fo[u] = make_float4(fn.x, fn.y, fn.z, 0.f);
+      const float3 fn = partner_forces(S, x, P, sF + j * MAXF, n, j);
+      v.x += (fo.x + fn.x) * hdtm; v.y += (fo.y + fn.y) * hdtm; v.z += (fo.z + fn.z) * hdtm;
+      fo = make_float4(fn.x, fn.y, fn.z, 0.f);
     }
   }
   int moved = 0, fast = 0;
-#pragma unroll
-  for (int u = 0; u < PER; ++u) {
-    const int j = tid + T * u;
-    if (j >= S.Nc) continue;
+  if (own) {
     const float4 x0 = S.xref[j], xs = S.X[j];
-    S.X[j] = x[u]; S.V[j] = v[u]; S.f[j] = fo[u];
-    S.W[j] = S.imp[2 * S.Nc + j]; S.ra[j] = S.imp[3 * S.Nc + j];
-    const float dx = wrapd(x[u].x - x0.x, S.L[0], S.iL[0]), dy = wrapd(x[u].y - x0.y, S.L[1], S.iL[1]),
-                dz = wrapd(x[u].z - x0.z, S.L[2], S.iL[2]);
-    moved |= dx * dx + dy * dy + dz * dz > S.half_skin2;
-    fast |= step_moved2(S, x[u], xs) > hs2;
-    atomicMax(&s_vmax, __float_as_uint(sqrtf(v[u].x * v[u].x + v[u].y * v[u].y + v[u].z * v[u].z)));
+    S.X[j] = x; S.V[j] = v; S.f[j] = fo;
+    moved = step_moved2(S, x, x0) > S.half_skin2;
+    fast = step_moved2(S, x, xs) > hs2;
+    atomicMax(&s_vmax, __float_as_uint(sqrtf(v.x * v.x + v.y * v.y + v.z * v.z)));
   }
   moved = __syncthreads_or(moved);
   fast = __syncthreads_or(fast);
@@ -896,8 +912,8 @@ __global__ void __launch_bounds__(1024) k_sur_md1(const Sur S) {
 // a colloid has moved more than half the skin since the candidate lists were built.
 constexpr int MDC = 8, MD_MAXT = MAXC / MDC;
 
+// The second cluster: the orientations.
 __global__ void __cluster_dims__(MDC, 1, 1) __launch_bounds__(MD_MAXT) k_sur_md(const Sur S) {
-  if (*S.err & 4) return;  // the network's outputs of this step are incomplete: the state stays as it was
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ float4 smem[];
@@ -906,11 +922,19 @@ __global__ void __cluster_dims__(MDC, 1, 1) __launch_bounds__(MD_MAXT) k_sur_md(
   int *sMoved = reinterpret_cast<int *>(sFn + MD_MAXT);                  // [MDC] (block 0)
   unsigned *sVmax = reinterpret_cast<unsigned *>(sMoved + MDC);         // [MDC] (block 0)
   __shared__ unsigned s_vmax;
-  const float hs = 0.5f * partner_skin(S), hs2 = hs * hs;
   const int tid = threadIdx.x, rank = (int)cl.block_rank();
   const int per = (S.Nc + MDC - 1) / MDC, j = rank * per + tid;
   const bool own = tid < per && j < S.Nc;
   if (tid == 0) s_vmax = 0u;
+  cl.sync();  // every block has started before any writes to its copies
+  wait_before();
+  let_dependents();
+  if (blockIdx.x >= MDC) {
+    if (own && !(*S.err & 4)) orient(S, j);
+    return;
+  }
+  const int err = *S.err;
+  const float hs = 0.5f * partner_skin(S), hs2 = hs * hs;
   float4 x = make_float4(0.f, 0.f, 0.f, 0.f), v = x, fo = x, pl = x;
   int n = 0;
   if (own) {
@@ -926,13 +950,13 @@ __global__ void __cluster_dims__(MDC, 1, 1) __launch_bounds__(MD_MAXT) k_sur_md(
     for (int i = 0; i < MAXF * 2 / 16; ++i) dst[i] = pp[i];
     v.x += S.v0 * a.x; v.y += S.v0 * a.y; v.z += S.v0 * a.z;
   }
-  cl.sync();  // every block has started before any writes to its copies
+  if (err & 4) return;  // the network's outputs of this step are incomplete: the state stays as it was
   const float hdt2m = 0.5f * S.dt * S.dt / S.M, hdtm = 0.5f * S.dt / S.M;
   for (int l = 0; l < S.n_sub; ++l) {
     const int nb = (l + 1) & 1;
     if (own) {  // update_pos_md
       x.x += v.x * S.dt + fo.x * hdt2m; x.y += v.y * S.dt + fo.y * hdt2m; x.z += v.z * S.dt + fo.z * hdt2m;
-      x.x -= S.L[0] * floorf(x.x * S.iL[0]); x.y -= S.L[1] * floorf(x.y * S.iL[1]); x.z -= S.L[2] * floorf(x.z * S.iL[2]);
+      x.x = boxed(x.x, S.L[0], S.iL[0]); x.y = boxed(x.y, S.L[1], S.iL[1]); x.z = boxed(x.z, S.L[2], S.iL[2]);
       float4 *mine = (nb ? smem + MAXC : smem) + j;
 #pragma unroll
       for (int b = 0; b < MDC; ++b) *cl.map_shared_rank(mine, b) = x;
@@ -952,10 +976,7 @@ __global__ void __cluster_dims__(MDC, 1, 1) __launch_bounds__(MD_MAXT) k_sur_md(
   if (own) {
     const float4 x0 = S.xref[j], xs = S.X[j];
     S.X[j] = x; S.V[j] = v; S.f[j] = fo;
-    S.W[j] = S.imp[2 * S.Nc + j]; S.ra[j] = S.imp[3 * S.Nc + j];
-    const float dx = wrapd(x.x - x0.x, S.L[0], S.iL[0]), dy = wrapd(x.y - x0.y, S.L[1], S.iL[1]),
-                dz = wrapd(x.z - x0.z, S.L[2], S.iL[2]);
-    moved = (dx * dx + dy * dy + dz * dz > S.half_skin2 ? 1 : 0) | (step_moved2(S, x, xs) > hs2 ? 2 : 0);
+    moved = (step_moved2(S, x, x0) > S.half_skin2 ? 1 : 0) | (step_moved2(S, x, xs) > hs2 ? 2 : 0);
     atomicMax(&s_vmax, __float_as_uint(sqrtf(v.x * v.x + v.y * v.y + v.z * v.z)));
   }
   moved = __syncthreads_or(moved & 1) | (__syncthreads_or(moved & 2) ? 2 : 0);
@@ -1015,7 +1036,7 @@ struct mpcd_surrogate {
   Sur S;
   mpcd_mlp *net = nullptr;
   cudaStream_t stream = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  cudaGraphExec_t exec[2] = {nullptr, nullptr};  // one step; GRAPH_STEPS steps
   uint4 *wpk = nullptr;
   float *outd = nullptr;  // the outputs in physical units (mpcd_surrogate_outputs)
   std::vector<void *> allocs;
@@ -1027,6 +1048,16 @@ namespace {
 int sfail(mpcd_surrogate *s, int code, const std::string &e) {
   if (s) s->err = e;
   return code;
+}
+
+constexpr int GRAPH_STEPS = 8;  // steps of a graph: within one, a kernel's start hides behind the kernel before it
+
+void drop_graphs(mpcd_surrogate *s) {
+  for (cudaGraphExec_t &g : s->exec)
+    if (g) {
+      cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
 }
 
 template <typename T>
@@ -1041,22 +1072,41 @@ T *salloc(mpcd_surrogate *s, size_t n) {
   return static_cast<T *>(p);
 }
 
-constexpr size_t kMd1Smem = 2 * MAXC * sizeof(float4) + MAXC * MAXF * sizeof(uint16_t) + MAXC;
-constexpr int kMdBlockMax = 1024;  // colloids up to which the substeps run in one block, else in a cluster
+constexpr size_t kMd1Smem = 2 * kMdBlockMax * sizeof(float4) + kMdBlockMax * MAXF * sizeof(uint16_t);
 constexpr size_t kMdSmem = 2 * MAXC * sizeof(float4) + MD_MAXT * MAXF * sizeof(uint16_t) + MD_MAXT + 2 * MDC * sizeof(int);
 constexpr size_t kNetSmem = sizeof(NetSmem);
 
-int enqueue_step(mpcd_surrogate *s) {
+// a launch that may start before the kernel before it on the stream has ended (early)
+template <typename K>
+cudaError_t launch_early(mpcd_surrogate *s, K *k, int grid, int block, size_t smem, bool early) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k, s->S);
+}
+
+// n steps
+int enqueue_steps(mpcd_surrogate *s, int n) {
   const Sur &S = s->S;
-  k_sur_net<<<(S.Nc + ROWS - 1) / ROWS, NET_THREADS, kNetSmem, s->stream>>>(S);
-  if (S.Nc <= kMdBlockMax) {
-    if (S.Nc <= 1024) k_sur_md1<1><<<1, (S.Nc + 31) / 32 * 32, kMd1Smem, s->stream>>>(S);
-    else k_sur_md1<2><<<1, 1024, kMd1Smem, s->stream>>>(S);
-  } else {
-    const int per = (S.Nc + MDC - 1) / MDC;
-    k_sur_md<<<MDC, (per + 31) / 32 * 32, kMdSmem, s->stream>>>(S);
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < n && e == cudaSuccess; ++i) {
+    e = launch_early(s, k_sur_net, (S.Nc + ROWS - 1) / ROWS, NET_THREADS, kNetSmem, i > 0);
+    if (e != cudaSuccess) break;
+    if (S.Nc <= kMdBlockMax) {
+      const int block = (S.Nc + 31) / 32 * 32;
+      e = launch_early(s, k_sur_md1, 2, block, kMd1Smem, true);
+    } else {
+      e = launch_early(s, k_sur_md, 2 * MDC, ((S.Nc + MDC - 1) / MDC + 31) / 32 * 32, kMdSmem, true);
+    }
   }
-  return cudaGetLastError() == cudaSuccess ? MPCD_OK : sfail(s, MPCD_ERR_CUDA, "step launch");
+  return e == cudaSuccess ? MPCD_OK : sfail(s, MPCD_ERR_CUDA, "step launch");
 }
 
 // the network's current weights in the order k_sur_net reads them
@@ -1121,7 +1171,7 @@ extern "C" int mpcd_surrogate_create(const mpcd_params *p, mpcd_mlp *net, mpcd_s
   S.X = salloc<float4>(s, Nc); S.V = salloc<float4>(s, Nc); S.W = salloc<float4>(s, Nc);
   S.ra = salloc<float4>(s, Nc); S.f = salloc<float4>(s, Nc);
   S.feat = salloc<float>(s, Nc * NF); S.out = salloc<float>(s, Nc * OUTP);
-  S.imp = salloc<float4>(s, 4 * Nc);
+  S.imp = salloc<float4>(s, 3 * Nc);
   S.nbl = salloc<uint16_t>(s, Nc * CAND); S.nbn = salloc<int>(s, Nc);
   S.xref = salloc<float4>(s, Nc); S.rebuild = salloc<int>(s, 1);
   if (S.rebuild) cudaMemset(S.rebuild, 1, sizeof(int));  // no candidate lists yet
@@ -1137,8 +1187,7 @@ extern "C" int mpcd_surrogate_create(const mpcd_params *p, mpcd_mlp *net, mpcd_s
   if (!s->err.empty() || cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaFuncSetAttribute(k_sur_net, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNetSmem) != cudaSuccess ||
       cudaFuncSetAttribute(k_sur_md, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMdSmem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_sur_md1<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMd1Smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_sur_md1<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMd1Smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sur_md1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMd1Smem) != cudaSuccess ||
       pack_weights(s) != MPCD_OK) {
     mpcd_surrogate_destroy(s);
     return MPCD_ERR_NOMEM;
@@ -1150,7 +1199,7 @@ extern "C" int mpcd_surrogate_create(const mpcd_params *p, mpcd_mlp *net, mpcd_s
 extern "C" int mpcd_surrogate_destroy(mpcd_surrogate *s) {
   if (!s) return MPCD_ERR_PARAM;
   if (s->stream) cudaStreamSynchronize(s->stream);
-  if (s->exec) cudaGraphExecDestroy(s->exec);
+  drop_graphs(s);
   for (void *a : s->allocs) cudaFree(a);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;
@@ -1246,23 +1295,17 @@ extern "C" int mpcd_surrogate_outputs(mpcd_surrogate *s, float *out) {
 }
 
 extern "C" int mpcd_surrogate_set_fault(mpcd_surrogate *s, int drop_chunk) {
-  if (!s || drop_chunk < -1 || drop_chunk >= NCHUNK || (drop_chunk >= 0 && drop_chunk < NSTAGE))
+  if (!s || drop_chunk < -1 || drop_chunk >= NCHUNK || (drop_chunk >= 0 && drop_chunk < FAULT_FIRST))
     return sfail(s, MPCD_ERR_PARAM, "drop_chunk: -1, or a weight chunk the producer loop issues");
   s->S.drop_chunk = drop_chunk;
-  if (s->exec) {  // the kernels take the parameters by value: capture again
-    cudaGraphExecDestroy(s->exec);
-    s->exec = nullptr;
-  }
+  drop_graphs(s);  // the kernels take the parameters by value: capture again
   return MPCD_OK;
 }
 
 extern "C" int mpcd_surrogate_set_noise(mpcd_surrogate *s, double scale) {
   if (!s || !(scale >= 0.0) || !(scale <= 1e3)) return sfail(s, MPCD_ERR_PARAM, "noise scale: 0 .. 1000");
   s->S.noise = (float)scale;
-  if (s->exec) {  // the kernels take the parameters by value: capture again
-    cudaGraphExecDestroy(s->exec);
-    s->exec = nullptr;
-  }
+  drop_graphs(s);  // the kernels take the parameters by value: capture again
   return MPCD_OK;
 }
 
@@ -1272,20 +1315,23 @@ extern "C" int mpcd_surrogate_step(mpcd_surrogate *s, int nsteps) {
   // before its failing step, and the next call may go on from there
   if (cudaMemsetAsync(s->S.err, 0, sizeof(int), s->stream) != cudaSuccess) return sfail(s, MPCD_ERR_CUDA, "step");
   if (nsteps > 0 && pack_weights(s) != MPCD_OK) return MPCD_ERR_CUDA;
-  if (!s->exec) {
-    cudaGraph_t g;
-    if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-      return sfail(s, MPCD_ERR_CUDA, "capture");
-    int r = enqueue_step(s);
-    cudaError_t e = cudaStreamEndCapture(s->stream, &g);
-    if (r) return r;
-    if (e != cudaSuccess) return sfail(s, MPCD_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&s->exec, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) return sfail(s, MPCD_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(e));
+  for (int left = nsteps; left > 0;) {
+    const int many = left >= GRAPH_STEPS ? 1 : 0, n = many ? GRAPH_STEPS : 1;
+    if (!s->exec[many]) {
+      cudaGraph_t g;
+      if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
+        return sfail(s, MPCD_ERR_CUDA, "capture");
+      int r = enqueue_steps(s, n);
+      cudaError_t e = cudaStreamEndCapture(s->stream, &g);
+      if (r) return r;
+      if (e != cudaSuccess) return sfail(s, MPCD_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
+      e = cudaGraphInstantiate(&s->exec[many], g, 0);
+      cudaGraphDestroy(g);
+      if (e != cudaSuccess) return sfail(s, MPCD_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(e));
+    }
+    if (cudaGraphLaunch(s->exec[many], s->stream) != cudaSuccess) return sfail(s, MPCD_ERR_CUDA, "graph launch");
+    left -= n;
   }
-  for (int i = 0; i < nsteps; ++i)
-    if (cudaGraphLaunch(s->exec, s->stream) != cudaSuccess) return sfail(s, MPCD_ERR_CUDA, "graph launch");
   int bits = 0;
   if (cudaMemcpyAsync(&bits, s->S.err, sizeof(int), cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||
       cudaStreamSynchronize(s->stream) != cudaSuccess)
