@@ -65,8 +65,8 @@ struct mpcd_ctx {
   cudaStream_t evs = nullptr;    // third stream (FP64 form): event passes and colloid finish
   cudaEvent_t ev_start = nullptr, ev_str = nullptr, ev_aux = nullptr, ev_finp[2] = {nullptr, nullptr};
 
-  cudaGraphExec_t step_exec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [sorts][fluid buffer]
-  int step_launches[2][2] = {{0, 0}, {0, 0}};
+  cudaGraphExec_t step_exec[3][2] = {};  // [does not sort; sorts; GRAPH_STEPS that do not][fluid buffer]
+  int step_launches[3][2] = {};
   int fbuf = 0;                  // fluid buffer holding the current state
   long long host_step = 0;       // completed steps (mirror of the device counter)
   int sort_every = 10;           // counting sort by cell every this many steps
@@ -709,7 +709,7 @@ static int check_device(mpcd_ctx *c) {
 }
 
 static int drop_graph(mpcd_ctx *c) {
-  for (int s = 0; s < 2; ++s)
+  for (int s = 0; s < 3; ++s)
     for (int b = 0; b < 2; ++b)
       if (c->step_exec[s][b]) {
         cudaGraphExecDestroy(c->step_exec[s][b]);
@@ -1342,6 +1342,8 @@ static void begin_steps(mpcd_ctx *c) {
   else ensure_tables(c);
 }
 
+constexpr int GRAPH_STEPS = 3;
+
 // nsteps steps enqueued on the context's stream (graph replays), nothing waited for
 static int enq_steps(mpcd_ctx *c, int nsteps) {
   int r;
@@ -1356,27 +1358,32 @@ static int enq_steps(mpcd_ctx *c, int nsteps) {
     }
     return MPCD_OK;
   }
-  for (int s = 0; s < nsteps; ++s) {
-    // one graph per (sorts this step, fluid buffer): the kernels' buffer arguments
-    // are fixed at capture
-    const int sort = sorts_at(c, c->host_step) ? 1 : 0, b = c->fbuf;
-    if (!c->step_exec[sort][b]) {
+  for (int s = 0; s < nsteps;) {
+    // one graph per (sorts this step, fluid buffer): the kernels' buffer arguments are fixed at
+    // capture; and one of GRAPH_STEPS steps none of which sorts (a graph's launch costs its first
+    // kernel more than a kernel's within one)
+    int n = 0;
+    while (n < GRAPH_STEPS && s + n < nsteps && !sorts_at(c, c->host_step + n)) ++n;
+    if (n < GRAPH_STEPS) n = 1;
+    const int kind = n > 1 ? 2 : (sorts_at(c, c->host_step) ? 1 : 0), b = c->fbuf;
+    if (!c->step_exec[kind][b]) {
       cudaGraph_t g;
       int64_t before = c->launches;
       CUDA_OK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-      enq_step(c, sort != 0);
+      for (int k = 0; k < n; ++k) enq_step(c, kind == 1);
       CUDA_OK(c, cudaStreamEndCapture(c->stream, &g));
       c->fbuf = b;  // capture only recorded the launches
-      c->step_launches[sort][b] = (int)(c->launches - before);
+      c->step_launches[kind][b] = (int)(c->launches - before);
       c->launches = before;
-      cudaError_t e = cudaGraphInstantiate(&c->step_exec[sort][b], g, 0);
+      cudaError_t e = cudaGraphInstantiate(&c->step_exec[kind][b], g, 0);
       cudaGraphDestroy(g);
       if (e != cudaSuccess) return fail(c, MPCD_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
     }
-    CUDA_OK(c, cudaGraphLaunch(c->step_exec[sort][b], c->stream));
-    c->launches += c->step_launches[sort][b];
-    if (sort) c->fbuf = 1 - b;
-    c->host_step += 1;
+    CUDA_OK(c, cudaGraphLaunch(c->step_exec[kind][b], c->stream));
+    c->launches += c->step_launches[kind][b];
+    if (kind == 1) c->fbuf = 1 - b;
+    c->host_step += n;
+    s += n;
   }
   return MPCD_OK;
 }

@@ -110,6 +110,30 @@ __device__ __forceinline__ long long sq_fix_f(float v, int k) {
   return (long long)r;
 }
 
+struct Fix2 { long long f, f2; };
+static __device__ __noinline__ Fix2 fix2_far(float v, int k) { return {to_fix_f(v, k), sq_fix_f(v, k)}; }
+
+// to_fix_f and sq_fix_f together, in 32-bit steps where the shifts allow it (2^(23 - k) <= |v| and about
+// 2^-11 <= |v| < 2^5 at the k of a usual system: 99.9 % of a thermal fluid's components): v 2^k as one
+// product of the significand with a power of two, v^2 2^k from m^2 2^8 by one funnel shift, the dropped
+// bits compared with one half in a word of their own.  About 20 instructions a component instead of 70.
+__device__ __forceinline__ void fix2(float v, int k, long long &f, long long &f2) {
+  const unsigned b = __float_as_uint(v);
+  const int e = (int)((b >> 23) & 0xFF), sh = e - 150 + k, s = 158 - e - sh;  // (s = 8 - (2 (e - 150) + k))
+  if ((unsigned)sh <= 30u && (unsigned)(s - 1) <= 30u) {
+    const unsigned m = (b & 0x7FFFFFu) | 0x800000u;
+    f = (long long)((int)b < 0 ? -(int)m : (int)m) * (long long)(1 << sh);
+    const unsigned long long q = (unsigned long long)m * (m << 8);
+    const unsigned lo = (unsigned)q, hi = (unsigned)(q >> 32), low = __funnelshift_r(lo, hi, s), rem = lo << (32 - s);
+    const unsigned long long r = ((unsigned long long)(hi >> s) << 32) | low;
+    f2 = (long long)(r + (rem > 0x80000000u - (low & 1u) ? 1ull : 0ull));
+  } else {
+    const Fix2 t = fix2_far(v, k);
+    f = t.f;
+    f2 = t.f2;
+  }
+}
+
 __device__ __forceinline__ BinTerm32 bin32_term(const SysF64 &S, const float *rr, int p, int cx, int cy, int cz,
                                                 float ox, float oy, float oz, float vx, float vy, float vz) {
   float tx = ox + rr[0], ty = oy + rr[1], tz = oz + rr[2];
@@ -124,8 +148,11 @@ __device__ __forceinline__ BinTerm32 bin32_term(const SysF64 &S, const float *rr
   if (!(fabsf(vx) <= S.vmaxf && fabsf(vy) <= S.vmaxf && fabsf(vz) <= S.vmaxf)) atomicOr(&S.ss->err, ERRB_VRANGE);
   BinTerm32 t;
   t.c = c;
-  t.fx = to_fix_f(vx, S.kw); t.fy = to_fix_f(vy, S.kw); t.fz = to_fix_f(vz, S.kw);
-  t.f2 = sq_fix_f(vx, S.kw) + sq_fix_f(vy, S.kw) + sq_fix_f(vz, S.kw);
+  long long x2, y2, z2;
+  fix2(vx, S.kw, t.fx, x2);
+  fix2(vy, S.kw, t.fy, y2);
+  fix2(vz, S.kw, t.fz, z2);
+  t.f2 = x2 + y2 + z2;
   return t;
 }
 
@@ -666,12 +693,12 @@ __global__ void __launch_bounds__(256) k_rotate_classify32_b(const SysF64 *Ss, c
 
 // n streaming substeps along one axis: the streaming passes' o = fma(v, dt, o) and carry, n
 // times, without a branch: carry's floor leaves an offset in [0, 1) as it is, so it is taken
-// every time (a warp nearly always has a lane that needs it), and the cells carried are added up
-// and wrapped into the box once at the end (integer sums, the same cell).  What carry does with
-// a NaN or runaway offset is left out: its particle fails the range test of the binning.
-static __device__ __forceinline__ void free_axis32(int &c, float &o, float v, float dt, int n, int L) {
+// every time, and the cells carried are added up and wrapped into the box once at the end
+// (integer sums, the same cell).  What carry does with a NaN or runaway offset is left out: its
+// particle fails the range test of the binning.
+static __device__ __noinline__ float2 free_axis32(float o, float v, float dt, int n) {
   float k = 0.f;
-#pragma unroll 2
+#pragma unroll 1
   for (int l = 0; l < n; ++l) {
     o = fmaf(v, dt, o);
     const float f = floorf(o);
@@ -679,11 +706,56 @@ static __device__ __forceinline__ void free_axis32(int &c, float &o, float v, fl
     k += f;
     if (o >= 1.f) { o = 0.f; k += 1.f; }
   }
-  c += (int)k;
-  if (c < 0 || c >= L) {
-    c %= L;
-    if (c < 0) c += L;
+  return make_float2(o, k);
+}
+
+// The same for the three axes where no substep's move reaches a cell's width (slow), without rounding
+// instructions: the offset leaves [0, 1) only on the side it moves to, by less than 1, so carry adds a =
+// -1 or 1 there (exactly floor's result); the cells carried are the whole number nearest to what the n
+// moves sum up to less what the offset shows.  An offset that rounds up to 1 on its way back
+// (carry makes it 0 and carries less) is left to free_axis32.  The unsigned comparison of the bits is true
+// for every offset outside [0, 1).
+static __device__ __forceinline__ void free_axes32(int &cx, int &cy, int &cz, float &ox, float &oy, float &oz, float vx,
+                                                   float vy, float vz, float dt, int n, bool slow, int Lx, int Ly,
+                                                   int Lz) {
+  const float x0 = ox, y0 = oy, z0 = oz;
+  float kx, ky, kz;
+  bool redo = !slow;
+  if (slow) {
+    const float ax = vx < 0.f ? 1.f : -1.f, ay = vy < 0.f ? 1.f : -1.f, az = vz < 0.f ? 1.f : -1.f;
+    float top = 0.f;
+    auto move = [&](float &o, float v, float a) {
+      o = fmaf(v, dt, o);
+      if (__float_as_uint(o) >= 0x3f800000u) o = __fadd_rn(o, a);
+      top = fmaxf(top, o);
+    };
+#pragma unroll 2
+    for (int l = 0; l < n; ++l) {
+      move(ox, vx, ax);
+      move(oy, vy, ay);
+      move(oz, vz, az);
+    }
+    const float T = (float)n * dt;
+    kx = rintf(fmaf(vx, T, x0) - ox);
+    ky = rintf(fmaf(vy, T, y0) - oy);
+    kz = rintf(fmaf(vz, T, z0) - oz);
+    redo = !(top < 1.f);
   }
+  if (redo) {
+    const float2 a = free_axis32(x0, vx, dt, n), b = free_axis32(y0, vy, dt, n), c = free_axis32(z0, vz, dt, n);
+    ox = a.x; oy = b.x; oz = c.x;
+    kx = a.y; ky = b.y; kz = c.y;
+  }
+  auto wrap = [](int c, int L) {
+    if (c < 0 || c >= L) {
+      c %= L;
+      if (c < 0) c += L;
+    }
+    return c;
+  };
+  cx = wrap(cx + (int)kx, Lx);
+  cy = wrap(cy + (int)ky, Ly);
+  cz = wrap(cz + (int)kz, Lz);
 }
 
 // the free particles' whole step: n_sub streaming substeps (update_pos_mpcd, the
@@ -699,6 +771,8 @@ static __device__ __forceinline__ void k_free_flight32_body(const SysF64 &S, int
   const Fluid32 F = fluid32_at(S, fb);
   const float rr[3] = {(float)S.ss->rrn[0], (float)S.ss->rrn[1], (float)S.ss->rrn[2]};
   const int n = S.n_sub;
+  // (a free particle's moves of a step sum up to flight_rv at most)
+  const bool slow = S.flight_rv <= 0.5f * (float)n;
   uint4 q = make_uint4(0, 0, 0, 0);
   float wx = 0.f, wy = 0.f, wz = 0.f;
   int fn = 255;
@@ -720,9 +794,7 @@ static __device__ __forceinline__ void k_free_flight32_body(const SysF64 &S, int
     load(p + stride);
     BinTerm32 bt{-1, 0, 0, 0, 0};
     if (free) {
-      free_axis32(cx, ox, vx, S.dtf, n, S.Lx);
-      free_axis32(cy, oy, vy, S.dtf, n, S.Ly);
-      free_axis32(cz, oz, vz, S.dtf, n, S.Lz);
+      free_axes32(cx, cy, cz, ox, oy, oz, vx, vy, vz, S.dtf, n, slow, S.Lx, S.Ly, S.Lz);
       bt = bin32_term(S, rr, p, cx, cy, cz, ox, oy, oz, vx, vy, vz);
       F.q[p] = pack(cx, cy, cz, ox, oy, oz);
     }
@@ -1237,7 +1309,7 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
     return (c == 0 ? O.vx : c == 1 ? O.vy : O.vz) + a0 + k;
   };
   auto idx = [&](int i) -> int * { return i < NEAR32_IDX ? &sm.idx[i] : O.id + a0 + i; };
-#pragma unroll 2
+#pragma unroll 4
   for (int k = t; k < cnt; k += NT) {
     const int p = S.act[a0 + k];
     const uint4 q = F.q[p];
@@ -1294,35 +1366,54 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
       }
       if (e) *idx(atomicAdd(&s_nchk, 1)) = k;
     };
-    // Two at a time and without a branch where they stay inside their cell (the addition then
-    // carries nothing) and have one candidate, which is not near: about 50 instructions each,
-    // interleaved.  Everything else takes the general path.
+    // Two at a time and without a branch where they have one or two candidates: carry's result for an
+    // offset in (-1, 2) (one that rounds up to 1 on its way back takes the general path, as do
+    // candidates from the flight table), both distances, about 120 instructions each, interleaved.
     const int kept = min(cnt, NEAR32_ACT);
+    const float chl = (ch + 1e-4f) * (ch + 1e-4f);
     for (int k0 = t; k0 < kept; k0 += 2 * NT) {
       unsigned cand[2];
-      bool away[2];
+      bool plain[2], close[2];
       uint4 q[2];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int k = min(k0 + u * NT, kept - 1);
         cand[u] = k0 + u * NT < kept ? sm.cand[k] : NEAR_GONE;
         q[u] = sm.q[k];
-        const NearCol32 &o = sm.col.d[min(cand[u] & 0xFFFFu, (unsigned)(NearCols<NearCol32>::MAX - 1))];
         int cx, cy, cz;
         float ox, oy, oz;
         unpack(q[u], cx, cy, cz, ox, oy, oz);
         ox = fmaf(sm.v[0][k], S.dtf, ox); oy = fmaf(sm.v[1][k], S.dtf, oy); oz = fmaf(sm.v[2][k], S.dtf, oz);
-        const float dx = rel(cx, ox, o.q.x, o.o.x, S.Lx), dy = rel(cy, oy, o.q.y, o.o.y, S.Ly),
-                    dz = rel(cz, oz, o.q.z, o.o.z, S.Lz);
-        away[u] = (cand[u] >> 16) == 0xFFFFu && ox >= 0.f && ox < 1.f && oy >= 0.f && oy < 1.f && oz >= 0.f &&
-                  oz < 1.f && dx * dx + dy * dy + dz * dz > (ch + 1e-4f) * (ch + 1e-4f);
+        plain[u] = (cand[u] >> 16) - (NEAR_STALE >> 16) > 2u;  // (none of the marks)
+        auto side = [&](int &c, float &o, int L) {
+          const bool up = o >= 1.f, down = o < 0.f;
+          const float a = up ? -1.f : (down ? 1.f : 0.f);
+          o = __fadd_rn(o, a);
+          c += up ? 1 : (down ? -1 : 0);
+          c = c < 0 ? L - 1 : (c >= L ? 0 : c);
+          plain[u] = plain[u] && o >= 0.f && o < 1.f;
+        };
+        side(cx, ox, S.Lx); side(cy, oy, S.Ly); side(cz, oz, S.Lz);
         q[u] = pack(cx, cy, cz, ox, oy, oz);
+        close[u] = false;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const unsigned j = h ? cand[u] >> 16 : cand[u] & 0xFFFFu;
+          const NearCol32 &o = sm.col.d[min(j, (unsigned)(NearCols<NearCol32>::MAX - 1))];
+          const float dx = rel(cx, ox, o.q.x, o.o.x, S.Lx), dy = rel(cy, oy, o.q.y, o.o.y, S.Ly),
+                      dz = rel(cz, oz, o.q.z, o.o.z, S.Lz);
+          close[u] = close[u] || (j != 0xFFFFu && dx * dx + dy * dy + dz * dz <= chl);
+        }
       }
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int k = k0 + u * NT;
-        if (away[u]) sm.q[k] = q[u];
-        else if (cand[u] != NEAR_GONE) one(k, cand[u]);
+        if (plain[u]) {
+          sm.q[k] = q[u];
+          if (close[u]) *idx(atomicAdd(&s_nchk, 1)) = k;
+        } else if (cand[u] != NEAR_GONE) {
+          one(k, cand[u]);
+        }
       }
     }
     for (int k = NEAR32_ACT + t; k < cnt; k += NT) one(k, NEAR_WILD);  // beyond shared memory
