@@ -17,6 +17,7 @@
 // whose arithmetic the colloid-only step's network reproduces bit for bit.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -274,14 +275,14 @@ struct WeightCopies {
 // Bound: latency, with four warps a scheduler: the chain of 35 weight stages (573 KB a CTA from L2)
 // with a barrier each and six epilogues between them (35 % of the issue slots, the tensor pipe a
 // quarter of the time).  Measured cold, 8,192 rows: nine launches, each staging its operands anew,
-// 130 us; this 46 us.  A training step, host side included: 305 -> 91 us (200 rows 228 -> 78 us,
-// 16,384 rows 440 -> 155 us).
+// 130 us; this 46 us.  A training step, host side included: 305 -> 95 us (200 rows 228 -> 71 us,
+// 16,384 rows 440 -> 165 us).
 struct LayersArgs {
   const float *x, *y, *xmean, *xistd, *ymean, *yistd, *bias;
   const bf16 *w[4], *wt[4];
   bf16 *X, *A[3], *dZ[3], *dO;
   __nv_bfloat162 *Z;  // pre-activations, in the order the threads hold them
-  double *loss;       // [CTA] sums of the loss
+  float *loss;        // [n] the rows' losses
   int n;
 };
 
@@ -292,7 +293,6 @@ struct Layers {
   bf16 W4[H][24], W4t[OUTP][LD];
   float O[TM][20];
   bf16 dO[TM][24];
-  float sum[16];
 };
 
 __global__ void __launch_bounds__(Layers::NTH) k_mlp_layers(const LayersArgs g) {
@@ -422,14 +422,11 @@ __global__ void __launch_bounds__(Layers::NTH) k_mlp_layers(const LayersArgs g) 
       const int cm = k < NY ? k : OUT + 2 * (k - NY), cs = k < NY ? NY + k : cm + 1;
       sm.dO[r][cm] = __float2bfloat16(dm);
       sm.dO[r][cs] = __float2bfloat16(ds);
-      for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, o);
-      if (lane == 0) sm.sum[warp] = loss;
+      float row = 0.f;  // the row's terms one after another
+#pragma unroll
+      for (int c = 0; c < NY; ++c) row += __shfl_sync(0xFFFFFFFFu, loss, (lane & 24) + c);
+      if (k == 0 && r < rows) g.loss[m0 + r] = row;
       __syncthreads();
-      if (tid == 0) {
-        double sum = 0;
-        for (int w = 0; w < NTH / 32; ++w) sum += (double)sm.sum[w];
-        g.loss[blockIdx.x] = sum;
-      }
       for (int v = tid; v < rows * 2; v += NTH)
         *reinterpret_cast<uint4 *>(g.dO + (size_t)(m0 + (v >> 1)) * OUTP + (v & 1) * 8) =
             *reinterpret_cast<const uint4 *>(&sm.dO[v >> 1][(v & 1) * 8]);
@@ -490,24 +487,29 @@ __global__ void __launch_bounds__(Layers::NTH) k_mlp_layers(const LayersArgs g) 
 //
 // dW_l = A_{l-1}^T dZ_l and db_l, the column sums of dZ_l, of all four layers in one launch, on the
 // 5th-generation tensor cores: a CTA takes one 128 x 128 tile (128 x 16 of the last layer; twelve
-// tiles) over one slice of the batch and leaves its partial sums in memory; k_adam adds the
-// slices in order, so a gradient has the same bits every time.  As many slices as give each SM a CTA.
+// tiles) over some of the batch's slices (up to 32 of whole stages).  Each slice is a sum of its own
+// in TMEM (two accumulators in turn), the CTA adds its slices in registers and leaves its partial sums in
+// memory; k_adam adds those in order, so a gradient has the same bits every time.  As many CTAs a tile
+// as give each SM one.
 // A row of the batch is contiguous along m (n), which is what the MN-major operand layout without
 // swizzle wants: core matrices of 8 k x 16 bytes, so the copies land where the MMA reads them
 // (blocks of 8 along m (n) SBO = 128 bytes apart, blocks of 8 k LBO apart).  Four stages of 64 k are
 // in flight; a buffer is filled again once the MMAs that read it have completed (one mbarrier a
 // buffer, every wait bounded: one that runs out sets *err and skips the output).  The column sums are
-// read from the staged tiles by the CTAs of the first m tile.  fault: the test hook, nothing issued.
-// Bound: latency (a CTA's eleven stages, each waiting for L2).  Measured cold, 8,192 rows: four
+// read from the staged tiles by the CTAs of the first m tile.  The CTAs past the tiles add the rows'
+// losses, 256 at a time.  fault: the test hook, nothing issued.
+// Bound: latency (a CTA's twelve stages, each waiting for L2).  Measured cold, 8,192 rows: four
 // launches that staged, waited, transposed and added with atomics, and four for the column sums,
-// 170 us; this 23 us.
-constexpr int TCW_K = 64, TCW_ST = 4, TCW_TILES = 12, TCW_TH = 256;
+// 170 us; this 27 us (23 us with a slice per CTA, whose sums are longer).
+constexpr int TCW_K = 64, TCW_ST = 4, TCW_TILES = 12, TCW_TH = 256, TCW_SLICES = 32;
 
 struct WgradArgs {
   const bf16 *A[4], *B[4];  // the layers' inputs and pre-activation gradients
-  float *part;              // [slices][total]
+  float *part;              // [gridDim.y][total]
   Layout L;
-  int n, kchunk;
+  int n, kchunk, slices;    // rows; rows of a slice (whole stages); slices
+  const float *loss;        // [n] the rows' losses
+  double *lsum;             // [n / 256] their sums
 };
 
 constexpr size_t TCW_BUF = (size_t)2 * TC_M * TCW_K * 2;  // one stage: A, then B
@@ -515,6 +517,21 @@ constexpr size_t TCW_SMEM = 1024 + TCW_ST * TCW_BUF;
 
 __global__ void __launch_bounds__(TCW_TH) k_gemm_tc_wgrad(const WgradArgs g, int *err, int fault) {
   extern __shared__ __align__(1024) uint8_t tc_smem[];
+  if (blockIdx.x == TCW_TILES) {
+    float *sh = reinterpret_cast<float *>(tc_smem);
+    for (int b = blockIdx.y; b * 256 < g.n; b += gridDim.y) {
+      const int r = b * 256 + (int)threadIdx.x;
+      sh[threadIdx.x] = r < g.n ? g.loss[r] : 0.f;
+      __syncthreads();
+      for (int o = 128; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+        __syncthreads();
+      }
+      if (threadIdx.x == 0) g.lsum[b] = (double)sh[0];
+      __syncthreads();
+    }
+    return;
+  }
   // this CTA's tile: layer l, rows m0.., columns n0.. (N of them)
   const int t = blockIdx.x;
   const int l = t < 2 ? 0 : t < 6 ? 1 : t < 10 ? 2 : 3;
@@ -522,12 +539,14 @@ __global__ void __launch_bounds__(TCW_TH) k_gemm_tc_wgrad(const WgradArgs g, int
   const int m0 = (l == 0 ? 0 : l == 3 ? u : u >> 1) * TC_M, n0 = l == 3 ? 0 : (u & 1) * 128, N = l == 3 ? OUTP : 128;
   const int lda = l == 0 ? INP : H, ldb = l == 3 ? OUTP : H;
   const bf16 *GA = g.A[l], *GB = g.B[l];
-  const int kbeg = blockIdx.y * g.kchunk, kend = min(g.n, kbeg + g.kchunk);
+  const int s0 = (int)((long long)blockIdx.y * g.slices / gridDim.y),
+            s1 = (int)((long long)(blockIdx.y + 1) * g.slices / gridDim.y);
+  const int kbeg = s0 * g.kchunk, kend = min(g.n, s1 * g.kchunk), sst = g.kchunk / TCW_K;  // (stages of a slice)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   unsigned long long *bar = reinterpret_cast<unsigned long long *>(tc_smem);  // one per buffer
   uint32_t *tslot = reinterpret_cast<uint32_t *>(tc_smem + 64);
   const uint32_t lboA = TC_M / 8 * 128u, lboB = (uint32_t)N / 8 * 128u;
-  const uint32_t ncols = 128u;
+  const uint32_t ncols = 256u;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)),
                  "r"(ncols)
@@ -575,6 +594,31 @@ __global__ void __launch_bounds__(TCW_TH) k_gemm_tc_wgrad(const WgradArgs g, int
   };
   for (int st = 0; st < TCW_ST - 1; ++st) load(st);
   bool ok = true;
+  float acc[64];  // row (warp & 3) 32 + lane, 16 columns of every 32
+#pragma unroll
+  for (int c = 0; c < 64; ++c) acc[c] = 0.f;
+  // a slice's sums (number i of this CTA) from TMEM: a row per thread, 16 columns at a time; two warps
+  // share a row's columns
+  auto gather = [&](int i) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c0 = q * 32 + (warp >> 2) * 16;
+      if (c0 >= N) continue;
+      uint32_t r[16];
+      const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((i & 1) * 128 + c0);
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+          : "r"(taddr)
+          : "memory");
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int c = 0; c < 16; ++c) acc[q * 16 + c] += __uint_as_float(r[c]);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  };
   float cs[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // column sums: columns 8 (tid / 16).., rows tid % 16..
   for (int st = 0; st < nst && ok; ++st) {
     const int q = st % TCW_ST;
@@ -587,11 +631,11 @@ __global__ void __launch_bounds__(TCW_TH) k_gemm_tc_wgrad(const WgradArgs g, int
       const uint32_t a0 = smem_addr(As), b0 = smem_addr(Bs);
       for (int kk = 0; kk < TCW_K / 16; ++kk) {
         const uint64_t ad = tc_desc(a0 + kk * 2 * lboA, lboA, 128), bd = tc_desc(b0 + kk * 2 * lboB, lboB, 128);
-        const uint32_t accumulate = (st > 0 || kk > 0) ? 1u : 0u;
+        const uint32_t accumulate = (st % sst > 0 || kk > 0) ? 1u : 0u;
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(tmem), "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate)
+            ::"r"(tmem + (uint32_t)((st / sst) & 1) * 128u), "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate)
             : "memory");
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar + q))
@@ -612,6 +656,7 @@ __global__ void __launch_bounds__(TCW_TH) k_gemm_tc_wgrad(const WgradArgs g, int
     if (st > 0) ok = tc_wait_bounded(smem_addr(bar + (st - 1) % TCW_ST), (uint32_t)(((st - 1) / TCW_ST) & 1));
     ok = __syncthreads_and(ok) != 0;
     if (ok) load(st + TCW_ST - 1);
+    if (ok && st > 0 && st % sst == 0) gather(st / sst - 1);  // (the slice before this one is complete)
   }
   // the last commit arrives when every MMA issued before it has completed
   if (ok && nst > 0) ok = tc_wait_bounded(smem_addr(bar + (nst - 1) % TCW_ST), (uint32_t)(((nst - 1) / TCW_ST) & 1));
@@ -622,25 +667,17 @@ __global__ void __launch_bounds__(TCW_TH) k_gemm_tc_wgrad(const WgradArgs g, int
   float *P = g.part + (size_t)blockIdx.y * g.L.total;
   const int nout = g.L.nout[l];
   if (all_ok) {
-    // TMEM -> registers (a row per thread, 16 columns at a time; two warps share a row's columns)
+    if (nst > 0) gather((nst - 1) / sst);
     const int m = m0 + (warp & 3) * 32 + lane;
-    for (int c0 = (warp >> 2) * 16; c0 < N; c0 += 32) {
-      uint32_t r[16];
-      const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(taddr)
-          : "memory");
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (m < g.L.kin[l]) {
+    if (m < g.L.kin[l]) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int c0 = q * 32 + (warp >> 2) * 16;
 #pragma unroll
         for (int c = 0; c < 16; c += 4)
-          if (n0 + c0 + c < nout)
+          if (c0 < N && n0 + c0 + c < nout)
             *reinterpret_cast<float4 *>(P + g.L.w[l] + (long long)m * nout + n0 + c0 + c) =
-                make_float4(__uint_as_float(r[c]), __uint_as_float(r[c + 1]), __uint_as_float(r[c + 2]),
-                            __uint_as_float(r[c + 3]));
+                make_float4(acc[q * 16 + c], acc[q * 16 + c + 1], acc[q * 16 + c + 2], acc[q * 16 + c + 3]);
       }
     }
     if (m0 == 0) {
@@ -662,7 +699,7 @@ __global__ void __launch_bounds__(TCW_TH) k_gemm_tc_wgrad(const WgradArgs g, int
   }
 }
 
-// A gradient from its slices' partial sums, in order; with update, unless a weight-gradient wait ran
+// A gradient from its partial sums, in order; with update, unless a weight-gradient wait ran
 // out, Adam on the FP32 masters and the BF16 copies (weights at [k][n] of a padded [kpad][npad] matrix
 // and transposed; biases stay FP32).  The last block adds the loss.
 struct TrainResult {
@@ -728,12 +765,13 @@ struct mpcd_mlp {
   int tc_fault = 0;                                                // test hook (mpcd_mlp_set_fault)
   float *bias = nullptr;                                           // padded biases [H][H][H][OUTP]
   float *xmean = nullptr, *xistd = nullptr, *ymean = nullptr, *yistd = nullptr;
-  // training: what the weight gradients read, the slices' partial sums and the CTAs' loss sums
+  // training: what the weight gradients read and their partial sums
   bf16 *X = nullptr, *A[3] = {nullptr, nullptr, nullptr}, *dZ[3] = {nullptr, nullptr, nullptr}, *dO = nullptr;
   __nv_bfloat162 *Z = nullptr;
   float *part = nullptr;
-  int max_slices = 1;
-  double *loss = nullptr;
+  int max_parts = 1;
+  float *loss = nullptr;    // [max_batch] the rows' losses
+  double *lsum = nullptr;   // their sums, 256 rows each
   int adam_t = 0;
   std::vector<void *> allocs;
   std::string err;
@@ -792,17 +830,19 @@ void gradients(mpcd_mlp *nn, const float *x, const float *y, int n, int update, 
   a.n = n;
   const int ctas = (n + Layers::TM - 1) / Layers::TM;
   k_mlp_layers<<<(unsigned)ctas, Layers::NTH, sizeof(Layers)>>>(a);
-  // slices of the batch: whole stages, a CTA per SM over all tiles
-  const int per = (n + nn->max_slices - 1) / nn->max_slices;
+  const int per = (n + TCW_SLICES - 1) / TCW_SLICES;
   w.part = nn->part;
   w.L = nn->L;
   w.n = n;
   w.kchunk = (per + TCW_K - 1) / TCW_K * TCW_K;
-  const int slices = (n + w.kchunk - 1) / w.kchunk;
-  k_gemm_tc_wgrad<<<dim3(TCW_TILES, (unsigned)slices), TCW_TH, TCW_SMEM>>>(w, &nn->res->err, nn->tc_fault);
+  w.slices = (n + w.kchunk - 1) / w.kchunk;
+  w.loss = nn->loss;
+  w.lsum = nn->lsum;
+  const int parts = std::min(w.slices, nn->max_parts);
+  k_gemm_tc_wgrad<<<dim3(TCW_TILES + 1, (unsigned)parts), TCW_TH, TCW_SMEM>>>(w, &nn->res->err, nn->tc_fault);
   const long long P = nn->L.total;
-  k_adam<<<(unsigned)((P + 255) / 256) + 1, 256>>>(nn->p, nn->part, slices, nn->g, nn->m, nn->v, P, update, lr, 0.9f,
-                                                  0.999f, 1e-8f, c1, c2, nn->L, copies(nn), nn->bias, nn->loss, ctas,
+  k_adam<<<(unsigned)((P + 255) / 256) + 1, 256>>>(nn->p, nn->part, parts, nn->g, nn->m, nn->v, P, update, lr, 0.9f,
+                                                  0.999f, 1e-8f, c1, c2, nn->L, copies(nn), nn->bias, nn->lsum, (n + 255) / 256,
                                                   nn->res);
 }
 
@@ -844,7 +884,7 @@ int upload_params(mpcd_mlp *nn, const float *h) {
   cudaMemset(nn->g, 0, sizeof(float) * nn->L.total);
   const long long n = nn->L.total;
   k_adam<<<(unsigned)((n + 255) / 256) + 1, 256>>>(nn->p, nn->g, 1, nn->g, nn->m, nn->v, n, 1, 0.f, 0.9f, 0.999f, 1e-8f,
-                                                  1.f, 1.f, nn->L, copies(nn), nn->bias, nn->loss, 0, nn->res);
+                                                  1.f, 1.f, nn->L, copies(nn), nn->bias, nn->lsum, 0, nn->res);
   cudaMemset(nn->m, 0, sizeof(float) * n);
   cudaMemset(nn->v, 0, sizeof(float) * n);
   return cudaDeviceSynchronize() == cudaSuccess ? MPCD_OK : mfail(nn, MPCD_ERR_CUDA, "parameter upload");
@@ -912,9 +952,10 @@ extern "C" int mpcd_mlp_create(int max_batch, uint64_t seed, mpcd_mlp **out) {
   }
   nn->dO = dalloc<bf16>(nn, B * OUTP);
   nn->Z = dalloc<__nv_bfloat162>(nn, (B + Layers::TM - 1) / Layers::TM * Layers::TM * 3 * (H / 2));
-  nn->max_slices = nn->n_sm / TCW_TILES > 0 ? nn->n_sm / TCW_TILES : 1;
-  nn->part = dalloc<float>(nn, (size_t)nn->max_slices * P);
-  nn->loss = dalloc<double>(nn, (B + Layers::TM - 1) / Layers::TM);
+  nn->max_parts = std::max(1, nn->n_sm / TCW_TILES);
+  nn->part = dalloc<float>(nn, (size_t)nn->max_parts * P);
+  nn->loss = dalloc<float>(nn, B);
+  nn->lsum = dalloc<double>(nn, (B + 255) / 256);
   if (!nn->err.empty()) {
     mpcd_mlp_destroy(nn);
     return MPCD_ERR_NOMEM;
