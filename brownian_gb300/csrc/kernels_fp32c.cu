@@ -191,7 +191,7 @@ static __device__ __forceinline__ float xdet(float a, float b, float c, float d)
 static __device__ __forceinline__ f3 xcross(f3 a, f3 b) {
   return fm(xdet(a.y, b.z, a.z, b.y), xdet(a.z, b.x, a.x, b.z), xdet(a.x, b.y, a.y, b.x));
 }
-static __device__ __forceinline__ void bounce32_draw(const SysF64 &S, long long gs, int j, int id, int part, int cx,
+static __device__ __noinline__ void bounce32_draw(const SysF64 &S, long long gs, int j, int id, int part, int cx,
                                                      int cy, int cz, float ox, float oy, float oz, float vx, float vy,
                                                      float vz, Bounce32 &o) {
   const uint32_t a = (uint32_t)(id + 1), b = (uint32_t)(j + 1), t = (uint32_t)gs;
@@ -1282,6 +1282,7 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
   __shared__ int s_hj[NT];
   __shared__ int s_nh, s_nchk, s_hits, s_fin;
   __shared__ int s_flag[2];
+  __shared__ NearPairs s_pairs;
   const int t = threadIdx.x;
   const int n = S.n_sub;
   if (t == 0) s_nh = s_nchk = s_hits = s_fin = 0;
@@ -1294,7 +1295,7 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
     return;
   }
   if (t >= NT) {
-    near_colloids(S, VB, G, t - NT, 2, &s_flag[1], &s_fin);
+    near_colloids(S, s_pairs, VB, G, t - NT, 2, &s_flag[1], &s_fin);
     return;
   }
   const long long step = S.ss->step, g0 = step * n;
@@ -1505,35 +1506,50 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
           };
           int hits = 0;
           int id = v ? v->id : -1;
-          // the collisions from colloid j on by the general routine
-          auto rest = [&](int j) {
+          if (!v || v->slow) {  // nothing listed: by the general routine
             const NearList q = near_list(S, step, c.lin, false);
-            for (; j >= 0; j = near_next(S, q, j, c, buf ^ 1)) {
+#pragma unroll 1
+            for (int j = near_next(S, q, -1, c, buf ^ 1); j >= 0; j = near_next(S, q, j, c, buf ^ 1)) {
               if (!inside(j)) continue;
               if (id < 0) id = F.id[S.act[a0 + k]];
               ++hits;
               bounce32(S, gs, j, Xq[j], Xo[j], id, vdump, cx, cy, cz, ox, oy, oz, vx, vy, vz);
             }
-          };
-          if (!v || v->slow) {
-            rest(near_next(S, near_list(S, step, c.lin, false), -1, c, buf ^ 1));
           } else {
+            // the listed colloids that hold it, one after another (they are all it can reach: a
+            // displacement beyond the margin fails the step)
             int m = 0, j = -1;
-            for (; m < v->nc; ++m) {
-              j = v->cd[m];
-              if (inside(j)) break;
-            }
-            if (m < v->nc && j != v->jc) {
-              rest(j);
-            } else if (m < v->nc) {
+            auto next = [&] {
+              for (; m < v->nc; ++m) {
+                j = v->cd[m];
+                if (inside(j)) break;
+              }
+            };
+            next();
+#pragma unroll 1
+            while (m < v->nc) {
+              if (j != v->jc) {
+                // not the colloid that was prepared for, or a second sphere (one in a few substeps
+                // somewhere, on one lane, with every block waiting for it): prepared now, by the
+                // instructions that every substep runs
+                v->jc = j;
+#pragma unroll 1
+                for (int part = 0; part < 3; ++part)
+                  bounce32_draw(S, gs, j, id, part, cx, cy, cz, ox, oy, oz, vx, vy, vz, v->b);
+              }
               ++hits;
               f3 dv, dl;
               bounce32_apply(S, j, Xq[j], Xo[j], vdump, v->b, cx, cy, cz, ox, oy, oz, vx, vy, vz, dv, dl);
               const int h = atomicAdd(&s_nh, 1);
-              s_hj[h] = j;
-              s_hx[h][0] = dv.x; s_hx[h][1] = dv.y; s_hx[h][2] = dv.z;
-              s_hx[h][3] = dl.x; s_hx[h][4] = dl.y; s_hx[h][5] = dl.z;
-              if (m + 1 < v->nc) rest(near_next(S, near_list(S, step, c.lin, false), j, c, buf ^ 1));
+              if (h < NT) {
+                s_hj[h] = j;
+                s_hx[h][0] = dv.x; s_hx[h][1] = dv.y; s_hx[h][2] = dv.z;
+                s_hx[h][3] = dl.x; s_hx[h][4] = dl.y; s_hx[h][5] = dl.z;
+              } else {
+                exch_add6(S.exch + j, mk(dv.x, dv.y, dv.z), mk(dl.x, dl.y, dl.z), &S.ss->err);
+              }
+              ++m;
+              next();
             }
           }
           if (hits) {
@@ -1566,7 +1582,7 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
       }
       sync();
       // the round's exchanges, a component per thread
-      const int nh = s_nh;
+      const int nh = min(s_nh, NT);
       for (int q = t; q < 6 * nh; q += NT) exch_add1(S.exch + s_hj[q / 6], q % 6, s_hx[q / 6][q % 6], &S.ss->err);
       sync();
       if (t == 0) {

@@ -1192,15 +1192,25 @@ static __device__ __forceinline__ void near_spheres64(const SysF64 &S, long long
   if (e.jc < 0) e.nc = 0;  // no first collision
 }
 
-// the collisions of a particle from colloid j on (j < 0: from the first), one after another, by
-// the general routine: the rare cases that nothing was prepared for
-static __device__ __noinline__ void near_collide_rest(const SysF64 &S, NearEv &e, int j, long long step, long long gs,
+// the collisions of a particle, one after another, by the general routine: the rare cases that
+// nothing was listed for
+static __device__ __noinline__ void near_collide_rest(const SysF64 &S, NearEv &e, long long step, long long gs,
                                                       int buf) {
   const NearList q = near_list(S, step, e.c.lin, e.c.alias);
-  if (j < 0) j = near_next(S, q, -1, e.c, buf ^ 1);
+  int j = near_next(S, q, -1, e.c, buf ^ 1);
   while (j >= 0) {
     if (within(S, S.X[buf], S.Xf[buf][j], j, e.x, e.y, e.z, S.r_coll, S.sig2q)) ev_collide(S, e, j, gs, buf);
     j = near_next(S, q, j, e.c, buf ^ 1);
+  }
+}
+
+// the same over the colloids listed for it, from number m on: they are all it can reach (a
+// displacement beyond the margin fails the step)
+static __device__ __noinline__ void near_collide_listed(const SysF64 &S, NearEv &e, int m, long long gs, int buf) {
+#pragma unroll 1
+  for (; m < e.nc; ++m) {
+    const int j = e.cd[m];
+    if (within(S, S.X[buf], S.Xf[buf][j], j, e.x, e.y, e.z, S.r_coll, S.sig2q)) ev_collide(S, e, j, gs, buf);
   }
 }
 
@@ -1269,6 +1279,7 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
   __shared__ int s_hj[NT];
   __shared__ int s_nh, s_np, s_fin;
   __shared__ int s_flag[2];
+  __shared__ NearPairs s_pairs;
   const int t = threadIdx.x, VB = blockIdx.x, G = gridDim.x;
   const int n = S.n_sub;
   if (t == 0) s_np = s_nh = s_fin = 0;
@@ -1281,7 +1292,7 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
     return;
   }
   if (t >= NT) {
-    near_colloids(S, VB, G, t - NT, 2, &s_flag[1], &s_fin);
+    near_colloids(S, s_pairs, VB, G, t - NT, 2, &s_flag[1], &s_fin);
     return;
   }
   const long long step = S.ss->step, g0 = step * n;
@@ -1377,7 +1388,7 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
       if (k < NEAR64_ACT) sm.cand[k] = NEAR_GONE;
     };
     // The active ones, two at a time and without a branch where they stay inside the box (so the
-    // additions need no mod) and have one candidate, which is not near: about 60 instructions
+    // additions need no mod) and have one or two candidates, which are not near: about 75 instructions
     // each, interleaved.  Everything else takes the general path.
     const int kept = min(cnt, NEAR64_ACT);
     for (int k0 = t; k0 < kept; k0 += 2 * NT) {
@@ -1388,9 +1399,10 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
       for (int u = 0; u < 2; ++u) {
         const int k = min(k0 + u * NT, kept - 1);
         cand[u] = k0 + u * NT < kept ? sm.cand[k] : NEAR_GONE;
-        const NearCol64 &o = sm.col.d[min(cand[u] & 0xFFFFu, (unsigned)(NearCols<NearCol64>::MAX - 1))];
-        float d2 = 0.f;
-        far[u] = (cand[u] >> 16) == 0xFFFFu;
+        const unsigned top = NearCols<NearCol64>::MAX - 1, j2 = cand[u] >> 16;
+        const float4 o = sm.col.d[min(cand[u] & 0xFFFFu, top)].x, o2 = sm.col.d[min(j2, top)].x;
+        float d2 = 0.f, e2 = 0.f;
+        far[u] = j2 - (NEAR_STALE >> 16) > 2u;  // (none of the marks)
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           const Dim &D = a == 0 ? S.dx : (a == 1 ? S.dy : S.dz);
@@ -1398,10 +1410,13 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
           x[u][a] = __dadd_rn(sm.st[a][k], sm.st[3 + a][k]);
           const long long b = dbits(x[u][a]);
           far[u] = far[u] && b >= D.lo_bits && b < D.L_bits;
-          const float d = wrap_half((a == 0 ? o.x.x : a == 1 ? o.x.y : o.x.z) - d2f_box(x[u][a]), L);
+          const float f = d2f_box(x[u][a]), d = wrap_half((a == 0 ? o.x : a == 1 ? o.y : o.z) - f, L),
+                      e = wrap_half((a == 0 ? o2.x : a == 1 ? o2.y : o2.z) - f, L);
           d2 = a == 0 ? d * d : fmaf(d, d, d2);
+          e2 = a == 0 ? e * e : fmaf(e, e, e2);
         }
-        far[u] = far[u] && d2 > (ch + 1e-4f) * (ch + 1e-4f);  // (the general path's rounding may differ)
+        const float lim = (ch + 1e-4f) * (ch + 1e-4f);  // (the general path's rounding may differ)
+        far[u] = far[u] && d2 > lim && (j2 == 0xFFFFu || e2 > lim);
       }
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
@@ -1519,7 +1534,7 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
       if (i < np) {
         e = &ev(i);
         if (e->slow) {
-          near_collide_rest(S, *e, -1, step, gs, buf);
+          near_collide_rest(S, *e, step, gs, buf);
           if (e->dumped) e->cand = NEAR_STALE;
         } else if (e->nc > 0) {
           int j = -1, c = 0;
@@ -1530,7 +1545,7 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
             if (within(S, S.X[buf], S.Xf[buf][j], j, e->x, e->y, e->z, S.r_coll, S.sig2q)) break;
           }
           if (c < e->nc && j != e->jc) {
-            near_collide_rest(S, *e, j, step, gs, buf);  // (not the colloid that was prepared for)
+            near_collide_listed(S, *e, c, gs, buf);  // (not the colloid that was prepared for)
             if (e->dumped) e->cand = NEAR_STALE;
           } else if (c < e->nc) {
             hit = true;
@@ -1552,8 +1567,7 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
             if (c + 1 < e->nc) {  // a second sphere may hold it now
               settle();
               hit = false;
-              near_collide_rest(S, *e, near_next(S, near_list(S, step, e->c.lin, e->c.alias), j, e->c, buf ^ 1), step,
-                                gs, buf);
+              near_collide_listed(S, *e, c + 1, gs, buf);
             }
           }
         }
