@@ -337,7 +337,7 @@ static bool sorts_at(const mpcd_ctx *c, long long step) { return c->sort_every >
 static void enq_rotation(mpcd_ctx *c, bool sort) {
   const SysF64 &S = c->S;
   const bool f32 = S.precision == MPCD_FP32C;
-  launch(c, "k_cell_prep", f32 ? k_cell_prep32 : k_cell_prep, prep_blocks(S), 256, S);
+  launch(c, "k_cell_prep", f32 ? k_cell_prep32 : k_cell_prep, prep_blocks(S), 256, S, sort ? 1 : 0);
   if (sort) {
     launch(c, "k_scan_blocks", k_scan_blocks, 1, 1024, S, c->nblk);
     launch(c, "k_rotate_sort", f32 ? k_rotate_sort32 : k_rotate_sort, blocks_for(S.N, 256), 256, S, c->fbuf,
@@ -381,7 +381,7 @@ static void enq_rotation_run(mpcd_ctx *c, bool sort) {
   cudaEventRecord(c->ev_join, c->aux);
   const SysF64 &S = c->S;
   const bool f32 = S.precision == MPCD_FP32C;
-  launch(c, "k_cell_prep", f32 ? k_cell_prep32 : k_cell_prep, prep_blocks(S), 256, S);
+  launch(c, "k_cell_prep", f32 ? k_cell_prep32 : k_cell_prep, prep_blocks(S), 256, S, sort ? 1 : 0);
   if (sort) {
     cudaStreamWaitEvent(c->stream, c->ev_join, 0);
     launch(c, "k_scan_blocks", k_scan_blocks, 1, 1024, S, c->nblk);
@@ -495,7 +495,7 @@ static void enq_step_flight32(mpcd_ctx *c, bool sort) {
   }
   if (S.Nc > 0) enq_run_shell(c, c->aux, c->fbuf);
   cudaEventRecord(c->ev_join, c->aux);
-  launch(c, "k_cell_prep", k_cell_prep32, prep_blocks(S), 256, S);
+  launch(c, "k_cell_prep", k_cell_prep32, prep_blocks(S), 256, S, sort ? 1 : 0);
   if (sort) enq_sort_scatter(c);
   cudaStreamWaitEvent(c->stream, c->ev_tab, 0);
   launch(c, "k_rotate_classify", classify_kernel32(!sort, false), blocks_for(S.N, 256 * CLASSIFY32_U), 256, S, c->fbuf);
@@ -531,7 +531,7 @@ static void enq_step_flight64(mpcd_ctx *c, bool sort) {
   }
   if (nc) enq_run_shell(c, c->aux, c->fbuf);
   cudaEventRecord(c->ev_join, c->aux);
-  launch(c, "k_cell_prep", k_cell_prep, prep_blocks(S), 256, S);
+  launch(c, "k_cell_prep", k_cell_prep, prep_blocks(S), 256, S, sort ? 1 : 0);
   if (sort) enq_sort_scatter(c);
   cudaStreamWaitEvent(c->stream, c->ev_tab, 0);
   launch(c, "k_rotate_classify", classify_kernel(!sort, false), blocks_for(S.N, 256), 256, S, c->fbuf);
@@ -600,7 +600,7 @@ static void enq_step_near(mpcd_ctx *c, bool sort) {
               M_KICK | M_ADVANCE | M_FLIGHT, 0);
   }
   cudaEventRecord(c->ev_aux, c->aux);
-  launch(c, "k_cell_prep", f32 ? k_cell_prep32 : k_cell_prep, prep_blocks(S), 256, S);
+  launch(c, "k_cell_prep", f32 ? k_cell_prep32 : k_cell_prep, prep_blocks(S), 256, S, sort ? 1 : 0);
   if (sort) enq_sort_scatter(c);
   cudaStreamWaitEvent(c->stream, c->ev_tab, 0);
   launch(c, "k_rotate_classify", f32 ? classify_kernel32(!sort, true) : classify_kernel(!sort, true),

@@ -60,6 +60,28 @@ static __device__ __forceinline__ int cell_of_pos(const SysF64 &S, double x, dou
   return lin_cell(S, ix, iy, iz);
 }
 
+// The sums of the block's 256 cells (from cell c0 on) into shared memory, and zeros in their place: in
+// consecutive words, where a thread per 40-byte record spreads each access over ten lines.  (The FP32
+// form's cell pass, with the prefix left out of steps that do not sort: 128^3 cells 184 -> 139 us, 64^3
+// 26 -> 17 us.  The FP64 form's is bound by its FP64 unit, and the shared memory this would take kept
+// the side stream's kernels off its SMs: 53x37x41 cells 344 -> 355 us a step.)
+static __device__ __forceinline__ void take_cells(const SysF64 &S, int c0, CellAcc *cells) {
+  constexpr int W = (int)(sizeof(CellAcc) / sizeof(unsigned long long));
+  static_assert(sizeof(CellAcc) % sizeof(unsigned long long) == 0, "whole words");
+  unsigned long long *from = reinterpret_cast<unsigned long long *>(S.acc + c0);
+  unsigned long long *to = reinterpret_cast<unsigned long long *>(cells);
+  const int words = min(256, S.Cpad - c0) * W;
+#pragma unroll
+  for (int k = 0; k < W; ++k) {
+    const int i = (int)threadIdx.x + 256 * k;
+    if (i < words) {
+      to[i] = from[i];
+      from[i] = 0ull;
+    }
+  }
+  __syncthreads();
+}
+
 // Base index in a shared list for the lanes in mask m of this warp, from one
 // global atomic per block (the whole block must call it): for the run() records
 // of a last substep, about one particle in sixteen, too many for one atomic per
@@ -74,6 +96,29 @@ static __device__ __forceinline__ int block_base_n(int *counter, int warp_count,
   if (threadIdx.x == 0) s_base = s_tot ? atomicAdd(counter, s_tot) : 0;
   __syncthreads();
   return s_base + __shfl_sync(FULL, off, 0);
+}
+
+// the same for two lists whose counters are the halves of one word (*a the base of the first,
+// low one): one round trip to L2 for both, where a block of the classification spends about a sixth of
+// its time on each (128^3 FP32 358 -> 322 us, 64^3 FP64 77 -> 72 us)
+static __device__ __forceinline__ void block_base2(int *counters, int warp_a, int warp_b, int lane, int *a, int *b) {
+  __shared__ int s_tot[2], s_base[2];
+  if (threadIdx.x < 2) s_tot[threadIdx.x] = 0;
+  __syncthreads();
+  int oa = 0, ob = 0;
+  if (lane == 0 && warp_a) oa = atomicAdd(&s_tot[0], warp_a);
+  if (lane == 0 && warp_b) ob = atomicAdd(&s_tot[1], warp_b);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_tot[0] + s_tot[1]) {
+    const unsigned long long was =
+        atomicAdd(reinterpret_cast<unsigned long long *>(counters),
+                  (unsigned long long)(unsigned)s_tot[0] | (unsigned long long)(unsigned)s_tot[1] << 32);
+    s_base[0] = (int)(unsigned)was;
+    s_base[1] = (int)(unsigned)(was >> 32);
+  }
+  __syncthreads();
+  *a = s_base[0] + __shfl_sync(FULL, oa, 0);
+  *b = s_base[1] + __shfl_sync(FULL, ob, 0);
 }
 
 static __device__ __forceinline__ int block_base(int *counter, unsigned m, int lane) {

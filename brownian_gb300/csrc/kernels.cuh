@@ -18,7 +18,7 @@ using StreamKernelB = void (*)(const SysF64 *, const int *, int, int, int);
 using EventKernelB = void (*)(const SysF64 *, const int *, int, int, int);
 StreamKernelB stream_kernel32_b(int flags);
 EventKernelB event_kernel32_b(int flags);
-__global__ void k_cell_prep32_b(const SysF64 *Ss, const int *boff, int nrep);
+__global__ void k_cell_prep32_b(const SysF64 *Ss, const int *boff, int nrep, int sort);
 __global__ void k_rotate32_b(const SysF64 *Ss, const int *boff, int nrep, int fb);
 __global__ void k_rotate_sort32_b(const SysF64 *Ss, const int *boff, int nrep, int src, int dst);
 __global__ void k_run_shell32_b(const SysF64 *Ss, const int *boff, int nrep, int fb);
@@ -37,7 +37,7 @@ __global__ void k_updown_table(const SysF64 S, unsigned long long *Tc, uint16_t 
 __global__ void k_updown(const SysF64 S, int fb, const unsigned long long *Tc, const uint16_t *Tl, long long epoch,
                          double rup2, int *cnt, ExchAcc *acc);
 EventKernel event_kernel32(int flags);
-__global__ void k_cell_prep32(__grid_constant__ const SysF64 S);
+__global__ void k_cell_prep32(__grid_constant__ const SysF64 S, int sort);
 __global__ void k_rotate32(__grid_constant__ const SysF64 S, int fb);
 __global__ void k_rotate_sort32(__grid_constant__ const SysF64 S, int src, int dst);
 // the FP32 free-flight schedule: flight table, rotation with the classification, the free
@@ -81,7 +81,8 @@ __global__ void k_run_shell32(__grid_constant__ const SysF64 S, int fb);
 __global__ void k_run_kick32(__grid_constant__ const SysF64 S, int fb, int split);
 __global__ void k_aos_to_q(const SysF64 S, const double *pos, const double *vel, int fb);
 __global__ void k_q_to_aos(const SysF64 S, double *pos, double *vel, int fb);
-__global__ void k_cell_prep(const SysF64 S);
+// (sort: the step sorts, and the counting sort's prefix is wanted)
+__global__ void k_cell_prep(const SysF64 S, int sort);
 __global__ void k_scan_blocks(__grid_constant__ const SysF64 S, int nblk);
 __global__ void k_rotate_sort(const SysF64 S, int src, int dst);
 __global__ void k_rotate(const SysF64 S, int fb);

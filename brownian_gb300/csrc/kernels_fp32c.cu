@@ -615,7 +615,7 @@ static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S,
     unpack(qq[u], cx, cy, cz, ox, oy, oz);
     const bool inb = cx < S.Lx && cy < S.Ly && cz < S.Lz;  // (a record within the box)
     const FlightCell *fc = S.ftab + (inb ? cx + S.Lx * (cy + S.Ly * cz) : 0);
-    const uint4 w0 = reinterpret_cast<const uint4 *>(fc)[0], w1 = reinterpret_cast<const uint4 *>(fc)[1];
+    const uint4 w0 = reinterpret_cast<const uint4 *>(fc)[0];
     if (ROT) {
       if (cc[u] < S.C) apply_map32(S.cell_ab32 + (size_t)cc[u] * 12, vx[u], vy[u], vz[u]);
       F.vx[p] = vx[u]; F.vy[p] = vy[u]; F.vz[p] = vz[u];
@@ -629,6 +629,8 @@ static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S,
     } else if (cnt > 0) {
       const float rad = near_radius(S, S.ss->cm, S.n_sub), T = (float)S.n_sub * S.dtf;
       const float r = S.r_shell + travel + (float)S.n_sub * S.ss->cm + 0.01f, r2 = r * r;
+      // (four ids lie in the first half of the record)
+      const uint4 w1 = cnt > 4 ? reinterpret_cast<const uint4 *>(fc)[1] : make_uint4(0, 0, 0, 0);
       const unsigned ids[6] = {w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
       const float4 *Xq = S.Xcq[b0], *Xo = S.Xco[b0];
       for (int k = 0; k < cnt; ++k) {
@@ -655,27 +657,29 @@ static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S,
     m[u] = __ballot_sync(FULL, near[u]);
     tot += __popc(m[u]);
   }
-  int base = block_base_n(&S.ss->nnear, tot, lane);
+  int base, ba = 0;
+  unsigned ma[U];
+  if (SPLIT) {
+    int tota = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      ma[u] = __ballot_sync(FULL, cand[u] != NEAR_NONE);
+      tota += __popc(ma[u]);
+    }
+    block_base2(&S.ss->nnear, tot, tota, lane, &base, &ba);
+  } else {
+    base = block_base_n(&S.ss->nnear, tot, lane);
+  }
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     if (near[u]) S.near[base + __popc(m[u] & lt)] = pp[u];
     base += __popc(m[u]);
-  }
-  if (!SPLIT) return;
-  tot = 0;
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    m[u] = __ballot_sync(FULL, cand[u] != NEAR_NONE);
-    tot += __popc(m[u]);
-  }
-  base = block_base_n(&S.ss->nact, tot, lane);
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
+    if (!SPLIT) continue;
     if (cand[u] != NEAR_NONE) {
-      S.act[base + __popc(m[u] & lt)] = pp[u];
-      S.actc[base + __popc(m[u] & lt)] = cand[u];
+      S.act[ba + __popc(ma[u] & lt)] = pp[u];
+      S.actc[ba + __popc(ma[u] & lt)] = cand[u];
     }
-    base += __popc(m[u]);
+    ba += __popc(ma[u]);
   }
 }
 
@@ -951,15 +955,16 @@ EventKernelB event_kernel32_b(int flags) {
 // SRD collision per cell (cpp/rotation_mpcd.cpp:14-49): cell mean from the exact
 // sums, thermostat factor in FP64, rotation about the random axis in FP32, stored
 // as the FP32 affine map v' = A v + b; plus the occupancy prefix of the counting sort.
-static __device__ __forceinline__ void k_cell_prep32_body(const SysF64 &S, const int VB, const int NVB) {
+static __device__ __forceinline__ void k_cell_prep32_body(const SysF64 &S, const int VB, int sort) {
   const int c = VB * blockDim.x + threadIdx.x;
+  __shared__ __align__(16) CellAcc cells[256];
+  take_cells(S, VB * 256, cells);
   CellAcc a = CellAcc{0, 0, 0, 0, 0, 0};
   if (c < S.Cpad) {
-    a = S.acc[c];
-    S.acc[c] = CellAcc{0, 0, 0, 0, 0, 0};
-    S.cursor[c] = 0;
+    a = cells[threadIdx.x];
+    if (sort) S.cursor[c] = 0;
   }
-  {
+  if (sort) {
     __shared__ int wsum[8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int v = a.n, incl = v;
@@ -1020,14 +1025,14 @@ static __device__ __forceinline__ void k_cell_prep32_body(const SysF64 &S, const
   ab4[2] = make_float4(A[8], b0, b1, b2);
 }
 
-__global__ void __launch_bounds__(256) k_cell_prep32(__grid_constant__ const SysF64 S) {
-  k_cell_prep32_body(S, blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(256) k_cell_prep32(__grid_constant__ const SysF64 S, int sort) {
+  k_cell_prep32_body(S, blockIdx.x, sort);
 }
 
 // the same over a batch of systems (persistent: batch_for)
-__global__ void __launch_bounds__(256) k_cell_prep32_b(const SysF64 *Ss, const int *boff, int nrep) {
+__global__ void __launch_bounds__(256) k_cell_prep32_b(const SysF64 *Ss, const int *boff, int nrep, int sort) {
   __shared__ SysF64 sS;
-  batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_cell_prep32_body(sS, VB, NVB); });
+  batch_for(Ss, boff, nrep, sS, [&](int VB, int) { k_cell_prep32_body(sS, VB, sort); });
 }
 
 static __device__ __forceinline__ void k_rotate32_body(const SysF64 &S, const int VB, const int NVB, int fb) {

@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(256) k_rotate_classify(const SysF64 S, int fb)
     // a position outside the box (a state that is not finite) reads no table: near
     const bool inb = cx >= 0 && cx < S.Lx && cy >= 0 && cy < S.Ly && cz >= 0 && cz < S.Lz;
     const FlightCell *fc = S.ftab + (inb ? cx + S.Lx * (cy + S.Ly * cz) : 0);
-    const uint4 w0 = reinterpret_cast<const uint4 *>(fc)[0], w1 = reinterpret_cast<const uint4 *>(fc)[1];
+    const uint4 w0 = reinterpret_cast<const uint4 *>(fc)[0];
     if (c < S.C) {
       const double2 *ab = reinterpret_cast<const double2 *>(S.cell_ab + (size_t)c * 12);
       double2 a01 = ab[0], a23 = ab[1], a45 = ab[2], a67 = ab[3], a8b0 = ab[4], b12 = ab[5];
@@ -445,6 +445,8 @@ __global__ void __launch_bounds__(256) k_rotate_classify(const SysF64 S, int fb)
     } else if (cnt > 0) {
       const float r = S.r_shell + travel + (float)S.n_sub * S.ss->cm + 0.01f, r2 = r * r;
       const float rad = near_radius(S, S.ss->cm, S.n_sub), fn = (float)S.n_sub;
+      // (four ids lie in the first half of the record)
+      const uint4 w1 = cnt > 4 ? reinterpret_cast<const uint4 *>(fc)[1] : make_uint4(0, 0, 0, 0);
       const unsigned ids[6] = {w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
       const float4 *Xf = S.Xf[b0];
       for (int k = 0; k < cnt; ++k) {
@@ -461,17 +463,20 @@ __global__ void __launch_bounds__(256) k_rotate_classify(const SysF64 S, int fb)
   }
   const int lane = threadIdx.x & 31;
   const unsigned m = __ballot_sync(FULL, near);
-  const int base = block_base_n(&S.ss->nnear, __popc(m), lane);
-  if (near) S.near[base + __popc(m & ((1u << lane) - 1u))] = p;
+  const unsigned lt = (1u << lane) - 1u;
+  int base, ba;
   if (SPLIT) {
     const bool active = cand != NEAR_NONE;
     const unsigned ma = __ballot_sync(FULL, active);
-    const int ba = block_base_n(&S.ss->nact, __popc(ma), lane) + __popc(ma & ((1u << lane) - 1u));
+    block_base2(&S.ss->nnear, __popc(m), __popc(ma), lane, &base, &ba);
     if (active) {
-      S.act[ba] = p;
-      S.actc[ba] = cand;
+      S.act[ba + __popc(ma & lt)] = p;
+      S.actc[ba + __popc(ma & lt)] = cand;
     }
+  } else {
+    base = block_base_n(&S.ss->nnear, __popc(m), lane);
   }
+  if (near) S.near[base + __popc(m & lt)] = p;
 }
 
 // n substeps of update_pos_mpcd along one axis for a free particle: x = mod(x + w, L) n
@@ -641,17 +646,17 @@ EventKernel event_kernel(int flags) {
 // cell's random axis (rho, phi), s the thermostat factor; the variance the
 // reference computes after rotating equals sum|w - u|^2 = S2 - n|u|^2 before.
 // Consumes (and clears) the exact sums k_stream accumulated.
-__global__ void __launch_bounds__(256) k_cell_prep(const SysF64 S) {
+__global__ void __launch_bounds__(256) k_cell_prep(const SysF64 S, int sort) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   CellAcc a = CellAcc{0, 0, 0, 0, 0, 0};
   if (c < S.Cpad) {
     a = S.acc[c];
     S.acc[c] = CellAcc{0, 0, 0, 0, 0, 0};
-    S.cursor[c] = 0;
+    if (sort) S.cursor[c] = 0;
   }
   // counting sort, first half: exclusive prefix of the occupancy within this block
   // of 256 cells, and the block's total
-  {
+  if (sort) {
     __shared__ int wsum[8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int v = a.n, incl = v;

@@ -70,9 +70,11 @@ struct StepState {
   // free-flight classification as the colloids' move over the step (n_sub cm)
   float cm;
   double cm2;
-  int nnear;        // free-flight schedule: particles listed for the near passes this step
+  // free-flight schedule: particles listed for the near passes this step, and of those whose path
+  // may meet a sphere (one word: the classification counts both with one atomic)
+  alignas(8) int nnear;
+  int nact;
   double rrn[3];    // free-flight schedule: the next step's grid shift (the free pass bins with it)
-  int nact;         // free-flight schedule: particles whose path may meet a sphere this step
   float cm_f;       // this step's cm and step number, for the end of the step, whose first block
   long long step_f; // sets the next step's while the others still record run() candidates
   long long crowd;  // step + 1 if some flight cell lists more colloids than a cell table holds
