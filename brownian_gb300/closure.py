@@ -477,8 +477,8 @@ def demo(colloids=500, fraction=0.1, steps=30, seed=5):
 
 def train_demo(batch=8192, steps=20, seed=0):
     """Training steps of the network on random data of `batch` rows (timing and profiling of
-    the training kernels): ms per step by CUDA events, and the FLOP rate of the layer products
-    that run on the tcgen05 path (forward and backward data: 2 x batch x 589,824 FLOP a step)."""
+    the training kernels): ms per step by CUDA events, and the FLOP of the layer products (forward
+    and backward data: 2 x batch x 589,824 FLOP a step)."""
     import torch
     rng = np.random.default_rng(seed)
     x = torch.from_numpy(rng.normal(0, 1, (batch, IN)).astype(np.float32)).cuda()

@@ -1202,7 +1202,7 @@ __global__ void k_run_kick32_b(const SysF64 *Ss, const int *boff, int nrep, int 
 
 // ------------------------------------------------- active particles' substeps (FP32 form)
 
-constexpr int NEAR32_ACT = 3584, NEAR32_CHK = 128, NEAR32_IDX = 1024;
+constexpr int NEAR32_CHK = 128, NEAR32_IDX = 1024;
 
 // what the tests need of a colloid
 struct __align__(16) NearCol32 {
