@@ -44,22 +44,22 @@ L, DENSITY, NC, RADIUS = 64, 10, 500, 2.0
 # the cell+offset record and the velocity (28 B) and writes the record and the cell (20 B).
 FREE_BYTES = {"fp64": 76, "fp32c": 48}
 # one MPCD step in that schedule, with a fraction f of near particles (density 10, per-cell
-# data per particle):
+# data per particle), every near one counted as active (taken through the substeps, its state
+# read and written once a step; the near ones that no sphere can reach are streamed by the free pass):
 #   FP64: rotation + classification 77 (rotcell 4, w 24 read and 24 written, x 24, flag 1)
 #         + SRD map 9.6 + flight table 3.2; free pass 1 + 76 (1 - f); cell pass 13.6 and the
-#         binning's cell sums 4; near passes 10 x 77 f (index 4, x and w 48, pending mark 1,
-#         x written 24) + near binning 57 f + list 4 f
+#         binning's cell sums 4; lists 12 f, substeps 80 f (list entry 8, x and w 48, x written 24),
+#         end of step 53 f (index 4, flag 1, x and w 48)
 #   FP32: rotation + classification 45 (rotcell 4, v 12 read and 12 written, record 16, flag 1)
-#         + map 4.8 + table 3.2; free pass 1 + 48 (1 - f); cell pass 8.8, cell sums 4; near
-#         passes 10 x 48 f (index 4, record 16 read and written, velocity 12) + 4 f + list 4 f
-#   (the near binning of the FP32 form is part of its last near pass)
-#   (with n substeps the near passes count n times: b = 77 n - 15 and 48 (n - 1) + 8)
+#         + map 4.8 + table 3.2; free pass 1 + 48 (1 - f); cell pass 8.8, cell sums 4; lists 12 f,
+#         substeps 52 f (list entry 8, record 16 read and written, velocity 12), end of step 41 f
+#         (index 4, flag 1, record 16, velocity 12, id 4, cell 4)
 STEP_BYTES_FLIGHT = {"fp64": 184.4, "fp32c": 114.8}
+NEAR_BYTES = {"fp64": 12.0 + 80.0 + 53.0 - 76.0, "fp32c": 12.0 + 52.0 + 41.0 - 48.0}
 
 
-def step_bytes(precision, near_frac, n_sub=10):
-    b = 77.0 * n_sub - 15.0 if precision == "fp64" else 48.0 * (n_sub - 1) + 8.0
-    return STEP_BYTES_FLIGHT[precision] + b * near_frac
+def step_bytes(precision, near_frac):
+    return STEP_BYTES_FLIGHT[precision] + NEAR_BYTES[precision] * near_frac
 
 
 def workload(seed=0):
@@ -526,11 +526,11 @@ def run_large(steps, warmup=3):
     peak = measured_peak_hbm()[0]
     # algorithmic bytes per fluid particle, FP32 form (the free-flight pass: the flag of every
     # particle and the free particles' record, velocity, record and cell; the cell pass: 88 B per
-    # cell at density 10; a near pass: index, record read and written, velocity of the near
-    # particles)
+    # cell at density 10; the substeps' kernel: list entry, record read and written, velocity of the
+    # near particles, once a step)
     per_particle = {"k_stream": 44, "k_rotate": 28, "k_rotate_sort": 64, "k_rotate_classify": 45,
                     "k_free_flight": 1.0 + (1.0 - near_frac) * FREE_BYTES["fp32c"], "k_cell_prep": 8.8,
-                    "k_stream_near": 48.0 * near_frac}
+                    "k_stream_near": 52.0 * near_frac}
     kernels = {}
     for k, (n, tms) in sorted(prof.items(), key=lambda kv: -kv[1][1]):
         us = tms / max(n, 1) * 1e3
@@ -541,7 +541,7 @@ def run_large(steps, warmup=3):
                         "frac_of_measured_copy": gbs / peak})
         kernels[k] = row
     sim.close()
-    b_step = step_bytes("fp32c", near_frac, NSUB)
+    b_step = step_bytes("fp32c", near_frac)
     ps = N / (ms / 1e3)
     return {"workload": "128^3 cells, density 10 (20,971,520 fluid particles), 2000 colloids r=3 (WCA sigma 6), "
                         "v0 0.02, Dr 0.0005, SRD angle 130 deg, 20 substeps; FP32 form",
