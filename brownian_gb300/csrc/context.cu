@@ -619,7 +619,9 @@ static void enq_step_near(mpcd_ctx *c, bool sort) {
   cudaEventRecord(c->ev_free, c->nst);
   cudaStreamWaitEvent(c->stream, c->ev_end, 0);
   cudaStreamWaitEvent(c->stream, c->ev_free, 0);
-  launch(c, "k_end_step", f32 ? k_end_flight32 : k_end_flight64, 1 + c->n_sm * 8, 256, S, c->fbuf);
+  // (as many blocks as are resident at once, 40 and 63 registers a thread: with eight an SM the second
+  // wave was a third full, 128^3 FP32 110 us against 83)
+  launch(c, "k_end_step", f32 ? k_end_flight32 : k_end_flight64, c->n_sm * (f32 ? 6 : 4), 256, S, c->fbuf);
 }
 
 // the cell table of the next step's first substep, for the schedules that read one, after a

@@ -1656,13 +1656,16 @@ static __device__ __forceinline__ void k_end_flight32_body(const SysF64 &S, cons
   const Fluid32 F = fluid32_at(S, fb);
   const float rr[3] = {(float)S.ss->rrn[0], (float)S.ss->rrn[1], (float)S.ss->rrn[2]};
   const int count = min(S.ss->nnear, S.N), lane = threadIdx.x & 31;
-  for (int base = (VB - 1) * 256; base < count; base += (NVB - 1) * 256) {
-    const int i = base + threadIdx.x;
+  const int stride = (NVB - 1) * 256;
+  int i = (VB - 1) * 256 + threadIdx.x;
+  int next = i < count ? S.near[i] : 0;
+  for (int base = (VB - 1) * 256; base < count; base += stride, i += stride) {
     ShellRec rec;
     rec.n = 0;
     BinTerm32 b{-1, 0, 0, 0, 0};
+    const int p = next;
+    if (i + stride < count) next = S.near[i + stride];
     if (i < count) {
-      const int p = S.near[i];
       const uint8_t fn = S.fnear[p];
       if (fn != FN_DONE) {
         int cx, cy, cz;

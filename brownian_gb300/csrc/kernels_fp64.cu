@@ -1664,14 +1664,17 @@ __global__ void __launch_bounds__(256) k_end_flight64(__grid_constant__ const Sy
   const int buf = (int)((step * S.n_sub + S.n_sub - 1) & 1);
   const Fluid F = fluid_at(S, fb);
   const int count = min(S.ss->nnear, S.N), lane = threadIdx.x & 31;
-  for (int base = (blockIdx.x - 1) * 256; base < count; base += (gridDim.x - 1) * 256) {
-    const int i = base + threadIdx.x;
+  const int stride = (gridDim.x - 1) * 256;
+  int i = (blockIdx.x - 1) * 256 + threadIdx.x;
+  int next = i < count ? S.near[i] : 0;
+  for (int base = (blockIdx.x - 1) * 256; base < count; base += stride, i += stride) {
     ShellRec rec;
     rec.n = 0;
     bool band = false;
     BinTerm b{-1, 0, 0, 0, 0};
+    const int p = next;
+    if (i + stride < count) next = S.near[i + stride];
     if (i < count) {
-      const int p = S.near[i];
       const uint8_t fn = S.fnear[p];
       if (fn != FN_DONE) {
         const double x = F.x[p], y = F.y[p], z = F.z[p];
