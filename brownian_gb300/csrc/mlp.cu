@@ -9,14 +9,13 @@
 // a colloid's per-step momentum and angular-momentum exchange with the fluid,
 // trained by the Gaussian negative log-likelihood.
 //
-// Inference (mpcd_mlp_forward) keeps a tile of rows on its SM through all layers, one kernel (k_mlp_infer) of
-// warp-level products, whose arithmetic the colloid-only step's network reproduces bit for bit.  A
-// training step runs its products on the 5th-generation tensor cores (tcgen05.mma with the accumulator
-// in tensor memory, TMEM): a launch for each layer's product forward and backward (k_gemm_tc), one for all
-// weight gradients, a reduction over the batch (k_gemm_tc_wgrad), and Adam (k_adam).
+// Training runs its products on the 5th-generation tensor cores (tcgen05.mma with the
+// accumulator in tensor memory, TMEM): the layer products (forward x W and backward dZ W^T, K and N
+// <= 256) on k_gemm_tc, the weight gradients (a reduction over the batch) on k_gemm_tc_wgrad.
+// Inference (mpcd_mlp_forward) is one kernel over all layers (k_mlp_infer) on warp-level products,
+// whose arithmetic the colloid-only step's network reproduces bit for bit.
 #include <cuda_bf16.h>
 
-#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -38,6 +37,27 @@ constexpr int IN = MPCD_MLP_IN, INP = MLP_IN_PADDED, H = MPCD_MLP_HIDDEN, OUT = 
 constexpr float kLogVarClamp = MLP_LOGVAR_CLAMP;
 constexpr float kInputClip = MLP_INPUT_CLIP;
 
+struct Gemm {
+  const bf16 *A;
+  long long sam, sak;
+  const bf16 *B;
+  long long sbk, sbn;
+  int M, N, K;
+  const float *bias;   // [N] or null
+  int silu;            // apply SiLU after the bias
+  const bf16 *dz;      // backward: multiply by silu'(dz[m, n]) (the layer's pre-activation)
+  long long lddz;
+  float *Cf;           // FP32 store
+  long long ldcf;
+  bf16 *Cb;            // BF16 store (after the activation)
+  long long ldcb;
+  bf16 *Zb;            // BF16 store of the pre-activation
+  long long ldzb;
+  float *Cacc;         // FP32 atomic accumulation
+  long long ldca;
+  int kchunk;          // K range of one blockIdx.z
+};
+
 // the logistic function, branch free (fast reciprocal: within 2 ulp, and 0 once e^-z overflows);
 // the colloid-only step evaluates the network with the same arithmetic
 __device__ __forceinline__ float sigm(float z) { return __fdividef(1.f, 1.f + __expf(-z)); }
@@ -50,8 +70,19 @@ __device__ __forceinline__ void mma_bf16(float c[4], const uint32_t a[4], const 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// ------------------------------------------------------------- tcgen05
-
+// ------------------------------------------------------------- tcgen05 products
+//
+// C[M x N] = A[M x K] B[K x N] for A with K contiguous (sak = 1) and B with K contiguous
+// (sbk = 1: B(k, n) at B[n sbn + k]), N and K multiples of 16 up to 256.  One CTA of four
+// warps per 128 rows and column tile (all N, or halves of it when the rows alone would leave
+// SMs idle): the A tile (128 x K) and the B tile (N x K) staged in shared memory in
+// the canonical K-major layout without swizzle (core matrices of 8 rows x 16 bytes, the K
+// direction LBO = 128 bytes apart, 8-row groups SBO = K/8 x 128 bytes apart), K/16
+// tcgen05.mma (kind::f16, BF16 x BF16 -> FP32, M = 128) issued by one thread into a TMEM
+// accumulator of 128 lanes x N columns, their completion signalled on an mbarrier
+// (tcgen05.commit) and waited for with a time limit (a wait that runs out sets *err and
+// skips the epilogue); then each warp reads its 32 TMEM lanes (rows) 16 columns at a time
+// (tcgen05.ld) into the epilogue.
 constexpr int TC_M = 128;
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -85,219 +116,6 @@ __device__ __forceinline__ bool tc_wait_bounded(uint32_t bar, uint32_t parity) {
   }
   return false;
 }
-
-// ------------------------------------------------------------------ inference
-//
-// The whole network for TM = 16 MT WM rows per CTA of eight warps (WM along the rows, 8 / WM
-// along the columns): normalisation, the four layers with the activations in shared memory, the
-// outputs in physical units, in one launch.  The weights stream from L2 through three stages
-// of 32 k rows by asynchronous copies, the next layer's first stages while this one's epilogue runs.
-// Each output element is K steps of 16 in ascending order into one FP32 accumulator, bias, SiLU and
-// the BF16 rounding between layers, as in the colloid-only step's network, whose bits these are.
-// Bound: L2 reads of the weights (311 KB a CTA) and the SiLU's two special-function operations
-// per element.  Measured, six launches with the activations through memory -> this: 16,384 rows
-// 197 -> 43 us a call, one row 50 -> 26.5 us (the rule at infer() has the rest).
-template <int MT, int WM, int ST>
-struct Infer {
-  static constexpr int TM = 16 * MT * WM, WN = 8 / WM, NT = H / WN / 8, LDA = H + 8, LDW = H + 8, KS = 32;
-  static constexpr size_t smem = (size_t)TM * LDA * 2 + (size_t)ST * KS * LDW * 2 + (size_t)H * 24 * 2;
-};
-
-__device__ __forceinline__ void ldsm4(uint32_t r[4], const void *p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"((uint32_t)__cvta_generic_to_shared(p)));
-}
-__device__ __forceinline__ void ldsm4t(uint32_t r[4], const void *p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"((uint32_t)__cvta_generic_to_shared(p)));
-}
-__device__ __forceinline__ void cp16(void *to, const void *from) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from)
-               : "memory");
-}
-
-struct InferArgs {
-  const float *x, *xmean, *xistd, *ymean, *yistd, *bias;
-  const bf16 *w[4];
-  float *out;
-  int n;
-};
-
-template <int MT, int WM, int ST>
-__global__ void __launch_bounds__(256) k_mlp_infer(const InferArgs g) {
-  using T = Infer<MT, WM, ST>;
-  extern __shared__ __align__(16) uint8_t tc_smem[];
-  bf16(*A)[T::LDA] = reinterpret_cast<bf16(*)[T::LDA]>(tc_smem);
-  bf16(*W)[T::KS][T::LDW] = reinterpret_cast<bf16(*)[T::KS][T::LDW]>(tc_smem + sizeof(bf16) * T::TM * T::LDA);
-  bf16(*W4)[24] = reinterpret_cast<bf16(*)[24]>(tc_smem + sizeof(bf16) * (T::TM * T::LDA + ST * T::KS * T::LDW));
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp % WM, wn = warp / WM;
-  const int gq = lane >> 2, q = lane & 3;
-  const int m0 = blockIdx.x * T::TM, rows = min(T::TM, g.n - m0);
-  // the weight stages in the order they are used: layer 1 (96 k rows), 2, 3
-  constexpr int S1 = INP / T::KS, S2 = H / T::KS, NS = S1 + 2 * S2;
-  auto stage = [&](int s) {
-    if (s < NS) {
-      const int k0 = (s < S1 ? s : (s - S1) % S2) * T::KS;
-      const bf16 *src = (s < S1 ? g.w[0] : s < S1 + S2 ? g.w[1] : g.w[2]) + (size_t)k0 * H;
-      for (int v = tid; v < T::KS * (H / 8); v += 256)
-        cp16(&W[s % ST][v / (H / 8)][(v % (H / 8)) * 8], src + (size_t)v * 8);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  for (int v = tid; v < H * 2; v += 256) cp16(&W4[v >> 1][(v & 1) * 8], g.w[3] + (size_t)v * 8);  // (the first group)
-#pragma unroll
-  for (int q = 0; q < ST - 1; ++q) stage(q);
-  // normalised inputs, clipped to six standard deviations so that inputs far outside the training
-  // data (a colloid the dynamics has thrown) meet the network's behaviour at the edge of that data
-  for (int i = tid; i < T::TM * INP; i += 256) {
-    const int r = i / INP, c = i % INP;
-    const float z = c < IN && r < rows ? (g.x[(size_t)(m0 + r) * IN + c] - g.xmean[c]) * g.xistd[c] : 0.f;
-    A[r][c] = __float2bfloat16(fminf(fmaxf(z, -kInputClip), kInputClip));
-  }
-  float acc[MT][T::NT][4];
-  int s = 0;
-#pragma unroll 1  // (straight-line code runs at the rate it is fetched)
-  for (int l = 0; l < 3; ++l) {
-#pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-      for (int j = 0; j < T::NT; ++j)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.f;
-    const int ns = l == 0 ? S1 : S2;
-    for (int t = 0; t < ns; ++t, ++s) {
-      asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
-      __syncthreads();  // stage s has arrived, and the buffer of stage s - 1 is free
-      stage(s + ST - 1);
-      const bf16(*Ws)[T::LDW] = W[s % ST];
-#pragma unroll
-      for (int kk = 0; kk < T::KS; kk += 16) {
-        uint32_t af[MT][4];
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-          ldsm4(af[i], &A[(wm * MT + i) * 16 + (lane & 15)][t * T::KS + kk + (lane >> 4) * 8]);
-#pragma unroll
-        for (int j = 0; j < T::NT; j += 2) {
-          uint32_t b[4];  // k 0-7 and 8-15 of the tile's first 8 columns, then of its next 8
-          ldsm4t(b, &Ws[kk + (lane & 15)][wn * T::NT * 8 + j * 8 + (lane >> 4) * 8]);
-#pragma unroll
-          for (int i = 0; i < MT; ++i) {
-            mma_bf16(acc[i][j], af[i], b);
-            mma_bf16(acc[i][j + 1], af[i], b + 2);
-          }
-        }
-      }
-    }
-    __syncthreads();  // every warp has read the layer's inputs
-    const float *bias = g.bias + l * H;
-#pragma unroll
-    for (int j = 0; j < T::NT; ++j) {
-      const int c = wn * T::NT * 8 + j * 8 + q * 2;
-      const float b0 = bias[c], b1 = bias[c + 1];
-#pragma unroll
-      for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int r = (wm * MT + i) * 16 + gq + h * 8;
-          float v0 = acc[i][j][2 * h] + b0, v1 = acc[i][j][2 * h + 1] + b1;
-          v0 = v0 * sigm(v0);
-          v1 = v1 * sigm(v1);
-          *reinterpret_cast<__nv_bfloat162 *>(&A[r][c]) = __nv_bfloat162(__float2bfloat16(v0), __float2bfloat16(v1));
-        }
-    }
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();
-  // the output layer: 16 rows x 8 columns a warp, in physical units (mean * std + mean, log-variance
-  // + 2 log std)
-  for (int p = warp; p < T::TM / 16 * 2; p += 8) {
-    const int r0 = (p >> 1) * 16, c0 = (p & 1) * 8;
-    float o[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int kk = 0; kk < H; kk += 32) {
-      uint32_t b[4], a0[4], a1[4];
-      ldsm4t(b, &W4[kk + lane][c0]);
-      ldsm4(a0, &A[r0 + (lane & 15)][kk + (lane >> 4) * 8]);
-      ldsm4(a1, &A[r0 + (lane & 15)][kk + 16 + (lane >> 4) * 8]);
-      mma_bf16(o, a0, b);
-      mma_bf16(o, a1, b + 2);
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int r = r0 + gq + (e >= 2 ? 8 : 0), k = c0 + q * 2 + (e & 1);
-      if (r >= rows || k >= OUT) continue;
-      const float v = o[e] + g.bias[3 * H + k];
-      g.out[(size_t)(m0 + r) * OUT + k] =
-          k < NY ? v / g.yistd[k] + g.ymean[k]
-                 : fminf(fmaxf(v, -kLogVarClamp), kLogVarClamp) - 2.f * __logf(g.yistd[k - NY]);
-    }
-  }
-}
-
-// the parameter layout: flat FP32 vector (W1 [IN][H], b1, W2 [H][H], b2, W3, b3, W4 [H][OUT], b4)
-// and the padded BF16 weights the GEMMs read
-struct Layout {
-  long long w[4], b[4], total;
-  int kin[4], nout[4];
-};
-
-Layout layout() {
-  Layout L;
-  const int kin[4] = {IN, H, H, H}, nout[4] = {H, H, H, OUT};
-  long long o = 0;
-  for (int l = 0; l < 4; ++l) {
-    L.kin[l] = kin[l];
-    L.nout[l] = nout[l];
-    L.w[l] = o;
-    o += (long long)kin[l] * nout[l];
-    L.b[l] = o;
-    o += nout[l];
-  }
-  L.total = o;
-  return L;
-}
-
-struct WeightCopies {
-  bf16 *w[4];   // [kpad][npad] (k major rows of n): inference, the forward pass
-  bf16 *wt[4];  // [npad][kpad] (n major rows of k): the backward pass
-};
-
-// ------------------------------------------------------------------ training: layers
-//
-// The products of the forward and the backward pass, a launch each: C[M x N] = A[M x K] B[K x N], A and B
-// with K contiguous (B(k, n) at B[n ldb + k]), N and K multiples of 16 up to 256.  One CTA of four
-// warps per 128 rows and column tile (all N, or halves of it when the rows alone would leave
-// SMs idle): the A tile (128 x K) and the B tile (N x K) staged in shared memory in
-// the canonical K-major layout without swizzle (core matrices of 8 rows x 16 bytes, the K
-// direction LBO = 128 bytes apart, 8-row groups SBO = K/8 x 128 bytes apart), K/16
-// tcgen05.mma (kind::f16, BF16 x BF16 -> FP32, M = 128) issued by one thread into a TMEM
-// accumulator of 128 lanes x N columns, their completion signalled on an mbarrier
-// (tcgen05.commit) and waited for with a time limit (a wait that runs out sets *err and
-// skips the epilogue); then each warp reads its 32 TMEM lanes (rows) 16 columns at a time
-// (tcgen05.ld) into the epilogue.  fault: the test hook, nothing issued.
-// Bound: each launch's latency, its staging, products and epilogue in sequence.  One kernel over all layers with
-// warp-level products took 46 us in place of these nine launches' 130 (cold, 8,192 rows), but mma.sync
-// rounds a few sums in a million the other way than tcgen05.mma: over 12 seeds, eight Adam steps of 8,192
-// rows then left the losses 1.1e-6 off (median), where two runs of this form with atomically added weight
-// gradients differ by 1.3e-7 and this form differs from those by 2.2e-7.
-struct Gemm {
-  const bf16 *A;
-  long long lda;
-  const bf16 *B;
-  long long ldb;
-  int M, N, K;
-  const float *bias;   // [N] or null
-  int silu;            // apply SiLU after the bias
-  const bf16 *dz;      // backward: multiply by silu'(dz[m, n]) (the layer's pre-activation)
-  long long lddz;
-  float *Cf;           // FP32 store
-  long long ldcf;
-  bf16 *Cb;            // BF16 store (after the activation)
-  long long ldcb;
-  bf16 *Zb;            // BF16 store of the pre-activation
-  long long ldzb;
-};
 
 // shared memory of k_gemm_tc: the mbarrier and the TMEM address, then from byte 1024 the
 // operand tiles (A: 128 x K, B: ntile x K, canonical layout) and, once the products are done,
@@ -349,7 +167,7 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const Gemm g, int ntile, int *e
   for (int v = tid; v < TC_M * kv; v += 128) {
     const int r = v / kv, j = v - r * kv;
     const bool in = r < rows;
-    const bf16 *src = in ? g.A + (long long)(m0 + r) * g.lda + j * 8 : g.A;
+    const bf16 *src = in ? g.A + (long long)(m0 + r) * g.sam + j * 8 : g.A;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(As + (r >> 3) * sbo + j * 128 + (r & 7) * 16)),
                  "l"(src), "r"(in ? 16 : 0)
                  : "memory");
@@ -357,7 +175,7 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const Gemm g, int ntile, int *e
   for (int v = tid; v < N * kv; v += 128) {
     const int r = v / kv, j = v - r * kv;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(Bs + (r >> 3) * sbo + j * 128 + (r & 7) * 16)),
-                 "l"(g.B + (long long)(n0 + r) * g.ldb + j * 8)
+                 "l"(g.B + (long long)(n0 + r) * g.sbn + j * 8)
                  : "memory");
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
@@ -458,6 +276,154 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const Gemm g, int ntile, int *e
   }
 }
 
+// The weight-gradient products on the tcgen05 path: C[M x N] += A[M x K] B[K x N] with A and B
+// contiguous along M and N (sam = 1, sbn = 1: the reduction runs over the batch rows, K; N
+// padded to a multiple of 16, the columns past it zero), the
+// K range split over blockIdx.z (kchunk each) and the results added to C with FP32 atomics.
+// The operands are staged row-major by 16-byte asynchronous copies, then transposed in shared
+// memory into the canonical K-major layout (a thread gathers 8 consecutive k of one row into
+// one 16-byte slot).  K runs in stages of 64 through two buffers; a buffer is staged
+// again only after the MMAs that read it have completed (one mbarrier per buffer, every wait
+// bounded).  fault: the test hook, nothing issued.
+constexpr int TCW_K = 64;
+
+__host__ __device__ inline size_t tcw_smem(int ntile) {
+  // two canonical buffers (A, B), then the row-major tiles the copies land in
+  return 1024 + 3 * ((size_t)TC_M * TCW_K * 2 + (size_t)ntile * TCW_K * 2);
+}
+
+__global__ void __launch_bounds__(128) k_gemm_tc_wgrad(const Gemm g, int ntile, int *err, int fault) {
+  extern __shared__ __align__(1024) uint8_t tc_smem[];
+  const int N = ntile, n0 = blockIdx.y * ntile, m0 = blockIdx.x * TC_M;
+  const int kbeg = blockIdx.z * g.kchunk, kend = min(g.K, kbeg + g.kchunk);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  unsigned long long *bar = reinterpret_cast<unsigned long long *>(tc_smem);  // one per buffer
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(tc_smem + 16);
+  const size_t a_bytes = (size_t)TC_M * TCW_K * 2, b_bytes = (size_t)N * TCW_K * 2;
+  const uint32_t sbo = (TCW_K / 8) * 128u;
+  const uint32_t ncols = N <= 32 ? 32u : (N <= 64 ? 64u : (N <= 128 ? 128u : 256u));
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)),
+                 "r"(ncols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar + 1)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tslot;
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+  const int nst = kbeg < kend ? (kend - kbeg + TCW_K - 1) / TCW_K : 0;
+  uint32_t phase[2] = {0u, 0u};
+  bool ok = true;
+  for (int st = 0; st < nst; ++st) {
+    const int q = st & 1;
+    uint8_t *As = tc_smem + 1024 + q * (a_bytes + b_bytes), *Bs = As + a_bytes;
+    if (st >= 2) {  // the MMAs of stage st - 2 read this buffer
+      if (ok) ok = tc_wait_bounded(smem_addr(bar + q), phase[q]);
+      phase[q] ^= 1u;
+    }
+    const int k0 = kbeg + st * TCW_K;
+    // the row-major tiles (64 k rows of 128 m, of N n) by 16-byte asynchronous copies, the
+    // bytes past M, N or the K range zero-filled
+    {
+      bf16 *Ra = reinterpret_cast<bf16 *>(tc_smem + 1024 + 2 * (a_bytes + b_bytes));
+      bf16 *Rb = Ra + TC_M * TCW_K;
+      for (int v = tid; v < TCW_K * (TC_M / 8); v += 128) {
+        const int k = v / (TC_M / 8), mv = (v - k * (TC_M / 8)) * 8, m = m0 + mv;
+        const int valid = (k0 + k < kend) ? max(0, min(8, g.M - m)) : 0;
+        const bf16 *src = valid ? g.A + (long long)(k0 + k) * g.sak + m : g.A;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(Ra + k * TC_M + mv)), "l"(src),
+                     "r"(valid * 2)
+                     : "memory");
+      }
+      for (int v = tid; v < TCW_K * (N / 8); v += 128) {
+        const int k = v / (N / 8), nv = (v - k * (N / 8)) * 8, n = n0 + nv;
+        const int valid = (k0 + k < kend) ? max(0, min(8, g.N - n)) : 0;
+        const bf16 *src = valid ? g.B + (long long)(k0 + k) * g.sbk + n : g.B;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(Rb + k * N + nv)), "l"(src),
+                     "r"(valid * 2)
+                     : "memory");
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      // transposed into the canonical K-major layout: 8 consecutive k of one row per 16 bytes
+      // (consecutive threads on consecutive rows: the shared-memory reads share words)
+      for (int v = tid; v < TC_M * (TCW_K / 8); v += 128) {
+        const int j = v / TC_M, r = v - j * TC_M;
+        bf16 e[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) e[t] = Ra[(j * 8 + t) * TC_M + r];
+        *reinterpret_cast<uint4 *>(As + (r >> 3) * sbo + j * 128 + (r & 7) * 16) = *reinterpret_cast<const uint4 *>(e);
+      }
+      for (int v = tid; v < N * (TCW_K / 8); v += 128) {
+        const int j = v / N, r = v - j * N;
+        bf16 e[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) e[t] = Rb[(j * 8 + t) * N + r];
+        *reinterpret_cast<uint4 *>(Bs + (r >> 3) * sbo + j * 128 + (r & 7) * 16) = *reinterpret_cast<const uint4 *>(e);
+      }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (tid == 0 && !fault) {
+      const uint32_t a0 = smem_addr(As), b0 = smem_addr(Bs);
+      for (int kk = 0; kk < TCW_K / 16; ++kk) {
+        const uint64_t ad = tc_desc(a0 + kk * 256, 128, sbo), bd = tc_desc(b0 + kk * 256, 128, sbo);
+        const uint32_t accumulate = (st > 0 || kk > 0) ? 1u : 0u;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(tmem), "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate)
+            : "memory");
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar + q))
+                   : "memory");
+    }
+  }
+  // the last commit arrives when every MMA issued before it has completed
+  if (nst > 0) {
+    const int q = (nst - 1) & 1;
+    if (ok) ok = tc_wait_bounded(smem_addr(bar + q), phase[q]);
+  }
+  if (!ok && lane == 0) atomicExch(err, 1);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const bool all_ok = __syncthreads_and(ok) != 0;
+  if (all_ok && nst > 0) {
+    const int m = m0 + warp * 32 + lane;
+    for (int c0 = 0; c0 < N; c0 += 16) {
+      uint32_t r[16];
+      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+          : "r"(taddr)
+          : "memory");
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (m < g.M) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+          if (n0 + c0 + q < g.N) atomicAdd(&g.Cacc[(long long)m * g.ldca + n0 + c0 + q], __uint_as_float(r[q]));
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+  }
+}
+
 // raw features [n][IN] -> normalised BF16 [n][INP] (zero padded), clipped to six
 // standard deviations so that inputs far outside the training data (a colloid the
 // dynamics has thrown) meet the network's behaviour at the edge of that data
@@ -470,12 +436,12 @@ __global__ void k_features_in(const float *x, int n, const float *mean, const fl
 }
 
 // Gaussian negative log-likelihood of normalised targets under (mean, log-variance)
-// outputs; writes d loss / d output (BF16, mean over the batch) and each row's loss
+// outputs; writes d loss / d output (BF16, mean over the batch) and adds the loss sum
 __global__ void k_nll(const float *o, const float *y, int n, const float *ymean, const float *yistd, bf16 *dout,
-                      float *loss) {
+                      double *loss) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  float l = 0.f;
   if (r < n) {
-    float l = 0.f;
     const float inv = 1.f / (float)n;
     for (int k = 0; k < NY; ++k) {
       const float t = (y[r * NY + k] - ymean[k]) * yistd[k];
@@ -487,258 +453,210 @@ __global__ void k_nll(const float *o, const float *y, int n, const float *ymean,
       dout[r * OUTP + k] = __float2bfloat16(-d * e * inv);
       dout[r * OUTP + NY + k] = __float2bfloat16((sraw == s) ? 0.5f * (1.f - d * d * e) * inv : 0.f);
     }
-    loss[r] = l;
     for (int k = OUT; k < OUTP; ++k) dout[r * OUTP + k] = __float2bfloat16(0.f);
   }
+  // block sum, one atomic per block
+  __shared__ float sh[256];
+  sh[threadIdx.x] = l;
+  __syncthreads();
+  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+    if ((int)threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) atomicAdd(loss, (double)sh[0]);
 }
 
-// ------------------------------------------------------------------ training: weight gradients
-//
-// dW_l = A_{l-1}^T dZ_l and db_l, the column sums of dZ_l, of all four layers in one launch, on the
-// 5th-generation tensor cores: a CTA takes one 128 x 128 tile (128 x 16 of the last layer; twelve
-// tiles) over some of the batch's slices (up to 32 of whole stages).  Each slice is a sum of its own
-// in TMEM (two accumulators in turn), the CTA adds its slices in registers and leaves its partial sums in
-// memory; k_adam adds those in order, so a gradient has the same bits every time.  As many CTAs a tile
-// as give each SM one.
-// A row of the batch is contiguous along m (n), which is what the MN-major operand layout without
-// swizzle wants: core matrices of 8 k x 16 bytes, so the copies land where the MMA reads them
-// (blocks of 8 along m (n) SBO = 128 bytes apart, blocks of 8 k LBO apart).  Four stages of 64 k are
-// in flight; a buffer is filled again once the MMAs that read it have completed (one mbarrier a
-// buffer, every wait bounded: one that runs out sets *err and skips the output).  The column sums are
-// read from the staged tiles by the CTAs of the first m tile.  The CTAs past the tiles add the rows'
-// losses, 256 at a time.  fault: the test hook, nothing issued.
-// Bound: latency (a CTA's twelve stages, each waiting for L2).  Measured cold, 8,192 rows: four
-// launches that staged, waited, transposed and added with atomics, and four for the column sums,
-// 170 us; this 27 us (23 us with a slice per CTA, whose sums are longer).  A training step, host side
-// included: 8,192 rows 305 -> 180 us, 777 rows 300 -> 143 us.
-constexpr int TCW_K = 64, TCW_ST = 4, TCW_TILES = 12, TCW_TH = 256, TCW_SLICES = 32;
+// column sums of a BF16 matrix into FP32 (bias gradients), one atomic per (block, column)
+__global__ void k_colsum(const bf16 *a, int n, int cols, long long lda, float *out) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  const int per = (n + gridDim.y - 1) / gridDim.y, r0 = blockIdx.y * per, r1 = min(n, r0 + per);
+  float s = 0.f;
+  for (int r = r0; r < r1; ++r) s += __bfloat162float(a[r * lda + c]);
+  atomicAdd(&out[c], s);
+}
 
-struct WgradArgs {
-  const bf16 *A[4], *B[4];  // the layers' inputs and pre-activation gradients
-  float *part;              // [gridDim.y][total]
-  Layout L;
-  int n, kchunk, slices;    // rows; rows of a slice (whole stages); slices
-  const float *loss;        // [n] the rows' losses
-  double *lsum;             // [n / 256] their sums
+// ------------------------------------------------------------------ inference
+//
+// The whole network for TM = 16 MT WM rows per CTA of eight warps (WM along the rows, 8 / WM
+// along the columns): normalisation, the four layers with the activations in shared memory, the
+// outputs in physical units, in one launch.  The weights stream from L2 through three stages
+// of 32 k rows by asynchronous copies, the next layer's first stages while this one's epilogue runs.
+// Each output element is K steps of 16 in ascending order into one FP32 accumulator, bias, SiLU and
+// the BF16 rounding between layers, as in the colloid-only step's network, whose bits these are.
+// Bound: L2 reads of the weights (311 KB a CTA) and the SiLU's two special-function operations
+// per element.  Measured, six launches with the activations through memory -> this: 16,384 rows
+// 197 -> 43 us a call, one row 50 -> 26.5 us (the rule at infer() has the rest).
+template <int MT, int WM, int ST>
+struct Infer {
+  static constexpr int TM = 16 * MT * WM, WN = 8 / WM, NT = H / WN / 8, LDA = H + 8, LDW = H + 8, KS = 32;
+  static constexpr size_t smem = (size_t)TM * LDA * 2 + (size_t)ST * KS * LDW * 2 + (size_t)H * 24 * 2;
 };
 
-constexpr size_t TCW_BUF = (size_t)2 * TC_M * TCW_K * 2;  // one stage: A, then B
-constexpr size_t TCW_SMEM = 1024 + TCW_ST * TCW_BUF;
+__device__ __forceinline__ void ldsm4(uint32_t r[4], const void *p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t r[4], const void *p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void cp16(void *to, const void *from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from)
+               : "memory");
+}
 
-__global__ void __launch_bounds__(TCW_TH) k_gemm_tc_wgrad(const WgradArgs g, int *err, int fault) {
-  extern __shared__ __align__(1024) uint8_t tc_smem[];
-  if (blockIdx.x == TCW_TILES) {
-    float *sh = reinterpret_cast<float *>(tc_smem);
-    for (int b = blockIdx.y; b * 256 < g.n; b += gridDim.y) {
-      const int r = b * 256 + (int)threadIdx.x;
-      sh[threadIdx.x] = r < g.n ? g.loss[r] : 0.f;
-      __syncthreads();
-      for (int o = 128; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-      }
-      if (threadIdx.x == 0) g.lsum[b] = (double)sh[0];
-      __syncthreads();
-    }
-    return;
-  }
-  // this CTA's tile: layer l, rows m0.., columns n0.. (N of them)
-  const int t = blockIdx.x;
-  const int l = t < 2 ? 0 : t < 6 ? 1 : t < 10 ? 2 : 3;
-  const int u = t - (l == 0 ? 0 : l == 1 ? 2 : l == 2 ? 6 : 10);
-  const int m0 = (l == 0 ? 0 : l == 3 ? u : u >> 1) * TC_M, n0 = l == 3 ? 0 : (u & 1) * 128, N = l == 3 ? OUTP : 128;
-  const int lda = l == 0 ? INP : H, ldb = l == 3 ? OUTP : H;
-  const bf16 *GA = g.A[l], *GB = g.B[l];
-  const int s0 = (int)((long long)blockIdx.y * g.slices / gridDim.y),
-            s1 = (int)((long long)(blockIdx.y + 1) * g.slices / gridDim.y);
-  const int kbeg = s0 * g.kchunk, kend = min(g.n, s1 * g.kchunk), sst = g.kchunk / TCW_K;  // (stages of a slice)
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  unsigned long long *bar = reinterpret_cast<unsigned long long *>(tc_smem);  // one per buffer
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(tc_smem + 64);
-  const uint32_t lboA = TC_M / 8 * 128u, lboB = (uint32_t)N / 8 * 128u;
-  const uint32_t ncols = 256u;
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)),
-                 "r"(ncols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (tid == 0) {
-    for (int q = 0; q < TCW_ST; ++q)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar + q)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tslot;
-  // instruction descriptor: FP32 accumulator (bit 4), A and B BF16 (bits 7, 10), both MN-major
-  // (bits 15, 16), N / 8 at bit 17, M / 16 at bit 24
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(N >> 3) << 17) |
-                         ((uint32_t)(TC_M >> 4) << 24);
-  const int nst = (kend - kbeg + TCW_K - 1) / TCW_K;
-  // stage st: 64 rows of 128 m and N n, 16 bytes per copy, what lies past the slice or the row's end
-  // zero-filled; eight lanes take eight rows (128 contiguous bytes of shared memory), four of them 64
-  // bytes of a row
-  auto load = [&](int st) {
-    if (st < nst) {
-      uint8_t *As = tc_smem + 1024 + (st % TCW_ST) * TCW_BUF, *Bs = As + TCW_BUF / 2;
-      const int k0 = kbeg + st * TCW_K;
-      auto copy = [&](uint8_t *to, const bf16 *from, int ld, int c0, int vecs, uint32_t lbo) {
-        const int quads = (vecs + 3) / 4;  // groups of four 16-byte vectors
-        for (int w = warp; w < TCW_K / 8 * quads; w += TCW_TH / 32) {
-          const int kb = w / quads, i = (w - kb * quads) * 4 + (lane >> 3), k = k0 + kb * 8 + (lane & 7);
-          if (i >= vecs) continue;
-          const int c = c0 + i * 8;
-          const bool in = k < kend && c < ld;
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                           smem_addr(to + kb * lbo + i * 128 + (lane & 7) * 16)),
-                       "l"(in ? from + (size_t)k * ld + c : from), "r"(in ? 16 : 0)
-                       : "memory");
-        }
-      };
-      copy(As, GA, lda, m0, TC_M / 8, lboA);
-      copy(Bs, GB, ldb, n0, N / 8, lboB);
+struct InferArgs {
+  const float *x, *xmean, *xistd, *ymean, *yistd, *bias;
+  const bf16 *w[4];
+  float *out;
+  int n;
+};
+
+template <int MT, int WM, int ST>
+__global__ void __launch_bounds__(256) k_mlp_infer(const InferArgs g) {
+  using T = Infer<MT, WM, ST>;
+  extern __shared__ __align__(16) uint8_t tc_smem[];
+  bf16(*A)[T::LDA] = reinterpret_cast<bf16(*)[T::LDA]>(tc_smem);
+  bf16(*W)[T::KS][T::LDW] = reinterpret_cast<bf16(*)[T::KS][T::LDW]>(tc_smem + sizeof(bf16) * T::TM * T::LDA);
+  bf16(*W4)[24] = reinterpret_cast<bf16(*)[24]>(tc_smem + sizeof(bf16) * (T::TM * T::LDA + ST * T::KS * T::LDW));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp % WM, wn = warp / WM;
+  const int gq = lane >> 2, q = lane & 3;
+  const int m0 = blockIdx.x * T::TM, rows = min(T::TM, g.n - m0);
+  // the weight stages in the order they are used: layer 1 (96 k rows), 2, 3
+  constexpr int S1 = INP / T::KS, S2 = H / T::KS, NS = S1 + 2 * S2;
+  auto stage = [&](int s) {
+    if (s < NS) {
+      const int k0 = (s < S1 ? s : (s - S1) % S2) * T::KS;
+      const bf16 *src = (s < S1 ? g.w[0] : s < S1 + S2 ? g.w[1] : g.w[2]) + (size_t)k0 * H;
+      for (int v = tid; v < T::KS * (H / 8); v += 256)
+        cp16(&W[s % ST][v / (H / 8)][(v % (H / 8)) * 8], src + (size_t)v * 8);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  for (int st = 0; st < TCW_ST - 1; ++st) load(st);
-  bool ok = true;
-  float acc[64];  // row (warp & 3) 32 + lane, 16 columns of every 32
+  for (int v = tid; v < H * 2; v += 256) cp16(&W4[v >> 1][(v & 1) * 8], g.w[3] + (size_t)v * 8);  // (the first group)
 #pragma unroll
-  for (int c = 0; c < 64; ++c) acc[c] = 0.f;
-  // a slice's sums (number i of this CTA) from TMEM: a row per thread, 16 columns at a time; two warps
-  // share a row's columns
-  auto gather = [&](int i) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  for (int q = 0; q < ST - 1; ++q) stage(q);
+  // normalised inputs, clipped (k_features_in)
+  for (int i = tid; i < T::TM * INP; i += 256) {
+    const int r = i / INP, c = i % INP;
+    const float z = c < IN && r < rows ? (g.x[(size_t)(m0 + r) * IN + c] - g.xmean[c]) * g.xistd[c] : 0.f;
+    A[r][c] = __float2bfloat16(fminf(fmaxf(z, -kInputClip), kInputClip));
+  }
+  float acc[MT][T::NT][4];
+  int s = 0;
+  for (int l = 0; l < 3; ++l) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c0 = q * 32 + (warp >> 2) * 16;
-      if (c0 >= N) continue;
-      uint32_t r[16];
-      const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((i & 1) * 128 + c0);
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(taddr)
-          : "memory");
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    for (int i = 0; i < MT; ++i)
 #pragma unroll
-      for (int c = 0; c < 16; ++c) acc[q * 16 + c] += __uint_as_float(r[c]);
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  };
-  float cs[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // column sums: columns 8 (tid / 16).., rows tid % 16..
-  for (int st = 0; st < nst && ok; ++st) {
-    const int q = st % TCW_ST;
-    const uint8_t *As = tc_smem + 1024 + q * TCW_BUF, *Bs = As + TCW_BUF / 2;
-    asm volatile("cp.async.wait_group %0;" ::"n"(TCW_ST - 2) : "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (tid == 0 && !fault) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a0 = smem_addr(As), b0 = smem_addr(Bs);
-      for (int kk = 0; kk < TCW_K / 16; ++kk) {
-        const uint64_t ad = tc_desc(a0 + kk * 2 * lboA, lboA, 128), bd = tc_desc(b0 + kk * 2 * lboB, lboB, 128);
-        const uint32_t accumulate = (st % sst > 0 || kk > 0) ? 1u : 0u;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(tmem + (uint32_t)((st / sst) & 1) * 128u), "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate)
-            : "memory");
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar + q))
-                   : "memory");
-    }
-    if (m0 == 0 && (tid >> 4) < N / 8) {
-      for (int r = tid & 15; r < TCW_K; r += 16) {
-        const uint4 v = *reinterpret_cast<const uint4 *>(Bs + (r >> 3) * lboB + (tid >> 4) * 128 + (r & 7) * 16);
-        const __nv_bfloat162 *e = reinterpret_cast<const __nv_bfloat162 *>(&v);
+      for (int j = 0; j < T::NT; ++j)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          cs[2 * c] += __low2float(e[c]);
-          cs[2 * c + 1] += __high2float(e[c]);
+        for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.f;
+    const int ns = l == 0 ? S1 : S2;
+    for (int t = 0; t < ns; ++t, ++s) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+      __syncthreads();  // stage s has arrived, and the buffer of stage s - 1 is free
+      stage(s + ST - 1);
+      const bf16(*Ws)[T::LDW] = W[s % ST];
+#pragma unroll
+      for (int kk = 0; kk < T::KS; kk += 16) {
+        uint32_t af[MT][4];
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+          ldsm4(af[i], &A[(wm * MT + i) * 16 + (lane & 15)][t * T::KS + kk + (lane >> 4) * 8]);
+#pragma unroll
+        for (int j = 0; j < T::NT; j += 2) {
+          uint32_t b[4];  // k 0-7 and 8-15 of the tile's first 8 columns, then of its next 8
+          ldsm4t(b, &Ws[kk + (lane & 15)][wn * T::NT * 8 + j * 8 + (lane >> 4) * 8]);
+#pragma unroll
+          for (int i = 0; i < MT; ++i) {
+            mma_bf16(acc[i][j], af[i], b);
+            mma_bf16(acc[i][j + 1], af[i], b + 2);
+          }
         }
       }
     }
-    // the buffer of stage st - 1 is free once its MMAs have completed
-    if (st > 0) ok = tc_wait_bounded(smem_addr(bar + (st - 1) % TCW_ST), (uint32_t)(((st - 1) / TCW_ST) & 1));
-    ok = __syncthreads_and(ok) != 0;
-    if (ok) load(st + TCW_ST - 1);
-    if (ok && st > 0 && st % sst == 0) gather(st / sst - 1);  // (the slice before this one is complete)
+    __syncthreads();  // every warp has read the layer's inputs
+    const float *bias = g.bias + l * H;
+#pragma unroll
+    for (int j = 0; j < T::NT; ++j) {
+      const int c = wn * T::NT * 8 + j * 8 + q * 2;
+      const float b0 = bias[c], b1 = bias[c + 1];
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = (wm * MT + i) * 16 + gq + h * 8;
+          float v0 = acc[i][j][2 * h] + b0, v1 = acc[i][j][2 * h + 1] + b1;
+          v0 = v0 * sigm(v0);
+          v1 = v1 * sigm(v1);
+          *reinterpret_cast<__nv_bfloat162 *>(&A[r][c]) = __nv_bfloat162(__float2bfloat16(v0), __float2bfloat16(v1));
+        }
+    }
   }
-  // the last commit arrives when every MMA issued before it has completed
-  if (ok && nst > 0) ok = tc_wait_bounded(smem_addr(bar + (nst - 1) % TCW_ST), (uint32_t)(((nst - 1) / TCW_ST) & 1));
-  if (!ok && lane == 0) atomicExch(err, 1);
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const bool all_ok = __syncthreads_and(ok) != 0;
-  float *P = g.part + (size_t)blockIdx.y * g.L.total;
-  const int nout = g.L.nout[l];
-  if (all_ok) {
-    if (nst > 0) gather((nst - 1) / sst);
-    const int m = m0 + (warp & 3) * 32 + lane;
-    if (m < g.L.kin[l]) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int c0 = q * 32 + (warp >> 2) * 16;
-#pragma unroll
-        for (int c = 0; c < 16; c += 4)
-          if (c0 < N && n0 + c0 + c < nout)
-            *reinterpret_cast<float4 *>(P + g.L.w[l] + (long long)m * nout + n0 + c0 + c) =
-                make_float4(acc[q * 16 + c], acc[q * 16 + c + 1], acc[q * 16 + c + 2], acc[q * 16 + c + 3]);
-      }
-    }
-    if (m0 == 0) {
-      // sixteen lanes hold a column's rows
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        float v = cs[c];
-        for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        const int col = (tid >> 4) * 8 + c;
-        if ((lane & 15) == 0 && col < N && n0 + col < nout) P[g.L.b[l] + n0 + col] = v;
-      }
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+  // the output layer: 16 rows x 8 columns a warp, in physical units (k_denorm)
+  for (int p = warp; p < T::TM / 16 * 2; p += 8) {
+    const int r0 = (p >> 1) * 16, c0 = (p & 1) * 8;
+    float o[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int kk = 0; kk < H; kk += 32) {
+      uint32_t b[4], a0[4], a1[4];
+      ldsm4t(b, &W4[kk + lane][c0]);
+      ldsm4(a0, &A[r0 + (lane & 15)][kk + (lane >> 4) * 8]);
+      ldsm4(a1, &A[r0 + (lane & 15)][kk + 16 + (lane >> 4) * 8]);
+      mma_bf16(o, a0, b);
+      mma_bf16(o, a1, b + 2);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int r = r0 + gq + (e >= 2 ? 8 : 0), k = c0 + q * 2 + (e & 1);
+      if (r >= rows || k >= OUT) continue;
+      const float v = o[e] + g.bias[3 * H + k];
+      g.out[(size_t)(m0 + r) * OUT + k] =
+          k < NY ? v / g.yistd[k] + g.ymean[k]
+                 : fminf(fmaxf(v, -kLogVarClamp), kLogVarClamp) - 2.f * __logf(g.yistd[k - NY]);
+    }
   }
 }
 
-// A gradient from its partial sums, in order; with update, unless a weight-gradient wait ran
-// out, Adam on the FP32 masters and the BF16 copies (weights at [k][n] of a padded [kpad][npad] matrix
-// and transposed; biases stay FP32).  The last block adds the loss.
-struct TrainResult {
-  double loss;
-  int err;
+// the parameter layout: flat FP32 vector (W1 [IN][H], b1, W2 [H][H], b2, W3, b3, W4 [H][OUT], b4)
+// and the padded BF16 weights the GEMMs read
+struct Layout {
+  long long w[4], b[4], total;
+  int kin[4], nout[4];
 };
 
-__global__ void __launch_bounds__(256) k_adam(float *p, const float *part, int slices, float *gr, float *m, float *v,
-                                              long long n, int update, float lr, float b1, float b2, float eps,
-                                              float c1, float c2, Layout L, WeightCopies W, float *bias,
-                                              const double *loss, int nloss, TrainResult *res) {
-  if (blockIdx.x == gridDim.x - 1) {
-    __shared__ double sh[256];
-    double s = 0;
-    for (int k = threadIdx.x; k < nloss; k += 256) s += loss[k];
-    sh[threadIdx.x] = s;
-    for (int o = 128; o > 0; o >>= 1) {
-      __syncthreads();
-      if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    }
-    if (threadIdx.x == 0) res->loss = sh[0];
-    return;
+Layout layout() {
+  Layout L;
+  const int kin[4] = {IN, H, H, H}, nout[4] = {H, H, H, OUT};
+  long long o = 0;
+  for (int l = 0; l < 4; ++l) {
+    L.kin[l] = kin[l];
+    L.nout[l] = nout[l];
+    L.w[l] = o;
+    o += (long long)kin[l] * nout[l];
+    L.b[l] = o;
+    o += nout[l];
   }
+  L.total = o;
+  return L;
+}
+
+// Adam on the FP32 masters, then the BF16 copies (weights at [k][n] of a padded
+// [kpad][npad] matrix; biases stay FP32)
+struct WeightCopies {
+  bf16 *w[4];   // [kpad][npad] (k major rows of n): the warp-level products, inference
+  bf16 *wt[4];  // [npad][kpad] (n major rows of k): the tcgen05 products of the forward pass
+};
+
+__global__ void k_adam(float *p, const float *gr, float *m, float *v, long long n, float lr, float b1, float b2,
+                       float eps, float c1, float c2, Layout L, WeightCopies W, float *bias) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float g = 0.f;
-  for (int k = 0; k < slices; ++k) g += part[k * n + i];
-  gr[i] = g;
-  if (!update || res->err) return;
+  const float g = gr[i];
   const float mi = b1 * m[i] + (1.f - b1) * g, vi = b2 * v[i] + (1.f - b2) * g * g;
   m[i] = mi;
   v[i] = vi;
@@ -771,18 +689,15 @@ struct mpcd_mlp {
   float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;  // flat FP32 params, grads, Adam moments
   bf16 *w[4] = {nullptr, nullptr, nullptr, nullptr};               // padded BF16 weights [k][n]
   bf16 *wt[4] = {nullptr, nullptr, nullptr, nullptr};              // the same transposed, [n][k]
-  TrainResult *res = nullptr;                                      // the loss; whether a tcgen05 wait ran out
+  int *tc_err = nullptr;                                           // a tcgen05 wait ran out
   int tc_fault = 0;                                                // test hook (mpcd_mlp_set_fault)
   float *bias = nullptr;                                           // padded biases [H][H][H][OUTP]
   float *xmean = nullptr, *xistd = nullptr, *ymean = nullptr, *yistd = nullptr;
-  // training: what the weight gradients read and their partial sums
-  bf16 *X = nullptr, *A[3] = {nullptr, nullptr, nullptr}, *dZ[3] = {nullptr, nullptr, nullptr}, *dO = nullptr;
-  bf16 *Z[3] = {nullptr, nullptr, nullptr};  // pre-activations
-  float *O = nullptr;                        // outputs
-  float *part = nullptr;
-  int max_parts = 1;
-  float *loss = nullptr;    // [max_batch] the rows' losses
-  double *lsum = nullptr;   // their sums, 256 rows each
+  bf16 *X = nullptr, *Z[3] = {nullptr, nullptr, nullptr}, *A[3] = {nullptr, nullptr, nullptr};
+  float *O = nullptr;
+  bf16 *dO = nullptr, *dA = nullptr, *dZ = nullptr;
+  double *loss = nullptr;
+  float *host_p = nullptr;
   int adam_t = 0;
   std::vector<void *> allocs;
   std::string err;
@@ -816,92 +731,113 @@ WeightCopies copies(const mpcd_mlp *nn) {
   return W;
 }
 
-const int kNpad[4] = {H, H, H, OUTP};
-const int kKpad[4] = {INP, H, H, H};
-
-void gemm_tc(mpcd_mlp *nn, const Gemm &g) {
+// a product on the tcgen05 path (A and B with K contiguous, N and K multiples of 16 up to 256)
+void gemm_tc(mpcd_mlp *nn, cudaStream_t s, const Gemm &g) {
   // at least 80 KB of shared memory per CTA, so that at most two CTAs share an SM and their
   // TMEM columns (256 each at most) always fit in its 512: an allocation never waits
   const int mt = (g.M + TC_M - 1) / TC_M;
   const int ntile = (mt < 120 && g.N % 32 == 0 && g.N >= 64) ? g.N / 2 : g.N;
   const size_t need = tc_smem_layout(g, ntile).total;
   const size_t smem = need > 80 * 1024 ? need : 80 * 1024;
-  k_gemm_tc<<<dim3((unsigned)mt, (unsigned)(g.N / ntile)), 128, smem>>>(g, ntile, &nn->res->err, nn->tc_fault);
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 + TC_M * 256 * 2 + 256 * 256 * 2);
+    attr = true;
+  }
+  k_gemm_tc<<<dim3((unsigned)mt, (unsigned)(g.N / ntile)), 128, smem, s>>>(g, ntile, nn->tc_err, nn->tc_fault);
 }
 
-Gemm product(const bf16 *A, int lda, const bf16 *B, int M, int N, int K) {
+// a weight-gradient product on the tcgen05 path (A and B contiguous along M and N, K the batch)
+void gemm_tc_wgrad(mpcd_mlp *nn, cudaStream_t s, Gemm g) {
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(k_gemm_tc_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tcw_smem(256));
+    attr = true;
+  }
+  const int mt = (g.M + TC_M - 1) / TC_M;
+  // (N padded to the MMA's multiple of 16; the columns past N read as zero and are not stored)
+  const int np = (g.N + 15) & ~15;
+  const int ntile = (np % 32 == 0 && np >= 64) ? np / 2 : np;
+  // about 32 K slices of at least one stage each
+  const int per = (g.K + 31) / 32;
+  g.kchunk = ((per + TCW_K - 1) / TCW_K) * TCW_K;
+  const int kz = (g.K + g.kchunk - 1) / g.kchunk;
+  const size_t need = tcw_smem(ntile);
+  const size_t smem = need > 80 * 1024 ? need : 80 * 1024;  // (two CTAs per SM at most: TMEM fits)
+  k_gemm_tc_wgrad<<<dim3((unsigned)mt, (unsigned)(np / ntile), (unsigned)kz), 128, smem, s>>>(g, ntile, nn->tc_err,
+                                                                                           nn->tc_fault);
+}
+
+Gemm base() {
   Gemm g;
   memset(&g, 0, sizeof g);
-  g.A = A; g.lda = lda;
-  g.B = B; g.ldb = K;
-  g.M = M; g.N = N; g.K = K;
   return g;
 }
 
-// gradients of the mean loss over n rows into nn->g, and with update an Adam step; the loss sum and the
-// status of the waits into nn->res
-void gradients(mpcd_mlp *nn, const float *x, const float *y, int n, int update, float lr, float c1, float c2) {
-  k_features_in<<<(unsigned)(((long long)n * INP + 255) / 256), 256>>>(x, n, nn->xmean, nn->xistd, nn->X);
+const int kNpad[4] = {H, H, H, OUTP};
+const int kKpad[4] = {INP, H, H, H};
+
+long long bias_off(int l) {
+  long long o = 0;
+  for (int i = 0; i < l; ++i) o += kNpad[i];
+  return o;
+}
+
+// forward of rows [0, n) of n->X; stores Z (pre-activations) and A (activations) for the backward
+// pass
+void forward(mpcd_mlp *nn, int n, cudaStream_t s) {
+  const bf16 *in = nn->X;
+  long long ldin = INP;
   for (int l = 0; l < 4; ++l) {
-    Gemm g = product(l ? nn->A[l - 1] : nn->X, kKpad[l], nn->wt[l], n, kNpad[l], kKpad[l]);
-    g.bias = nn->bias + l * H;
+    Gemm g = base();
+    g.A = in; g.sam = ldin; g.sak = 1;
+    g.B = nn->wt[l]; g.sbk = 1; g.sbn = kKpad[l];
+    g.M = n; g.N = kNpad[l]; g.K = kKpad[l];
+    g.bias = nn->bias + bias_off(l);
     if (l < 3) {
       g.silu = 1;
       g.Zb = nn->Z[l]; g.ldzb = H;
       g.Cb = nn->A[l]; g.ldcb = H;
+      in = nn->A[l];
+      ldin = H;
     } else {
       g.Cf = nn->O; g.ldcf = OUTP;
     }
-    gemm_tc(nn, g);
+    gemm_tc(nn, s, g);
   }
-  k_nll<<<(unsigned)((n + 255) / 256), 256>>>(nn->O, y, n, nn->ymean, nn->yistd, nn->dO, nn->loss);
-  // d/d(pre-activation of layer l - 1) = (d/d(pre-activation of layer l) W_l^T) * silu'(Z_{l-1})
-  for (int l = 3; l > 0; --l) {
-    Gemm g = product(l < 3 ? nn->dZ[l] : nn->dO, kNpad[l], nn->w[l], n, H, kNpad[l]);
-    g.dz = nn->Z[l - 1]; g.lddz = H;
-    g.Cb = nn->dZ[l - 1]; g.ldcb = H;
-    gemm_tc(nn, g);
-  }
-  WgradArgs w;
-  for (int l = 0; l < 4; ++l) {
-    w.A[l] = l ? nn->A[l - 1] : nn->X;
-    w.B[l] = l < 3 ? nn->dZ[l] : nn->dO;
-  }
-  const int per = (n + TCW_SLICES - 1) / TCW_SLICES;
-  w.part = nn->part;
-  w.L = nn->L;
-  w.n = n;
-  w.kchunk = (per + TCW_K - 1) / TCW_K * TCW_K;
-  w.slices = (n + w.kchunk - 1) / w.kchunk;
-  w.loss = nn->loss;
-  w.lsum = nn->lsum;
-  const int parts = std::min(w.slices, nn->max_parts);
-  k_gemm_tc_wgrad<<<dim3(TCW_TILES + 1, (unsigned)parts), TCW_TH, TCW_SMEM>>>(w, &nn->res->err, nn->tc_fault);
-  const long long P = nn->L.total;
-  k_adam<<<(unsigned)((P + 255) / 256) + 1, 256>>>(nn->p, nn->part, parts, nn->g, nn->m, nn->v, P, update, lr, 0.9f,
-                                                  0.999f, 1e-8f, c1, c2, nn->L, copies(nn), nn->bias, nn->lsum, (n + 255) / 256,
-                                                  nn->res);
 }
 
-// gradients() and its status; loss: the mean over the batch
-int train(mpcd_mlp *nn, const float *x, const float *y, int n, int update, float lr, float c1, float c2, float *grad,
-          double *loss) {
-  if (!nn || !x || !y) return MPCD_ERR_PARAM;
-  if (n < 1 || n > nn->max_batch) return mfail(nn, MPCD_ERR_CAPACITY, "batch larger than max_batch");
-  gradients(nn, x, y, n, update, lr, c1, c2);
-  if (cudaGetLastError() != cudaSuccess) return mfail(nn, MPCD_ERR_CUDA, "training launch");
-  if (grad && cudaMemcpy(grad, nn->g, sizeof(float) * nn->L.total, cudaMemcpyDeviceToHost) != cudaSuccess)
-    return mfail(nn, MPCD_ERR_CUDA, "gradient download");
-  TrainResult r;
-  if (cudaMemcpy(&r, nn->res, sizeof r, cudaMemcpyDeviceToHost) != cudaSuccess)
-    return mfail(nn, MPCD_ERR_CUDA, "loss download");
-  if (r.err) {
-    // reported once; the next call starts afresh
-    cudaMemset(&nn->res->err, 0, sizeof(int));
-    return mfail(nn, MPCD_ERR_CUDA, "a tensor-core product did not complete within its time limit");
+// gradients of the mean loss over rows [0, n) into n->g (zeroed first)
+void backward(mpcd_mlp *nn, int n, cudaStream_t s) {
+  cudaMemsetAsync(nn->g, 0, sizeof(float) * nn->L.total, s);
+  const bf16 *dcur = nn->dO;  // gradient w.r.t. the output of layer l (after its activation)
+  long long ldd = OUTP;
+  for (int l = 3; l >= 0; --l) {
+    const int kin = nn->L.kin[l], nout = nn->L.nout[l];
+    const bf16 *act = l > 0 ? nn->A[l - 1] : nn->X;
+    const long long ldact = l > 0 ? H : INP;
+    // dW[k][c] = sum_b act[b][k] dcur[b][c]  (dcur is already d/d(pre-activation) of layer l)
+    Gemm gw = base();
+    gw.A = act; gw.sam = 1; gw.sak = ldact;
+    gw.B = dcur; gw.sbk = ldd; gw.sbn = 1;
+    gw.M = kin; gw.N = nout; gw.K = n;
+    gw.Cacc = nn->g + nn->L.w[l]; gw.ldca = nout;
+    gemm_tc_wgrad(nn, s, gw);
+    dim3 cg((nout + 127) / 128, n >= 4096 ? 32 : 1);
+    k_colsum<<<cg, 128, 0, s>>>(dcur, n, nout, ldd, nn->g + nn->L.b[l]);
+    if (l == 0) break;
+    // d/d(pre-activation of layer l-1) = (dcur W_l^T) * silu'(Z_{l-1})
+    Gemm gd = base();
+    gd.A = dcur; gd.sam = ldd; gd.sak = 1;
+    gd.B = nn->w[l]; gd.sbk = 1; gd.sbn = kNpad[l];  // B(k = c, n = i) = W_l[i][c]
+    gd.M = n; gd.N = H; gd.K = kNpad[l];
+    gd.dz = nn->Z[l - 1]; gd.lddz = H;
+    bf16 *dst = (l % 2) ? nn->dA : nn->dZ;
+    gd.Cb = dst; gd.ldcb = H;
+    gemm_tc(nn, s, gd);
+    dcur = dst;
+    ldd = H;
   }
-  if (loss) *loss = r.loss / n;
-  return MPCD_OK;
 }
 
 void init_params(mpcd_mlp *nn, uint64_t seed, std::vector<float> &h) {
@@ -920,8 +856,8 @@ int upload_params(mpcd_mlp *nn, const float *h) {
   // zero gradient, zero learning rate: writes the BF16 copies and biases from the masters
   cudaMemset(nn->g, 0, sizeof(float) * nn->L.total);
   const long long n = nn->L.total;
-  k_adam<<<(unsigned)((n + 255) / 256) + 1, 256>>>(nn->p, nn->g, 1, nn->g, nn->m, nn->v, n, 1, 0.f, 0.9f, 0.999f, 1e-8f,
-                                                  1.f, 1.f, nn->L, copies(nn), nn->bias, nn->lsum, 0, nn->res);
+  k_adam<<<(unsigned)((n + 255) / 256), 256>>>(nn->p, nn->g, nn->m, nn->v, n, 0.f, 0.9f, 0.999f, 1e-8f, 1.f, 1.f,
+                                              nn->L, copies(nn), nn->bias);
   cudaMemset(nn->m, 0, sizeof(float) * n);
   cudaMemset(nn->v, 0, sizeof(float) * n);
   return cudaDeviceSynchronize() == cudaSuccess ? MPCD_OK : mfail(nn, MPCD_ERR_CUDA, "parameter upload");
@@ -959,6 +895,13 @@ void infer(mpcd_mlp *nn, const float *x, int n, float *out, cudaStream_t s) {
   else infer_launch<4, 1, 3>(g, s);
 }
 
+int stage_inputs(mpcd_mlp *nn, const float *x, int n, cudaStream_t s) {
+  if (n < 1 || n > nn->max_batch) return mfail(nn, MPCD_ERR_CAPACITY, "batch larger than max_batch");
+  const long long tot = (long long)n * INP;
+  k_features_in<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(x, n, nn->xmean, nn->xistd, nn->X);
+  return MPCD_OK;
+}
+
 }  // namespace
 
 extern "C" int mpcd_mlp_create(int max_batch, uint64_t seed, mpcd_mlp **out) {
@@ -977,23 +920,21 @@ extern "C" int mpcd_mlp_create(int max_batch, uint64_t seed, mpcd_mlp **out) {
     nn->w[l] = dalloc<bf16>(nn, (size_t)kKpad[l] * kNpad[l]);
     nn->wt[l] = dalloc<bf16>(nn, (size_t)kKpad[l] * kNpad[l]);
   }
-  nn->res = dalloc<TrainResult>(nn, 1);
+  nn->tc_err = dalloc<int>(nn, 1);
   nn->bias = dalloc<float>(nn, 3 * H + OUTP);
   nn->xmean = dalloc<float>(nn, IN); nn->xistd = dalloc<float>(nn, IN);
   nn->ymean = dalloc<float>(nn, NY); nn->yistd = dalloc<float>(nn, NY);
   const size_t B = (size_t)max_batch;
   nn->X = dalloc<bf16>(nn, B * INP);
   for (int l = 0; l < 3; ++l) {
-    nn->A[l] = dalloc<bf16>(nn, B * H);
-    nn->dZ[l] = dalloc<bf16>(nn, B * H);
     nn->Z[l] = dalloc<bf16>(nn, B * H);
+    nn->A[l] = dalloc<bf16>(nn, B * H);
   }
-  nn->dO = dalloc<bf16>(nn, B * OUTP);
   nn->O = dalloc<float>(nn, B * OUTP);
-  nn->max_parts = std::max(1, nn->n_sm / TCW_TILES);
-  nn->part = dalloc<float>(nn, (size_t)nn->max_parts * P);
-  nn->loss = dalloc<float>(nn, B);
-  nn->lsum = dalloc<double>(nn, (B + 255) / 256);
+  nn->dO = dalloc<bf16>(nn, B * OUTP);
+  nn->dA = dalloc<bf16>(nn, B * H);
+  nn->dZ = dalloc<bf16>(nn, B * H);
+  nn->loss = dalloc<double>(nn, 1);
   if (!nn->err.empty()) {
     mpcd_mlp_destroy(nn);
     return MPCD_ERR_NOMEM;
@@ -1001,11 +942,7 @@ extern "C" int mpcd_mlp_create(int max_batch, uint64_t seed, mpcd_mlp **out) {
   std::vector<float> one(IN, 1.f), zero(IN, 0.f);
   cudaMemcpy(nn->xistd, one.data(), sizeof(float) * IN, cudaMemcpyHostToDevice);
   cudaMemcpy(nn->yistd, one.data(), sizeof(float) * NY, cudaMemcpyHostToDevice);
-  if (!infer_attr<1, 1, 6>() || !infer_attr<2, 1, 4>() || !infer_attr<4, 1, 3>() ||
-      cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           1024 + TC_M * 256 * 2 + 256 * 256 * 2) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(k_gemm_tc_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TCW_SMEM) != cudaSuccess) {
+  if (!infer_attr<1, 1, 6>() || !infer_attr<2, 1, 4>() || !infer_attr<4, 1, 3>()) {
     mpcd_mlp_destroy(nn);
     return MPCD_ERR_CUDA;
   }
@@ -1067,7 +1004,28 @@ extern "C" int mpcd_mlp_forward(mpcd_mlp *nn, const float *x, int n, float *out,
 }
 
 extern "C" int mpcd_mlp_grad(mpcd_mlp *nn, const float *x, const float *y, int n, float *grad, double *loss) {
-  return train(nn, x, y, n, 0, 0.f, 1.f, 1.f, grad, loss);
+  if (!nn || !x || !y) return MPCD_ERR_PARAM;
+  int r = stage_inputs(nn, x, n, nullptr);
+  if (r) return r;
+  forward(nn, n, nullptr);
+  cudaMemset(nn->loss, 0, sizeof(double));
+  k_nll<<<(n + 255) / 256, 256>>>(nn->O, y, n, nn->ymean, nn->yistd, nn->dO, nn->loss);
+  backward(nn, n, nullptr);
+  if (grad && cudaMemcpy(grad, nn->g, sizeof(float) * nn->L.total, cudaMemcpyDeviceToHost) != cudaSuccess)
+    return mfail(nn, MPCD_ERR_CUDA, "gradient download");
+  double l = 0;
+  if (cudaMemcpy(&l, nn->loss, sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess)
+    return mfail(nn, MPCD_ERR_CUDA, "loss download");
+  int te = 0;
+  if (cudaMemcpy(&te, nn->tc_err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+    return mfail(nn, MPCD_ERR_CUDA, "status download");
+  if (te) {
+    // reported once; the next call starts afresh
+    cudaMemset(nn->tc_err, 0, sizeof(int));
+    return mfail(nn, MPCD_ERR_CUDA, "a tensor-core product did not complete within its time limit");
+  }
+  if (loss) *loss = l / n;
+  return MPCD_OK;
 }
 
 extern "C" int mpcd_mlp_set_fault(mpcd_mlp *nn, int on) {
@@ -1077,12 +1035,15 @@ extern "C" int mpcd_mlp_set_fault(mpcd_mlp *nn, int on) {
 }
 
 extern "C" int mpcd_mlp_train_step(mpcd_mlp *nn, const float *x, const float *y, int n, float lr, double *loss) {
-  if (!nn) return MPCD_ERR_PARAM;
-  const float t = (float)(nn->adam_t + 1);
-  const float c1 = 1.f / (1.f - std::pow(0.9f, t)), c2 = 1.f / (1.f - std::pow(0.999f, t));
-  const int r = train(nn, x, y, n, 1, lr, c1, c2, nullptr, loss);
-  if (r == MPCD_OK) nn->adam_t += 1;
-  return r;
+  int r = mpcd_mlp_grad(nn, x, y, n, nullptr, loss);
+  if (r) return r;
+  nn->adam_t += 1;
+  const float b1 = 0.9f, b2 = 0.999f;
+  const float c1 = 1.f / (1.f - std::pow(b1, (float)nn->adam_t)), c2 = 1.f / (1.f - std::pow(b2, (float)nn->adam_t));
+  const long long P = nn->L.total;
+  k_adam<<<(unsigned)((P + 255) / 256), 256>>>(nn->p, nn->g, nn->m, nn->v, P, lr, b1, b2, 1e-8f, c1, c2, nn->L,
+                                              copies(nn), nn->bias);
+  return cudaGetLastError() == cudaSuccess ? MPCD_OK : mfail(nn, MPCD_ERR_CUDA, "adam launch");
 }
 
 MlpIO mlp_io(mpcd_mlp *nn) {
