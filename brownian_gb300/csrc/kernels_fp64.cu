@@ -1059,6 +1059,7 @@ __global__ void __launch_bounds__(128) k_colloid_setup(const SysF64 S) {
     S.ss->nevents = 0;
     S.ss->nnew[0] = S.ss->nnew[1] = 0;
     S.ss->npend = 0;
+    S.ss->crowd = 0;
     S.ss->cm = S.cmarginf;  // the static bound until a step has measured the colloids
     S.ss->cm2 = S.cmargin2;
   }
@@ -1644,6 +1645,7 @@ __global__ void __launch_bounds__(256) k_rotdiff_step_b(const SysF64 *Ss, const 
 __global__ void __launch_bounds__(256) k_table_next(const SysF64 S) {
   const int j = blockIdx.x;
   if (j >= S.Nc) return;
+  if (S.ss->crowd == S.ss->step) return;  // (a step with crowded cells has built it)
   const long long g = S.ss->step * S.n_sub;
   const int b = (int)(g & 1);
   int *err = &S.ss->err;

@@ -1,0 +1,121 @@
+"""Cells that list more colloids than a cell table holds (16) in a step's flight table, whose reach
+is longer: the free-flight step then builds the cell tables for their capacity check.  A run that
+goes from it to a schedule that reads them goes on with the bits of one that never left that
+schedule."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+STATE = ("pos_fl", "vel_fl", "pos_colloid", "vel_colloid", "ang_vel_colloid", "ra")
+
+
+def _outside(X):
+    """Uniform positions in the 32^3 box outside the spheres."""
+    pos = np.random.default_rng(1).uniform(0.01, 31.99, (200_000, 3))
+    free = np.ones(len(pos), bool)
+    for x in X:
+        d = pos - x
+        d -= 32 * np.round(d / 32)
+        free &= (d * d).sum(1) > 9.2
+    return pos[free][:90_000]
+
+
+def _crowd(form, as_params=False):
+    """32^3 cells, 41 spheres of radius 3 (free to overlap) in a cube of side 10.33: up to 14 colloids in
+    a cell table, 23 in a flight cell, and no particle in the run() shells of more than 6."""
+    import brownian_gb300 as bg
+    rng = np.random.default_rng(206)
+    n, side = rng.integers(20, 60), rng.uniform(8, 14)
+    X = 16 - side / 2 + rng.uniform(0, side, (n, 3))
+    rng = np.random.default_rng(1)
+    M = bg.displaced_mass(3.0, 10)
+    pos = _outside(X)
+    ra = rng.normal(0, 1, (n, 3))
+    state = dict(pos_fl=pos, vel_fl=rng.normal(0, 1, pos.shape), pos_colloid=X,
+                 vel_colloid=rng.normal(0, M ** -0.5, (n, 3)), ang_vel_colloid=np.zeros((n, 3)),
+                 ra=ra / np.linalg.norm(ra, axis=1, keepdims=True))
+    kw = dict(n_sub=10, mass_colloid=M, sig_colloid=0.01, sigma=6.0, I_colloid=0.4 * M * 9.0, v0=0.0, theta_deg=90.0,
+              Dr=0.001, seed=3, precision=bg.FP64 if form == "fp64" else bg.FP32C)
+    p = bg.make_params(32, len(pos), int(n), **kw)
+    return (p, state) if as_params else (_start(bg.Simulation(32, len(pos), int(n), **kw), state), state)
+
+
+def _start(sim, state):
+    sim.set_state(*[state[k] for k in STATE])
+    sim.setup()
+    return sim
+
+
+def _same(a, b):
+    x, y = a.get_state(), b.get_state()
+    for k in x:
+        assert np.array_equal(x[k], y[k]), k
+
+
+def _by_routine(sim, form):
+    sim.rotation_mpcd()
+    sim.run()
+    for l in range(1, 11):
+        sim.substep_routines() if form == "fp64" else sim.substep(l)
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp32c"])
+def test_a_schedule_that_reads_the_tables_goes_on_from_a_crowded_step(form):
+    a, _ = _crowd(form)
+    b, _ = _crowd(form)
+    b.set_flight(False)
+    for flight, k in ((True, 1), (False, 2), (True, 3), (False, 1)):
+        a.set_flight(flight)
+        a.step(k)
+        b.step(k)
+        _same(a, b)
+    a.set_flight(True)
+    for _ in range(2):
+        a.step(1)
+        b.step(1)
+        _by_routine(a, form)
+        _by_routine(b, form)
+        _same(a, b)
+    a.close()
+    b.close()
+
+
+def test_an_ensemble_goes_on_from_a_crowded_step():
+    import brownian_gb300 as bg
+    p, state = _crowd("fp32c", as_params=True)
+    a, b = bg.Ensemble([p, p]), bg.Ensemble([p, p])
+    b.set_flight(False)
+    for e in (a, b):
+        for s in e:
+            _start(s, state)
+    for flight, k in ((True, 2), (False, 1), (True, 1), (False, 2)):
+        a.set_flight(flight)
+        a.step(k)
+        b.step(k)
+        for x, y in zip(a, b):
+            _same(x, y)
+    a.close()
+    b.close()
+
+
+def test_another_state_at_the_step_after_a_crowded_one():
+    # the mark of the crowded step does not outlive the state that it was made for
+    a, state = _crowd("fp64")
+    a.step(6)
+    spread = dict(state)
+    grid = np.stack(np.meshgrid(*[np.arange(4) * 8.0 + 4.3] * 3), -1).reshape(-1, 3)
+    spread["pos_colloid"] = grid[:len(state["pos_colloid"])]
+    spread["pos_fl"] = _outside(spread["pos_colloid"])
+    b, _ = _crowd("fp64")
+    b.set_flight(False)
+    for s in (a, b):
+        s.step_count = 5
+        _start(s, spread)
+        s.step(1)
+    a.set_flight(False)
+    for s in (a, b):
+        s.step(2)
+    _same(a, b)
+    a.close()
+    b.close()
