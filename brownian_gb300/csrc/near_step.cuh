@@ -339,6 +339,16 @@ static __device__ __forceinline__ void near_forces(const SysF64 &S, NearPairs &p
   }
 }
 
+// The cell table that the per-substep passes would read in substep e, from the positions before it,
+// the block's colloids (thread t of nt).  The step's last one is that of the next step's first
+// substep (k_table_next then has none to build).
+static __device__ __noinline__ void near_tables(const SysF64 &S, int VB, int G, long long e, int t, int nt) {
+  const int b = (int)((e - 1) & 1);
+  for (int j = VB; j < S.Nc; j += G)
+    for_reach_cells(S, S.cbox[b][j], S.Xf[b][j], table_reach(S, e), t, nt,
+                    [&](int cell) { tappend(S.Tcnt[e & 1], S.Tlist[e & 1], cell, e, j, &S.ss->err); });
+}
+
 // The colloid group of a block (t: thread of the group): colloids VB, VB + G, ... through the
 // substeps.  A colloid has eight lanes (four colloids a warp): lane k < 3 the linear component
 // k, lane 3 + k the angular one, so that an FP64 instruction, which occupies the SM's FP64 unit
@@ -359,6 +369,8 @@ static __device__ __forceinline__ void near_colloids(const SysF64 &S, NearPairs 
   const bool crowd = S.ss->crowd == step + 1;
   const Dim &D = k == 0 ? S.dx : (k == 1 ? S.dy : S.dz);
   const int Lk = k == 0 ? S.Lx : (k == 1 ? S.Ly : S.Lz);
+  // some cell may hold more colloids than a cell table: the tables are built for their capacity check
+  if (crowd) near_tables(S, VB, G, g0 + 1, t, NT);
   for (int l = 1; l <= n; ++l) {
     const long long g = g0 + (l - 1);
     const int cur = (int)(g & 1), nxt = cur ^ 1;
@@ -439,16 +451,7 @@ static __device__ __forceinline__ void near_colloids(const SysF64 &S, NearPairs 
       *fin = l;  // (the orientation warp follows)
     }
     if (l == n) return;
-    if (crowd) {
-      // some cell may hold more colloids than a cell table: build the tables the per-substep
-      // passes would read, for their capacity check
-      const long long e = g + 2;
-      for (int s = 0; s < M; ++s) {
-        const int j = VB + G * s;
-        for_reach_cells(S, S.cbox[nxt][j], S.Xf[nxt][j], table_reach(S, e), t, NT,
-                        [&](int cell) { tappend(S.Tcnt[e & 1], S.Tlist[e & 1], cell, e, j, &S.ss->err); });
-      }
-    }
+    if (crowd) near_tables(S, VB, G, g + 2, t, NT);
     if (t == 0) bar_arrive(S.bar + BAR_MOVE);
   }
   if (t == 0) *fin = -1;  // (a wait ran out)

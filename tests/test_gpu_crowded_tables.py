@@ -1,7 +1,7 @@
 """Cells that list more colloids than a cell table holds (16) in a step's flight table, whose reach
 is longer: the free-flight step then builds the cell tables for their capacity check.  A run that
 goes from it to a schedule that reads them goes on with the bits of one that never left that
-schedule."""
+schedule, and a table that overflows is refused in the same step."""
 import numpy as np
 import pytest
 
@@ -119,3 +119,34 @@ def test_another_state_at_the_step_after_a_crowded_one():
     _same(a, b)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp32c"])
+@pytest.mark.parametrize("n_sub", [2, 3, 10])
+def test_a_table_that_overflows_is_refused_in_the_same_step(form, n_sub):
+    # 16 spheres around one point and one that comes within reach of a cell of the last substep's table
+    # (whose reach is the run() shell's), never of the others'
+    import brownian_gb300 as bg
+    rng = np.random.default_rng(7)
+    M = 200.0
+    X = np.concatenate([10.5 + rng.uniform(-0.02, 0.02, (16, 3)), [[14.75, 10.5, 10.5]]])
+    V = np.zeros((17, 3))
+    V[16, 0] = -0.15
+    pos = rng.uniform(0, 1, (2000, 3)) * [4.0, 23.9, 23.9] + [18.5, 0.05, 0.05]
+    state = dict(pos_fl=pos, vel_fl=0.5 * rng.normal(0, 1, pos.shape), pos_colloid=X, vel_colloid=V,
+                 ang_vel_colloid=np.zeros((17, 3)), ra=np.tile([1.0, 0.0, 0.0], (17, 1)))
+    refused = []
+    for flight in (True, False):
+        sim = bg.Simulation(24, 2000, 17, n_sub=n_sub, mass_colloid=M, sig_colloid=0.001, sigma=2.0, I_colloid=80.0,
+                            theta_deg=90.0, seed=3, precision=bg.FP64 if form == "fp64" else bg.FP32C)
+        sim.set_flight(flight)
+        _start(sim, state)
+        for k in range(12):
+            try:
+                sim.step(1)
+            except bg.MPCDError as e:
+                assert e.code == bg.ERR_CAPACITY and "table" in str(e)
+                refused.append(k)
+                break
+        sim.close()
+    assert len(refused) == 2 and refused[0] == refused[1] > 0, refused
