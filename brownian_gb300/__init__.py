@@ -27,6 +27,7 @@ EXPORTS = ["mpcd_create", "mpcd_destroy", "mpcd_last_error", "mpcd_set_stream", 
            "mpcd_neighbour_list_mpcd", "mpcd_fluid_colloid_collision", "mpcd_update_activity_direction",
            "mpcd_compute_force_md", "mpcd_update_velocity_colloid", "mpcd_get_neighbour_md", "mpcd_get_box_binning",
            "mpcd_step", "mpcd_step_async", "mpcd_sync", "mpcd_set_flight", "mpcd_get_flight", "mpcd_diag", "mpcd_get_rotation_binning", "mpcd_get_shell_count",
+           "mpcd_set_fault", "mpcd_ensemble_set_fault",
            "mpcd_profile_enable", "mpcd_profile_read", "mpcd_trace_step", "mpcd_launch_count", "mpcd_set_launch",
            "mpcd_fluid_sums_noalloc", "mpcd_ensemble_create", "mpcd_ensemble_destroy", "mpcd_ensemble_last_error",
            "mpcd_ensemble_system", "mpcd_ensemble_step", "mpcd_ensemble_set_launch", "mpcd_ensemble_launch_count",
@@ -47,6 +48,7 @@ ENS_EVENTS, ENS_RUN, ENS_FIN, ENS_AUX, ENS_FREE = 0, 1, 2, 3, 4
 NOALLOC_MAX_PARTICLES = 33554432
 PHYSICS_REFERENCE, PHYSICS_FIXED = 0, 1
 LAUNCH_EVENTS, LAUNCH_FIN, LAUNCH_AUX, LAUNCH_FREE = 0, 1, 2, 3
+FAULT_LAUNCH = 0
 
 
 class MPCDError(RuntimeError):
@@ -123,6 +125,7 @@ def lib():
         L.mpcd_launch_count.argtypes = [vp]
         L.mpcd_launch_count.restype = C.c_int64
         L.mpcd_set_launch.argtypes = [vp, C.c_int, C.c_int, C.c_int]
+        L.mpcd_set_fault.argtypes = [vp, C.c_int, C.c_int]
         L.mpcd_fluid_sums_noalloc.argtypes = [vp, C.c_int64, C.c_double, vp, vp]
         L.mpcd_exchange_read.argtypes = [vp, dp, C.c_int]
         L.mpcd_updown_velocity.argtypes = [vp, C.POINTER(C.c_int32), C.POINTER(C.c_int32), dp, dp]
@@ -149,6 +152,7 @@ def lib():
         L.mpcd_ensemble_launch_count.restype = C.c_int64
         L.mpcd_ensemble_set_flight.argtypes = [vp, C.c_int]
         L.mpcd_ensemble_get_flight.argtypes = [vp]
+        L.mpcd_ensemble_set_fault.argtypes = [vp, C.c_int, C.c_int]
         _lib = L
     return _lib
 
@@ -518,6 +522,10 @@ class Simulation:
         32 for the finish)."""
         self._ck(lib().mpcd_set_launch(self.h, which, grid, block))
 
+    def set_fault(self, what, value):
+        """Test hook: makes a check of the step fail from the host (FAULT_*)."""
+        self._ck(lib().mpcd_set_fault(self.h, what, value))
+
     @property
     def launch_count(self):
         return lib().mpcd_launch_count(self.h)
@@ -558,6 +566,10 @@ class Ensemble:
         """The batched step's schedule: free flight (default) or one pass per substep
         over every particle; both leave the same bits."""
         self._ck(lib().mpcd_ensemble_set_flight(self.h, 1 if on else 0))
+
+    def set_fault(self, what, value):
+        """Test hook: makes a check of the step fail from the host (FAULT_*)."""
+        self._ck(lib().mpcd_ensemble_set_fault(self.h, what, value))
 
     @property
     def flight(self):

@@ -74,6 +74,8 @@ struct mpcd_ctx {
   bool tables_stale = false;     // the last step was a free-flight one on k_near_step: the cell table of the next
                                  // step's first substep is not built (ensure_tables)
   std::string err;
+  cudaError_t launch_err = cudaSuccess;  // the first launch that was refused since launch_status
+  bool fault_launch = false;     // test hook (mpcd_set_fault)
   int64_t launches = 0;
   bool profile = false;
   std::vector<ProfEvent> pending;
@@ -154,30 +156,15 @@ static cudaEvent_t pool_event(mpcd_ctx *c) {
   return e;
 }
 
-template <typename... KArgs, typename... Args>
-static void launch_on(mpcd_ctx *c, cudaStream_t s, const char *name, void (*k)(KArgs...), dim3 g, dim3 b,
-                      Args... args) {
-  ProfEvent pe{name, nullptr, nullptr};
-  if (c->profile || c->tracing) {
-    pe.a = pool_event(c);
-    pe.b = pool_event(c);
-    // (in a traced capture the records become nodes of the graph)
-    cudaEventRecordWithFlags(pe.a, s, c->tracing ? cudaEventRecordExternal : cudaEventRecordDefault);
-  }
-  k<<<g, b, 0, s>>>(args...);
-  c->launches++;
-  if (c->profile || c->tracing) {
-    cudaEventRecordWithFlags(pe.b, s, c->tracing ? cudaEventRecordExternal : cudaEventRecordDefault);
-    (c->tracing ? c->trace : c->pending).push_back(pe);
-  }
-}
+// PLAIN; COOP: cooperative (its blocks wait on one another); DEPENDENT: it starts when every block of
+// the kernel before it on the stream has let it, not when that has ended
+enum LaunchKind { PLAIN, COOP, DEPENDENT };
 
-// a launch with one launch attribute: cooperative (its blocks wait on one another), or dependent (it
-// starts when every block of the kernel before it on the stream has let it, not when that has ended)
 template <typename... KArgs, typename... Args>
-static void launch_with(cudaStream_t s, bool coop, void (*k)(KArgs...), int grid, int block, size_t smem, Args... args) {
+static cudaError_t launch_with(cudaStream_t s, LaunchKind kind, void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                               Args... args) {
   cudaLaunchAttribute at;
-  if (coop) {
+  if (kind == COOP) {
     at.id = cudaLaunchAttributeCooperative;
     at.val.cooperative = 1;
   } else {
@@ -185,25 +172,29 @@ static void launch_with(cudaStream_t s, bool coop, void (*k)(KArgs...), int grid
     at.val.programmaticStreamSerializationAllowed = 1;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k, args...);
+  cfg.numAttrs = kind == PLAIN ? 0 : 1;
+  return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
+// a launch's status is kept until launch_status asks for it
 template <typename... KArgs, typename... Args>
-static void launch_attr(mpcd_ctx *c, cudaStream_t s, const char *name, bool coop, void (*k)(KArgs...), int grid,
-                        int block, size_t smem, Args... args) {
+static void launch_attr(mpcd_ctx *c, cudaStream_t s, const char *name, LaunchKind kind, void (*k)(KArgs...), dim3 grid,
+                        dim3 block, size_t smem, Args... args) {
   ProfEvent pe{name, nullptr, nullptr};
   if (c->profile || c->tracing) {
     pe.a = pool_event(c);
     pe.b = pool_event(c);
+    // (in a traced capture the records become nodes of the graph)
     cudaEventRecordWithFlags(pe.a, s, c->tracing ? cudaEventRecordExternal : cudaEventRecordDefault);
   }
-  launch_with(s, coop, k, grid, block, smem, args...);
+  const cudaError_t e = kind == COOP && c->fault_launch ? cudaErrorCooperativeLaunchTooLarge
+                                                        : launch_with(s, kind, k, grid, block, smem, args...);
+  if (e != cudaSuccess && c->launch_err == cudaSuccess) c->launch_err = e;
   c->launches++;
   if (c->profile || c->tracing) {
     cudaEventRecordWithFlags(pe.b, s, c->tracing ? cudaEventRecordExternal : cudaEventRecordDefault);
@@ -212,8 +203,23 @@ static void launch_attr(mpcd_ctx *c, cudaStream_t s, const char *name, bool coop
 }
 
 template <typename... KArgs, typename... Args>
+static void launch_on(mpcd_ctx *c, cudaStream_t s, const char *name, void (*k)(KArgs...), dim3 g, dim3 b,
+                      Args... args) {
+  launch_attr(c, s, name, PLAIN, k, g, b, 0, args...);
+}
+
+template <typename... KArgs, typename... Args>
 static void launch(mpcd_ctx *c, const char *name, void (*k)(KArgs...), dim3 g, dim3 b, Args... args) {
   launch_on(c, c->stream, name, k, g, b, args...);
+}
+
+// whether every launch since the last call was taken
+static int launch_status(mpcd_ctx *c) {
+  const cudaError_t e = c->launch_err;
+  if (e == cudaSuccess) return MPCD_OK;
+  c->launch_err = cudaSuccess;
+  cudaGetLastError();  // (the same one: reported here)
+  return fail(c, MPCD_ERR_CUDA, std::string("a launch was refused: ") + cudaGetErrorString(e));
 }
 
 // a copy ordered on the context's stream (which does not synchronise with the
@@ -611,10 +617,10 @@ static void enq_step_near(mpcd_ctx *c, bool sort) {
   cudaStreamWaitEvent(c->nst, c->ev_cls, 0);
   cudaStreamWaitEvent(c->nst, c->ev_aux, 0);
   cudaStreamWaitEvent(c->nst, c->ev_str, 0);
-  launch_attr(c, c->nst, "k_stream_near", true, f32 ? k_near_step32 : k_near_step64, c->n_sm,
+  launch_attr(c, c->nst, "k_stream_near", COOP, f32 ? k_near_step32 : k_near_step64, c->n_sm,
               f32 ? NEAR32_BLOCK : NEAR64_BLOCK, f32 ? near_step32_smem() : near_step64_smem(), S, c->fbuf);
   cudaEventRecord(c->ev_end, c->nst);
-  launch_attr(c, c->nst, "k_free_flight", false, f32 ? k_free_flight32 : k_free_flight, free_blocks(c), 256, 0, S,
+  launch_attr(c, c->nst, "k_free_flight", DEPENDENT, f32 ? k_free_flight32 : k_free_flight, free_blocks(c), 256, 0, S,
               c->fbuf, 2);
   cudaEventRecord(c->ev_free, c->nst);
   cudaStreamWaitEvent(c->stream, c->ev_end, 0);
@@ -698,6 +704,7 @@ static int err_code(int bits) {
 static int check_device(mpcd_ctx *c) {
   CUDA_OK(c, cudaMemcpyAsync(c->ss_host, c->S.ss, sizeof(StepState), cudaMemcpyDeviceToHost, c->stream));
   CUDA_OK(c, cudaStreamSynchronize(c->stream));
+  if (int r = launch_status(c)) return r;
   CUDA_OK(c, cudaGetLastError());
   if (c->profile) collect_profile(c);
   int bits = c->ss_host->err;
@@ -1239,6 +1246,13 @@ extern "C" int mpcd_set_launch(mpcd_ctx *c, int which, int grid, int block) {
   return drop_graph(c);
 }
 
+extern "C" int mpcd_set_fault(mpcd_ctx *c, int what, int value) {
+  if (!c) return MPCD_ERR_PARAM;
+  if (what != MPCD_FAULT_LAUNCH) return fail(c, MPCD_ERR_PARAM, "unknown fault");
+  c->fault_launch = value != 0;
+  return drop_graph(c);
+}
+
 extern "C" int mpcd_set_flight(mpcd_ctx *c, int on) {
   if (!c) return MPCD_ERR_PARAM;
   c->flight = on != 0;
@@ -1338,10 +1352,44 @@ extern "C" int mpcd_substep(mpcd_ctx *c, int l) {
   return check_device(c);
 }
 
-// before whole steps are enqueued: the table their schedule reads, or the note that they leave none
-static void begin_steps(mpcd_ctx *c) {
+// before whole steps are enqueued: the table their schedule reads; once they are, the note that
+// they leave none
+static int begin_steps(mpcd_ctx *c) {
+  if (!(c->flight && c->near_step)) ensure_tables(c);
+  return launch_status(c);
+}
+
+static void end_steps(mpcd_ctx *c, int n) {
+  c->host_step += n;
   if (c->flight && c->near_step) c->tables_stale = true;
-  else ensure_tables(c);
+}
+
+// n steps captured into a graph (`sort`: one that sorts), after a record of `start` if there is one;
+// nothing is kept of one with a refused launch
+static int capture_steps(mpcd_ctx *c, int n, bool sort, cudaGraphExec_t *exec, int *launches,
+                         cudaEvent_t start = nullptr) {
+  const int b = c->fbuf;
+  const int64_t before = c->launches;
+  cudaGraph_t g = nullptr;
+  CUDA_OK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+  if (start) cudaEventRecordWithFlags(start, c->stream, cudaEventRecordExternal);
+  for (int k = 0; k < n; ++k) enq_step(c, sort);
+  cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+  c->fbuf = b;  // capture only recorded the launches
+  *launches = (int)(c->launches - before);
+  c->launches = before;
+  int r = launch_status(c);
+  if (!r && e == cudaSuccess) {
+    cudaGraphExec_t x = nullptr;
+    e = cudaGraphInstantiate(&x, g, 0);
+    if (e == cudaSuccess) *exec = x;
+  }
+  if (g) cudaGraphDestroy(g);
+  if (!r && e != cudaSuccess) {
+    cudaGetLastError();
+    r = fail(c, MPCD_ERR_CUDA, std::string("capture of a step: ") + cudaGetErrorString(e));
+  }
+  return r;
 }
 
 constexpr int GRAPH_STEPS = 3;
@@ -1352,13 +1400,13 @@ static int enq_steps(mpcd_ctx *c, int nsteps) {
   if ((r = need_setup(c))) return r;
   if (nsteps < 0) return MPCD_ERR_PARAM;
   if (c->phase != 0) return fail(c, MPCD_ERR_STATE, "a step begun routine by routine is unfinished");
-  if (nsteps > 0) begin_steps(c);
+  if (nsteps > 0 && (r = begin_steps(c))) return r;
   if (c->profile) {
     for (int s = 0; s < nsteps; ++s) {
       enq_step(c, sorts_at(c, c->host_step));
-      c->host_step += 1;
+      end_steps(c, 1);
     }
-    return MPCD_OK;
+    return launch_status(c);
   }
   for (int s = 0; s < nsteps;) {
     // one graph per (sorts this step, fluid buffer): the kernels' buffer arguments are fixed at
@@ -1368,23 +1416,13 @@ static int enq_steps(mpcd_ctx *c, int nsteps) {
     while (n < GRAPH_STEPS && s + n < nsteps && !sorts_at(c, c->host_step + n)) ++n;
     if (n < GRAPH_STEPS) n = 1;
     const int kind = n > 1 ? 2 : (sorts_at(c, c->host_step) ? 1 : 0), b = c->fbuf;
-    if (!c->step_exec[kind][b]) {
-      cudaGraph_t g;
-      int64_t before = c->launches;
-      CUDA_OK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-      for (int k = 0; k < n; ++k) enq_step(c, kind == 1);
-      CUDA_OK(c, cudaStreamEndCapture(c->stream, &g));
-      c->fbuf = b;  // capture only recorded the launches
-      c->step_launches[kind][b] = (int)(c->launches - before);
-      c->launches = before;
-      cudaError_t e = cudaGraphInstantiate(&c->step_exec[kind][b], g, 0);
-      cudaGraphDestroy(g);
-      if (e != cudaSuccess) return fail(c, MPCD_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-    }
+    if (!c->step_exec[kind][b] &&
+        (r = capture_steps(c, n, kind == 1, &c->step_exec[kind][b], &c->step_launches[kind][b])))
+      return r;
     CUDA_OK(c, cudaGraphLaunch(c->step_exec[kind][b], c->stream));
     c->launches += c->step_launches[kind][b];
     if (kind == 1) c->fbuf = 1 - b;
-    c->host_step += n;
+    end_steps(c, n);
     s += n;
   }
   return MPCD_OK;
@@ -1430,6 +1468,7 @@ extern "C" int mpcd_diag(mpcd_ctx *c, mpcd_diag_t *out) {
   }
   CUDA_OK(c, cudaMemsetAsync(&S.ss->ev_total, 0, sizeof(long long), c->stream));
   CUDA_OK(c, cudaStreamSynchronize(c->stream));
+  if ((r = launch_status(c))) return r;
   CUDA_OK(c, cudaGetLastError());
   if (c->profile) collect_profile(c);
   if (int bits = c->ss_host->err) {
@@ -1536,31 +1575,23 @@ extern "C" int mpcd_trace_step(mpcd_ctx *c, char names[][48], double *t0_ms, dou
   if ((r = need_setup(c))) return r;
   if (c->phase != 0) return fail(c, MPCD_ERR_STATE, "a step begun routine by routine is unfinished");
   if (c->profile) return fail(c, MPCD_ERR_STATE, "profiling is on");
-  begin_steps(c);
+  if ((r = begin_steps(c))) return -r;
   const int sort = sorts_at(c, c->host_step) ? 1 : 0, b = c->fbuf;
   cudaEvent_t start = pool_event(c);
-  cudaGraph_t g;
   cudaGraphExec_t x = nullptr;
+  int launches = 0;
   c->trace.clear();
-  CUDA_OK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  cudaEventRecordWithFlags(start, c->stream, cudaEventRecordExternal);
   c->tracing = true;
-  const int64_t before = c->launches;
-  enq_step(c, sort != 0);
+  r = capture_steps(c, 1, sort != 0, &x, &launches, start);
   c->tracing = false;
-  c->launches = before;
-  c->fbuf = b;
-  CUDA_OK(c, cudaStreamEndCapture(c->stream, &g));
-  cudaError_t e = cudaGraphInstantiate(&x, g, 0);
-  cudaGraphDestroy(g);
-  if (e != cudaSuccess) return fail(c, MPCD_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-  e = cudaGraphLaunch(x, c->stream);
+  if (r) return -r;
+  cudaError_t e = cudaGraphLaunch(x, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   cudaGraphExecDestroy(x);
   if (e != cudaSuccess) return fail(c, MPCD_ERR_CUDA, std::string("traced step: ") + cudaGetErrorString(e));
   c->launches += (int64_t)c->trace.size();
   if (sort) c->fbuf = 1 - b;
-  c->host_step += 1;
+  end_steps(c, 1);
   int i = 0;
   for (auto &pe : c->trace) {
     if (i < cap) {

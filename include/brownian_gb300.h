@@ -228,6 +228,12 @@ enum { MPCD_LAUNCH_EVENTS = 0, /* wall-collision events: grid, block (<= 128, mu
  * whose substeps are one kernel has none of these launches. */
 int mpcd_set_launch(mpcd_ctx *c, int which, int grid, int block);
 
+/* ---- failure detection (test hooks: each makes a check fail from the host) ---------------- */
+enum { MPCD_FAULT_LAUNCH = 0 }; /* value 1: the substeps' cooperative launch is refused (0: it is
+                                   launched): a step fails with MPCD_ERR_CUDA, nothing of it runs
+                                   and nothing of its capture is kept */
+int mpcd_set_fault(mpcd_ctx *c, int what, int value);
+
 /* ---- exchange record (no counterpart in the reference) ------------------------------- */
 /* The momentum (m sum dv, 3) and angular momentum (m sum r x dv, 3) the fluid gave each colloid
  * in the stochastic reflections (cpp/fluid_colloid_collision.cpp:46-47) since the last reset:
@@ -295,6 +301,8 @@ int64_t mpcd_ensemble_launch_count(const mpcd_ensemble *e);
  * leave the same bits. */
 int mpcd_ensemble_set_flight(mpcd_ensemble *e, int on);
 int mpcd_ensemble_get_flight(const mpcd_ensemble *e);
+/* mpcd_set_fault for the batched step */
+int mpcd_ensemble_set_fault(mpcd_ensemble *e, int what, int value);
 
 /* ---- learned closure network (no counterpart in the reference) ----------------------- */
 /* MLP 81 -> 256 -> 256 -> 256 -> 12 with SiLU, BF16 weights on the tensor cores with FP32
