@@ -61,7 +61,8 @@ struct mpcd_ctx {
   cudaStream_t nst = nullptr;
   cudaEvent_t ev_tab = nullptr, ev_cls = nullptr, ev_end = nullptr, ev_list = nullptr, ev_free = nullptr;
   bool flight = true;
-  bool near_step = false;        // its substeps in one cooperative kernel (enq_step_near)
+  bool near_sized = false;       // the system's sizes let its substeps run in one cooperative kernel
+  bool near_step = false;        // and that kernel can be launched: it is (enq_step_near)
   cudaStream_t evs = nullptr;    // third stream (FP64 form): event passes and colloid finish
   cudaEvent_t ev_start = nullptr, ev_str = nullptr, ev_aux = nullptr, ev_finp[2] = {nullptr, nullptr};
 
@@ -727,6 +728,32 @@ static int drop_graph(mpcd_ctx *c) {
   return MPCD_OK;
 }
 
+// ---------------------------------------------------------------- the substeps' kernel
+
+// whether cooperative kernel k (block threads, smem bytes) can be launched with a block on every SM;
+// ff, the free-flight pass that shares the SMs with it, gets the same shared-memory split
+static bool near_fits(const void *k, int block, size_t smem, const void *ff) {
+  int dev = 0, coop = 0, blocks = 0;
+  const bool ok =
+      cudaGetDevice(&dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+      cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess &&
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, block, smem) == cudaSuccess && blocks >= 1 &&
+      cudaFuncSetAttribute(ff, cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+
+// the substeps in one cooperative kernel where the system's sizes and the device allow it (no_room: as if
+// the device did not), else a launch per stage
+static void choose_near_step(mpcd_ctx *c, bool no_room) {
+  const bool f32 = c->S.precision == MPCD_FP32C;
+  c->near_step = c->near_sized && !no_room &&
+                 (f32 ? near_fits((const void *)k_near_step32, NEAR32_BLOCK, near_step32_smem(), (const void *)k_free_flight32)
+                      : near_fits((const void *)k_near_step64, NEAR64_BLOCK, near_step64_smem(), (const void *)k_free_flight));
+}
+
 // ---------------------------------------------------------------- lifetime
 
 extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
@@ -903,11 +930,11 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
     // substep; substep numbers in 16 bits.)
     const double reach = S.r_shell + S.flight_rx + S.n_sub * cmargin + 0.02 + 0.62;  // + a cell's radius as a ball
     const double expected = (double)S.Nc / (double)S.C * 4.0 / 3.0 * M_PI * reach * reach * reach;
-    c->near_step =
+    c->near_sized =
         S.Nc > 0 && S.n_sub >= 2 && S.n_sub <= 4096 && expected <= 8.0 && (long long)S.Nc * S.n_sub <= (1ll << 24);
-    if (c->near_step && p.Dr > 0) S.xi_all = m.get<double>(3 * Nc * (size_t)S.n_sub);
-    if (c->near_step) S.w_all = m.get<double>(3 * Nc * (size_t)S.n_sub);
-    if (c->near_step && p.precision == MPCD_FP64) {
+    if (c->near_sized && p.Dr > 0) S.xi_all = m.get<double>(3 * Nc * (size_t)S.n_sub);
+    if (c->near_sized) S.w_all = m.get<double>(3 * Nc * (size_t)S.n_sub);
+    if (c->near_sized && p.precision == MPCD_FP64) {
       S.evx_cap = S.events_cap;
       S.evx = m.get<char>((size_t)EV_STATE_BYTES * S.evx_cap);
     }
@@ -982,22 +1009,8 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && nsm > 0)
       c->n_sm = nsm;
-    int coop = 0;
-    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) c->near_step = false;
   }
-  if (c->near_step) {
-    // the free-flight pass shares the SMs with the substeps' kernel: the same shared-memory split
-    const bool f32 = p.precision == MPCD_FP32C;
-    const void *k = f32 ? (const void *)k_near_step32 : (const void *)k_near_step64;
-    const void *ff = f32 ? (const void *)k_free_flight32 : (const void *)k_free_flight;
-    const int smem = (int)(f32 ? near_step32_smem() : near_step64_smem());
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess ||
-        cudaFuncSetAttribute(ff, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess) {
-      mpcd_destroy(c);
-      return MPCD_ERR_CUDA;
-    }
-  }
+  choose_near_step(c, false);
   cudaDeviceSynchronize();
   *out = c;
   return MPCD_OK;
@@ -1248,8 +1261,9 @@ extern "C" int mpcd_set_launch(mpcd_ctx *c, int which, int grid, int block) {
 
 extern "C" int mpcd_set_fault(mpcd_ctx *c, int what, int value) {
   if (!c) return MPCD_ERR_PARAM;
-  if (what != MPCD_FAULT_LAUNCH) return fail(c, MPCD_ERR_PARAM, "unknown fault");
-  c->fault_launch = value != 0;
+  if (what == MPCD_FAULT_LAUNCH) c->fault_launch = value != 0;
+  else if (what == MPCD_FAULT_ROOM) choose_near_step(c, value != 0);
+  else return fail(c, MPCD_ERR_PARAM, "unknown fault");
   return drop_graph(c);
 }
 

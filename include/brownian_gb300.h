@@ -229,9 +229,11 @@ enum { MPCD_LAUNCH_EVENTS = 0, /* wall-collision events: grid, block (<= 128, mu
 int mpcd_set_launch(mpcd_ctx *c, int which, int grid, int block);
 
 /* ---- failure detection (test hooks: each makes a check fail from the host) ---------------- */
-enum { MPCD_FAULT_LAUNCH = 0 }; /* value 1: the substeps' cooperative launch is refused (0: it is
-                                   launched): a step fails with MPCD_ERR_CUDA, nothing of it runs
-                                   and nothing of its capture is kept */
+enum { MPCD_FAULT_LAUNCH = 0, /* value 1: the substeps' cooperative launch is refused (0: it is
+                                 launched): a step fails with MPCD_ERR_CUDA, nothing of it runs
+                                 and nothing of its capture is kept */
+       MPCD_FAULT_ROOM = 1 }; /* value 1: as on a device without room for a block of that kernel on
+                                 every SM: the steps take a launch per stage, the same bits */
 int mpcd_set_fault(mpcd_ctx *c, int what, int value);
 
 /* ---- exchange record (no counterpart in the reference) ------------------------------- */

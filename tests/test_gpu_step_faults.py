@@ -1,6 +1,7 @@
 """Failure detection of the cooperative substeps, provoked from the host: a launch that is refused
 fails the step and every step after it until it is taken, runs nothing and leaves no captured
-graph; the steps that follow give the bits of a run that never failed."""
+graph; the steps that follow give the bits of a run that never failed; and a device without room
+for the kernel takes a launch per stage."""
 import numpy as np
 import pytest
 
@@ -87,6 +88,21 @@ def test_another_schedule_goes_on_after_a_refused_launch(form):
         e.set_flight(False)
         e.step(3)
     _same(_state(a), _state(b))
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp32c", "ensemble"])
+def test_a_device_without_room_takes_a_launch_per_stage(form):
+    import brownian_gb300 as bg
+    a, b = _start(form), _start(form)
+    a.set_fault(bg.FAULT_LAUNCH, 1)  # (the cooperative kernel is not launched)
+    for room, k in ((1, 6), (0, 3), (1, 2)):
+        a.set_fault(bg.FAULT_ROOM, room)
+        a.set_fault(bg.FAULT_LAUNCH, room)
+        a.step(k)
+        b.step(k)
+        _same(_state(a), _state(b))
     a.close()
     b.close()
 
