@@ -48,7 +48,7 @@ ENS_EVENTS, ENS_RUN, ENS_FIN, ENS_AUX, ENS_FREE = 0, 1, 2, 3, 4
 NOALLOC_MAX_PARTICLES = 33554432
 PHYSICS_REFERENCE, PHYSICS_FIXED = 0, 1
 LAUNCH_EVENTS, LAUNCH_FIN, LAUNCH_AUX, LAUNCH_FREE = 0, 1, 2, 3
-FAULT_LAUNCH, FAULT_ROOM = 0, 1
+FAULT_LAUNCH, FAULT_ROOM, FAULT_WAIT, FAULT_ORIENT = 0, 1, 2, 3
 
 
 class MPCDError(RuntimeError):

@@ -682,6 +682,7 @@ static int collect_profile(mpcd_ctx *c) {
 }
 
 static const char *err_text(int bits) {
+  if (bits & ERRB_WAIT) return "a wait of the near particles' substeps did not end within its limit";
   if (bits & ERRB_TTABLE) return "more colloids reach one cell than the fluid-to-colloid table holds";
   if (bits & ERRB_SHELL) return "run() candidate records overflowed";
   if (bits & ERRB_VRANGE) return "a fluid velocity exceeded vmax (range of the exact cell sums)";
@@ -692,7 +693,6 @@ static const char *err_text(int bits) {
   if (bits & ERRB_SHELLSLOTS) return "a particle lies in more rear shells than a record holds";
   if (bits & ERRB_DELTA) return "a colloid momentum exchange left the range of the exact sums";
   if (bits & ERRB_EVENTS) return "the wall-collision event lists overflowed";
-  if (bits & ERRB_WAIT) return "a grid-wide wait of the near particles' substeps did not end within its limit";
   if (bits & ERRB_NBR) return "a colloid has more pair-list partners than the list holds";
   return "device error";
 }
@@ -921,6 +921,8 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
   S.act = m.get<int>(N);
   S.actc = m.get<unsigned>(N);
   S.bar = m.get<unsigned>(BAR_WORDS);
+  S.near_polls = NEAR_POLLS;
+  S.orient_polls = ORIENT_POLLS;
   {
     // A free-flight step takes the active particles through its substeps in one cooperative
     // kernel where there are colloids and at least two substeps, unless the flight table's cells
@@ -1263,6 +1265,8 @@ extern "C" int mpcd_set_fault(mpcd_ctx *c, int what, int value) {
   if (!c) return MPCD_ERR_PARAM;
   if (what == MPCD_FAULT_LAUNCH) c->fault_launch = value != 0;
   else if (what == MPCD_FAULT_ROOM) choose_near_step(c, value != 0);
+  else if (what == MPCD_FAULT_WAIT) c->S.near_polls = value >= 0 && value < NEAR_POLLS ? value : NEAR_POLLS;
+  else if (what == MPCD_FAULT_ORIENT) c->S.orient_polls = value >= 0 && value < ORIENT_POLLS ? value : ORIENT_POLLS;
   else return fail(c, MPCD_ERR_PARAM, "unknown fault");
   return drop_graph(c);
 }

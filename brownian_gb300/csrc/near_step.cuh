@@ -38,7 +38,6 @@
 namespace bgb {
 
 constexpr int NEAR_CW = 3;         // colloid warps of a block (and one for the orientations)
-constexpr int NEAR_WAIT = 1 << 20; // polls of a wait before it gives up (about a second)
 
 // a particle's candidate colloids for the rest of the step, packed: up to two ids (0xFFFF:
 // none); NEAR_WILD: look the flight table up in every substep; NEAR_GONE: kept elsewhere
@@ -58,8 +57,8 @@ static __device__ __forceinline__ void bar_arrive(unsigned *c) {
   asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(c) : "memory");
 }
 
-static __device__ __forceinline__ bool bar_wait(const unsigned *c, unsigned target) {
-  for (int it = 0; it < NEAR_WAIT; ++it) {
+static __device__ __forceinline__ bool bar_wait(const unsigned *c, unsigned target, int polls) {
+  for (int it = 0; it < polls; ++it) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(c) : "memory");
     if (v >= target) return true;
@@ -72,7 +71,7 @@ static __device__ __forceinline__ bool bar_wait(const unsigned *c, unsigned targ
 static __device__ __forceinline__ bool group_wait(const SysF64 &S, int which, unsigned target, int t, int id, int n,
                                                   volatile int *flag) {
   if (t == 0) {
-    const bool ok = bar_wait(S.bar + which, target);
+    const bool ok = bar_wait(S.bar + which, target, S.near_polls);
     if (!ok) atomicOr(&S.ss->err, ERRB_WAIT);
     *flag = ok ? 1 : 0;
   }
@@ -468,12 +467,16 @@ static __device__ __forceinline__ void near_orient(const SysF64 &S, const int VB
   const int k8 = lane & 7, k = k8 < 3 ? k8 : 0;
   for (int l = 1; l <= S.n_sub && M > 0; ++l) {
     int f = 0;
-    for (int it = 0; it < 16 * NEAR_WAIT; ++it) {
+    for (int it = 0; it < S.orient_polls; ++it) {
       f = *fin;
       if (f < 0 || f >= l) break;
       __nanosleep(64);
     }
-    if (!__all_sync(FULL, f >= l)) return;  // (the colloid warps have reported their wait)
+    if (!__all_sync(FULL, f >= l)) {
+      // this wait ran out, or (f < 0, reported already) one of the colloid warps'
+      if (lane == 0) atomicOr(&S.ss->err, ERRB_WAIT);
+      return;
+    }
     __threadfence_block();
     for (int s0 = 0; s0 < M; s0 += 4) {
       const int s = s0 + (lane >> 3);

@@ -213,6 +213,7 @@ struct SysF64 {
   unsigned *actc;               // [N] and the colloids their paths come near (NEAR_*)
   uint8_t *fnear;               // [N] the slot's particle this step: FN_*
   unsigned *bar;                // k_near_step's counters, 128 bytes apart (BAR_*)
+  int near_polls, orient_polls; // polls of its waits before they give up (NEAR_POLLS, ORIENT_POLLS)
   double *xi_all;               // [n_sub][Nc][3] rotational-diffusion normals of the step's substeps
   double *w_all;                // [n_sub][Nc][3] Omega after each substep of the step
   void *evx;                    // [evx_cap] records of pending particles beyond a block's shared
@@ -237,6 +238,9 @@ struct SysF64 {
   int *bkt_list;       // [Nc] colloids by bucket
 };
 
+// Limits of k_near_step's waits: polls of a grid-wide counter (each a read of L2), and of the block's own
+// orientation warp, which sleeps between two; both many times what a step takes.
+constexpr int NEAR_POLLS = 1 << 20, ORIENT_POLLS = 1 << 24;
 // k_near_step's counters in SysF64::bar: blocks whose particles are through the substep's
 // collisions, blocks whose colloids have moved on, overflow records taken
 constexpr int EV_STATE_BYTES = 256;

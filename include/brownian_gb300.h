@@ -232,8 +232,11 @@ int mpcd_set_launch(mpcd_ctx *c, int which, int grid, int block);
 enum { MPCD_FAULT_LAUNCH = 0, /* value 1: the substeps' cooperative launch is refused (0: it is
                                  launched): a step fails with MPCD_ERR_CUDA, nothing of it runs
                                  and nothing of its capture is kept */
-       MPCD_FAULT_ROOM = 1 }; /* value 1: as on a device without room for a block of that kernel on
+       MPCD_FAULT_ROOM = 1,   /* value 1: as on a device without room for a block of that kernel on
                                  every SM: the steps take a launch per stage, the same bits */
+       MPCD_FAULT_WAIT = 2,   /* value >= 0: polls after which that kernel's grid-wide waits give up
+                                 (< 0: its own limit), and the step fails with MPCD_ERR_CUDA */
+       MPCD_FAULT_ORIENT = 3 }; /* the same for the waits of its orientation warps */
 int mpcd_set_fault(mpcd_ctx *c, int what, int value);
 
 /* ---- exchange record (no counterpart in the reference) ------------------------------- */

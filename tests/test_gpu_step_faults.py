@@ -1,7 +1,8 @@
 """Failure detection of the cooperative substeps, provoked from the host: a launch that is refused
 fails the step and every step after it until it is taken, runs nothing and leaves no captured
 graph; the steps that follow give the bits of a run that never failed; and a device without room
-for the kernel takes a launch per stage."""
+for the kernel takes a launch per stage.  A wait that runs out (its limit set to a few polls) fails
+the step, and with the state set again the steps give those bits too."""
 import numpy as np
 import pytest
 
@@ -103,6 +104,35 @@ def test_a_device_without_room_takes_a_launch_per_stage(form):
         a.step(k)
         b.step(k)
         _same(_state(a), _state(b))
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp32c", "ensemble"])
+@pytest.mark.parametrize("what", ["WAIT", "ORIENT"])
+def test_a_wait_that_runs_out_is_reported(form, what):
+    import brownian_gb300 as bg
+    keys = ("pos_fl", "vel_fl", "pos_colloid", "vel_colloid", "ang_vel_colloid", "ra")
+    a, b = _start(form), _start(form)
+    first = _state(a)
+    fault = getattr(bg, "FAULT_" + what)
+    for polls, steps in ((0, 1), (0, 4)) + (((1, 2),) if what == "WAIT" else ()):
+        a.set_fault(fault, polls)
+        with pytest.raises(bg.MPCDError) as err:
+            a.step(steps)
+        assert err.value.code == bg.ERR_CUDA and "did not end within its limit" in str(err.value)
+        if form != "ensemble":
+            with pytest.raises(bg.MPCDError) as err:
+                a.sim.diag()
+            assert err.value.code == bg.ERR_CUDA
+        a.set_fault(fault, -1)
+        for s, x in zip(a, first):
+            s.step_count = 0
+            s.set_state(*[x[k] for k in keys])
+            s.setup()
+    a.step(5)
+    b.step(5)
+    _same(_state(a), _state(b))
     a.close()
     b.close()
 
