@@ -918,8 +918,6 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
   S.near = m.get<int>(N);
   S.fnear = m.get<uint8_t>(N);
   S.ftab = m.get<FlightCell>(S.C);
-  S.act = m.get<int>(N);
-  S.actc = m.get<unsigned>(N);
   S.bar = m.get<unsigned>(BAR_WORDS);
   S.near_polls = NEAR_POLLS;
   S.orient_polls = ORIENT_POLLS;
@@ -934,18 +932,27 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
     const double expected = (double)S.Nc / (double)S.C * 4.0 / 3.0 * M_PI * reach * reach * reach;
     c->near_sized =
         S.Nc > 0 && S.n_sub >= 2 && S.n_sub <= 4096 && expected <= 8.0 && (long long)S.Nc * S.n_sub <= (1ll << 24);
+    // (in an ensemble the others' kernel takes a system without colloids along)
+    if (c->near_sized || (S.Nc == 0 && p.precision == MPCD_FP32C)) {
+      S.act = m.get<int>(N);
+      S.actc = m.get<unsigned>(N);
+    }
     if (c->near_sized && p.Dr > 0) S.xi_all = m.get<double>(3 * Nc * (size_t)S.n_sub);
     if (c->near_sized) S.w_all = m.get<double>(3 * Nc * (size_t)S.n_sub);
-    if (c->near_sized && p.precision == MPCD_FP64) {
-      S.evx_cap = S.events_cap;
-      S.evx = m.get<char>((size_t)EV_STATE_BYTES * S.evx_cap);
-    }
   }
   if (S.precision == MPCD_FP64) {
-    S.newrec[0] = m.get<EventRec>(S.events_cap);
-    S.newrec[1] = m.get<EventRec>(S.events_cap);
+    // the event passes' lists and, in the same place, the cooperative kernel's records of pending
+    // particles (no step uses both, and none leaves anything in them)
+    const size_t cap = S.events_cap, lists = 3 * sizeof(EventRec);
+    EventRec *ev = (EventRec *)m.get<double2>(cap * std::max<size_t>(lists, c->near_sized ? EV_STATE_BYTES : 0) / sizeof(double2));
+    S.newrec[0] = ev;
+    S.newrec[1] = ev + cap;
+    S.prec = ev + 2 * cap;
     S.pend_cap = S.events_cap;
-    S.prec = m.get<EventRec>(S.pend_cap);
+    if (c->near_sized) {
+      S.evx = ev;
+      S.evx_cap = S.events_cap;
+    }
     S.pend = m.get<uint8_t>(S.N);
   }
   S.ss = m.get<StepState>(1);
