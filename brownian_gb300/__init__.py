@@ -31,7 +31,7 @@ EXPORTS = ["mpcd_create", "mpcd_destroy", "mpcd_last_error", "mpcd_set_stream", 
            "mpcd_profile_enable", "mpcd_profile_read", "mpcd_trace_step", "mpcd_launch_count", "mpcd_set_launch",
            "mpcd_fluid_sums_noalloc", "mpcd_ensemble_create", "mpcd_ensemble_destroy", "mpcd_ensemble_last_error",
            "mpcd_ensemble_system", "mpcd_ensemble_step", "mpcd_ensemble_set_launch", "mpcd_ensemble_launch_count",
-           "mpcd_ensemble_set_flight", "mpcd_ensemble_get_flight",
+           "mpcd_ensemble_set_flight", "mpcd_ensemble_get_flight", "mpcd_ensemble_one_kernel",
            "mpcd_exchange_read", "mpcd_mlp_create", "mpcd_mlp_destroy", "mpcd_mlp_last_error", "mpcd_mlp_param_count",
            "mpcd_mlp_set_normalisation", "mpcd_mlp_get_params", "mpcd_mlp_set_params", "mpcd_mlp_forward",
            "mpcd_mlp_grad", "mpcd_mlp_train_step", "mpcd_mlp_set_fault", "mpcd_surrogate_create", "mpcd_surrogate_destroy",
@@ -152,6 +152,7 @@ def lib():
         L.mpcd_ensemble_launch_count.restype = C.c_int64
         L.mpcd_ensemble_set_flight.argtypes = [vp, C.c_int]
         L.mpcd_ensemble_get_flight.argtypes = [vp]
+        L.mpcd_ensemble_one_kernel.argtypes = [vp]
         L.mpcd_ensemble_set_fault.argtypes = [vp, C.c_int, C.c_int]
         _lib = L
     return _lib
@@ -574,6 +575,11 @@ class Ensemble:
     @property
     def flight(self):
         return bool(lib().mpcd_ensemble_get_flight(self.h))
+
+    @property
+    def one_kernel(self):
+        """whether a step's substeps run in one cooperative kernel (ENS_EVENTS and ENS_AUX then shape nothing)"""
+        return bool(lib().mpcd_ensemble_one_kernel(self.h))
 
     @property
     def launch_count(self):

@@ -2,9 +2,11 @@
 
 Coordinate descent over the knobs of mpcd_ensemble_set_launch (event blocks per
 system, run() blocks per system, colloid-finish block size, threads per colloid
-of the colloid side work, resident blocks per SM of the free-flight pass): each candidate is timed over a few whole ensemble
-steps (the step call synchronises, so wall time is device time plus one host
-round trip), the fastest is kept, and every timing is logged.  The results do
+of the colloid side work, resident blocks per SM of the free-flight pass): each
+candidate is timed over a few whole ensemble steps (the step call synchronises,
+so wall time is device time plus one host round trip), the fastest is kept, and
+every timing is logged.  A knob that shapes nothing in the ensemble's schedule
+keeps its default: a choice among its timings would be noise.  The results do
 not depend on the shapes (every sum is exact), so tuning can run on the warm-up
 steps of a production run.
 """
@@ -19,6 +21,8 @@ CANDIDATES = {
     "aux_threads_per_colloid": (ENS_AUX, [(1, 64), (1, 128), (1, 256)]),
     "free_blocks_per_sm": (ENS_FREE, [(2, 256), (4, 256), (8, 256)]),
 }
+# the substeps in one cooperative kernel have no event pass and no side work
+PER_STAGE_ONLY = ("events_blocks_per_system", "aux_threads_per_colloid")
 DEFAULTS = {"events_blocks_per_system": (2, 32), "run_blocks_per_system": (4, 32), "fin_threads_per_block": (1, 128),
             "aux_threads_per_colloid": (1, 128), "free_blocks_per_sm": (4, 256)}
 
@@ -40,6 +44,8 @@ def autotune(ens, steps=3, rounds=1):
     log.append({"start": dict(choice), "ms_per_step": best * 1e3})
     for _ in range(rounds):
         for name, (which, cands) in CANDIDATES.items():
+            if name in PER_STAGE_ONLY and getattr(ens, "one_kernel", False):
+                continue
             for cand in cands:
                 if cand == choice[name]:
                     continue

@@ -306,6 +306,9 @@ int64_t mpcd_ensemble_launch_count(const mpcd_ensemble *e);
  * leave the same bits. */
 int mpcd_ensemble_set_flight(mpcd_ensemble *e, int on);
 int mpcd_ensemble_get_flight(const mpcd_ensemble *e);
+/* 1 where a step's substeps run in one cooperative kernel: it has no event pass and no side work
+ * (MPCD_ENS_EVENTS and MPCD_ENS_AUX then shape nothing) */
+int mpcd_ensemble_one_kernel(const mpcd_ensemble *e);
 /* mpcd_set_fault for the batched step */
 int mpcd_ensemble_set_fault(mpcd_ensemble *e, int what, int value);
 

@@ -85,6 +85,18 @@ def test_launch_shapes_of_an_ensembles_stages_leave_the_same_bits(schedule):
     b.close()
 
 
+def test_an_ensemble_says_whether_its_substeps_are_one_kernel():
+    import brownian_gb300 as bg
+    e = _ens([_params("fp32c", L=12, nc=2)])
+    assert e.one_kernel
+    e.set_flight(False)
+    assert not e.one_kernel
+    e.set_flight(True)
+    e.set_fault(bg.FAULT_ROOM, 1)
+    assert not e.one_kernel
+    e.close()
+
+
 @pytest.mark.parametrize("sort_every", [-1, 1, 2, 3, 4, 5])
 @pytest.mark.parametrize("form", ["fp64", "fp32c"])
 def test_steps_of_one_call_are_those_of_many(form, sort_every):
