@@ -25,20 +25,33 @@ struct ProfEvent {
   cudaEvent_t a, b;
 };
 
+// Zeroed device memory of a context.  Arrays of up to 64 KB share chunks of 512 KB: a small system has
+// some forty of them, and an allocation and its clearing cost several us each.
 struct DevAlloc {
+  static constexpr size_t SMALL = 64 << 10, CHUNK = 512 << 10;
   std::vector<void *> ptrs;
+  char *chunk = nullptr;
+  size_t used = CHUNK;
   cudaError_t err = cudaSuccess;
+  void *fresh(size_t bytes) {
+    void *p = nullptr;
+    if (err == cudaSuccess) err = cudaMalloc(&p, bytes);
+    if (err != cudaSuccess) return nullptr;
+    ptrs.push_back(p);
+    cudaMemset(p, 0, bytes);
+    return p;
+  }
   template <typename T>
   T *get(size_t n) {
-    void *p = nullptr;
-    if (err == cudaSuccess) {
-      err = cudaMalloc(&p, n * sizeof(T) + 16);
-      if (err == cudaSuccess) {
-        ptrs.push_back(p);
-        cudaMemset(p, 0, n * sizeof(T) + 16);
-      }
+    const size_t bytes = (n * sizeof(T) + 16 + 255) / 256 * 256;
+    if (bytes > SMALL) return (T *)fresh(bytes);
+    if (used + bytes > CHUNK) {
+      chunk = (char *)fresh(CHUNK);
+      used = 0;
     }
-    return (T *)p;
+    if (!chunk) return nullptr;
+    used += bytes;
+    return (T *)(chunk + used - bytes);
   }
   void release() {
     for (void *p : ptrs) cudaFree(p);
