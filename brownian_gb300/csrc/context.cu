@@ -648,7 +648,10 @@ static void enq_step_near(mpcd_ctx *c, bool sort) {
 // step that left none
 static void ensure_tables(mpcd_ctx *c) {
   if (!c->tables_stale) return;
-  if (c->S.Nc) launch(c, "k_table_next", k_table_next, c->S.Nc, 256, c->S);
+  if (c->S.Nc) {
+    launch(c, "k_table_next", k_table_next, c->S.Nc, 256, c->S);
+    launch(c, "k_table_next", k_table_mark, 1, 1, c->S);
+  }
   c->tables_stale = false;
 }
 

@@ -945,6 +945,14 @@ static __device__ __forceinline__ float table_reach(const SysF64 &S, long long e
   return (e % S.n_sub) == S.n_sub - 1 ? S.rT_shell : S.rT_coll;
 }
 
+// colloid j in the cell table of substep e, from its position before it (thread t of nt; out of line: for
+// steps with crowded cells)
+static __device__ __noinline__ void table_of(const SysF64 &S, int j, long long e, int t, int nt) {
+  const int b = (int)((e - 1) & 1);
+  for_reach_cells(S, S.cbox[b][j], S.Xf[b][j], table_reach(S, e), t, nt,
+                  [&](int cell) { tappend(S.Tcnt[e & 1], S.Tlist[e & 1], cell, e, j, &S.ss->err); });
+}
+
 // update_activity_direction (cpp/update.cpp:34-46) of colloid j on lanes k = 0-2 of
 // group grp: lane k takes sin and cos of (Omega dt)_k, all three gather them, lane 0
 // stores the turned orientation (with the rotational-diffusion normals S.xi[j])

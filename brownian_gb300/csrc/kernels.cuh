@@ -70,7 +70,8 @@ size_t near_step64_smem();
 size_t near_step32_smem();
 __global__ void k_rotdiff_step(__grid_constant__ const SysF64 S);
 __global__ void k_rotdiff_step_b(const SysF64 *Ss, const int *boff, int nrep);
-__global__ void k_table_next(const SysF64 S);
+__global__ void k_table_next(__grid_constant__ const SysF64 S);
+__global__ void k_table_mark(__grid_constant__ const SysF64 S);
 __global__ void k_end_flight64(__grid_constant__ const SysF64 S, int fb);
 __global__ void k_end_flight32(__grid_constant__ const SysF64 S, int fb);
 __global__ void k_end_flight32_b(const SysF64 *Ss, const int *boff, int nrep, int fb);

@@ -562,7 +562,9 @@ static __device__ __forceinline__ void k_flight_table32_body(const SysF64 &S, co
     atomicMax(&fc->tc, tag);
     const int slot = (int)(unsigned)atomicAdd(&fc->tc, 1ull);
     if (slot < FLIGHT_CAP) fc->id[slot] = (uint16_t)j;
-    if (slot == TCAP) S.ss->crowd = step + 1;  // (a cell table, whose reach is shorter, may overflow)
+    // the particles of a crowded cell find their colloids in the cell tables (near_list), which are built in
+    // this step; one may overflow, too
+    if (slot == FLIGHT_CAP) S.ss->crowd = step + 1;
   }
 }
 
@@ -1101,12 +1103,13 @@ static __device__ __forceinline__ unsigned near_cand32(const SysF64 &S, long lon
   const float T = (float)rem * S.dtf;
   const float wx = T * vx, wy = T * vy, wz = T * vz;
   if (!(sqrtf(wx * wx + wy * wy + wz * wz) <= S.flight_rv)) return NEAR_WILD;
-  const NearList q = near_list(S, step, lin_cell(S, cx, cy, cz), false);
-  if (q.brute) return NEAR_WILD;
+  const FlightCell *fc = S.ftab + lin_cell(S, cx, cy, cz);
+  const int cnt = tcount(fc->tc, step);
+  if (cnt > FLIGHT_CAP) return NEAR_WILD;
   const float rad = near_radius(S, S.ss->cm, rem);
   unsigned cand = NEAR_NONE;
-  for (int k = 0; k < q.cnt; ++k) {
-    const int j = q.ids[k];
+  for (int k = 0; k < cnt; ++k) {
+    const int j = fc->id[k];
     const float4 cq = S.Xcq[b][j], co = S.Xco[b][j];
     if (path_meets(rel(cx, ox, cq.x, co.x, S.Lx), rel(cy, oy, cq.y, co.y, S.Ly), rel(cz, oz, cq.z, co.z, S.Lz), wx,
                    wy, wz, rad))
@@ -1247,7 +1250,7 @@ struct Near32 {
 static __device__ __forceinline__ void near_shell32(const SysF64 &S, long long step, int buf, int cx, int cy, int cz,
                                                     float ox, float oy, float oz, const NearCell &c, int id, bool hit,
                                                     ShellRec &rec) {
-  const NearList q = near_list(S, step, c.lin, false);
+  const NearList q = near_list(S, step, step * S.n_sub + S.n_sub - 1, c.lin, false);
   const float rs2 = S.r_shell * S.r_shell;
   rec.p = id;
   rec.n = 0;
@@ -1363,7 +1366,7 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
       };
       bool e = false;
       if (cand == NEAR_WILD) {
-        const NearList c = near_list(S, step, lin_cell(S, cx, cy, cz), false);
+        const NearList c = near_list(S, step, gs, lin_cell(S, cx, cy, cz), false);
         for (int m = 0; m < (c.brute ? S.Nc : c.cnt) && !e; ++m)
           e = dist2(sm.col.at(S, xb, c.brute ? m : c.ids[m])) <= ch * ch;
       } else {
@@ -1434,7 +1437,7 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
       int cx, cy, cz;
       float ox, oy, oz;
       unpack(*pq(k), cx, cy, cz, ox, oy, oz);
-      const NearList c = near_list(S, step, lin_cell(S, cx, cy, cz), false);
+      const NearList c = near_list(S, step, gs, lin_cell(S, cx, cy, cz), false);
       v.k = k;
       v.id = F.id[S.act[a0 + k]];
       v.jc = -1;
@@ -1512,7 +1515,7 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
           int hits = 0;
           int id = v ? v->id : -1;
           if (!v || v->slow) {  // nothing listed: by the general routine
-            const NearList q = near_list(S, step, c.lin, false);
+            const NearList q = near_list(S, step, gs, c.lin, false);
 #pragma unroll 1
             for (int j = near_next(S, q, -1, c, buf ^ 1); j >= 0; j = near_next(S, q, j, c, buf ^ 1)) {
               if (!inside(j)) continue;
@@ -1648,7 +1651,7 @@ size_t near_step32_smem() { return sizeof(Near32); }
 // ones among them (the others)
 static __device__ __forceinline__ void k_end_flight32_body(const SysF64 &S, const int VB, const int NVB, int fb) {
   if (VB == 0) {
-    k_end_step_body(S, 0, 1);
+    k_end_step_body(S, 0, S.ss->crowd == S.ss->step + 1);
     return;
   }
   const long long step = S.ss->step_f;

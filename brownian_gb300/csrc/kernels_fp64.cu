@@ -818,12 +818,13 @@ static __device__ __forceinline__ unsigned near_cand64(const SysF64 &S, long lon
   const float fr = (float)rem;
   const float fx = fr * d2f_trunc(wx), fy = fr * d2f_trunc(wy), fz = fr * d2f_trunc(wz);
   if (!(sqrtf(fx * fx + fy * fy + fz * fz) <= S.flight_rv)) return NEAR_WILD;
-  const NearList q = near_list(S, step, lin_cell(S, cx, cy, cz), false);
-  if (q.brute) return NEAR_WILD;
+  const FlightCell *fc = S.ftab + lin_cell(S, cx, cy, cz);
+  const int cnt = tcount(fc->tc, step);
+  if (cnt > FLIGHT_CAP) return NEAR_WILD;
   const float rad = near_radius(S, S.ss->cm, rem);
   unsigned cand = NEAR_NONE;
-  for (int k = 0; k < q.cnt; ++k) {
-    const int j = q.ids[k];
+  for (int k = 0; k < cnt; ++k) {
+    const int j = fc->id[k];
     const float4 c = S.Xf[b][j];
     const float dx = wrap_half(c.x - px, S.Lxf), dy = wrap_half(c.y - py, S.Lyf), dz = wrap_half(c.z - pz, S.Lzf);
     if (path_meets(-dx, -dy, -dz, fx, fy, fz, rad)) cand = near_add(cand, j);
@@ -947,6 +948,12 @@ static __device__ __forceinline__ void k_fin_body(const SysF64 &S, const int VB,
   if (j >= S.Nc) return;  // (j is the block's or the warp's)
   if (!S.fin_table) {
     if (lane < 6) k_fin_colloid(S, j, lane, mode, g, gn);
+    if ((mode & M_FLIGHT) && S.ss->crowd == step + 1) {
+      // a crowded flight cell: the cell tables of the step's first two substeps
+      __syncwarp();
+      if (S.ss->tab != gn) table_of(S, j, gn, lane, 32);
+      table_of(S, j, gn + 1, lane, 32);
+    }
     return;
   }
   if (threadIdx.x < 6) k_fin_colloid(S, j, lane, mode, g, gn);
@@ -1060,6 +1067,7 @@ __global__ void __launch_bounds__(128) k_colloid_setup(const SysF64 S) {
     S.ss->nnew[0] = S.ss->nnew[1] = 0;
     S.ss->npend = 0;
     S.ss->crowd = 0;
+    S.ss->tab = g0;
     S.ss->cm = S.cmarginf;  // the static bound until a step has measured the colloids
     S.ss->cm2 = S.cmargin2;
   }
@@ -1092,13 +1100,13 @@ __global__ void __launch_bounds__(128) k_colloid_pot(const SysF64 S, int b) {
 }
 
 __global__ void k_end_step(__grid_constant__ const SysF64 S) {
-  k_end_step_body(S, blockIdx.x, gridDim.x);
+  k_end_step_body(S, blockIdx.x, true);
 }
 
 // the same over a batch of systems (persistent: batch_for)
 __global__ void k_end_step_b(const SysF64 *Ss, const int *boff, int nrep) {
   __shared__ SysF64 sS;
-  batch_for(Ss, boff, nrep, sS, [&](int VB, int NVB) { k_end_step_body(sS, VB, NVB); });
+  batch_for(Ss, boff, nrep, sS, [&](int VB, int) { k_end_step_body(sS, VB, true); });
 }
 
 // fluid diagnostics from the exact cell sums of the last binning: per block the
@@ -1161,8 +1169,8 @@ static __device__ __forceinline__ NearCell near_cell64(const SysF64 &S, double x
 // (mg) alone allow, among the ones its path comes near; where there is one, all those within a
 // wall collision's displacement of that as well (a second sphere is reached through a collision
 // with the first).
-static __device__ __forceinline__ void near_spheres64(const SysF64 &S, long long step, NearEv &e, int prev, float mg,
-                                                      const NearCols<NearCol64> &cols) {
+static __device__ __forceinline__ void near_spheres64(const SysF64 &S, long long step, long long gs, NearEv &e, int prev,
+                                                      float mg, const NearCols<NearCol64> &cols) {
   const float px = d2f_trunc(e.x), py = d2f_trunc(e.y), pz = d2f_trunc(e.z);
   const float ch = S.r_coll + 1e-3f + mg, far = ch + S.disp_marginf + 1e-3f;
   auto dist2 = [&](float4 c) {
@@ -1179,7 +1187,7 @@ static __device__ __forceinline__ void near_spheres64(const SysF64 &S, long long
       any = dist2(cols.d[r & 0xFFFFu].x) <= ch * ch;
     if (!any) return;
   }
-  const NearList q = near_list(S, step, e.c.lin, e.c.alias);
+  const NearList q = near_list(S, step, gs, e.c.lin, e.c.alias);
   e.slow = q.brute;
   for (int k = 0; k < q.cnt && !e.slow; ++k) {
     const int j = q.ids[k];
@@ -1202,7 +1210,7 @@ static __device__ __forceinline__ void near_spheres64(const SysF64 &S, long long
 // nothing was listed for
 static __device__ __noinline__ void near_collide_rest(const SysF64 &S, NearEv &e, long long step, long long gs,
                                                       int buf) {
-  const NearList q = near_list(S, step, e.c.lin, e.c.alias);
+  const NearList q = near_list(S, step, gs, e.c.lin, e.c.alias);
   int j = near_next(S, q, -1, e.c, buf ^ 1);
   while (j >= 0) {
     if (within(S, S.X[buf], S.Xf[buf][j], j, e.x, e.y, e.z, S.r_coll, S.sig2q)) ev_collide(S, e, j, gs, buf);
@@ -1227,7 +1235,7 @@ static __device__ __noinline__ void near_collide_listed(const SysF64 &S, NearEv 
 static __device__ __forceinline__ void near_shell64(const SysF64 &S, long long step, int buf, float mg, double x,
                                                     double y, double z, const NearCell &c, int id, ShellRec &rec,
                                                     bool *band) {
-  const NearList q = near_list(S, step, c.lin, c.alias);
+  const NearList q = near_list(S, step, step * S.n_sub + S.n_sub - 1, c.lin, c.alias);
   const float px = d2f_trunc(x), py = d2f_trunc(y), pz = d2f_trunc(z);
   const float sl = S.r_shell - 1e-3f - mg, sh = S.r_shell + 1e-3f + mg;
   rec.p = id;
@@ -1361,7 +1369,7 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
       auto block = [&](int4 cc, int j) { return c.alias ? near_in_block(S, j, c, xb) : in_block3(S, cc, c.ix, c.iy, c.iz); };
       bool e = c.alias;
       if (cand == NEAR_WILD) {
-        const NearList q = near_list(S, step, c.lin, c.alias);
+        const NearList q = near_list(S, step, gs, c.lin, c.alias);
         for (int m = 0; m < (q.brute ? S.Nc : q.cnt) && !e; ++m) {
           const int j = q.brute ? m : q.ids[m];
           e = close(sm.col.at(S, xb, j).x) && near_in_block(S, j, c, xb);
@@ -1462,7 +1470,7 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
       e.alias = e.c.alias;
       e.x0 = e.x; e.y0 = e.y; e.z0 = e.z;
       e.dumped = false;
-      near_spheres64(S, step, e, xb, mg, sm.col);
+      near_spheres64(S, step, gs, e, xb, mg, sm.col);
     }
     sync();
     // the preparations of 32 pending particles at a time, the three independent FP64 chains on
@@ -1641,24 +1649,22 @@ __global__ void __launch_bounds__(256) k_rotdiff_step_b(const SysF64 *Ss, const 
 }
 
 // the cell table of a step's first substep at the present positions (the free-flight steps
-// leave none; the per-substep passes read it), one block per colloid
-__global__ void __launch_bounds__(256) k_table_next(const SysF64 S) {
+// leave none, unless a flight cell is crowded; the per-substep passes read it), one block per colloid
+__global__ void __launch_bounds__(256) k_table_next(__grid_constant__ const SysF64 S) {
   const int j = blockIdx.x;
-  if (j >= S.Nc) return;
-  if (S.ss->crowd == S.ss->step) return;  // (a step with crowded cells has built it)
   const long long g = S.ss->step * S.n_sub;
-  const int b = (int)(g & 1);
-  int *err = &S.ss->err;
-  for_reach_cells(S, S.cbox[b ^ 1][j], S.Xf[b ^ 1][j], table_reach(S, g), threadIdx.x, blockDim.x,
-                  [&](int cell) { tappend(S.Tcnt[b], S.Tlist[b], cell, g, j, err); });
+  if (j < S.Nc && S.ss->tab != g) table_of(S, j, g, threadIdx.x, blockDim.x);
 }
+
+// (behind it: the table is built)
+__global__ void k_table_mark(__grid_constant__ const SysF64 S) { S.ss->tab = S.ss->step * S.n_sub; }
 
 // The end of a free-flight step: the step counter and the next step's margin (block 0), and, in
 // the other blocks, the run() candidate records of the near particles and the binning of the
 // active ones among them (k_near_step64 wrote their final state).
 __global__ void __launch_bounds__(256) k_end_flight64(__grid_constant__ const SysF64 S, int fb) {
   if (blockIdx.x == 0) {
-    k_end_step_body(S, 0, 1);
+    k_end_step_body(S, 0, S.ss->crowd == S.ss->step + 1);
     return;
   }
   const long long step = S.ss->step_f;

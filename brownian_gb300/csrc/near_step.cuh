@@ -85,15 +85,23 @@ static __device__ __forceinline__ void near_let_dependents() { asm volatile("gri
 
 // ---------------------------------------------------------------- candidates
 
-// colloids the flight table lists for cell lin of this step; brute: all colloids (an aliased
-// cell, or one with more than the table holds)
+// The colloids that may matter to a particle of cell lin in substep g of this step: the flight table's, or
+// where it lists more than it holds, the cell table's of that substep, which such a step builds;
+// brute: all colloids (an aliased cell).  (Scanning all of them in crowded cells, too: 300 spheres of
+// radius 0.5 in a cube of side 12, 5,532 us a step FP64 and 2,882 FP32; this 395 and 333, a launch per
+// stage 357 and 250.  With 28 ids a flight cell, whose lists are longer than the cell tables', 411 and 352.)
 struct NearList {
   const uint16_t *ids;
   int cnt;
   bool brute;
 };
 
-static __device__ __forceinline__ NearList near_list(const SysF64 &S, long long step, int lin, bool alias) {
+// the cell table's (rare, out of line)
+static __device__ __noinline__ int near_table(const SysF64 &S, long long g, int lin) {
+  return min(tcount(S.Tcnt[g & 1][lin], g), TCAP);
+}
+
+static __device__ __forceinline__ NearList near_list(const SysF64 &S, long long step, long long g, int lin, bool alias) {
   NearList q;
   q.ids = nullptr;
   q.cnt = 0;
@@ -102,7 +110,10 @@ static __device__ __forceinline__ NearList near_list(const SysF64 &S, long long 
     const FlightCell *fc = S.ftab + lin;
     q.ids = fc->id;
     q.cnt = tcount(fc->tc, step);
-    q.brute = q.cnt > FLIGHT_CAP;
+    if (q.cnt > FLIGHT_CAP) {
+      q.ids = S.Tlist[g & 1] + (size_t)lin * TCAP;
+      q.cnt = near_table(S, g, lin);
+    }
   }
   return q;
 }
@@ -338,16 +349,6 @@ static __device__ __forceinline__ void near_forces(const SysF64 &S, NearPairs &p
   }
 }
 
-// The cell table that the per-substep passes would read in substep e, from the positions before it,
-// the block's colloids (thread t of nt).  The step's last one is that of the next step's first
-// substep (k_table_next then has none to build).
-static __device__ __noinline__ void near_tables(const SysF64 &S, int VB, int G, long long e, int t, int nt) {
-  const int b = (int)((e - 1) & 1);
-  for (int j = VB; j < S.Nc; j += G)
-    for_reach_cells(S, S.cbox[b][j], S.Xf[b][j], table_reach(S, e), t, nt,
-                    [&](int cell) { tappend(S.Tcnt[e & 1], S.Tlist[e & 1], cell, e, j, &S.ss->err); });
-}
-
 // The colloid group of a block (t: thread of the group): colloids VB, VB + G, ... through the
 // substeps.  A colloid has eight lanes (four colloids a warp): lane k < 3 the linear component
 // k, lane 3 + k the angular one, so that an FP64 instruction, which occupies the SM's FP64 unit
@@ -368,8 +369,6 @@ static __device__ __forceinline__ void near_colloids(const SysF64 &S, NearPairs 
   const bool crowd = S.ss->crowd == step + 1;
   const Dim &D = k == 0 ? S.dx : (k == 1 ? S.dy : S.dz);
   const int Lk = k == 0 ? S.Lx : (k == 1 ? S.Ly : S.Lz);
-  // some cell may hold more colloids than a cell table: the tables are built for their capacity check
-  if (crowd) near_tables(S, VB, G, g0 + 1, t, NT);
   for (int l = 1; l <= n; ++l) {
     const long long g = g0 + (l - 1);
     const int cur = (int)(g & 1), nxt = cur ^ 1;
@@ -450,7 +449,13 @@ static __device__ __forceinline__ void near_colloids(const SysF64 &S, NearPairs 
       *fin = l;  // (the orientation warp follows)
     }
     if (l == n) return;
-    if (crowd) near_tables(S, VB, G, g + 2, t, NT);
+    // the cell table of substep g + 2 (those of the step's first two are k_fin's): near_list reads it once this
+    // count is complete, and its capacity is checked as in the per-substep passes.  (It takes the place of
+    // substep g's, whose collisions are over in every block.)
+    if (crowd) {
+      for (int j = VB; j < S.Nc; j += G) table_of(S, j, g + 2, t, NT);
+      group_sync(bar_id, NT);
+    }
     if (t == 0) bar_arrive(S.bar + BAR_MOVE);
   }
   if (t == 0) *fin = -1;  // (a wait ran out)
@@ -516,9 +521,10 @@ static __device__ __forceinline__ void near_orient(const SysF64 &S, const int VB
   }
 }
 
-// completes a step: bumps the step counter
-static __device__ __forceinline__ void k_end_step_body(const SysF64 &S, const int VB, const int NVB) {
+// completes a step: bumps the step counter (tables: the cell table of the next step's first substep is built)
+static __device__ __forceinline__ void k_end_step_body(const SysF64 &S, const int VB, bool tables) {
   if (VB != 0) return;
+  if (threadIdx.x == 0 && tables) S.ss->tab = (S.ss->step + 1) * S.n_sub;
   // run()'s shell counts start from zero for the next step (its rear-shell test runs beside
   // the next step's cell pass, so the cell pass cannot clear them)
   for (int j = threadIdx.x; j < S.Nc; j += blockDim.x) S.shell_cnt[j] = 0;

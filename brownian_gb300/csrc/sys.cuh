@@ -77,7 +77,8 @@ struct StepState {
   double rrn[3];    // free-flight schedule: the next step's grid shift (the free pass bins with it)
   float cm_f;       // this step's cm and step number, for the end of the step, whose first block
   long long step_f; // sets the next step's while the others still record run() candidates
-  long long crowd;  // step + 1 if some flight cell lists more colloids than a cell table holds
+  long long crowd;  // step + 1 if some flight cell lists more colloids than it holds
+  long long tab;    // the last substep that is a step's first and whose cell table is built
 };
 
 // a particle in a free-flight step: free; near; of the near ones active, those of them that

@@ -150,3 +150,48 @@ def test_a_table_that_overflows_is_refused_in_the_same_step(form, n_sub):
                 break
         sim.close()
     assert len(refused) == 2 and refused[0] == refused[1] > 0, refused
+
+
+def _cluster(form, nc=300, side=12.0, L=48):
+    """Small spheres on a jittered lattice in a corner of the box: seventeen expected within a flight cell's
+    reach, one to five in a cell table."""
+    import brownian_gb300 as bg
+    rng = np.random.default_rng(2)
+    m = int(np.ceil(nc ** (1 / 3)))
+    a = side / m
+    g = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)[rng.permutation(m ** 3)[:nc]]
+    X = 3 + (g + 0.5) * a + rng.uniform(-0.1, 0.1, (nc, 3)) * (a - 1.0)
+    M = 50.0
+    pos = rng.uniform(0.01, L - 0.01, (L ** 3 * 6, 3))
+    near = (pos < side + 6).all(1)
+    free = np.ones(len(pos), bool)
+    free[near] = np.array([((X - p) ** 2).sum(1).min() > 0.26 for p in pos[near]])
+    pos = pos[free]
+    ra = rng.normal(0, 1, (nc, 3))
+    state = dict(pos_fl=pos, vel_fl=rng.normal(0, 1, pos.shape), pos_colloid=X,
+                 vel_colloid=rng.normal(0, M ** -0.5, (nc, 3)), ang_vel_colloid=np.zeros((nc, 3)),
+                 ra=ra / np.linalg.norm(ra, axis=1, keepdims=True))
+    sim = bg.Simulation(L, len(pos), nc, n_sub=10, mass_colloid=M, sig_colloid=0.9, sigma=1.0, I_colloid=5.0, v0=0.02,
+                        theta_deg=90.0, Dr=0.001, seed=3, precision=bg.FP64 if form == "fp64" else bg.FP32C)
+    return _start(sim, state)
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp32c"])
+def test_a_cluster_of_small_spheres_is_no_scan_of_all_spheres(form):
+    # (the particles of its cells, which list more spheres than a flight cell holds, once scanned all 300 in
+    # every substep: ten times the per-substep schedule's time)
+    import time
+    a, b = _cluster(form), _cluster(form)
+    b.set_flight(False)
+    took = []
+    for s in (a, b):
+        s.step(6)
+        t = time.perf_counter()
+        s.step(20)
+        took.append(time.perf_counter() - t)
+    _same(a, b)
+    da, db = a.diag(), b.diag()
+    assert da["events"] == db["events"] > 0 and da["shell_records"] == db["shell_records"] > 0
+    assert took[0] < 2.0 * took[1], took
+    a.close()
+    b.close()
