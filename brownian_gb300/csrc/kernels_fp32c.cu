@@ -1364,14 +1364,15 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
                     dz = rel(cz, oz, o.q.z, o.o.z, S.Lz);
         return dx * dx + dy * dy + dz * dz;
       };
+      // (inside a sphere that its boxes leave out, a particle needs no exact test: the box rule first)
+      auto reached = [&](const NearCol32 &o) { return dist2(o) <= ch * ch && in_block3(S, o.c, cx, cy, cz); };
       bool e = false;
       if (cand == NEAR_WILD) {
         const NearList c = near_list(S, step, gs, lin_cell(S, cx, cy, cz), false);
-        for (int m = 0; m < (c.brute ? S.Nc : c.cnt) && !e; ++m)
-          e = dist2(sm.col.at(S, xb, c.brute ? m : c.ids[m])) <= ch * ch;
+        for (int m = 0; m < (c.brute ? S.Nc : c.cnt) && !e; ++m) e = reached(sm.col.at(S, xb, c.brute ? m : c.ids[m]));
       } else {
         for (unsigned r = cand; (r & 0xFFFFu) != 0xFFFFu && !e; r = (r >> 16) | 0xFFFF0000u)
-          e = dist2(sm.col.d[r & 0xFFFFu]) <= ch * ch;
+          e = reached(sm.col.d[r & 0xFFFFu]);
       }
       if (e) *idx(atomicAdd(&s_nchk, 1)) = k;
     };
@@ -1411,7 +1412,7 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
           const NearCol32 &o = sm.col.d[min(j, (unsigned)(NearCols<NearCol32>::MAX - 1))];
           const float dx = rel(cx, ox, o.q.x, o.o.x, S.Lx), dy = rel(cy, oy, o.q.y, o.o.y, S.Ly),
                       dz = rel(cz, oz, o.q.z, o.o.z, S.Lz);
-          close[u] = close[u] || (j != 0xFFFFu && dx * dx + dy * dy + dz * dz <= chl);
+          if (j != 0xFFFFu && dx * dx + dy * dy + dz * dz <= chl) close[u] = close[u] || in_block3(S, o.c, cx, cy, cz);
         }
       }
 #pragma unroll
