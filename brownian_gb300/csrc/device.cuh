@@ -386,7 +386,9 @@ static __device__ __forceinline__ double refl_speed(const SysF64 &S, uint4 r0) {
 // (2 ran - 1 is exact: pm1 builds it from the draw's bits); only two rejections
 // in a row (1 in 22) branch.
 // (refl_try: the accepted try's x1, x2 and, returned, its z)
-static __device__ __noinline__ double refl_more(uint2 key, uint32_t a, uint32_t b, uint32_t t, double &x1, double &x2) {
+// (refl_more in line: out of line, an event pass of a crowded system took 41 us instead of 37, its step
+// 600 instead of 557; the cooperative substeps are the same)
+static __device__ __forceinline__ double refl_more(uint2 key, uint32_t a, uint32_t b, uint32_t t, double &x1, double &x2) {
   CollDraw d;
   d.key = key; d.a = a; d.b = b; d.t = t; d.idx = 8;
   double z = 2.0;
