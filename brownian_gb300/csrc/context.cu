@@ -881,6 +881,12 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
   S.inv_sw = ldexp(1.0, -S.kw);
   S.wlim_bits = dbits_h(wmax);
 
+  {
+    int dev = 0, nsm = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && nsm > 0)
+      c->n_sm = nsm;
+  }
   DevAlloc &m = c->mem;
   const size_t N = S.N, Nc = S.Nc > 0 ? S.Nc : 1;
   for (int b = 0; b < 2; ++b) {
@@ -929,8 +935,7 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
   double est = (double)S.Nc * (4.0 / 3.0 * M_PI * rsh * rsh * rsh * density * 2.0 + 64.0);
   S.shell_cap = (int)(est < (double)S.N ? est : (double)S.N) + 1024;
   S.shell = m.get<ShellRec>(S.shell_cap);
-  S.events_cap = S.N / 16 + 65536;
-  S.events = m.get<int>(S.events_cap);
+  double listed = (double)S.N / 16.0 + 65536.0;  // room of the event passes' lists
   S.near = m.get<int>(N);
   S.fnear = m.get<uint8_t>(N);
   S.ftab = m.get<FlightCell>(S.C);
@@ -941,13 +946,35 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
     // A free-flight step takes the active particles through its substeps in one cooperative
     // kernel where there are colloids and at least two substeps, unless the flight table's cells
     // would overflow as a rule: with more than eight colloids expected within its reach of a cell
-    // (12 fit), the particles of overflowing cells would scan every colloid, which the
-    // per-substep cell tables avoid.  (The normals and spins of a step: 48 bytes per colloid and
+    // (12 fit), most particles would look their colloids up in the cell tables in every substep, as the
+    // passes of a launch per stage do.  (The normals and spins of a step: 48 bytes per colloid and
     // substep; substep numbers in 16 bits.)
     const double reach = S.r_shell + S.flight_rx + S.n_sub * cmargin + 0.02 + 0.62;  // + a cell's radius as a ball
     const double expected = (double)S.Nc / (double)S.C * 4.0 / 3.0 * M_PI * reach * reach * reach;
     c->near_sized =
         S.Nc > 0 && S.n_sub >= 2 && S.n_sub <= 4096 && expected <= 8.0 && (long long)S.Nc * S.n_sub <= (1ll << 24);
+    // And in the FP64 form, unless the active particles expected are more than 1.1 times what the blocks hold in
+    // shared memory (the rest take a path of several us a substep for every 128 of a block), than a
+    // fiftieth of the fluid (below it the free pass hides them) and than 40 a colloid (the passes of a launch per
+    // stage cost more with many colloids).  Expected: around each sphere the shell that the colloids' moves
+    // add to it and what the fluid's mean speed sweeps (the count is within 30 % of it).  Measured, us a step,
+    // one kernel / a launch per stage, with the number expected per SM: 48^3 at density 60, 300 / 450 / 600
+    // spheres of radius 2 (753 / 1,130 / 1,506) 1,077 / 1,133, 1,483 / 1,481, 2,091 / 1,837; 64^3, steps of 1.0,
+    // 200 / 300 / 500 spheres (896 / 1,343 / 2,239) 1,265 / 1,302, 1,975 / 1,597, 4,016 / 2,135; 128^3, 4,000 of
+    // radius 2 and 3,700 of radius 3 (1,673 / 3,422; 1.2 and 2.5 % of the fluid) 3,136 / 3,716, 5,884 / 5,260; with
+    // many colloids, 25,000 of radius 1 and 14,800 of 1.5 in 128^3 (5,226 / 4,376) 8,406 / 9,383, 7,409 / 7,530.
+    // The FP32 form is faster in one kernel in all of these.
+    if (c->near_sized && p.precision == MPCD_FP64) {
+      const double cm = fmin(cmargin, fmax(0.005, 2.0 * dt * (4.0 * sqrt(p.kbt / p.mass_colloid) + fabs(p.v0))));
+      const double r = p.sigma * 0.5, rad = r + (S.n_sub + 2) * cm + 0.02;
+      const double swept = 4.0 / 3.0 * M_PI * (rad * rad * rad - r * r * r) + M_PI * rad * rad * 1.6 * vth * p.ndt;
+      const double active = (double)S.Nc * swept * (double)S.N / (double)S.C;
+      c->near_sized = active <= fmax(fmax(1.1 * NEAR64_ACT * c->n_sm, (double)S.N / 50.0), 40.0 * S.Nc);
+      // (a launch per stage lists the active particles that come near a sphere)
+      if (!c->near_sized) listed = fmax(listed, fmin((double)S.N, 1.75 * active));
+    }
+    S.events_cap = (int)listed;
+    S.events = m.get<int>(S.events_cap);
     // (in an ensemble the others' kernel takes a system without colloids along)
     if (c->near_sized || (S.Nc == 0 && p.precision == MPCD_FP32C)) {
       S.act = m.get<int>(N);
@@ -1028,12 +1055,6 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
       cudaEventCreateWithFlags(&c->ev_finp[1], cudaEventDisableTiming) != cudaSuccess) {
     mpcd_destroy(c);
     return MPCD_ERR_CUDA;
-  }
-  {
-    int dev = 0, nsm = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && nsm > 0)
-      c->n_sm = nsm;
   }
   choose_near_step(c, false);
   cudaDeviceSynchronize();

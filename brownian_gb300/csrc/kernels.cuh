@@ -65,7 +65,8 @@ __global__ void k_near_step64(__grid_constant__ const SysF64 S, int fb);
 __global__ void k_near_step32(__grid_constant__ const SysF64 S, int fb);
 __global__ void k_near_step32_b(const SysF64 *Ss, const int *boff, int nrep, int first, int fb);
 constexpr int NEAR64_BLOCK = 256, NEAR32_BLOCK = 384;
-constexpr int NEAR32_ACT = 3584;  // active particles a block of k_near_step32 keeps in shared memory
+// active particles a block of k_near_step64 / k_near_step32 keeps in shared memory
+constexpr int NEAR64_ACT = 1024, NEAR32_ACT = 3584;
 size_t near_step64_smem();
 size_t near_step32_smem();
 __global__ void k_rotdiff_step(__grid_constant__ const SysF64 S);

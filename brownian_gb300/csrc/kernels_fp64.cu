@@ -1271,7 +1271,7 @@ static __device__ __forceinline__ void near_shell64(const SysF64 &S, long long s
 
 // Particles per block kept in shared memory: NEAR64_ACT active ones (52 bytes each; more stay
 // in the other fluid buffer, which is free between sorts) and NEAR64_EV pending ones.
-constexpr int NEAR64_ACT = 1024, NEAR64_EV = 160;
+constexpr int NEAR64_EV = 160;
 struct Near64 {
   double st[6][NEAR64_ACT];
   unsigned cand[NEAR64_ACT];
