@@ -115,9 +115,10 @@ struct Dim {
 // a - L lround((a - h) / L): the bands of mod and img that need the division, out of line (inlined
 // at every wrap it is most of the kernels' code, and the kernels run at the rate their code is
 // fetched)
-static __device__ __noinline__ double far_mod(double a, double L, double h) {
+static __device__ __forceinline__ double far_mod_in(double a, double L, double h) {
   return __dsub_rn(a, __dmul_rn(L, (double)llround(__ddiv_rn(__dsub_rn(a, h), L))));
 }
+static __device__ __noinline__ double far_mod(double a, double L, double h) { return far_mod_in(a, L, h); }
 
 // The reference's mod(a, L) = a - L*lround((a - L/2)/L) (cpp/parameters.hpp:75).
 // The quotient rounds to 0 for a in [2^-30 L, L) (result a), to 1 for a in
@@ -125,23 +126,26 @@ static __device__ __noinline__ double far_mod(double a, double L, double h) {
 // a - L*(-1)); those subtractions are the reference's own, so the results are
 // bit-identical.  Only a in [0, 2^-30 L), where rounding decides, and values
 // further out take the reference's division (mod(0, L) == L comes from there).
+// (IN: the division in line)
+template <bool IN = false>
 __device__ __forceinline__ double ref_mod(double a, const Dim &d) {
   long long b = dbits(a);
   if (b >= d.lo_bits && b < d.L_bits) return a;
   if (b >= d.L_bits && b < d.img2_bits) return __dsub_rn(a, d.L);
   if (b < 0 && (b & 0x7FFFFFFFFFFFFFFFll) < d.img_bits) return __dsub_rn(a, -d.L);
-  return far_mod(a, d.L, d.halfL);
+  return IN ? far_mod_in(a, d.L, d.halfL) : far_mod(a, d.L, d.halfL);
 }
 
 // The reference's img(a, L) = a - L*lround(a/L) (cpp/parameters.hpp:76).  For
 // |a| < 0.49 L the quotient rounds to 0 (result a); for 0.51 L < |a| < 1.49 L it
 // rounds to sign(a) (result a - L sign(a), one subtraction as in the reference);
 // only the bands around L/2 and beyond take the division.
+template <bool IN = false>
 __device__ __forceinline__ double ref_img(double a, const Dim &d) {
   long long b = dbits(a) & 0x7FFFFFFFFFFFFFFFll;
   if (b < d.img_bits) return a;
   if (b > d.img1_bits && b < d.img2_bits) return __dsub_rn(a, a > 0 ? d.L : -d.L);
-  return far_mod(a, d.L, 0.0);
+  return IN ? far_mod_in(a, d.L, 0.0) : far_mod(a, d.L, 0.0);
 }
 
 // (x*x + y*y) + z*z with separately rounded products, as point::sum() of a*a.
