@@ -631,6 +631,7 @@ static void enq_step_near(mpcd_ctx *c, bool sort) {
   cudaStreamWaitEvent(c->nst, c->ev_cls, 0);
   cudaStreamWaitEvent(c->nst, c->ev_aux, 0);
   cudaStreamWaitEvent(c->nst, c->ev_str, 0);
+  // (under the name of the pass that it takes the place of: the near particles' substeps)
   launch_attr(c, c->nst, "k_stream_near", COOP, f32 ? k_near_step32 : k_near_step64, c->n_sm,
               f32 ? NEAR32_BLOCK : NEAR64_BLOCK, f32 ? near_step32_smem() : near_step64_smem(), S, c->fbuf);
   cudaEventRecord(c->ev_end, c->nst);

@@ -164,7 +164,6 @@ __device__ __forceinline__ void bin32(const SysF64 &S, int p, int cx, int cy, in
 
 struct f3 { float x, y, z; };
 __device__ __forceinline__ f3 fm(float x, float y, float z) { f3 r; r.x = x; r.y = y; r.z = z; return r; }
-__device__ __forceinline__ f3 fcross(f3 a, f3 b) { return fm(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x); }
 
 // One wall collision of a particle in two halves.  bounce32_draw: everything that the colloid's
 // state does not enter, into Bounce32: the point half a substep back (cell and offset) and, from
@@ -552,7 +551,7 @@ static __device__ __forceinline__ float flight_reach(const SysF64 &S) {
 // the flight table of this step (both forms: the colloids' cell + offset copies are kept by
 // both): colloid j (its position at the start of the step) in every cell whose box comes
 // within the flight reach of it, the own box included.  A cell
-// with more than FLIGHT_CAP colloids keeps counting; its particles are all near.  Block 0
+// with more than FLIGHT_CAP colloids keeps counting; its particles are all near (near_list).  Block 0
 // also empties the near list and draws the next step's grid shift for the free pass.
 static __device__ __forceinline__ void k_flight_table32_body(const SysF64 &S, const int j) {
   const long long step = S.ss->step;

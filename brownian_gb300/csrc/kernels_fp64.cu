@@ -1285,7 +1285,7 @@ struct Near64 {
 // FP64 unit 16 of them however many lanes are active, so a substep's collisions run one per lane
 // on as few warps as hold them, and everything that does not wait for the colloids (the
 // logarithms of the draws above all) is prepared beside the colloids' finish.
-// (112 registers: the free-flight pass's two blocks fit beside it)
+// (128 registers: with the free-flight pass's two blocks of 64 beside it all that an SM has)
 __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant__ const SysF64 S, int fb) {
   constexpr int NT = NEAR64_BLOCK - 32 * (NEAR_CW + 1), NW = NT / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -480,13 +480,13 @@ __global__ void k_colsum(const bf16 *a, int n, int cols, long long lda, float *o
 //
 // The whole network for TM = 16 MT WM rows per CTA of eight warps (WM along the rows, 8 / WM
 // along the columns): normalisation, the four layers with the activations in shared memory, the
-// outputs in physical units, in one launch.  The weights stream from L2 through three stages
+// outputs in physical units, in one launch.  The weights stream from L2 through ST stages
 // of 32 k rows by asynchronous copies, the next layer's first stages while this one's epilogue runs.
 // Each output element is K steps of 16 in ascending order into one FP32 accumulator, bias, SiLU and
 // the BF16 rounding between layers, as in the colloid-only step's network, whose bits these are.
 // Bound: L2 reads of the weights (311 KB a CTA) and the SiLU's two special-function operations
-// per element.  Measured, six launches with the activations through memory -> this: 16,384 rows
-// 197 -> 43 us a call, one row 50 -> 26.5 us (the rule at infer() has the rest).
+// per element.  Measured, six launches with the activations through memory -> this, us a call among
+// others: 16,384 rows 184 -> 30.4, one row 34 -> 12.4 (the rule at infer() has the rest).
 template <int MT, int WM, int ST>
 struct Infer {
   static constexpr int TM = 16 * MT * WM, WN = 8 / WM, NT = H / WN / 8, LDA = H + 8, LDW = H + 8, KS = 32;
@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(256) k_mlp_infer(const InferArgs g) {
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  // the output layer: 16 rows x 8 columns a warp, in physical units (k_denorm)
+  // the output layer: 16 rows x 8 columns a warp, in physical units (mean * std + mean, log-variance + 2 log std)
   for (int p = warp; p < T::TM / 16 * 2; p += 8) {
     const int r0 = (p >> 1) * 16, c0 = (p & 1) * 8;
     float o[4] = {0.f, 0.f, 0.f, 0.f};
@@ -877,10 +877,10 @@ bool infer_attr() {
 
 // Rows per CTA: the smallest of 16, 32 and 64 that gives the device at most one CTA per SM (the
 // weights are then read the fewest times that keep every SM busy), and 64 beyond, where two CTAs share an
-// SM and one's epilogue runs under the other's products.  Measured per call, layer by layer -> 16 /
-// 32 / 64 rows a CTA: 1 row 50 -> 26.5 / 26.9 / 32 us, 2,432 rows 62 -> 29 / 30 / 34, 4,864 rows 90
-// -> 40 / 32 / 34, 16,384 rows 197 -> 96 / 54 / 43, 65,536 rows 663 -> 311 / 141 / 108 (128 rows a
-// CTA, one per SM: 47 and 136).
+// SM and one's epilogue runs under the other's products.  Measured, us a call among others, layer by layer
+// -> 16 / 32 / 64 rows a CTA: 1 row 34 -> 12.4 / 14.5 / 20.1, 2,432 rows 51 -> 16.5 / 16.5 / 20.6, 4,864 rows
+// 76 -> 26.8 / 18.5 / 20.6, 16,384 rows 184 -> 81 / 39 / 30.4, 65,536 rows 648 -> 297 / 125 / 92.5 (a call
+// that is waited for takes 9 us more).
 void infer(mpcd_mlp *nn, const float *x, int n, float *out, cudaStream_t s) {
   InferArgs g;
   g.x = x;

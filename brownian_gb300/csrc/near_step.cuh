@@ -22,16 +22,17 @@
 // cycle (fence and counter 1.2 us twice, exact collisions 2 us FP32 / 4 us FP64, colloid finish
 // 2 us), and with that the rate at which the code of a cycle is fetched: what is rarely taken is
 // out of line, and the common test runs two particles at a time without a branch.  Measured per
-// step, launches per stage -> this (with the free-flight pass as it is beside it): 24^3 FP32
-// system (30 colloids) 204 -> 134 us, 20^3 FP64 (20 colloids) 251 -> 167 us, 64^3 (500 colloids)
-// FP32 388 -> 280 us, FP64 605 -> 461 us, 128^3 FP32 (2,000 colloids, 20 substeps) 3.08 -> 1.81 ms;
-// 32 FP32 systems of 16^3 to 48^3 stepped together, each on blocks of its own, 2.28 -> 1.74 ms.
+// step, before it -> with it and the passes around it as they are now: 24^3 FP32 system (30
+// colloids) 204 -> 131 us, 20^3 FP64 (20 colloids) 251 -> 164 us, 64^3 (500 colloids) FP32
+// 390 -> 269 us, FP64 605 -> 450 us, 128^3 FP32 (2,000 colloids, 20 substeps) 3.08 -> 1.41 ms;
+// 32 FP32 systems of 16^3 to 48^3 stepped together, each on blocks of its own, 2.29 -> 1.59 ms.
+// Which systems take it: near_sized in context.cu.
 //
 // The arithmetic is that of the per-substep passes, in their order: the results are theirs
 // bit for bit.  The candidates of a particle come from the flight table of its cell (every
 // colloid that can come near in the step) with the reference's box rule (in_block) instead of
-// a cell table rebuilt each substep.  Waits are bounded: one that runs out sets ERRB_WAIT and
-// its group returns.
+// a cell table rebuilt each substep (where a cell lists more than it holds, with it: near_list).
+// Waits are bounded: one that runs out sets ERRB_WAIT and its group returns.
 #pragma once
 #include "device.cuh"
 
@@ -40,7 +41,7 @@ namespace bgb {
 constexpr int NEAR_CW = 3;         // colloid warps of a block (and one for the orientations)
 
 // a particle's candidate colloids for the rest of the step, packed: up to two ids (0xFFFF:
-// none); NEAR_WILD: look the flight table up in every substep; NEAR_GONE: kept elsewhere
+// none); NEAR_WILD: look the tables up in every substep (near_list); NEAR_GONE: kept elsewhere
 constexpr unsigned NEAR_NONE = 0xFFFFFFFFu, NEAR_WILD = 0xFFFEFFFEu, NEAR_GONE = 0xFFFDFFFDu,
                    NEAR_STALE = 0xFFFCFFFCu;  // (after a collision: to be looked up)
 

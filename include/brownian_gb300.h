@@ -178,8 +178,10 @@ int mpcd_sync(mpcd_ctx *c);
  * beside the substeps of the other (near) particles, which the substep passes walk alone.  The
  * results are those of the schedule without it, bit for bit.  The near particles whose path may
  * meet a sphere go through the substeps, with the colloids, in one cooperative kernel (its waits
- * are bounded: MPCD_ERR_CUDA if one runs out); in a system without colloids, with one substep, or
- * with more colloids around a cell than its tables are made for, in launches per substep.
+ * are bounded: MPCD_ERR_CUDA if one runs out); in a system without colloids, with one substep,
+ * with more colloids around a cell than its tables are made for, in the FP64 form with far more such
+ * particles than the SMs' shared memory holds, or on a device without room for it, in launches per
+ * substep.
  * mpcd_get_flight gives the near particles of the last step that used it. */
 int mpcd_set_flight(mpcd_ctx *c, int on);
 int mpcd_get_flight(mpcd_ctx *c, int32_t *near);
