@@ -1292,12 +1292,12 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
   Near64 &sm = *reinterpret_cast<Near64 *>(smem_raw);
   __shared__ double s_hx[NT][6];  // the exchanges of a round's collisions, and their colloids
   __shared__ int s_hj[NT];
-  __shared__ int s_nh, s_np, s_fin;
+  __shared__ int s_nh, s_np, s_nx, s_fin;  // (s_np: pending particles; s_nx: of them, beyond NEAR64_EV)
   __shared__ int s_flag[2];
   __shared__ NearPairs s_pairs;
   const int t = threadIdx.x, VB = blockIdx.x, G = gridDim.x;
   const int n = S.n_sub;
-  if (t == 0) s_np = s_nh = s_fin = 0;
+  if (t == 0) s_np = s_nx = s_nh = s_fin = 0;
   sm.col.clear(S, t, NEAR64_BLOCK);
   if (VB == 0 && t == NT) set_shift(S, S.ss->step + 2);  // (the records of this step are all kicked)
   near_let_dependents();
@@ -1385,16 +1385,22 @@ __global__ void __launch_bounds__(NEAR64_BLOCK, 2) k_near_step64(__grid_constant
         *px = x; *py = y; *pz = z;
         return;
       }
-      const int i = atomicAdd(&s_np, 1), p = S.act[a0 + k];
-      if (i >= NEAR64_EV) {
-        int o = (int)atomicAdd(S.bar + BAR_EVX, 1u);
-        if (o >= S.evx_cap) {
-          atomicOr(&S.ss->err, ERRB_EVENTS);
-          o = S.evx_cap - 1;
-        }
-        O.id[a0 + i] = o;
-      }
       *px = x; *py = y; *pz = z;
+      int i = atomicAdd(&s_np, 1);
+      const int p = S.act[a0 + k];
+      if (i >= NEAR64_EV) {
+        const unsigned o = atomicAdd(S.bar + BAR_EVX, 1u);
+        if (o >= (unsigned)S.evx_cap) {
+          // no record left: the step fails, and the particle goes on unlisted (a record of two particles
+          // would be changed by both their blocks)
+          atomicOr(&S.ss->err, ERRB_EVENTS);
+          atomicSub(S.bar + BAR_EVX, 1u);
+          atomicSub(&s_np, 1);
+          return;
+        }
+        i = NEAR64_EV + atomicAdd(&s_nx, 1);  // (s_np also counts those that find none)
+        O.id[a0 + i] = (int)o;
+      }
       NearEv &v = ev(i);
       v.j = k;  // (the record is made below)
       v.p = p;
