@@ -870,6 +870,7 @@ extern "C" int mpcd_create(const mpcd_params *pp, mpcd_ctx **out) {
   // free flight: a particle moving further than 5 thermal speeds' worth in a step is near
   S.flight_rv = (float)(5.0 * vth * p.ndt);
   S.flight_rx = (float)fmax(5.0 * vth * p.ndt, pmargin + cmargin + 0.05);
+  S.near_img = 0.5f * (float)std::min(p.Lx, std::min(p.Ly, p.Lz)) - 1.001f;
   // the free-flight steps' forces from a pair list built at the start of each step
   S.vlist = p.n_colloid > 1 ? 1 : 0;
   S.step_geo = nlist_geo(c, S.r_cutoff + 2.0 * S.n_sub * sqrt(S.cmargin2) + 0.05);

@@ -650,7 +650,7 @@ static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S,
       F.vx[p] = vx[u]; F.vy[p] = vy[u]; F.vz[p] = vz[u];
     }
     const float travel = (float)S.n_sub * S.dtf * sqrtf(vx[u] * vx[u] + vy[u] * vy[u] + vz[u] * vz[u]);
-    const int cnt = tcount(((unsigned long long)w0.y << 32) | w0.x, step);
+    int cnt = tcount(((unsigned long long)w0.y << 32) | w0.x, step);
     bool nr = false;
     if (!inb || !(travel <= S.flight_rv) || cnt > FLIGHT_CAP) {
       nr = true;  // faster than the table allows (or not finite), or a crowded cell
@@ -658,6 +658,11 @@ static __device__ __forceinline__ void k_rotate_classify32_body(const SysF64 &S,
     } else if (cnt > 0) {
       const float rad = near_radius(S, S.ss->cm, S.n_sub), T = (float)S.n_sub * S.dtf;
       const float r = S.r_shell + travel + (float)S.n_sub * S.ss->cm + 0.01f, r2 = r * r;
+      if (r > S.near_img) {  // (a box as narrow as that: other copies of the spheres matter)
+        nr = true;
+        cand[u] = NEAR_WILD;
+        cnt = 0;
+      }
       // (four ids lie in the first half of the record)
       const uint4 w1 = cnt > 4 ? reinterpret_cast<const uint4 *>(fc)[1] : make_uint4(0, 0, 0, 0);
       const unsigned ids[6] = {w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
@@ -1129,11 +1134,11 @@ static __device__ __forceinline__ unsigned near_cand32(const SysF64 &S, long lon
   if (!(cx < S.Lx && cy < S.Ly && cz < S.Lz)) return NEAR_WILD;
   const float T = (float)rem * S.dtf;
   const float wx = T * vx, wy = T * vy, wz = T * vz;
-  if (!(sqrtf(wx * wx + wy * wy + wz * wz) <= S.flight_rv)) return NEAR_WILD;
+  const float travel = sqrtf(wx * wx + wy * wy + wz * wz), rad = near_radius(S, S.ss->cm, rem);
+  if (!(travel <= S.flight_rv) || rad + travel > S.near_img) return NEAR_WILD;
   const FlightCell *fc = S.ftab + lin_cell(S, cx, cy, cz);
   const int cnt = tcount(fc->tc, step);
   if (cnt > FLIGHT_CAP) return NEAR_WILD;
-  const float rad = near_radius(S, S.ss->cm, rem);
   unsigned cand = NEAR_NONE;
   for (int k = 0; k < cnt; ++k) {
     const int j = fc->id[k];
@@ -1376,6 +1381,7 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
     const long long gs = g0 + (l - 1);
     const int xb = (int)(gs & 1) ^ 1;
     const float ch = S.r_coll + 1e-3f + cm, far = ch + S.disp_marginf + 1e-3f;
+    const bool wide = ch > S.near_img;  // (a colloid's move may turn a distance into that of a nearer copy)
     // particle k by the general path
     auto one = [&](int k, unsigned cand) {
       uint4 *q = pq(k);
@@ -1392,7 +1398,9 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
         return dx * dx + dy * dy + dz * dz;
       };
       // (inside a sphere that its boxes leave out, a particle needs no exact test: the box rule first)
-      auto reached = [&](const NearCol32 &o) { return dist2(o) <= ch * ch && in_block3(S, o.c, cx, cy, cz); };
+      auto reached = [&](const NearCol32 &o) {
+        return (wide || dist2(o) <= ch * ch) && in_block3(S, o.c, cx, cy, cz);
+      };
       bool e = false;
       if (cand == NEAR_WILD) {
         const NearList c = near_list(S, step, gs, lin_cell(S, cx, cy, cz), false);
@@ -1470,7 +1478,7 @@ static __device__ __forceinline__ void near_step32(const SysF64 &S, const int VB
       v.id = F.id[S.act[a0 + k]];
       v.jc = -1;
       v.nc = 0;
-      v.slow = c.brute;
+      v.slow = c.brute || far > S.near_img;
       for (int m = 0; m < c.cnt && !v.slow; ++m) {
         const int j = c.ids[m];
         const NearCol32 o = sm.col.at(S, xb, j);

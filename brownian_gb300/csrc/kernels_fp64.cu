@@ -438,13 +438,18 @@ __global__ void __launch_bounds__(256) k_rotate_classify(const SysF64 S, int fb)
     // the travel under it, which the slack covers)
     const float fx = d2f_trunc(wx), fy = d2f_trunc(wy), fz = d2f_trunc(wz);
     const float travel = (float)S.n_sub * sqrtf(fx * fx + fy * fy + fz * fz);
-    const int cnt = tcount(((unsigned long long)w0.y << 32) | w0.x, step);
+    int cnt = tcount(((unsigned long long)w0.y << 32) | w0.x, step);
     if (!inb || !(travel <= S.flight_rv) || cnt > FLIGHT_CAP) {
       near = true;  // faster than the table allows (or not finite), or a crowded cell
       cand = NEAR_WILD;
     } else if (cnt > 0) {
       const float r = S.r_shell + travel + (float)S.n_sub * S.ss->cm + 0.01f, r2 = r * r;
       const float rad = near_radius(S, S.ss->cm, S.n_sub), fn = (float)S.n_sub;
+      if (r > S.near_img) {  // (a box as narrow as that: other copies of the spheres matter)
+        near = true;
+        cand = NEAR_WILD;
+        cnt = 0;
+      }
       // (four ids lie in the first half of the record)
       const uint4 w1 = cnt > 4 ? reinterpret_cast<const uint4 *>(fc)[1] : make_uint4(0, 0, 0, 0);
       const unsigned ids[6] = {w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
@@ -817,11 +822,11 @@ static __device__ __forceinline__ unsigned near_cand64(const SysF64 &S, long lon
   if (!(cx >= 0 && cx < S.Lx && cy >= 0 && cy < S.Ly && cz >= 0 && cz < S.Lz)) return NEAR_WILD;
   const float fr = (float)rem;
   const float fx = fr * d2f_trunc(wx), fy = fr * d2f_trunc(wy), fz = fr * d2f_trunc(wz);
-  if (!(sqrtf(fx * fx + fy * fy + fz * fz) <= S.flight_rv)) return NEAR_WILD;
+  const float travel = sqrtf(fx * fx + fy * fy + fz * fz), rad = near_radius(S, S.ss->cm, rem);
+  if (!(travel <= S.flight_rv) || rad + travel > S.near_img) return NEAR_WILD;
   const FlightCell *fc = S.ftab + lin_cell(S, cx, cy, cz);
   const int cnt = tcount(fc->tc, step);
   if (cnt > FLIGHT_CAP) return NEAR_WILD;
-  const float rad = near_radius(S, S.ss->cm, rem);
   unsigned cand = NEAR_NONE;
   for (int k = 0; k < cnt; ++k) {
     const int j = fc->id[k];

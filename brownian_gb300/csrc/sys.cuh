@@ -224,6 +224,9 @@ struct SysF64 {
   float flight_rv;              // travel allowance: particles moving further in a step are near
   float flight_rx;              // the table's reach beyond the run() shell: the travel allowance, and
                                 // at least a wall collision's and a colloid's displacement bounds
+  float near_img;               // half the shortest side less a cell: a sphere within it of a particle, the
+                                // particle's path included, has no nearer copy at any point of the path, and the
+                                // FP32 form's distances (rel) are to the nearest copy; beyond it, no sphere is ruled out
   int vlist;                    // the free-flight steps compute the forces from a pair list built
                                 // at the start of the step
   NListGeo step_geo;            // its bucket grid
