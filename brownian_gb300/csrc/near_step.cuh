@@ -564,7 +564,9 @@ static __device__ __forceinline__ void k_end_step_body(const SysF64 &S, const in
         dm = fmaxf(dm, s_dm[k]);
       }
       float cm = fminf(fmaxf(2.f * (float)S.dt * sqrtf(vm), 0.005f), S.cmarginf);
-      cm = fmaxf(cm, sqrtf(dm) + 2e-5f);
+      // (capped: in a step that has failed a colloid may have moved anywhere, and the steps enqueued behind it
+      // would take that for the reach of their tables)
+      cm = fmaxf(cm, fminf(sqrtf(dm) + 2e-5f, fmaxf(2.f * S.cmarginf, 0.1f)));
       S.ss->cm = cm;
       S.ss->cm2 = (double)cm * (double)cm;
     }
