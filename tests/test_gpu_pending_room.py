@@ -57,7 +57,10 @@ def test_more_pending_particles_than_records(flight):
     a.set_flight(flight)
     with pytest.raises(bg.MPCDError) as e:
         a.step(3)
-    assert e.value.code == 3 and int(re.search(r"bits (0x[0-9a-f]+)", str(e.value))[1], 16) & 0x80
+    # (which particles find no room depends on the order of the blocks, and so does what else the two steps
+    # behind that one report: a range bit, 4 or 64, makes it code 4)
+    bits = int(re.search(r"bits (0x[0-9a-f]+)", str(e.value))[1], 16)
+    assert bits & 0x80 and e.value.code == (4 if bits & 0x44 else 3), str(e.value)
     _steps(b, flight, 3)  # (the draws are keyed by the step)
     refused = [_steps(s, flight, 4) for s in (a, b)]
     assert refused[0] == refused[1] and "event lists" not in refused[0], refused
